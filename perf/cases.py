@@ -230,3 +230,47 @@ def tolerance(case):
         return {"rel": 1.2e-2, "max": 0.08}
     # rows move unchanged; the weighted sum is taken in 32 bits and rounded to BF16 once: measured 1.7e-3 against 64 bits
     return {"rel": 6.6e-3, "max": 1.6e-2}
+
+
+# ---------------------------------------------------------------------------------------------------- the values themselves
+def _fp8_rows(rows):
+    """Rows as the E4M3 codes of the wire format hold them (scale = largest magnitude / 448, one per row)."""
+    rows = rows.float()
+    peak = rows.abs().amax(dim=-1, keepdim=True)
+    scale = torch.where(peak == 0, torch.ones_like(peak), (peak / 448.0).clamp_min(torch.finfo(torch.float32).tiny))
+    return (rows * (1.0 / scale)).clamp(-448.0, 448.0).to(torch.float8_e4m3fn).double() * scale.double()
+
+
+def exact(case, seed):
+    """What ``run`` returns for these inputs, in 64 bits; ``None`` stands for rows and whole numbers that only move."""
+    if case["kind"] == "keep_fp8":
+        return None
+    state = prepare(case, seed)
+    x, idx, weights = state.x, state.idx, state.weights.double()
+    if case["kind"] == "layer":
+        fp8, inter = case["fp8"], case["inter"]
+        rows = _fp8_rows(x) if fp8 else x.double()
+        out = torch.zeros(x.shape, dtype=torch.float64, device=x.device)
+        for expert in range(case["experts"]):
+            token, slot = torch.nonzero(idx == expert, as_tuple=True)
+            if token.numel() == 0:
+                continue
+            w = state.layer.w_gate_up[expert]
+            gate_up = rows[token] @ (_fp8_rows(w) if fp8 else w.double()).t()
+            hidden = torch.nn.functional.silu(gate_up[:, :inter]) * gate_up[:, inter:]
+            out.index_add_(0, token, hidden @ state.layer.w_down[expert].double().t() * weights[token, slot].unsqueeze(1))
+        return out
+    result = dict(recv_x=None, recv_idx=None, recv_w=None, counts=None, offsets=None)
+    if case.get("expand", True):
+        # an expert's rows follow each other in token order, the experts in theirs
+        order = torch.argsort(idx.reshape(-1), stable=True)
+        row_of = torch.empty_like(order)
+        row_of[order] = torch.arange(order.numel(), device=order.device)
+        row_of = row_of.view(idx.shape)
+        combined = torch.zeros(x.shape, dtype=torch.float64, device=x.device)
+        for slot in range(case["topk"]):
+            combined += state.y[row_of[:, slot]].double() * weights[:, slot:slot + 1]
+        result["combined"] = combined
+    else:
+        result["combined"] = state.y.double()
+    return result
