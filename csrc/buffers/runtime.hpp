@@ -245,6 +245,8 @@ struct PreparedCombine {
     at::Tensor out;
     bool inline_kernel = false;  // one cooperative launch does both sides
     CombinePushArgs push{};    // expert side as an ordinary launch (the default)
+    int max_rows = 1;          // most rows an entry of the combine map can have
+    CombineLocalArgs local{};  // one rank: its reduced rows are the result, one ordinary launch
     bool reduce_needed = false;  // more than one rank: the owner-side sum follows as a second ordinary launch
     FusedReduceArgs reduce{};
 };
@@ -293,6 +295,7 @@ class Runtime {
         grid_ctas_ = options_.channels + options_.send_ctas;
         if (smem_ > static_cast<std::size_t>(max_optin)) throw std::runtime_error("dispatch kernel needs more shared memory than the device offers");
         cuda_check(configure_kernels(smem_), "configure kernels");
+        max_smem_ = static_cast<std::size_t>(max_optin);
 
         const auto i32 = at::TensorOptions().dtype(at::kInt).device(at::kCUDA, device);
         const auto i64 = at::TensorOptions().dtype(at::kLong).device(at::kCUDA, device);
@@ -446,11 +449,11 @@ class Runtime {
                                              std::int64_t stream) {
         c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device_));
         PreparedDispatch p = prepare_dispatch(x, topk_idx, topk_weights, alignment, expand, zero_padding, cached, graph_pool);
+        cudaStream_t launch_stream = stream != 0 ? reinterpret_cast<cudaStream_t>(stream)
+                                                 : at::cuda::getCurrentCUDAStream(device_).stream();
         DispatchLaunch launch{};
         launch.num_virtual = 1;
         launch.r[0] = p.args;
-        cudaStream_t launch_stream = stream != 0 ? reinterpret_cast<cudaStream_t>(stream)
-                                                 : at::cuda::getCurrentCUDAStream(device_).stream();
         cuda_check(launch_dispatch(launch, grid_ctas_, threads_, smem_, launch_stream), "dispatch launch");
         return p.result;
     }
@@ -495,46 +498,61 @@ class Runtime {
         p.inline_kernel = combine_is_inline();
         if (p.inline_kernel) return p;
         unsigned long long* counters = reinterpret_cast<unsigned long long*>(fused_counters_.data_ptr<std::int64_t>());
+        if (combine_is_local()) {
+            CombineLocalArgs& local = p.local;
+            local.rc = a.rc;
+            local.y = a.y;
+            local.comb_map = a.comb_map;
+            local.recv_chan_counts = a.recv_chan_counts;
+            local.plan_mask = a.plan_mask;
+            local.num_tokens = T;
+            local.weighted = a.weighted;
+            local.out = a.out;
+            local.error = a.error;
+            local.stats = a.stats;
+            local.cta_done = counters + 3;
+            local.first_start = counters + 6;
+            local.next_unit = counters + 9;
+            local.num_channels = lay_.num_channels;
+            local.slots_full = lay_.slots_full;
+            local.num_topk = lay_.num_topk;
+            local.hidden = lay_.hidden;
+            p.max_rows = expand ? std::min(lay_.num_topk, lay_.num_local_experts) : 1;
+            return p;
+        }
         CombinePushArgs& push = p.push;
         push.rc = a.rc;
         push.y = a.y;
         push.comb_map = a.comb_map;
         push.recv_chan_counts = a.recv_chan_counts;
-        push.plan_mask = a.plan_mask;
-        push.num_tokens = T;
         push.weighted = a.weighted;
-        push.out = a.out;
         push.error = a.error;
         push.stats = a.stats;
         push.cta_done = counters + 3;
         push.stat_scratch = counters + 4;
         push.next_unit = counters + 9;
         push.forwarder_sms = counters + 16;
-        push.forward_ctas = lay_.num_ranks > 1 ? combine_forward_ctas_ : 0;
-        if (push.forward_ctas > 0) {
-            ensure_outbox();
-            push.outbox = outbox_.data_ptr<std::uint8_t>();
-            push.outbox_units = reinterpret_cast<unsigned long long*>(outbox_units_.data_ptr<std::int64_t>());
-        }
-        p.reduce_needed = lay_.num_ranks > 1;
-        if (p.reduce_needed) {
-            FusedReduceArgs& r = p.reduce;
-            r.rc = a.rc;
-            r.expert_ord = nullptr;
-            r.rank_mask = a.plan_mask;
-            r.gemm_status = nullptr;
-            r.num_tokens = T;
-            r.epoch = 0;  // the combine epoch the push launch has just advanced on the device
-            r.cta_done = counters + 2;
-            r.stage_off = lay_.cstage_off;
-            r.sig_off = lay_.csig_off;
-            r.done_off = lay_.cdone_off;
-            r.slot_stride = static_cast<std::size_t>(lay_.num_max_tokens) * lay_.crow_stride;
-            r.token_stride = static_cast<std::size_t>(lay_.crow_stride);
-            r.slots = lay_.num_ranks;
-            r.out = a.out;
-            r.error = a.error;
-        }
+        push.forward_ctas = combine_forward_ctas_;
+        ensure_outbox();
+        push.outbox = outbox_.data_ptr<std::uint8_t>();
+        push.outbox_units = reinterpret_cast<unsigned long long*>(outbox_units_.data_ptr<std::int64_t>());
+        p.reduce_needed = true;
+        FusedReduceArgs& r = p.reduce;
+        r.rc = a.rc;
+        r.expert_ord = nullptr;
+        r.rank_mask = a.plan_mask;
+        r.gemm_status = nullptr;
+        r.num_tokens = T;
+        r.epoch = 0;  // the combine epoch the push launch has just advanced on the device
+        r.cta_done = counters + 2;
+        r.stage_off = lay_.cstage_off;
+        r.sig_off = lay_.csig_off;
+        r.done_off = lay_.cdone_off;
+        r.slot_stride = static_cast<std::size_t>(lay_.num_max_tokens) * lay_.crow_stride;
+        r.token_stride = static_cast<std::size_t>(lay_.crow_stride);
+        r.slots = lay_.num_ranks;
+        r.out = a.out;
+        r.error = a.error;
         return p;
     }
 
@@ -550,7 +568,13 @@ class Runtime {
         return per_sm * std::max(1, sms);
     }
 
+    // the launch that reads the expert rows: everything with a single rank, else the expert side
     void launch_combine_push(PreparedCombine& prepared, cudaStream_t stream, int num_sms = 0) {
+        if (combine_is_local()) {
+            prepared.local.shape = combine_local_shape(prepared.local.num_tokens, lay_.hidden, prepared.max_rows, combine_ctas(1, num_sms), max_smem_);
+            cuda_check(launch_combine_local(prepared.local, stream), "combine launch");
+            return;
+        }
         const int forward = prepared.push.forward_ctas;
         // two reducer CTAs per SM; with `num_sms` the whole launch (forwarders included) stays inside that many SMs
         // forwarders + reducers together never exceed what is resident at once (a reducer CTA that had to wait for a
@@ -860,7 +884,7 @@ class Runtime {
     RankConst rc_{};
     bool use_tma_ = false;
     int threads_ = 0;
-    std::size_t smem_ = 0;
+    std::size_t smem_ = 0, max_smem_ = 0;
     at::Tensor epochs_, grid_bar_, done_ctas_, block_hist_, sticky_, chan_stats_, plan_flags_, rank_const_;
     int grid_ctas_ = 0;
     std::vector<std::shared_ptr<OutputSet>> pools_;

@@ -1,0 +1,279 @@
+// Combine of a group of one rank: every token's expert rows, weighted, become its result row in one ordinary launch.
+//
+// What bounds it: reading the expert rows from HBM (4096 tokens, hidden 7168, top-8: 470 MB in, 59 MB out).  The rows of a
+// token lie far apart, so how they are asked for matters more than how many loads are in flight: pieces of 1 KB per row
+// through 16-byte register loads read 4.3 TB/s however many of them were outstanding (110 us).  Here a piece is as long as
+// two stages in shared memory allow -- a whole row of 7168 with top-8 -- and one bulk copy: 95 us, and 104 us with half rows.
+//
+// Work unit = (entry of the combine map, slice of its rows).  A CTA's first units are its own, the others come from a
+// counter: SMs do not all get the same share of HBM, and equal shares waited for the slowest (125 us).  The producer warp
+// keeps the claim after next and the map entries of the next units on their way while it starts the copies of the present
+// ones; a round of that takes 1.4 us, so small units are claimed four at a time (2048 tokens, a row each: 25.5 -> 21.9 us).
+// Before, through the multi-rank reducers (combine_push.cuh): 111 us, 139 us for 8192 tokens top-4 (now 103), 22 us for 128
+// tokens (now 11).  The other warps add the rows out of shared memory in the order of the entry, in FP32, a thread per 16-byte chunk.
+#pragma once
+
+#include "protocol.cuh"
+
+namespace bep {
+
+// How a launch cuts its work (host): slices per row and the ring of stages that fits shared memory.
+struct CombineLocalShape {
+    int slice_chunks = 0;  // 16-byte chunks of a slice
+    int slices = 0;        // per row
+    int stages = 0;
+    int stage_bytes = 0;   // rows of a unit, one slice each
+    int ctas = 0;
+    int batch = 1;         // consecutive units per claim: 1 or 4
+    std::size_t bytes = 0; // dynamic shared memory
+};
+
+struct CombineLocalArgs {
+    const RankConst* rc;
+    const __nv_bfloat16* y;          // expert outputs in the layout of the dispatch's recv_x
+    const int* comb_map;             // [C][slots_full][2 + 2K]: token, n, then (row, weight bits) pairs
+    const int* recv_chan_counts;     // [C] entries per channel
+    const std::uint32_t* plan_mask;  // [Tmax] 0: the token was routed nowhere, its result is zero
+    int num_tokens;
+    int weighted;
+    __nv_bfloat16* out;              // [T, H]
+    int* error;                      // [8]
+    std::int64_t* stats;             // [8]: rows written, 0, ns from the first CTA's start to the last one's end
+    unsigned long long* cta_done;    // CTAs of this launch that have finished; the last one puts it back to zero
+    unsigned long long* first_start; // earliest start; all ones between launches
+    unsigned long long* next_unit;   // units handed out beyond every CTA's first; zero between launches
+    int num_channels, slots_full, num_topk, hidden;
+    CombineLocalShape shape;
+};
+
+constexpr int kCombineLocalMaxStages = 8;
+constexpr int kCombineLocalConsumers = 14;  // warps that add, behind the producer warp: 448 threads, half a row of 7168
+constexpr int kCombineLocalThreads = 32 * (1 + kCombineLocalConsumers);
+constexpr int kCombineLocalSmallStage = 32 * 1024;  // stages up to this size: units are claimed four at a time, given a dozen per CTA
+
+struct CombineLocalHeader {
+    int token, n, first_chunk, chunks;  // n < 0: no more units
+    float weight[kMaxTopk];
+};
+struct CombineLocalShared {
+    unsigned long long full[kCombineLocalMaxStages], empty[kCombineLocalMaxStages];
+    CombineLocalHeader header[kCombineLocalMaxStages];
+};
+constexpr int kCombineLocalTiles = 2048;  // offset of the stages
+static_assert(sizeof(CombineLocalShared) <= kCombineLocalTiles, "the stages start behind the barriers and headers");
+
+// `max_rows`: most rows an entry can have.  Slices are as long as two stages allow, but short enough that a few tokens
+// reach every SM (units of at least 1 KB per row).
+inline CombineLocalShape combine_local_shape(int tokens, int hidden, int max_rows, int sms, std::size_t smem_limit) {
+    CombineLocalShape s;
+    const int chunks = hidden / 8;
+    auto slices_for = [chunks](int slice) { return (chunks + slice - 1) / slice; };
+    int slice = static_cast<int>((smem_limit - kCombineLocalTiles) / 2 - 128) / 16 / max_rows;
+    if (slice > chunks) slice = chunks;
+    int slices = slices_for(slice);
+    while (static_cast<long long>(tokens) * slices < 2ll * sms && slice >= 128) {
+        slice = (slice + 1) / 2;
+        slices = slices_for(slice);
+    }
+    s.slice_chunks = (chunks + slices - 1) / slices;  // equal slices
+    s.slices = slices_for(s.slice_chunks);
+    s.stage_bytes = static_cast<int>(align_up(static_cast<std::size_t>(max_rows) * s.slice_chunks * 16, 128));
+    const std::size_t room = (smem_limit - kCombineLocalTiles) / static_cast<std::size_t>(s.stage_bytes);
+    s.stages = room < 2 ? 2 : room > kCombineLocalMaxStages ? kCombineLocalMaxStages : static_cast<int>(room);
+    s.bytes = kCombineLocalTiles + static_cast<std::size_t>(s.stages) * s.stage_bytes;
+    const long long units = static_cast<long long>(tokens) * s.slices;
+    s.ctas = units < 1 ? 1 : units < sms ? static_cast<int>(units) : sms;
+    s.batch = s.stage_bytes <= kCombineLocalSmallStage && units >= 12ll * sms ? 4 : 1;
+    return s;
+}
+
+#ifdef __CUDACC__
+
+// kBatch: consecutive units per claim
+template <int kBatch>
+__global__ void __launch_bounds__(kCombineLocalThreads, 1) local_combine_push_kernel(const __grid_constant__ CombineLocalArgs a) {
+    const RankConst* __restrict__ rc = a.rc;
+    const int C = a.num_channels, K = a.num_topk, H = a.hidden, T = a.num_tokens;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int chunks = H / 8, stages = a.shape.stages;
+    const std::size_t row_bytes = static_cast<std::size_t>(H) * 2;
+    extern __shared__ __align__(128) unsigned char combine_smem[];
+    auto* sh = reinterpret_cast<CombineLocalShared*>(combine_smem);
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < stages; ++s) {
+            ptx::mbar_init(reinterpret_cast<std::uint64_t*>(&sh->full[s]), 1);
+            ptx::mbar_init(reinterpret_cast<std::uint64_t*>(&sh->empty[s]), kCombineLocalConsumers);
+        }
+        ptx::mbar_fence_init();
+        atomicMin(a.first_start, ptx::globaltimer_ns());
+    }
+    const bool aborted = ptx::ld_volatile(&rc->sticky[0]) != 0;
+    if (aborted && threadIdx.x == 0 && blockIdx.x == 0) atomicCAS(&a.error[0], 0, kErrAlreadyAborted);
+    Health health(rc, a.error);
+    __syncthreads();
+
+    bool ok = true;
+    auto wait = [&](unsigned long long* bar, unsigned parity) {
+        while (!ptx::mbar_try_wait(reinterpret_cast<std::uint64_t*>(bar), parity))
+            if (health.give_up(kErrCopyEngine, static_cast<int>(blockIdx.x), 1)) return false;
+        return true;
+    };
+    const int Tc = max(1, (T + C - 1) / C);  // tokens per channel: no channel has more entries
+    if (aborted || T == 0) {
+        // nothing to do
+    } else if (warp == 0) {
+        // ---- producer ----------------------------------------------------------------------------------------------
+        const int map_stride = 2 + 2 * K;
+        const long long units = static_cast<long long>((T + Tc - 1) / Tc) * Tc * a.shape.slices;
+        struct Entry {
+            int count, j;  // the entry exists if j < count
+            int2 head;     // token, rows
+            int2 pair;     // lane i: row and weight of the entry's i-th row
+        };
+        auto load_entry = [&](long long u) {
+            Entry e{};
+            if (u >= units) return e;
+            const int entry = static_cast<int>(u / a.shape.slices), c = entry / Tc;
+            e.j = entry % Tc;
+            // (entries beyond the channel's count hold what an earlier dispatch left: read, not used)
+            const int* map = a.comb_map + (static_cast<std::size_t>(c) * a.slots_full + e.j) * map_stride;
+            e.count = __ldg(a.recv_chan_counts + c);
+            e.head = __ldg(reinterpret_cast<const int2*>(map));
+            if (lane < K) e.pair = __ldg(reinterpret_cast<const int2*>(map) + 1 + lane);
+            return e;
+        };
+        auto claim = [&]() {
+            unsigned long long got = 0;
+            if (lane == 0) got = atomicAdd(a.next_unit, 1ull);
+            return got;  // lane 0's value counts
+        };
+        long long u = static_cast<long long>(blockIdx.x) * kBatch;
+        Entry e[kBatch];
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i) e[i] = load_entry(u + i);
+        unsigned long long claimed = claim();
+        int filled = 0;  // stages handed to the consumers
+        while (ok && u < units) {
+            const long long next_u = (static_cast<long long>(gridDim.x) + static_cast<long long>(__shfl_sync(0xffffffffu, claimed, 0))) * kBatch;
+            Entry next[kBatch];
+#pragma unroll
+            for (int i = 0; i < kBatch; ++i) next[i] = load_entry(next_u + i);
+            if (next_u < units) claimed = claim();
+#pragma unroll
+            for (int i = 0; i < kBatch; ++i) {
+                if (!ok || e[i].j >= e[i].count) continue;
+                const int stage = filled % stages;
+                ok = __all_sync(0xffffffffu, wait(&sh->empty[stage], (static_cast<unsigned>(filled / stages) & 1u) ^ 1u)) != 0;
+                if (!ok) continue;
+                const int n = e[i].head.y, first = static_cast<int>((u + i) % a.shape.slices) * a.shape.slice_chunks;
+                const int len = min(a.shape.slice_chunks, chunks - first);
+                CombineLocalHeader& header = sh->header[stage];
+                if (lane < n) header.weight[lane] = a.weighted ? __int_as_float(e[i].pair.y) : 1.0f;
+                if (lane == 0) {
+                    header.token = e[i].head.x;
+                    header.n = n;
+                    header.first_chunk = first;
+                    header.chunks = len;
+                }
+                __syncwarp();
+                auto* bar = reinterpret_cast<std::uint64_t*>(&sh->full[stage]);
+                if (lane == 0) ptx::mbar_expect_tx(bar, static_cast<unsigned>(n * len) * 16u);
+                __syncwarp();
+                if (lane < n)
+                    ptx::bulk_g2s(combine_smem + kCombineLocalTiles + static_cast<std::size_t>(stage) * a.shape.stage_bytes + static_cast<std::size_t>(lane) * len * 16,
+                                  reinterpret_cast<const std::uint8_t*>(a.y) + static_cast<std::size_t>(e[i].pair.x) * row_bytes + static_cast<std::size_t>(first) * 16,
+                                  static_cast<unsigned>(len) * 16u, bar);
+                ++filled;
+            }
+            u = next_u;
+#pragma unroll
+            for (int i = 0; i < kBatch; ++i) e[i] = next[i];
+        }
+        if (ok) {  // tell the consumers that this was all
+            const int stage = filled % stages;
+            ok = __all_sync(0xffffffffu, wait(&sh->empty[stage], (static_cast<unsigned>(filled / stages) & 1u) ^ 1u)) != 0;
+            if (ok && lane == 0) {
+                sh->header[stage].n = -1;
+                ptx::mbar_arrive(reinterpret_cast<std::uint64_t*>(&sh->full[stage]));
+            }
+        }
+        if (!ok)  // copies that are still under way: a bounded time to land before shared memory goes away
+            for (int f = max(0, filled - stages); f < filled; ++f)
+                for (unsigned polls = 0; !ptx::mbar_try_wait(reinterpret_cast<std::uint64_t*>(&sh->full[f % stages]), static_cast<unsigned>(f / stages) & 1u) &&
+                                         polls < (1u << 20); ++polls)
+                    ptx::nanosleep(64);
+    } else {
+        // ---- consumers ---------------------------------------------------------------------------------------------
+        const int consumer = warp - 1, rank = consumer * 32 + lane;  // first chunk of this thread in a slice
+        const int first_zero = blockIdx.x * kCombineLocalConsumers + consumer, zero_step = gridDim.x * kCombineLocalConsumers;
+        const std::uint32_t first_mask = first_zero < T ? __ldg(a.plan_mask + first_zero) : 1u;  // needed at the end
+        for (int f = 0;; ++f) {
+            const int stage = f % stages;
+            ok = __all_sync(0xffffffffu, wait(&sh->full[stage], static_cast<unsigned>(f / stages) & 1u)) != 0;
+            if (!ok) break;
+            const CombineLocalHeader& header = sh->header[stage];
+            const int n = header.n, len = header.chunks;
+            if (n < 0) break;
+            const unsigned char* tile = combine_smem + kCombineLocalTiles + static_cast<std::size_t>(stage) * a.shape.stage_bytes;
+            std::uint8_t* dst = reinterpret_cast<std::uint8_t*>(a.out) + static_cast<std::size_t>(header.token) * row_bytes + static_cast<std::size_t>(header.first_chunk) * 16;
+            for (int q = rank; q < len; q += kCombineLocalConsumers * 32) {
+                float acc[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 4
+                for (int r = 0; r < n; ++r) {
+                    const uint4 v = *reinterpret_cast<const uint4*>(tile + (static_cast<std::size_t>(r) * len + q) * 16);
+                    const float w = header.weight[r];
+                    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) {
+                        const float2 p = __bfloat1622float2(h[x]);
+                        acc[2 * x] = fmaf(w, p.x, acc[2 * x]);
+                        acc[2 * x + 1] = fmaf(w, p.y, acc[2 * x + 1]);
+                    }
+                }
+                uint4 packed;
+                __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&packed);
+#pragma unroll
+                for (int x = 0; x < 4; ++x) h[x] = __floats2bfloat162_rn(acc[2 * x], acc[2 * x + 1]);
+                ptx::st_v4(dst + static_cast<std::size_t>(q) * 16, packed);
+            }
+            __syncwarp();
+            if (lane == 0) ptx::mbar_arrive(reinterpret_cast<std::uint64_t*>(&sh->empty[stage]));
+        }
+        // tokens that were routed nowhere have no entry: their result is zero
+        for (int t = first_zero; ok && t < T; t += zero_step) {
+            if ((t == first_zero ? first_mask : __ldg(a.plan_mask + t)) != 0) continue;
+            for (int q = lane; q < chunks; q += 32)
+                ptx::st_v4(reinterpret_cast<std::uint8_t*>(a.out) + static_cast<std::size_t>(t) * row_bytes + static_cast<std::size_t>(q) * 16, make_uint4(0u, 0u, 0u, 0u));
+        }
+    }
+
+    __syncthreads();
+    if (warp == 0) {
+        unsigned long long finished = 0;
+        if (lane == 0) {
+            __threadfence();
+            finished = atomicAdd(a.cta_done, 1ull) + 1ull;
+        }
+        if (__shfl_sync(0xffffffffu, finished, 0) == gridDim.x) {
+            // launches that share these counters are stream-ordered
+            int rows = 0;
+            if (!aborted)
+                for (int c = lane; c < C; c += 32) rows += __ldg(a.recv_chan_counts + c);
+            rows = __reduce_add_sync(0xffffffffu, rows);
+            if (lane == 0) {
+                __threadfence();
+                *a.cta_done = 0ull;
+                *a.next_unit = 0ull;
+                a.stats[0] = rows;
+                a.stats[2] = static_cast<std::int64_t>(ptx::globaltimer_ns() - __ldcg(a.first_start));
+                a.stats[1] = a.stats[3] = a.stats[4] = a.stats[5] = a.stats[6] = a.stats[7] = 0;
+                *a.first_start = ~0ull;
+                if (ptx::ld_volatile(&rc->sticky[0]) == 0) rc->epochs[1] += 1;
+            }
+        }
+    }
+}
+
+#endif  // __CUDACC__
+
+}  // namespace bep

@@ -5,8 +5,9 @@
 #include <mutex>
 
 #include "combine.cuh"
-#include "dispatch.cuh"
+#include "combine_local.cuh"
 #include "combine_push.cuh"
+#include "dispatch.cuh"
 #include "fused_reduce.cuh"
 
 namespace bep {
@@ -83,6 +84,28 @@ cudaError_t launch_dispatch(const DispatchLaunch& launch, int ctas, int threads,
     const dim3 grid(ctas, launch.num_virtual, 1);
     if (threads <= kSmallCtaThreads) return cooperative_launch(dispatch_kernel<kSmallCtaThreads>, launch, grid, threads, smem, stream);
     return cooperative_launch(dispatch_kernel<kMaxWarps * 32>, launch, grid, threads, smem, stream);
+}
+
+cudaError_t launch_combine_local(const CombineLocalArgs& args, cudaStream_t stream) {
+    const auto kernel = args.shape.batch == 1 ? local_combine_push_kernel<1> : local_combine_push_kernel<4>;
+    static std::mutex mutex;
+    static std::size_t configured[64] = {0};
+    {
+        std::lock_guard<std::mutex> guard(mutex);
+        int device = 0;
+        cudaError_t status = cudaGetDevice(&device);
+        if (status != cudaSuccess) return status;
+        if (device < 0 || device >= 64) return cudaErrorInvalidDevice;
+        if (args.shape.bytes > configured[device]) {
+            status = cudaFuncSetAttribute(local_combine_push_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(args.shape.bytes));
+            if (status == cudaSuccess)
+                status = cudaFuncSetAttribute(local_combine_push_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(args.shape.bytes));
+            if (status != cudaSuccess) return status;
+            configured[device] = args.shape.bytes;
+        }
+    }
+    kernel<<<args.shape.ctas, kCombineLocalThreads, args.shape.bytes, stream>>>(args);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_combine(const CombineLaunch& launch, int channels, std::size_t crow_stride, cudaStream_t stream) {

@@ -6,6 +6,7 @@
 
 #include <cuda_runtime.h>
 
+#include "combine_local.cuh"
 #include "combine_push.cuh"
 #include "fused_reduce.cuh"
 #include "protocol.cuh"
@@ -27,6 +28,9 @@ int combine_resident_ctas(int threads);
 cudaError_t launch_dispatch(const DispatchLaunch& launch, int ctas, int threads, std::size_t smem,
                             cudaStream_t stream);
 cudaError_t launch_combine(const CombineLaunch& launch, int channels, std::size_t crow_stride, cudaStream_t stream);
+
+// Combine of a group of one rank: an ordinary launch.
+cudaError_t launch_combine_local(const CombineLocalArgs& args, cudaStream_t stream);
 
 // Ordinary launches of the combine paths: expert-side gather-reduce-push, owner-side sum.  Any grid size works.
 // `reduce_ctas` reducer CTAs follow the args.forward_ctas forwarder CTAs in one grid.
