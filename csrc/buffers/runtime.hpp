@@ -304,7 +304,13 @@ class Runtime {
         epochs_ = at::zeros({4}, i64);
         grid_bar_ = at::zeros({2}, i64);
         done_ctas_ = at::zeros({2}, i64);
-        block_hist_ = at::zeros({static_cast<std::int64_t>(hist_scratch_ints(C, E + P))}, i32);
+        // scratch of the layout phase; with a single rank the local kernel's counters and scratch lie in front of it
+        if (num_ranks == 1) {
+            cuda_check(cudaDeviceGetAttribute(&local_sms_, cudaDevAttrMultiProcessorCount, device), "query the device");
+            local_plan_ = plan_dispatch_local(lay_, local_sms_, max_smem_);
+            if (local_plan_.usable) local_ints_ = static_cast<std::int64_t>(align_up(kLocalCounterInts + dispatch_local_hist_ints(lay_, local_sms_), 32));
+        }
+        block_hist_ = at::zeros({local_ints_ + static_cast<std::int64_t>(hist_scratch_ints(C, E + P))}, i32);
         sticky_ = at::zeros({8}, i32);
         chan_stats_ = at::zeros({2, C + options_.send_ctas, 10}, i64);
         plan_flags_ = at::zeros({C}, i64);
@@ -334,7 +340,7 @@ class Runtime {
         rc_.epochs = reinterpret_cast<std::uint64_t*>(epochs_.data_ptr<std::int64_t>());
         rc_.grid_bar = reinterpret_cast<unsigned long long*>(grid_bar_.data_ptr<std::int64_t>());
         rc_.done_ctas = reinterpret_cast<unsigned long long*>(done_ctas_.data_ptr<std::int64_t>());
-        rc_.block_hist = block_hist_.data_ptr<int>();
+        rc_.block_hist = block_hist_.data_ptr<int>() + local_ints_;
         rc_.sticky = sticky_.data_ptr<int>();
         rc_.chan_stats = chan_stats_.data_ptr<std::int64_t>();
         rc_.delay_meta_ns = options_.delay_meta_ns;
@@ -451,11 +457,25 @@ class Runtime {
         PreparedDispatch p = prepare_dispatch(x, topk_idx, topk_weights, alignment, expand, zero_padding, cached, graph_pool);
         cudaStream_t launch_stream = stream != 0 ? reinterpret_cast<cudaStream_t>(stream)
                                                  : at::cuda::getCurrentCUDAStream(device_).stream();
+        if (dispatch_is_local()) {
+            cuda_check(launch_dispatch_local(p.args, rc_, local_plan_, block_hist_.data_ptr<int>() + kLocalCounterInts,
+                                             reinterpret_cast<unsigned long long*>(block_hist_.data_ptr<int>()), local_sms_, launch_stream),
+                       "dispatch launch");
+            return p.result;
+        }
         DispatchLaunch launch{};
         launch.num_virtual = 1;
         launch.r[0] = p.args;
         cuda_check(launch_dispatch(launch, grid_ctas_, threads_, smem_, launch_stream), "dispatch launch");
         return p.result;
+    }
+
+    // A single rank whose rows move with bulk copies takes the kernel without the protocol (dispatch_local.cuh), unless a
+    // test hook or delay of the protocol is set or the library counts what the protocol's roles do.
+    bool dispatch_is_local() const {
+        return local_plan_.usable && use_tma_ && !role_profiling_enabled() && rc_.delay_meta_ns == 0 && rc_.delay_tx_ns == 0 &&
+               rc_.delay_rx_ns == 0 && rc_.delay_scatter_ns == 0 && rc_.delay_prefix_ns == 0 && rc_.test_skip_done_to == -1 &&
+               rc_.test_withhold_counts == 0 && rc_.test_corrupt_sequence == 0 && rc_.test_abort_after_ns == 0;
     }
 
     // ---- combine --------------------------------------------------------------------------------
@@ -887,6 +907,10 @@ class Runtime {
     std::size_t smem_ = 0, max_smem_ = 0;
     at::Tensor epochs_, grid_bar_, done_ctas_, block_hist_, sticky_, chan_stats_, plan_flags_, rank_const_;
     int grid_ctas_ = 0;
+    // single rank: shared-memory plan of the local dispatch kernel, CTAs it may use, ints of its counters and scratch
+    LocalPlan local_plan_{};
+    int local_sms_ = 0;
+    std::int64_t local_ints_ = 0;
     std::vector<std::shared_ptr<OutputSet>> pools_;
     std::vector<std::shared_ptr<Layout>> plans_;
     std::vector<at::Tensor> combine_pool_;

@@ -1,0 +1,554 @@
+// Dispatch of a group of one rank.  Nothing crosses a link, so of the protocol in dispatch.cuh only the routing layout and
+// the expansion are left: no counts message, no READY flags, no send role, no control warp.  Results, routing plan and
+// combine map are the ones dispatch.cuh leaves behind, bit for bit; the two kernels may alternate on one buffer.
+//
+// Grid: one CTA per SM, or one per token where there are fewer tokens; CTA b owns the tokens [T*b/G, T*(b+1)/G).  (The
+// channels of the configuration only number the combine map here: few CTAs would keep a barrier between ranks short, but
+// the SMs that write the rows are what sets the pace.)
+//   1. token rows are on their way into shared memory before anything about the layout is known;
+//   2. expert ids -> histogram and stable ordinals inside the CTA's tokens, 32 tokens at a time, one thread per (token, k);
+//   3. one grid barrier; then a prefix over the CTAs before this one and a scan over experts, one thread per bin.  A cached
+//      layout skips 2 and the barrier, and its launch is an ordinary one;
+//   4. a warp per token: every lane k < K whose expert is valid starts the bulk store of the row to its expert's segment.
+//
+// What bounds it.  Large batches: writing the expanded rows to HBM.  4096 tokens, hidden 7168, top-8 move 528 MB.
+// Small ones: the chain launch -> ids -> barrier -> prefix -> rows.  Launch to end with a cold L2, general kernel -> this
+// one: 128 tokens 46 -> 19 us (no flags to wait for, no prefix by a single warp), 4096 tokens 131 ->
+// 110 us, the same with E4M3 rows 106 -> 73 us (fourteen row buffers per SM on all SMs instead of eight on 128), 256 tokens
+// with a cached layout 45 -> 17 us.
+#pragma once
+
+#include "dispatch_common.cuh"
+
+namespace bep {
+
+constexpr int kLocalThreads = 512;
+constexpr int kLocalWarps = kLocalThreads / 32;
+constexpr int kLocalMaxStages = 3;      // row buffers per warp
+constexpr int kLocalMinWarps = 4;       // fewer row buffers than this: rows too long, dispatch.cuh takes the call
+constexpr int kLocalMaxPairBytes = 64 * 1024;
+
+struct LocalDispatchArgs {
+    DispatchArgs a;
+    LocalPlan plan;
+    int* hist;                     // [G][E + 1] counts per CTA, then two copies of [groups][E + 1 + C] sums, then their generation
+    unsigned long long* counters;  // barrier arrivals, finished CTAs, complement of the first start (zero between launches)
+    int hist_ctas;                 // CTAs the scratch has room for
+    int num_experts, num_channels, num_topk, hidden, slots_full, expanded_cap, unique_cap, recv_fp8;  // as in the rank's constants
+};
+
+inline std::size_t local_hist_ints(int ctas, int experts, int channels) {
+    const std::size_t groups = static_cast<std::size_t>((ctas + kHistGroup - 1) / kHistGroup);
+    return static_cast<std::size_t>(ctas) * (experts + 1) + 2 * groups * (experts + 1 + channels) + 1;
+}
+
+struct LocalShared {
+    unsigned long long mbar[kLocalWarps * kLocalMaxStages];
+    unsigned long long warp_sum[kLocalWarps];
+    int flag;        // the CTA leaves without rows
+    int routed;      // routed tokens of this CTA
+    int first_unique;  // routed tokens of earlier CTAs
+    int unique_total;
+};
+
+// header | base[E] | total[E] | eoff[E + 1] | chan_base[C] | pair_e[cap*K] | pair_ord[cap*K] | unique[cap] | row buffers
+inline LocalPlan make_local_plan(int experts, int channels, int topk, int hidden, int max_tokens, int sms, std::size_t smem_limit) {
+    LocalPlan p;
+    p.token_cap = (max_tokens + sms - 1) / sms + 1;
+    const std::size_t pair_bytes = static_cast<std::size_t>(p.token_cap) * (8 * topk + 4);
+    std::size_t bytes = align_up(sizeof(LocalShared), 16) + static_cast<std::size_t>(experts) * 12 + 4 + static_cast<std::size_t>(channels) * 4;
+    bytes = align_up(bytes + pair_bytes, 128);
+    p.rows_off = bytes;
+    p.slot_bytes = static_cast<int>(align_up(static_cast<std::size_t>(hidden) * 2, 128));
+    if (pair_bytes > static_cast<std::size_t>(kLocalMaxPairBytes) || bytes >= smem_limit) return p;
+    const int slots = static_cast<int>((smem_limit - bytes) / static_cast<std::size_t>(p.slot_bytes));
+    p.warps = slots < kLocalWarps ? slots : kLocalWarps;
+    p.stages = slots / kLocalWarps < 1 ? 1 : slots / kLocalWarps < kLocalMaxStages ? slots / kLocalWarps : kLocalMaxStages;
+    p.bytes = bytes + static_cast<std::size_t>(p.warps) * p.stages * p.slot_bytes;
+    p.usable = p.warps >= kLocalMinWarps;
+    return p;
+}
+
+#ifdef __CUDACC__
+
+namespace detail {
+
+__device__ __forceinline__ void local_wait_read(int groups_left) {
+    if (groups_left <= 0) bulk_wait_group_read<0>();
+    else if (groups_left == 1) bulk_wait_group_read<1>();
+    else bulk_wait_group_read<2>();
+}
+
+}  // namespace detail
+
+__global__ void __launch_bounds__(kLocalThreads, 1) local_dispatch_kernel(const __grid_constant__ LocalDispatchArgs args) {
+    using namespace detail;
+    const DispatchArgs& a = args.a;
+    const RankConst* __restrict__ rc = a.rc;
+    const int E = args.num_experts, C = args.num_channels, K = args.num_topk, H = args.hidden, Qf = args.slots_full;
+    const int T = a.num_tokens, G = gridDim.x, b = blockIdx.x;
+    const int Tc = max(1, (T + C - 1) / C);
+    const int t0 = static_cast<int>(static_cast<long long>(T) * b / G), t1 = static_cast<int>(static_cast<long long>(T) * (b + 1) / G);
+    const int nt = t1 - t0;
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const unsigned lane = ptx::lane_id(), full = 0xffffffffu, lt_mask = (1u << lane) - 1u;
+    const bool recv_fp8 = args.recv_fp8 != 0, expand = a.do_expand != 0, cached = a.cached != 0;
+    const int row_warps = args.plan.warps, stages = args.plan.stages, slot_bytes = args.plan.slot_bytes;
+    const unsigned in_bytes = static_cast<unsigned>(H) * 2u;
+
+    extern __shared__ __align__(128) unsigned char local_smem[];
+    auto* sh = reinterpret_cast<LocalShared*>(local_smem);
+    int* base = reinterpret_cast<int*>(local_smem + align_up(sizeof(LocalShared), 16));  // [E] rows of earlier CTAs in the expert
+    int* total = base + E;         // [E] rows of the expert; the bit sets of a 32-token chunk before that
+    int* eoff = total + E;         // [E + 1]
+    int* chan_base = eoff + E + 1; // [C] routed tokens of earlier channels
+    int* pair_e = chan_base + C;   // [cap * K] expert of (token, k), -1: none
+    int* pair_ord = pair_e + args.plan.token_cap * K;  // stable ordinal of the pair in its expert: inside the CTA (fresh layout) or overall (cached)
+    int* unique = pair_ord + args.plan.token_cap * K;  // [cap] ordinal of the routed token: inside the CTA (fresh) or in its channel (cached); else the complement of it
+    unsigned char* rows_sm = local_smem + args.plan.rows_off;
+
+    // what thread 0 has to know about the rank (asked for now, looked at after the histogram)
+    const int sticky_before = tid == 0 ? ptx::ld_volatile(&rc->sticky[0]) : 0;
+    const std::uint64_t epoch_before = tid == 0 ? __ldcg(rc->epochs) : 0;
+    const unsigned long long t_start = ptx::globaltimer_ns();
+    if (tid == 0) atomicMax(&args.counters[2], ~t_start);
+    // profile rows are per channel: CTA b fills the rows b, b + G, ...
+#define BEP_PROF(point)                                                                                          \
+    do {                                                                                                         \
+        const std::int64_t now_ = static_cast<std::int64_t>(ptx::globaltimer_ns());                              \
+        for (int r_ = b; r_ < C; r_ += G) a.profile[static_cast<std::size_t>(r_) * 16 + (point)] = now_;         \
+    } while (0)
+    if (tid == 0)
+        for (int r = b; r < C; r += G) {
+            std::int64_t* prof = a.profile + static_cast<std::size_t>(r) * 16;
+            prof[kProfStart] = prof[kProfGuardDone] = static_cast<std::int64_t>(t_start);
+            prof[kProfFirstTxDone] = prof[kProfFirstRxRow] = 0;
+        }
+    Health health(rc, a.error);
+
+    if (tid < row_warps * stages) {
+        ptx::mbar_init(reinterpret_cast<std::uint64_t*>(&sh->mbar[tid]), 1);
+        ptx::mbar_fence_init();
+    }
+    // ids of the first chunk are asked for now; they arrive while shared memory is cleared
+    const int first_pairs = min(32, nt) * K;
+    const std::int64_t first_id = tid < first_pairs ? __ldg(a.topk_idx + static_cast<std::size_t>(t0) * K + tid) : -1;
+    const int W = E + 1, S = W + C;
+    const int groups = (args.hist_ctas + kHistGroup - 1) / kHistGroup;
+    int* const sums_base = args.hist + static_cast<std::size_t>(args.hist_ctas) * W;
+    int* const generation_at = sums_base + static_cast<std::size_t>(2) * groups * S;
+    const int generation = cached ? 0 : __ldcg(generation_at);
+    if (tid == 0) {
+        sh->flag = 0;
+        sh->routed = 0;
+        sh->first_unique = 0;
+    }
+    for (int i = tid; i < E; i += kLocalThreads) {
+        base[i] = 0;
+        total[i] = 0;
+    }
+    if (!cached) {
+        // the sums this CTA will add to have been driven out of L2 by the rows of the last launch: fetch both copies' lines
+        for (int i = tid * 32; i < S; i += kLocalThreads * 32)
+            for (int copy = 0; copy < 2; ++copy)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(sums_base + (static_cast<std::size_t>(copy) * groups + b / kHistGroup) * S + i));
+    }
+    __syncthreads();
+
+    // ---- 1. the first rows of every warp start their way into shared memory ----------------------------------
+    auto start_load = [&](int n) {  // the warp's n-th token (lane 0 only)
+        const int i = warp + n * row_warps;
+        auto* bar = reinterpret_cast<std::uint64_t*>(&sh->mbar[warp * stages + n % stages]);
+        ptx::mbar_expect_tx(bar, in_bytes);
+        ptx::bulk_g2s(rows_sm + static_cast<std::size_t>(warp * stages + n % stages) * slot_bytes, a.x + static_cast<std::size_t>(t0 + i) * H, in_bytes, bar);
+    };
+    int started = 0;  // loads of this warp that are under way or done
+    auto start_first_loads = [&]() {
+        if (warp >= row_warps) return;
+        for (; started < stages && warp + started * row_warps < nt; ++started)
+            if (lane == 0) start_load(started);
+    };
+
+    // a rank that has failed, or has run out of epochs, leaves without rows
+    auto leaves = [&]() {  // thread 0
+        if (sticky_before != 0) {
+            if (b == 0) atomicCAS(&a.error[0], 0, kErrAlreadyAborted);
+            return true;
+        }
+        if (epoch_before + 1 >= (1ull << 32)) record_error(rc, a.error, kErrEpochExhausted, 0, 0);
+        return epoch_before + 1 >= (1ull << 32);
+    };
+
+    // ---- 2. ordinals inside the CTA ------------------------------------------------------------------------------
+    if (!cached) {
+        unsigned* bits = reinterpret_cast<unsigned*>(total);
+        constexpr int kLastFlag = 1 << 30;  // the pair of the chunk's last token in its expert carries the count forward
+        int routed_before = 0;              // (last warp) routed tokens of earlier chunks
+        for (int c0 = 0; c0 < nt; c0 += 32) {
+            const int pairs = min(32, nt - c0) * K;
+            for (int p = tid; p < pairs; p += kLocalThreads) {
+                const std::int64_t e = (c0 == 0 && p == tid) ? first_id : __ldg(a.topk_idx + static_cast<std::size_t>(t0 + c0) * K + p);
+                const int tl = p / K, k = p % K;
+                int mine = -1;
+                if (e < -1 || e >= E) {
+                    record_error(rc, a.error, kErrInvalidRouting, t0 + c0 + tl, k);
+                } else if (e >= 0) {
+                    if (atomicOr(&bits[e], 1u << tl) >> tl & 1u) {  // the token names this expert twice
+                        int at = k;
+                        for (int k2 = k + 1; k2 < K; ++k2)
+                            if (a.topk_idx[static_cast<std::size_t>(t0 + c0 + tl) * K + k2] == e) at = k2;
+                        record_error(rc, a.error, kErrInvalidRouting, t0 + c0 + tl, at);
+                    } else {
+                        mine = static_cast<int>(e);
+                    }
+                }
+                pair_e[c0 * K + p] = mine;
+            }
+            __syncthreads();
+            for (int p = tid; p < pairs; p += kLocalThreads) {
+                const int e = pair_e[c0 * K + p], tl = p / K;
+                if (e < 0) continue;
+                const unsigned set = bits[e];
+                const int ord = base[e] + __popc(set & ((1u << tl) - 1u));
+                pair_ord[c0 * K + p] = ord | (tl == 31 - __clz(set) ? kLastFlag : 0);
+            }
+            if (warp == kLocalWarps - 1) {
+                bool routed = false;
+                if (c0 + static_cast<int>(lane) < nt)
+                    for (int k = 0; k < K; ++k) routed = routed || pair_e[(c0 + lane) * K + k] >= 0;
+                const unsigned m = __ballot_sync(full, routed);
+                if (c0 + static_cast<int>(lane) < nt) unique[c0 + lane] = routed ? routed_before + __popc(m & lt_mask) : ~(routed_before + __popc(m & lt_mask));
+                routed_before += __popc(m);
+                if (lane == 0) sh->routed = routed_before;
+            }
+            __syncthreads();
+            for (int p = tid; p < pairs; p += kLocalThreads) {
+                const int e = pair_e[c0 * K + p];
+                if (e < 0) continue;
+                const int ord = pair_ord[c0 * K + p];
+                if (ord & kLastFlag) {
+                    pair_ord[c0 * K + p] = ord & ~kLastFlag;
+                    base[e] = (ord & ~kLastFlag) + 1;
+                    bits[e] = 0;
+                }
+            }
+            __syncthreads();
+        }
+        // ---- 3. prefix over the CTAs before this one.  Two levels (groups of kHistGroup CTAs, then the CTAs of the group),
+        // as in dispatch.cuh: a CTA reads G / kHistGroup + kHistGroup rows, all at once, instead of G.
+        int* const sums = sums_base + static_cast<std::size_t>(generation & 1) * groups * S;
+        int* const sums_next = sums_base + static_cast<std::size_t>((generation + 1) & 1) * groups * S;
+        const int my_group = b / kHistGroup;
+        for (int i = tid; i < W; i += kLocalThreads) {
+            const int v = i < E ? base[i] : sh->routed;
+            args.hist[static_cast<std::size_t>(b) * W + i] = v;
+            if (v != 0) atomicAdd(sums + static_cast<std::size_t>(my_group) * S + i, v);
+        }
+        if (nt > 0) {  // routed tokens per channel: a thread per channel that this CTA's tokens touch
+            auto routed_before = [&](int i) { return i >= nt ? sh->routed : unique[i] >= 0 ? unique[i] : ~unique[i]; };
+            for (int ch = t0 / Tc + tid; ch <= (t1 - 1) / Tc; ch += kLocalThreads) {
+                const int v = routed_before(min(t1, (ch + 1) * Tc) - t0) - routed_before(max(t0, ch * Tc) - t0);
+                if (v != 0) atomicAdd(sums + static_cast<std::size_t>(my_group) * S + W + ch, v);
+            }
+        }
+        for (int i = b * kLocalThreads + tid; i < groups * S; i += G * kLocalThreads) sums_next[i] = 0;
+        __threadfence();  // every thread's own stores and reductions, before the CTA arrives
+        if (tid == 0) BEP_PROF(kProfHistDone);
+        start_first_loads();
+        __syncthreads();
+        if (tid == 0) {
+            __threadfence();
+            atomicAdd(&args.counters[0], 1ull);
+            while (ptx::ld_acquire_gpu(reinterpret_cast<const std::uint64_t*>(&args.counters[0])) < static_cast<std::uint64_t>(G))
+                if (health.give_up(kErrGridBarrier, b, 0)) break;
+            __threadfence();
+            sh->flag = leaves() || health.failed() ? 1 : 0;
+            BEP_PROF(kProfBarrierDone);
+        }
+        __syncthreads();
+        if (!sh->flag) {
+            for (int i = tid; i < S; i += kLocalThreads) {
+                int before = 0, all = 0;
+                for (int g0 = 0; g0 < groups; g0 += 10) {
+                    int v[10];
+#pragma unroll
+                    for (int u = 0; u < 10; ++u) v[u] = g0 + u < groups ? __ldcg(sums + static_cast<std::size_t>(g0 + u) * S + i) : 0;
+#pragma unroll
+                    for (int u = 0; u < 10; ++u) {
+                        all += v[u];
+                        before += g0 + u < my_group ? v[u] : 0;
+                    }
+                }
+                if (i >= W) {  // a channel's routed tokens
+                    chan_base[i - W] = all;
+                    continue;
+                }
+                int v[kHistGroup];
+#pragma unroll
+                for (int u = 0; u < kHistGroup; ++u) {
+                    const int b2 = my_group * kHistGroup + u;
+                    v[u] = b2 < b ? __ldcg(args.hist + static_cast<std::size_t>(b2) * W + i) : 0;
+                }
+#pragma unroll
+                for (int u = 0; u < kHistGroup; ++u) before += v[u];
+                if (i < E) {
+                    base[i] = before;
+                    total[i] = all;
+                } else {
+                    sh->first_unique = before;
+                    sh->unique_total = all;
+                }
+            }
+        }
+    } else {
+        start_first_loads();
+        if (tid == 0 && leaves()) sh->flag = 1;
+        for (int p = tid; p < nt * K; p += kLocalThreads) {
+            const std::int64_t e = p == tid && p < first_pairs ? first_id : __ldg(a.topk_idx + static_cast<std::size_t>(t0) * K + p);
+            pair_e[p] = e >= 0 && e < E ? static_cast<int>(e) : -1;
+            pair_ord[p] = a.plan_expert_ord[static_cast<std::size_t>(t0) * K + p];
+        }
+        for (int i = tid; i < nt; i += kLocalThreads) unique[i] = (a.plan_mask[t0 + i] & 1u) ? a.plan_slot[t0 + i] : -1;
+        for (int i = tid; i < 1 + E + C; i += kLocalThreads) {
+            const int v = a.plan_counts[i];
+            if (i == 0) sh->unique_total = v;
+            else if (i <= E) total[i - 1] = v;
+            else chan_base[i - 1 - E] = v;
+        }
+    }
+    __syncthreads();
+    bool failed = sh->flag != 0;
+    if (tid == 0) BEP_PROF(kProfPrefixScan);
+
+    // ---- aligned scan over experts (a thread takes consecutive bins), scan over channels (last warp) ----------
+    int own_from = 0, own_to = 0;
+    unsigned long long run = 0;  // padded rows in the upper half, true rows in the lower
+    auto padded = [&](int count) { return a.alignment == 1 ? count : (count + a.alignment - 1) / a.alignment * a.alignment; };
+    if (!failed) {
+        const int per = (E + kLocalThreads - 1) / kLocalThreads;
+        own_from = min(E, tid * per);
+        own_to = min(E, own_from + per);
+        for (int i = own_from; i < own_to; ++i) run += static_cast<unsigned long long>(padded(total[i])) << 32 | static_cast<unsigned>(total[i]);
+        unsigned long long incl = run;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long v = __shfl_up_sync(full, incl, o);
+            if (lane >= static_cast<unsigned>(o)) incl += v;
+        }
+        if (lane == 31) sh->warp_sum[warp] = incl;
+        run = incl - run;  // what comes before this thread's bins inside the warp
+    }
+    __syncthreads();
+    unsigned long long all_rows = 0;
+    if (!failed) {
+#pragma unroll
+        for (int w = 0; w < kLocalWarps; ++w) {
+            const unsigned long long s = sh->warp_sum[w];
+            if (w < warp) run += s;
+            all_rows += s;
+        }
+        int at = static_cast<int>(run >> 32);
+        for (int i = own_from; i < own_to; ++i) {
+            eoff[i] = at;
+            at += padded(total[i]);
+        }
+        if (tid == 0) eoff[E] = static_cast<int>(all_rows >> 32);
+        if (warp == kLocalWarps - 1) {
+            int before = 0;
+            for (int c0 = 0; c0 < C; c0 += 32) {
+                const int v = c0 + static_cast<int>(lane) < C ? chan_base[c0 + lane] : 0;
+                if (b == G - 1 && c0 + static_cast<int>(lane) < C) {
+                    a.recv_chan_counts[c0 + lane] = v;
+                    if (!cached) a.plan_counts[1 + E + c0 + lane] = v;
+                }
+                int incl = v;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int up = __shfl_up_sync(full, incl, o);
+                    if (lane >= static_cast<unsigned>(o)) incl += up;
+                }
+                if (c0 + static_cast<int>(lane) < C) chan_base[c0 + lane] = before + incl - v;
+                before += __shfl_sync(full, incl, 31);
+            }
+        }
+    }
+    __syncthreads();
+    if (!failed && (static_cast<int>(all_rows >> 32) > args.expanded_cap || sh->unique_total > args.unique_cap)) {
+        if (tid == 0) record_error(rc, a.error, kErrCapacity, static_cast<int>(all_rows >> 32), sh->unique_total);
+        failed = true;
+    }
+    if (tid == 0) {
+        const std::int64_t now = static_cast<std::int64_t>(ptx::globaltimer_ns());
+        for (int r = b; r < C; r += G) {
+            std::int64_t* prof = a.profile + static_cast<std::size_t>(r) * 16;
+            prof[kProfCountsSent] = prof[kProfOrdinalsDone] = prof[kProfRolesSplit] = now;
+            prof[kProfCountsArrived] = prof[kProfPrefixReady] = prof[kProfTxDone] = now;
+        }
+        if (b == G - 1) {
+            a.prefix_tx_ts[0] = static_cast<std::int64_t>(t_start);
+            a.prefix_tx_ts[1] = now;
+        }
+        for (int r = b; r < C; r += G) {
+            a.prefix_tx_ts[(r + 1) * 2 + 0] = 0;
+            a.prefix_tx_ts[(r + 1) * 2 + 1] = now;
+        }
+    }
+
+    // ---- 4. rows -------------------------------------------------------------------------------------------------------
+    const std::size_t out_row_bytes = static_cast<std::size_t>(H) * (recv_fp8 ? 1 : 2);
+    auto* const recv_bytes = reinterpret_cast<std::uint8_t*>(a.recv_x);
+    const int map_stride = 2 + 2 * K;
+    if (warp < row_warps && !failed) {
+        for (int n = 0, i = warp; i < nt; ++n, i += row_warps) {
+            const int t = t0 + i;
+            int e = -1, ord = -1;
+            float wgt = 1.0f;
+            if (lane < static_cast<unsigned>(K)) {
+                if (a.topk_w) wgt = __ldg(a.topk_w + static_cast<std::size_t>(t) * K + lane);
+                e = pair_e[i * K + lane];
+                if (e >= 0) ord = pair_ord[i * K + lane] + base[e];
+            }
+            const unsigned valid = __ballot_sync(full, e >= 0);
+            const int u = unique[i], c = t / Tc;
+            const bool routed = u >= 0;
+            const int j = cached ? u : u + sh->first_unique - chan_base[c];  // ordinal in the channel
+            int row = -1;  // this lane's output row
+            if (routed) {
+                if (expand) row = e >= 0 ? eoff[e] + ord : -1;
+                else if (lane == 0) row = chan_base[c] + j;
+            }
+            const int buffer = warp * stages + n % stages;
+            unsigned char* slot = rows_sm + static_cast<std::size_t>(buffer) * slot_bytes;
+            if (!__all_sync(full, mbar_wait_bounded(&sh->mbar[buffer], static_cast<unsigned>(n / stages) & 1u, health))) {
+                failed = true;
+                break;
+            }
+            float scale = 1.0f;
+            if (recv_fp8 && routed) {
+                scale = quantise_row_in_place(slot, H);
+                ptx::fence_proxy_async_smem();
+                __syncwarp();
+            }
+            // every lane with a row starts its own copy: the bulk groups are the lanes' own
+            if (row >= 0) ptx::bulk_s2g(recv_bytes + static_cast<std::size_t>(row) * out_row_bytes, slot, static_cast<unsigned>(out_row_bytes));
+            ptx::bulk_commit();
+            if (routed) {
+                int* map = a.comb_map + (static_cast<std::size_t>(c) * Qf + j) * map_stride;
+                if (lane == 0) *reinterpret_cast<int2*>(map) = make_int2(t, expand ? __popc(valid) : 1);
+                if (expand) {
+                    if (row >= 0) {
+                        if (recv_fp8) a.recv_scale[row] = scale;
+                        a.recv_idx[row] = e;
+                        a.recv_w[row] = wgt;
+                        std::int64_t* meta = a.source_meta + static_cast<std::size_t>(row) * 3;
+                        meta[0] = 0;
+                        meta[1] = t;
+                        meta[2] = lane;
+                        *reinterpret_cast<int2*>(map + 2 + 2 * __popc(valid & lt_mask)) = make_int2(row, __float_as_int(wgt));
+                    }
+                } else {
+                    const int r = __shfl_sync(full, row, 0);
+                    if (lane < static_cast<unsigned>(K)) {
+                        a.recv_idx[static_cast<std::size_t>(r) * K + lane] = e;
+                        a.recv_w[static_cast<std::size_t>(r) * K + lane] = e >= 0 ? wgt : 0.0f;
+                    }
+                    if (lane == 0) {
+                        if (recv_fp8) a.recv_scale[r] = scale;
+                        std::int64_t* meta = a.source_meta + static_cast<std::size_t>(r) * 3;
+                        meta[0] = 0;
+                        meta[1] = t;
+                        meta[2] = -1;
+                        *reinterpret_cast<int2*>(map + 2) = make_int2(r, __float_as_int(1.0f));
+                    }
+                }
+            }
+            if (!cached) {
+                if (lane < static_cast<unsigned>(K)) a.plan_expert_ord[static_cast<std::size_t>(t) * K + lane] = ord;
+                if (lane == 0) {
+                    a.plan_mask[t] = routed ? 1u : 0u;
+                    a.plan_slot[t] = routed ? j : -1;
+                }
+            }
+            // the next token's load goes into the oldest buffer, once its copies have left it
+            if (warp + started * row_warps < nt) {
+                local_wait_read(stages - 1);
+                __syncwarp();
+                if (n + 1 >= stages) {
+                    if (lane == 0) start_load(started);
+                    ++started;
+                }
+            }
+        }
+    }
+    if (failed && warp < row_warps) {
+        // loads that are still under way: give them a bounded time to land before shared memory goes away
+        for (int n = max(0, started - stages); n < started; ++n)
+            for (unsigned polls = 0; !ptx::mbar_try_wait(reinterpret_cast<std::uint64_t*>(&sh->mbar[warp * stages + n % stages]),
+                                                         static_cast<unsigned>(n / stages) & 1u) && polls < (1u << 20); ++polls)
+                ptx::nanosleep(64);
+    }
+    if (!failed) {
+        if (expand && a.zero_padding) {  // rows between the experts' segments
+            for (int el = b * kLocalWarps + warp; el < E; el += G * kLocalWarps) {
+                for (int row = eoff[el] + total[el]; row < eoff[el + 1]; ++row) {
+                    if (recv_fp8) {
+                        for (int x = lane; x < H; x += 32) recv_bytes[static_cast<std::size_t>(row) * H + x] = 0;
+                        if (lane == 0) a.recv_scale[row] = 0.0f;
+                    } else {
+                        zero_row(recv_bytes + static_cast<std::size_t>(row) * out_row_bytes, H, true);
+                    }
+                    if (lane == 0) {
+                        a.recv_idx[row] = -1;
+                        a.recv_w[row] = 0.0f;
+                    }
+                    if (lane < 3) a.source_meta[static_cast<std::size_t>(row) * 3 + lane] = -1;
+                }
+            }
+        }
+        if (b == G - 1) {
+            for (int i = tid; i < E; i += kLocalThreads) {
+                a.expert_counts[i] = total[i];
+                a.expert_offsets[i] = eoff[i];
+                a.expert_prefix[i] = eoff[i] + total[i];
+                a.source_expert_prefix[i] = 0;
+                if (!cached) a.plan_counts[1 + i] = total[i];
+            }
+            if (tid == 0) {
+                a.expert_offsets[E] = eoff[E];
+                a.source_offsets[0] = 0;
+                a.source_offsets[1] = sh->unique_total;
+                a.unique_count[0] = sh->unique_total;
+                a.expanded_count[0] = static_cast<std::int64_t>(all_rows & 0xffffffffull);
+                if (!cached) a.plan_counts[0] = sh->unique_total;
+            }
+        }
+    }
+    bulk_wait_group_read<0>();  // the row buffers have been read; the rows themselves are complete when the launch is
+    const bool any_failed = __syncthreads_or(failed ? 1 : 0) != 0;
+
+    // ---- epilogue: the last CTA settles the launch ---------------------------------------------------------------
+    if (tid == 0) {
+        BEP_PROF(kProfRxDone);
+        BEP_PROF(kProfEnd);
+        if (any_failed) return;  // the rank has failed: nothing of it is used again
+        __threadfence();
+        if (atomicAdd(&args.counters[1], 1ull) + 1ull == static_cast<unsigned long long>(G)) {
+            __threadfence();
+            for (int i = 0; i < 8; ++i) a.stats[i] = i == kStatLocalRows ? sh->unique_total : 0;
+            a.timestamps[0] = static_cast<std::int64_t>(~__ldcg(&args.counters[2]));
+            a.timestamps[1] = static_cast<std::int64_t>(ptx::globaltimer_ns());
+            args.counters[0] = args.counters[1] = args.counters[2] = 0ull;
+            if (ptx::ld_volatile(&rc->sticky[0]) == 0) {
+                const std::uint64_t epoch = epoch_before + 1;
+                ptx::st_release_sys(flag_ptr(rc->seg[rc->rank], rc->lay.done_off, rc->rank), epoch);
+                rc->epochs[0] = epoch;
+                if (!cached) *generation_at = generation + 1;
+            }
+        }
+    }
+#undef BEP_PROF
+}
+
+#endif  // __CUDACC__
+
+}  // namespace bep

@@ -8,6 +8,7 @@
 #include "combine_local.cuh"
 #include "combine_push.cuh"
 #include "dispatch.cuh"
+#include "dispatch_local.cuh"
 #include "fused_reduce.cuh"
 
 namespace bep {
@@ -84,6 +85,36 @@ cudaError_t launch_dispatch(const DispatchLaunch& launch, int ctas, int threads,
     const dim3 grid(ctas, launch.num_virtual, 1);
     if (threads <= kSmallCtaThreads) return cooperative_launch(dispatch_kernel<kSmallCtaThreads>, launch, grid, threads, smem, stream);
     return cooperative_launch(dispatch_kernel<kMaxWarps * 32>, launch, grid, threads, smem, stream);
+}
+
+LocalPlan plan_dispatch_local(const SegmentLayout& lay, int sms, std::size_t smem_limit) {
+    return make_local_plan(lay.num_experts, lay.num_channels, lay.num_topk, lay.hidden, lay.num_max_tokens, sms, smem_limit);
+}
+
+std::size_t dispatch_local_hist_ints(const SegmentLayout& lay, int ctas) { return local_hist_ints(ctas, lay.num_experts, lay.num_channels); }
+
+cudaError_t launch_dispatch_local(const DispatchArgs& a, const RankConst& rc, const LocalPlan& plan, int* hist, unsigned long long* counters, int sms, cudaStream_t stream) {
+    static std::mutex mutex;
+    static std::size_t configured[64] = {0};
+    {
+        std::lock_guard<std::mutex> guard(mutex);
+        int device = 0;
+        cudaError_t status = cudaGetDevice(&device);
+        if (status != cudaSuccess) return status;
+        if (device < 0 || device >= 64) return cudaErrorInvalidDevice;
+        if (plan.bytes > configured[device]) {
+            status = cudaFuncSetAttribute(local_dispatch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(plan.bytes));
+            if (status != cudaSuccess) return status;
+            configured[device] = plan.bytes;
+        }
+    }
+    LocalDispatchArgs args{a, plan, hist, counters, sms, rc.lay.num_experts, rc.lay.num_channels, rc.lay.num_topk, rc.lay.hidden,
+                           rc.lay.slots_full, rc.expanded_cap, rc.unique_cap, rc.recv_fp8};
+    const int ctas = std::max(1, std::min(sms, a.num_tokens));
+    // a fresh layout has a grid barrier and needs every CTA resident; with a cached one no CTA waits for another
+    if (!a.cached) return cooperative_launch(local_dispatch_kernel, args, dim3(ctas), kLocalThreads, plan.bytes, stream);
+    local_dispatch_kernel<<<ctas, kLocalThreads, plan.bytes, stream>>>(args);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_combine_local(const CombineLocalArgs& args, cudaStream_t stream) {

@@ -282,6 +282,17 @@ struct DispatchLaunch {
     DispatchArgs r[kMaxVirtualRanks];
 };
 
+// Dispatch of a group of one rank (dispatch_local.cuh): how a CTA's shared memory is cut up.
+constexpr int kLocalCounterInts = 32;  // its counters, in front of its scratch
+struct LocalPlan {
+    int token_cap = 0;   // tokens a CTA may own
+    int warps = 0;       // warps that move rows
+    int stages = 0;      // row buffers per such warp
+    int slot_bytes = 0;  // bytes of a row buffer
+    std::size_t rows_off = 0, bytes = 0;
+    bool usable = false;
+};
+
 // One combine of one (virtual) rank: the inverse of a finished dispatch.
 struct CombineArgs {
     const RankConst* rc;

@@ -199,6 +199,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         .def("fused_status", &Runtime::fused_status)
         .def("combine_is_split", &Runtime::combine_is_split)
         .def("combine_is_local", &Runtime::combine_is_local)
+        .def("dispatch_is_local", &Runtime::dispatch_is_local)
         .def("combine_is_inline", &Runtime::combine_is_inline)
         .def("send_stages", &Runtime::send_stages)
         .def("send_ctas", &Runtime::send_ctas)

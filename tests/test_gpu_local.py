@@ -1,0 +1,98 @@
+"""A group of one rank: the kernels without the exchange protocol against the general dispatch kernel, field by field, and
+the combine against a sum in 64 bits, where tiles, slices and chunks end."""
+
+import os
+import tempfile
+
+import pytest
+import torch
+import torch.distributed as dist
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def one_rank(ext):
+    if not dist.is_initialized():
+        store = dist.FileStore(os.path.join(tempfile.mkdtemp(prefix="local-store-"), "store"), 1)
+        dist.init_process_group("gloo", store=store, rank=0, world_size=1)
+    if dist.get_world_size() != 1:
+        pytest.skip("needs a process group of one")
+    return dist.group.WORLD
+
+
+# tokens, capacity, experts, top-k, hidden, channels, FP8 rows, expand, alignment
+CASES = [
+    (0, 16, 8, 2, 64, 4, False, True, 1),            # nothing to send
+    (1, 1, 1, 1, 8, 1, False, True, 256),            # one chunk per row, one expert
+    (149, 149, 32, 4, 136, 32, False, True, 16),     # one CTA with two tokens, a row that is no multiple of 128 bytes
+    (148 * 33, 148 * 33, 16, 2, 64, 128, False, True, 1),  # more than one 32-token chunk per CTA
+    (77, 300, 600, 32, 1024, 3, False, True, 7),     # more experts than threads, widest top-k
+    (300, 300, 40, 6, 2880, 64, True, True, 8),      # FP8 rows, several row buffers per warp
+    (130, 256, 64, 8, 7168, 32, False, False, 1),    # a row per token, fewer row buffers than warps
+    (200, 256, 64, 3, 1024, 128, True, False, 1),
+]
+FIELDS = ["unique_count", "expanded_count", "expert_counts", "expert_offsets", "expert_prefix", "source_offsets", "source_expert_prefix",
+          "recv_chan_counts"]
+
+
+@pytest.mark.parametrize("tokens,capacity,experts,topk,hidden,channels,fp8,expand,alignment", CASES)
+def test_local_dispatch_and_combine(one_rank, tokens, capacity, experts, topk, hidden, channels, fp8, expand, alignment):
+    from pcie_ep_b200 import HostStagedConfig, HostStagedEPBuffer
+
+    gen = torch.Generator().manual_seed(tokens + topk)
+    x = torch.randn(tokens, hidden, generator=gen).to(torch.bfloat16)
+    idx = torch.rand(tokens, experts, generator=gen).topk(topk, dim=1).indices.to(torch.int64)
+    idx[torch.rand(tokens, topk, generator=gen) < 0.2] = -1
+    if tokens > 2:
+        idx[tokens // 2] = -1  # a token that goes nowhere
+    w = torch.rand(tokens, topk, generator=gen)
+    wire = "fp8_e4m3" if fp8 else "bf16"
+    config = HostStagedConfig(stage=7 if fp8 else 6, channels=channels, wire_dtype=wire, recv_dtype=wire, output_pool_size=4)
+    options = dict(do_expand=expand, expert_alignment=alignment, do_zero_padding=expand)
+    with HostStagedEPBuffer(one_rank, capacity, hidden, topk, experts, config) as buffer:
+        args = (x.cuda(), idx.cuda(), w.cuda())
+        assert buffer.runtime.dispatch_is_local()
+        local = buffer.dispatch(*args, **options)
+        buffer.runtime.set_test_prefix_delay_ns(1)  # a hook of the protocol: the general kernel takes the call
+        assert not buffer.runtime.dispatch_is_local()
+        general = buffer.dispatch(*args, **options)
+        buffer.runtime.set_test_prefix_delay_ns(0)
+        cached = buffer.dispatch(args[0], None, args[2], handle=buffer.cache_layout(general[3]), **options)
+        for result in (general, cached, local):
+            buffer.check_errors(result[3])
+        rows = int(general[3].expert_offsets[-1]) if expand else int(general[3].unique_count[0])
+        entries = (idx >= 0).any(1)
+        per_channel = max(1, -(-tokens // channels))
+        for got in (local, cached):
+            for field in FIELDS:
+                assert torch.equal(got[3]._result[field], general[3]._result[field]), field
+            for mine, theirs in zip(got[:3], general[:3]):
+                assert torch.equal(mine[:rows].view(torch.uint8), theirs[:rows].view(torch.uint8))
+            assert torch.equal(got[3].source_meta[:rows], general[3].source_meta[:rows])
+            if fp8:
+                assert torch.equal(got[3]._result["recv_x_scales"][:rows], general[3]._result["recv_x_scales"][:rows])
+            assert int(got[3].stats[6]) == int(entries.sum())
+            # the combine map: token, rows, then (row, weight) pairs, for the entries that exist
+            slots = got[3]._result["comb_map"].shape[0] // channels
+            for channel in range(channels):
+                first = channel * per_channel
+                for j in range(int(entries[first:first + per_channel].sum())):
+                    a, b = (r[3]._result["comb_map"][channel * slots + j].cpu() for r in (got, general))
+                    assert torch.equal(a[:2 + 2 * int(a[1])], b[:2 + 2 * int(b[1])])
+        y = torch.randn(max(1, rows), hidden, generator=gen).to(torch.bfloat16)
+        for result, weighted, num_sms in ((local, expand, 0), (cached, False, 3)):
+            out = buffer.combine(y.cuda(), result[3], weighted=weighted, num_sms=num_sms)[0].cpu().double()
+            meta = result[3].source_meta[:rows].cpu()
+            used = meta[:, 1] >= 0
+            token, slot = meta[used, 1], meta[used, 2].clamp_min(0)
+            factor = w[token, slot].double() if weighted else torch.ones(int(used.sum()), dtype=torch.float64)
+            terms = y[:rows][used].double() * factor.unsqueeze(1)
+            want = torch.zeros(tokens, hidden, dtype=torch.float64).index_add_(0, token, terms)
+            size = torch.zeros(tokens, hidden, dtype=torch.float64).index_add_(0, token, terms.abs())
+            # one rounding to BF16 (half a unit in the last of 8 bits), and one FP32 rounding per added row
+            assert bool(((out - want).abs() <= want.abs() * 2.0 ** -8 + size * topk * 2.0 ** -23).all())
+            assert int(result[3]._result["combine_stats"][0]) == int(entries.sum())
+            del out
+        buffer.check_errors(local[3])
+        del local, general, cached, result, got
