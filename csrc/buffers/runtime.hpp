@@ -38,6 +38,20 @@ inline bool tensor_unowned(const at::Tensor& t) {
     return t.use_count() == 1 && t.unsafeGetTensorImpl()->unsafe_storage().use_count() == 1;
 }
 
+// A tensor of its own over the memory of a contiguous pool tensor (from its first element on), as narrow / view / alias make
+// one, without the dispatcher: 1.2 us -> 0.3 us for each of the tensors that every dispatch hands out.
+inline at::Tensor pool_alias(const at::Tensor& base, at::IntArrayRef sizes) {
+    // (in inference mode a new tensor would be an inference tensor, a view of a pool tensor is not)
+    if (c10::InferenceMode::is_enabled()) return base.view({-1}).narrow(0, 0, c10::multiply_integers(sizes)).view(sizes);
+    at::TensorImpl* from = base.unsafeGetTensorImpl();
+    at::Tensor t = at::detail::make_tensor<at::TensorImpl>(c10::Storage(base.storage()), from->key_set(), base.dtype());
+    at::TensorImpl* to = t.unsafeGetTensorImpl();
+    to->set_storage_offset(base.storage_offset());
+    to->set_sizes_contiguous(sizes);
+    to->set_version_counter(from->version_counter());
+    return t;
+}
+
 struct TensorRefs {
     std::int64_t tensor_use_count, storage_use_count;
 };
@@ -155,7 +169,7 @@ class DispatchResult {
     }
 
     bool contains(const std::string& key) const {
-        if (overrides_.contains(key.c_str())) return true;
+        if (!overrides_.empty() && overrides_.contains(key.c_str())) return true;
         if (key == "_layout" || key == "_expand" || key == "_num_tokens") return true;
         for (const auto& k : tensor_keys())
             if (k == key) return true;
@@ -163,7 +177,7 @@ class DispatchResult {
     }
 
     py::object get(const std::string& key) {
-        if (overrides_.contains(key.c_str())) return overrides_[key.c_str()];
+        if (!overrides_.empty() && overrides_.contains(key.c_str())) return overrides_[key.c_str()];
         if (key == "_layout") return py::cast(layout_);
         if (key == "_expand") return py::cast(expand_);
         if (key == "_num_tokens") return py::cast(num_tokens_);
@@ -183,7 +197,13 @@ class DispatchResult {
         return out;
     }
 
+    // recv_x, recv_topk_idx and (with weights) recv_topk_weights in one go: what every dispatch returns
+    py::tuple received(bool with_weights) {
+        return py::make_tuple(get("recv_x"), get("recv_topk_idx"), with_weights ? get("recv_topk_weights") : py::object(py::none()));
+    }
+
     const OutputSet& set_ref() const { return *set_; }
+    int capacity() const { return expand_ ? expanded_cap_ : unique_cap_; }
     const std::shared_ptr<Layout>& layout() const { return layout_; }
     bool expand() const { return expand_; }
     int num_tokens() const { return num_tokens_; }
@@ -194,7 +214,7 @@ class DispatchResult {
         const std::int64_t K = topk_;
         if (key == "recv_x") {
             const std::int64_t cap = expand_ ? expanded_cap_ : unique_cap_;
-            if (!recv_fp8_) return s.recv_x.narrow(0, 0, cap);
+            if (!recv_fp8_) return pool_alias(s.recv_x, {cap, s.recv_x.size(1)});
             // E4M3 rows occupy the first half of the BF16-sized pool tensor, one byte per element
             const std::int64_t hidden = s.recv_x.size(1);
             return s.recv_x.view(at::kByte).reshape({-1}).narrow(0, 0, cap * hidden).view({cap, hidden}).view(at::kFloat8_e4m3fn);
@@ -202,15 +222,15 @@ class DispatchResult {
         if (key == "recv_x_scales") return recv_fp8_ ? s.recv_scale.narrow(0, 0, expand_ ? expanded_cap_ : unique_cap_) : at::alias(s.recv_scale);
         if (key == "source_meta") return s.source_meta.narrow(0, 0, expand_ ? expanded_cap_ : unique_cap_);
         if (key == "recv_topk_idx")
-            return expand_ ? s.recv_idx.narrow(0, 0, expanded_cap_) : s.recv_idx.narrow(0, 0, unique_cap_ * K).view({unique_cap_, K});
+            return expand_ ? pool_alias(s.recv_idx, {expanded_cap_}) : pool_alias(s.recv_idx, {unique_cap_, K});
         if (key == "recv_topk_weights")
-            return expand_ ? s.recv_w.narrow(0, 0, expanded_cap_) : s.recv_w.narrow(0, 0, unique_cap_ * K).view({unique_cap_, K});
+            return expand_ ? pool_alias(s.recv_w, {expanded_cap_}) : pool_alias(s.recv_w, {unique_cap_, K});
         if (key == "comb_map") return at::alias(s.comb_map);
         if (key == "recv_chan_counts") return at::alias(s.recv_chan_counts);
         if (key == "unique_count") return at::alias(s.unique_count);
         if (key == "expanded_count") return at::alias(s.expanded_count);
-        if (key == "expert_counts") return at::alias(s.expert_counts);
-        if (key == "expert_offsets") return at::alias(s.expert_offsets);
+        if (key == "expert_counts") return pool_alias(s.expert_counts, s.expert_counts.sizes());
+        if (key == "expert_offsets") return pool_alias(s.expert_offsets, s.expert_offsets.sizes());
         if (key == "expert_prefix") return at::alias(s.expert_prefix);
         if (key == "source_offsets") return at::alias(s.source_offsets);
         if (key == "source_expert_prefix") return at::alias(s.source_expert_prefix);
@@ -385,6 +405,24 @@ class Runtime {
     const SegmentLayout& layout() const { return lay_; }
     int unique_capacity() const { return rc_.unique_cap; }
     int expanded_capacity() const { return rc_.expanded_cap; }
+
+    // ---- argument checks of the Python layer, answered in one call ---------------------------------
+    // True when the tensors of a dispatch are what the layer's rules ask for; the rules themselves (which know what to say
+    // about a wrong argument) only run when this says no.
+    bool accepts_inputs(const py::handle& x, const py::handle& idx, const py::handle& w) const {
+        if (!THPVariable_Check(x.ptr()) || !THPVariable_Check(idx.ptr()) || !(w.is_none() || THPVariable_Check(w.ptr()))) return false;
+        const at::Tensor& tx = THPVariable_Unpack(x.ptr());
+        const at::Tensor& ti = THPVariable_Unpack(idx.ptr());
+        if (!matches(tx, at::kBFloat16, -1, lay_.hidden) || tx.size(0) > lay_.num_max_tokens) return false;
+        if (!matches(ti, at::kLong, tx.size(0), lay_.num_topk)) return false;
+        return w.is_none() || matches(THPVariable_Unpack(w.ptr()), at::kFloat, tx.size(0), lay_.num_topk);
+    }
+    // the same for the expert rows of a combine
+    bool accepts_rows(const py::handle& y, const DispatchResult& result) const {
+        if (!THPVariable_Check(y.ptr())) return false;
+        const at::Tensor& ty = THPVariable_Unpack(y.ptr());
+        return matches(ty, at::kBFloat16, -1, lay_.hidden) && ty.size(0) <= result.capacity();
+    }
 
     // ---- dispatch -------------------------------------------------------------------------------
     PreparedDispatch prepare_dispatch(const at::Tensor& x, const at::Tensor& topk_idx,
@@ -782,6 +820,11 @@ class Runtime {
         cuda_check(cudaStreamSynchronize(at::cuda::getCurrentCUDAStream(device_)), "upload rank constants");
     }
 
+    bool matches(const at::Tensor& t, at::ScalarType dtype, std::int64_t rows, std::int64_t columns) const {
+        return t.defined() && t.layout() == at::kStrided && t.is_cuda() && t.get_device() == device_ && t.scalar_type() == dtype && t.dim() == 2 &&
+               t.is_contiguous() && (rows < 0 || t.size(0) == rows) && t.size(1) == columns;
+    }
+
     void validate_inputs(const at::Tensor& x, const at::Tensor& idx, const std::optional<at::Tensor>& w, int alignment,
                          bool expand, bool zero_padding) const {
         auto on_device = [this](const at::Tensor& t) { return t.is_cuda() && t.get_device() == device_; };
@@ -884,7 +927,7 @@ class Runtime {
             const int index = (next_combine_ + i) % n;
             if (tensor_unowned(combine_pool_[index])) {
                 next_combine_ = (index + 1) % n;
-                return combine_pool_[index].narrow(0, 0, num_tokens);
+                return pool_alias(combine_pool_[index], {num_tokens, lay_.hidden});
             }
         }
         throw std::runtime_error("combine output pool exhausted: every preallocated output is still referenced");

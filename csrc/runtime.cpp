@@ -182,6 +182,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         .def("__setitem__", &DispatchResult::set)
         .def("__contains__", &DispatchResult::contains)
         .def("keys", &DispatchResult::keys)
+        .def("received", &DispatchResult::received, py::arg("with_weights"))
         .def("get", [](DispatchResult& r, const std::string& key, py::object fallback) {
             return r.contains(key) ? r.get(key) : fallback;
         }, py::arg("key"), py::arg("default") = py::none());
@@ -197,6 +198,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
              py::arg("dispatch_result"), py::arg("stream") = 0)
         .def("fused_reduce", &Runtime::fused_reduce, py::arg("dispatch_result"), py::arg("out"), py::arg("stream") = 0)
         .def("fused_status", &Runtime::fused_status)
+        .def("accepts_inputs", &Runtime::accepts_inputs, py::arg("x"), py::arg("topk_idx"), py::arg("topk_weights"))
+        .def("accepts_rows", &Runtime::accepts_rows, py::arg("y"), py::arg("dispatch_result"))
         .def("combine_is_split", &Runtime::combine_is_split)
         .def("combine_is_local", &Runtime::combine_is_local)
         .def("dispatch_is_local", &Runtime::dispatch_is_local)

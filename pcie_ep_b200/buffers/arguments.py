@@ -108,13 +108,15 @@ def build_dispatch_request(owner: Any, x: Any, topk_idx: Any, topk_weights: Any,
         if given is not None and given != prepared:
             raise ValueError(f"{name}={given} contradicts the buffer, which was built for {prepared}")
     device, on_gpu = owner.device, owner.on_gpu
-    TensorRule("x", torch.bfloat16 if on_gpu else None, (None, owner.hidden)).check(x, device=device, on_gpu=on_gpu)
-    tokens = x.shape[0]
-    if tokens > owner.num_max_tokens_per_rank:
-        raise ValueError(f"x has {tokens} tokens, the buffer holds at most {owner.num_max_tokens_per_rank} per rank")
-    TensorRule("topk_idx", torch.int64, (tokens, owner.num_topk)).check(topk_idx, device=device, on_gpu=on_gpu)
-    if topk_weights is not None:
-        TensorRule("topk_weights", torch.float32, (tokens, owner.num_topk)).check(topk_weights, device=device, on_gpu=on_gpu)
+    # the runtime answers "all as the rules below want it" in one call; the rules say what is wrong if it is not
+    if not (on_gpu and owner.runtime.accepts_inputs(x, topk_idx, topk_weights)):
+        TensorRule("x", torch.bfloat16 if on_gpu else None, (None, owner.hidden)).check(x, device=device, on_gpu=on_gpu)
+        tokens = x.shape[0]
+        if tokens > owner.num_max_tokens_per_rank:
+            raise ValueError(f"x has {tokens} tokens, the buffer holds at most {owner.num_max_tokens_per_rank} per rank")
+        TensorRule("topk_idx", torch.int64, (tokens, owner.num_topk)).check(topk_idx, device=device, on_gpu=on_gpu)
+        if topk_weights is not None:
+            TensorRule("topk_weights", torch.float32, (tokens, owner.num_topk)).check(topk_weights, device=device, on_gpu=on_gpu)
     if cumulative is not None:
         TensorRule("cumulative_local_expert_recv_stats", torch.int32, (owner.num_experts // owner.num_ranks,)).check(
             cumulative, device=device, on_gpu=on_gpu)

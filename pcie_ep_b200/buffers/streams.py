@@ -46,11 +46,22 @@ class StreamPolicy:
         self.device = device
         self.comm = torch.cuda.Stream(device=device) if on_gpu else NullStream()
         self.consumers: Dict[Tuple[int, int], Any] = {}
+        # stream objects by raw handle: torch builds a new one per query (1.3 us), and with one object per stream "the only
+        # reader is the stream itself" is a comparison of identities
+        self._known: Dict[int, Any] = {}
         # work was queued on the communication stream that the compute stream has not waited for yet
         self._comm_ahead = False
 
     def current(self) -> Any:
-        return torch.cuda.current_stream(self.device) if self.on_gpu else NullStream()
+        if not self.on_gpu:
+            return NullStream()
+        raw = torch._C._cuda_getCurrentRawStream(self.device)
+        stream = self._known.get(raw)
+        if stream is None:
+            if len(self._known) >= 64:
+                self._known.clear()
+            stream = self._known[raw] = torch.cuda.current_stream(self.device)
+        return stream
 
     # -- readers of result pools ---------------------------------------------------------------
     def add_consumer(self, stream: Any) -> None:
@@ -63,6 +74,8 @@ class StreamPolicy:
 
     def _after_consumers(self, target: Any, *already_ordered: Any) -> None:
         """Make ``target`` wait for every registered reader except the streams given."""
+        if len(self.consumers) == 1 and target in self.consumers.values():
+            return
         done = {stream_key(s) for s in already_ordered}
         done.add(stream_key(target))
         for key, reader in self.consumers.items():
@@ -106,7 +119,8 @@ class StreamPolicy:
         if launched_on is not compute and event is not None:
             compute.wait_event(event)
             self._comm_ahead = False
-        self.add_consumer(compute)
+        if not (len(self.consumers) == 1 and compute in self.consumers.values()):
+            self.add_consumer(compute)
 
     def drain(self, last_event: Optional[Any]) -> None:
         """Blocking: used by ``close`` only."""

@@ -96,3 +96,29 @@ def test_local_dispatch_and_combine(one_rank, tokens, capacity, experts, topk, h
             del out
         buffer.check_errors(local[3])
         del local, general, cached, result, got
+
+
+@pytest.mark.parametrize("inference", [False, True])
+def test_results_are_ordinary_tensors_over_the_pool(one_rank, inference):
+    """What a dispatch and a combine hand out shares the pool's memory and version counter, also in inference mode."""
+    from pcie_ep_b200 import HostStagedConfig, HostStagedEPBuffer
+
+    with HostStagedEPBuffer(one_rank, 32, 64, 2, 8, HostStagedConfig(channels=4)) as buffer:
+        x = torch.randn(20, 64).to(torch.bfloat16).cuda()
+        idx = torch.rand(20, 8).topk(2, dim=1).indices.cuda()
+        with torch.inference_mode(inference):
+            recv_x, recv_idx, recv_w, handle, _ = buffer.dispatch(x, idx, torch.ones(20, 2, device="cuda"), do_expand=True)
+            out = buffer.combine(recv_x, handle)[0]
+        buffer.check_errors(handle)
+        assert torch.equal(out, 2 * x) and torch.equal(recv_x[:40], x[handle.source_meta[:40, 1]])
+        for t in (recv_x, recv_idx, recv_w, out, handle.expert_counts):
+            assert t.is_contiguous() and not t.is_inference() and not t.requires_grad
+        version = recv_x._version
+        recv_x[:1].zero_()
+        assert recv_x._version == version + 1
+        with pytest.raises(ValueError, match="expected dtype"):
+            buffer.dispatch(x.float(), idx)
+        with pytest.raises(TypeError, match="expected a torch.Tensor"):
+            buffer.dispatch(x, [1])
+        with pytest.raises(ValueError, match="contiguous"):
+            buffer.combine(recv_x[:, :32], handle)
