@@ -14,7 +14,7 @@
 // What bounds it.  Large batches: writing the expanded rows to HBM.  4096 tokens, hidden 7168, top-8 move 528 MB.
 // Small ones: the chain launch -> ids -> barrier -> prefix -> rows.  Launch to end with a cold L2, general kernel -> this
 // one: 128 tokens 46 -> 19 us (no flags to wait for, no prefix by a single warp), 4096 tokens 131 ->
-// 110 us, the same with E4M3 rows 106 -> 73 us (fourteen row buffers per SM on all SMs instead of eight on 128), 256 tokens
+// 104 us, the same with E4M3 rows 106 -> 71 us (fourteen row buffers per SM on all SMs instead of eight on 128), 256 tokens
 // with a cached layout 45 -> 17 us.
 #pragma once
 
@@ -32,7 +32,7 @@ struct LocalDispatchArgs {
     DispatchArgs a;
     LocalPlan plan;
     int* hist;                     // [G][E + 1] counts per CTA, then two copies of [groups][E + 1 + C] sums, then their generation
-    unsigned long long* counters;  // barrier arrivals, finished CTAs, complement of the first start (zero between launches)
+    unsigned long long* counters;  // barrier arrivals, finished CTAs, complement of the first start, CTAs whose plan is written, tokens claimed (zero between launches)
     int hist_ctas;                 // CTAs the scratch has room for
     int num_experts, num_channels, num_topk, hidden, slots_full, expanded_cap, unique_cap, recv_fp8;  // as in the rank's constants
 };
@@ -47,6 +47,7 @@ struct LocalShared {
     unsigned long long warp_sum[kLocalWarps];
     int flag;        // the CTA leaves without rows
     int routed;      // routed tokens of this CTA
+    int token[kLocalWarps * kLocalMaxStages];  // of the row in each buffer
     int first_unique;  // routed tokens of earlier CTAs
     int unique_total;
 };
@@ -156,18 +157,23 @@ __global__ void __launch_bounds__(kLocalThreads, 1) local_dispatch_kernel(const 
     __syncthreads();
 
     // ---- 1. the first rows of every warp start their way into shared memory ----------------------------------
-    auto start_load = [&](int n) {  // the warp's n-th token (lane 0 only)
-        const int i = warp + n * row_warps;
+    auto start_load = [&](int n, int t) {  // token t as the warp's n-th (lane 0 only)
         auto* bar = reinterpret_cast<std::uint64_t*>(&sh->mbar[warp * stages + n % stages]);
         ptx::mbar_expect_tx(bar, in_bytes);
-        ptx::bulk_g2s(rows_sm + static_cast<std::size_t>(warp * stages + n % stages) * slot_bytes, a.x + static_cast<std::size_t>(t0 + i) * H, in_bytes, bar);
+        ptx::bulk_g2s(rows_sm + static_cast<std::size_t>(warp * stages + n % stages) * slot_bytes, a.x + static_cast<std::size_t>(t) * H, in_bytes, bar);
+        sh->token[warp * stages + n % stages] = t;
     };
     int started = 0;  // loads of this warp that are under way or done
     auto start_first_loads = [&]() {
         if (warp >= row_warps) return;
         for (; started < stages && warp + started * row_warps < nt; ++started)
-            if (lane == 0) start_load(started);
+            if (lane == 0) start_load(started, t0 + warp + started * row_warps);
     };
+    // Large batches: what does not fit a CTA's row buffers at once is handed out through a counter, a token at a time over
+    // all CTAs (SMs do not all get the same share of HBM: with equal shares the slowest finished 17 us behind the others
+    // at 4096 tokens: 110 -> 104 us, 8192 tokens top-4 122 -> 117, 4096 with E4M3 rows 73 -> 71).
+    const int own_tokens = row_warps * stages, most_tokens = (T + G - 1) / G;
+    const bool pooled = most_tokens > own_tokens;  // then every CTA has at least own_tokens tokens
 
     // a rank that has failed, or has run out of epochs, leaves without rows
     auto leaves = [&]() {  // thread 0
@@ -394,30 +400,60 @@ __global__ void __launch_bounds__(kLocalThreads, 1) local_dispatch_kernel(const 
         }
     }
 
+    if (pooled && !cached && !failed) {
+        // the plan of the tokens that any CTA may move, before the first of them is claimed
+        for (int q = own_tokens * K + tid; q < nt * K; q += kLocalThreads)
+            a.plan_expert_ord[static_cast<std::size_t>(t0) * K + q] = pair_e[q] >= 0 ? pair_ord[q] + base[pair_e[q]] : -1;
+        for (int i = own_tokens + tid; i < nt; i += kLocalThreads) {
+            const bool routed = unique[i] >= 0;
+            a.plan_mask[t0 + i] = routed ? 1u : 0u;
+            a.plan_slot[t0 + i] = routed ? unique[i] + sh->first_unique - chan_base[(t0 + i) / Tc] : -1;
+        }
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) {
+            __threadfence();
+            atomicAdd(&args.counters[3], 1ull);
+        }
+    }
+
     // ---- 4. rows -------------------------------------------------------------------------------------------------------
     const std::size_t out_row_bytes = static_cast<std::size_t>(H) * (recv_fp8 ? 1 : 2);
     auto* const recv_bytes = reinterpret_cast<std::uint8_t*>(a.recv_x);
     const int map_stride = 2 + 2 * K;
     if (warp < row_warps && !failed) {
-        for (int n = 0, i = warp; i < nt; ++n, i += row_warps) {
-            const int t = t0 + i;
-            int e = -1, ord = -1;
+        bool plans_seen = !pooled || cached, more = pooled;
+        for (int n = 0; n < started; ++n) {
+            const int buffer = warp * stages + n % stages;
+            const int t = sh->token[buffer], c = t / Tc, i = t - t0;
+            const bool own = n < stages;  // from this CTA's tables, else from the plan in global memory
+            int e = -1, ord = -1, j = -1;
             float wgt = 1.0f;
             if (lane < static_cast<unsigned>(K)) {
-                if (a.topk_w) wgt = __ldg(a.topk_w + static_cast<std::size_t>(t) * K + lane);
-                e = pair_e[i * K + lane];
-                if (e >= 0) ord = pair_ord[i * K + lane] + base[e];
+                const std::size_t at = static_cast<std::size_t>(t) * K + lane;
+                if (a.topk_w) wgt = __ldg(a.topk_w + at);
+                if (own) {
+                    e = pair_e[i * K + lane];
+                    if (e >= 0) ord = pair_ord[i * K + lane] + base[e];
+                } else {
+                    const std::int64_t e64 = __ldg(a.topk_idx + at);
+                    ord = __ldcg(a.plan_expert_ord + at);
+                    e = e64 >= 0 && e64 < E ? static_cast<int>(e64) : -1;
+                }
             }
+            if (own) {
+                if (unique[i] >= 0) j = cached ? unique[i] : unique[i] + sh->first_unique - chan_base[c];
+            } else {
+                const int slot = __ldcg(a.plan_slot + t);
+                if (__ldcg(a.plan_mask + t) & 1u) j = slot;
+            }
+            const bool routed = j >= 0;  // j: ordinal in the channel
             const unsigned valid = __ballot_sync(full, e >= 0);
-            const int u = unique[i], c = t / Tc;
-            const bool routed = u >= 0;
-            const int j = cached ? u : u + sh->first_unique - chan_base[c];  // ordinal in the channel
             int row = -1;  // this lane's output row
             if (routed) {
                 if (expand) row = e >= 0 ? eoff[e] + ord : -1;
                 else if (lane == 0) row = chan_base[c] + j;
             }
-            const int buffer = warp * stages + n % stages;
             unsigned char* slot = rows_sm + static_cast<std::size_t>(buffer) * slot_bytes;
             if (!__all_sync(full, mbar_wait_bounded(&sh->mbar[buffer], static_cast<unsigned>(n / stages) & 1u, health))) {
                 failed = true;
@@ -432,6 +468,10 @@ __global__ void __launch_bounds__(kLocalThreads, 1) local_dispatch_kernel(const 
             // every lane with a row starts its own copy: the bulk groups are the lanes' own
             if (row >= 0) ptx::bulk_s2g(recv_bytes + static_cast<std::size_t>(row) * out_row_bytes, slot, static_cast<unsigned>(out_row_bytes));
             ptx::bulk_commit();
+            // the next token: claimed now, its number arrives while this row's copies drain
+            const bool refill = more && n + 1 >= stages;
+            unsigned long long claim = 0;
+            if (refill && lane == 0) claim = atomicAdd(&args.counters[4], 1ull);
             if (routed) {
                 int* map = a.comb_map + (static_cast<std::size_t>(c) * Qf + j) * map_stride;
                 if (lane == 0) *reinterpret_cast<int2*>(map) = make_int2(t, expand ? __popc(valid) : 1);
@@ -462,20 +502,46 @@ __global__ void __launch_bounds__(kLocalThreads, 1) local_dispatch_kernel(const 
                     }
                 }
             }
-            if (!cached) {
+            if (!cached && own) {
                 if (lane < static_cast<unsigned>(K)) a.plan_expert_ord[static_cast<std::size_t>(t) * K + lane] = ord;
                 if (lane == 0) {
                     a.plan_mask[t] = routed ? 1u : 0u;
                     a.plan_slot[t] = routed ? j : -1;
                 }
             }
-            // the next token's load goes into the oldest buffer, once its copies have left it
-            if (warp + started * row_warps < nt) {
-                local_wait_read(stages - 1);
-                __syncwarp();
-                if (n + 1 >= stages) {
-                    if (lane == 0) start_load(started);
+            // its load goes into the oldest buffer, once the copies have left that
+            if (refill) {
+                if (!plans_seen) {  // every CTA has written its part of the plan (they all do before their first row)
+                    bool seen = true;
+                    if (lane == 0)
+                        while (ptx::ld_acquire_gpu(reinterpret_cast<const std::uint64_t*>(&args.counters[3])) < static_cast<std::uint64_t>(G))
+                            if (health.give_up(kErrGridBarrier, b, 1)) {
+                                seen = false;
+                                break;
+                            }
+                    plans_seen = __all_sync(full, seen) != 0;
+                    if (!plans_seen) {
+                        failed = true;
+                        break;
+                    }
+                }
+                int next_t = -1;
+                while (true) {
+                    claim = __shfl_sync(full, claim, 0);
+                    const int f = static_cast<int>(claim % G), next_i = own_tokens + static_cast<int>(claim / G);
+                    more = next_i < most_tokens;
+                    const int f_t0 = static_cast<int>(static_cast<long long>(T) * f / G), f_t1 = static_cast<int>(static_cast<long long>(T) * (f + 1) / G);
+                    if (more && f_t0 + next_i < f_t1) next_t = f_t0 + next_i;
+                    if (!more || next_t >= 0) break;
+                    // a CTA with one token less than the others leaves a gap in the numbering: claim again
+                    if (lane == 0) claim = atomicAdd(&args.counters[4], 1ull);
+                }
+                if (next_t >= 0) {
+                    local_wait_read(stages - 1);
+                    __syncwarp();
+                    if (lane == 0) start_load(started, next_t);
                     ++started;
+                    __syncwarp();
                 }
             }
         }
@@ -537,7 +603,7 @@ __global__ void __launch_bounds__(kLocalThreads, 1) local_dispatch_kernel(const 
             for (int i = 0; i < 8; ++i) a.stats[i] = i == kStatLocalRows ? sh->unique_total : 0;
             a.timestamps[0] = static_cast<std::int64_t>(~__ldcg(&args.counters[2]));
             a.timestamps[1] = static_cast<std::int64_t>(ptx::globaltimer_ns());
-            args.counters[0] = args.counters[1] = args.counters[2] = 0ull;
+            for (int i = 0; i < 5; ++i) args.counters[i] = 0ull;
             if (ptx::ld_volatile(&rc->sticky[0]) == 0) {
                 const std::uint64_t epoch = epoch_before + 1;
                 ptx::st_release_sys(flag_ptr(rc->seg[rc->rank], rc->lay.done_off, rc->rank), epoch);

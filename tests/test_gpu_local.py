@@ -31,6 +31,9 @@ CASES = [
     (300, 300, 40, 6, 2880, 64, True, True, 8),      # FP8 rows, several row buffers per warp
     (130, 256, 64, 8, 7168, 32, False, False, 1),    # a row per token, fewer row buffers than warps
     (200, 256, 64, 3, 1024, 128, True, False, 1),
+    (148 * 49 + 5, 148 * 49 + 5, 16, 2, 64, 128, False, True, 1),  # more tokens than row buffers: the rest is claimed, with gaps
+    (2400, 2500, 12, 3, 7168, 64, False, True, 8),   # the same with one row buffer per warp
+    (2400, 2400, 8, 2, 7168, 100, True, False, 1),   # and with FP8 rows, a row per token
 ]
 FIELDS = ["unique_count", "expanded_count", "expert_counts", "expert_offsets", "expert_prefix", "source_offsets", "source_expert_prefix",
           "recv_chan_counts"]
@@ -75,10 +78,11 @@ def test_local_dispatch_and_combine(one_rank, tokens, capacity, experts, topk, h
             assert int(got[3].stats[6]) == int(entries.sum())
             # the combine map: token, rows, then (row, weight) pairs, for the entries that exist
             slots = got[3]._result["comb_map"].shape[0] // channels
+            maps = [r[3]._result["comb_map"].cpu() for r in (got, general)]
             for channel in range(channels):
                 first = channel * per_channel
                 for j in range(int(entries[first:first + per_channel].sum())):
-                    a, b = (r[3]._result["comb_map"][channel * slots + j].cpu() for r in (got, general))
+                    a, b = (m[channel * slots + j] for m in maps)
                     assert torch.equal(a[:2 + 2 * int(a[1])], b[:2 + 2 * int(b[1])])
         y = torch.randn(max(1, rows), hidden, generator=gen).to(torch.bfloat16)
         for result, weighted, num_sms in ((local, expand, 0), (cached, False, 3)):
