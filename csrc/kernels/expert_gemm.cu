@@ -2,6 +2,7 @@
 #include "expert_gemm.cuh"
 
 #include <mutex>
+#include <type_traits>
 
 #include "expert_gemm.hpp"
 #include "ptx.cuh"
@@ -163,7 +164,7 @@ struct TileCursor {
 // the gate and the up rows of the same 128 output columns, for the plain GEMM 256 adjacent output columns.
 template <bool kSwiGLU, bool kFp8, int kBoxesB, bool kScatter>
 __global__ void __launch_bounds__(kThreads, 1)
-grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_a, const __grid_constant__ CUtensorMap map_b,
                     const GroupedGemmParams p) {
     static_assert(kBoxesB == 2 || !kSwiGLU, "SwiGLU stages carry the gate and the up box");
     static_assert(!kScatter || (kBoxesB == 2 && !kSwiGLU && !kFp8), "the scatter epilogue exists for the plain BF16 256-column tile");
@@ -201,6 +202,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const int n_tiles = p.n / kOutN;
     const int k_blocks = p.k / kBlockK;
     const int w_rows_per_expert = kSwiGLU ? 2 * p.n : p.n;
+    // gate/up tiles with few rows swap the operands (see ActivationMaps)
+    auto flips = [](int box) { return kSwiGLU && box != kBoxesA - 1; };
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
@@ -236,14 +239,18 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 const int row0 = p.expert_offsets[cursor.expert] + m_tile * kBlockM;
                 const int wrow0 = cursor.expert * w_rows_per_expert + n_tile * kOutN;
                 const int wrow1 = wrow0 + (kSwiGLU ? p.n : kBlockN);
+                // a tile with few valid rows loads only those (rows of the box beyond them are never written out)
+                const int box = box_of_rows(p.expert_counts[cursor.expert] - m_tile * kBlockM);
+                const CUtensorMap* map_a = &maps_a.box[box];
+                const unsigned stage_bytes = static_cast<unsigned>(Plan::kStageBytes - Plan::kTileA + box_rows_a(box) * kBlockKBytes);
                 for (int kb = 0; kb < k_blocks; ++kb) {
                     if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort)) {
                         ok = false;
                         break;
                     }
                     unsigned char* stage_base = tiles + stage * Plan::kStageBytes;
-                    mbar_expect_tx(&full_bar[stage], Plan::kStageBytes);
-                    tma_load_2d(stage_base, &map_a, kb * kBlockK, row0, &full_bar[stage]);
+                    mbar_expect_tx(&full_bar[stage], stage_bytes);
+                    tma_load_2d(stage_base, map_a, kb * kBlockK, row0, &full_bar[stage]);
                     tma_load_2d(stage_base + Plan::kTileA, &map_b, kb * kBlockK, wrow0, &full_bar[stage]);
                     if (kBoxesB == 2)
                         tma_load_2d(stage_base + Plan::kTileA + Plan::kTileB, &map_b, kb * kBlockK, wrow1, &full_bar[stage]);
@@ -257,24 +264,22 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     } else if (warp == 1) {
         // ===== MMA issuer =====
         if (lane == 0) {
-            constexpr std::uint32_t idesc = kFp8 ? make_idesc_e4m3(kBlockM, kAccCols) : make_idesc_bf16(kBlockM, kAccCols);
             TileCursor cursor;
             int stage = 0;
             unsigned phase = 0;
             bool ok = true;
             int it = 0;
-            for (int tile = blockIdx.x; ok; tile += gridDim.x, ++it) {
-                int m_tile, n_tile;
-                if (!cursor.locate(tile, p, n_tiles, m_tile, n_tile)) break;
-                const int buf = it & 1;
-                const unsigned acc_phase = (it >> 1) & 1u;
-                if (!mbar_wait(&tmem_empty[buf], acc_phase ^ 1u, abort)) break;
-                tc_fence_after();
-                const std::uint32_t acc = tmem_base + buf * kAccCols;
+            // The K loop exists once per box height: with the operand order and the instruction descriptor chosen at run time
+            // inside it, every tile was 28 % slower.  kBox = kBoxesA - 1: not swapped.
+            auto multiply = [&](auto box, std::uint32_t acc) {
+                constexpr int kBox = decltype(box)::value;
+                constexpr bool kFlip = kBox != kBoxesA - 1;
+                constexpr int kM = kFlip ? kBlockN : kBlockM, kN = kFlip ? box_rows_a(kBox) : kAccCols;
+                constexpr std::uint32_t idesc = kFp8 ? make_idesc_e4m3(kM, kN) : make_idesc_bf16(kM, kN);
                 for (int kb = 0; kb < k_blocks; ++kb) {
                     if (!mbar_wait(&full_bar[stage], phase, abort)) {
                         ok = false;
-                        break;
+                        return;
                     }
                     tc_fence_after();
                     unsigned char* stage_base = tiles + stage * Plan::kStageBytes;
@@ -286,8 +291,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                         // 32 bytes further along K inside the swizzle atom: +2 in the address field
                         const std::uint64_t step = static_cast<std::uint64_t>(k * kUmmaKBytes) >> 4;
                         const std::uint32_t accumulate = (kb | k) != 0 ? 1u : 0u;
-                        if (kFp8) umma_f8(acc, desc_a + step, desc_b + step, idesc, accumulate);
-                        else umma_f16(acc, desc_a + step, desc_b + step, idesc, accumulate);
+#pragma unroll
+                        for (int bx = 0; bx < (kFlip ? kBoxesB : 1); ++bx) {
+                            const std::uint64_t first = kFlip ? desc_b + step + (static_cast<std::uint64_t>(bx * Plan::kTileB) >> 4) : desc_a + step;
+                            const std::uint64_t second = kFlip ? desc_a + step : desc_b + step;
+                            if (kFp8) umma_f8(acc + bx * kBlockN, first, second, idesc, accumulate);
+                            else umma_f16(acc + bx * kBlockN, first, second, idesc, accumulate);
+                        }
                     }
                     umma_commit(&empty_bar[stage]);  // the stage is free once these MMAs have read it
                     if (++stage == kStages) {
@@ -295,6 +305,20 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                         phase ^= 1u;
                     }
                 }
+            };
+            for (int tile = blockIdx.x; ok; tile += gridDim.x, ++it) {
+                int m_tile, n_tile;
+                if (!cursor.locate(tile, p, n_tiles, m_tile, n_tile)) break;
+                const int buf = it & 1;
+                const unsigned acc_phase = (it >> 1) & 1u;
+                if (!mbar_wait(&tmem_empty[buf], acc_phase ^ 1u, abort)) break;
+                tc_fence_after();
+                const std::uint32_t acc = tmem_base + buf * kAccCols;
+                const int box = box_of_rows(p.expert_counts[cursor.expert] - m_tile * kBlockM);
+                if constexpr (!kSwiGLU) multiply(std::integral_constant<int, kBoxesA - 1>{}, acc);
+                else if (!flips(box)) multiply(std::integral_constant<int, kBoxesA - 1>{}, acc);
+                else if (box == 0) multiply(std::integral_constant<int, 0>{}, acc);
+                else multiply(std::integral_constant<int, 1>{}, acc);
                 if (ok) umma_commit(&tmem_full[buf]);
             }
         }
@@ -338,6 +362,36 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             const float a_scale = (kFp8 && valid) ? p.a_scales[out_row] : 1.0f;
             const float* w_scale = kFp8 ? p.w_scales + static_cast<long long>(cursor.expert) * w_rows_per_expert + n_tile * kOutN : nullptr;
             const std::uint32_t lane_base = tmem_base + (static_cast<std::uint32_t>(q * 32) << 16) + buf * kAccCols;
+            const int tile_rows = p.expert_counts[cursor.expert] - m_tile * kBlockM;
+            if (flips(box_of_rows(tile_rows))) {
+                // swapped tile: TMEM lane = output channel, column = row; a warp stores 32 channels of a row
+                const long long row0 = static_cast<long long>(p.expert_offsets[cursor.expert]) + m_tile * kBlockM;
+                const int channel = q * 32 + lane;
+                const float w_gate = kFp8 ? __ldg(w_scale + channel) : 1.0f, w_up = kFp8 ? __ldg(w_scale + p.n + channel) : 1.0f;
+#pragma unroll 1
+                for (int c0 = 0; c0 < tile_rows; c0 += 32) {
+                    const float a_scale_of_lane = (kFp8 && c0 + lane < tile_rows) ? p.a_scales[row0 + c0 + lane] : 1.0f;
+                    std::uint32_t g[32], u[32];
+                    tmem_ld_32x32(lane_base + c0, g);
+                    tmem_ld_32x32(lane_base + kBlockN + c0, u);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) {
+                        float gate = __uint_as_float(g[i]), up = __uint_as_float(u[i]);
+                        if (kFp8) {
+                            const float a_scale_i = __shfl_sync(0xffffffffu, a_scale_of_lane, i);
+                            gate *= a_scale_i * w_gate;
+                            up *= a_scale_i * w_up;
+                        }
+                        const float v = gate / (1.0f + __expf(-gate)) * up;
+                        if (c0 + i < tile_rows) p.out[(row0 + c0 + i) * p.n + n_tile * kOutN + channel] = __float2bfloat16_rn(v);
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&tmem_empty[buf]);
+                continue;
+            }
             if (kScatter) {
                 int owner = -1, token = 0, slot = -1;
                 float weight = 1.0f;
@@ -503,7 +557,7 @@ bool make_map(CUtensorMap* map, const void* base, std::uint64_t rows, std::uint6
 }
 
 template <bool kSwiGLU, bool kFp8, int kBoxesB, bool kScatter = false>
-cudaError_t launch(const CUtensorMap& map_a, const CUtensorMap& map_b, const GroupedGemmParams& p, int ctas, cudaStream_t stream) {
+cudaError_t launch(const ActivationMaps& map_a, const CUtensorMap& map_b, const GroupedGemmParams& p, int ctas, cudaStream_t stream) {
     static bool configured[64] = {false};
     int device = 0;
     cudaError_t status = cudaGetDevice(&device);
@@ -545,9 +599,13 @@ const char* run_grouped_gemm(const void* a, const void* w, void* out, const floa
             return "scatter target: bad landing-area description";
     }
     if (fp8 && (a_scales == nullptr || w_scales == nullptr)) return "fp8 operands need their scales";
-    CUtensorMap map_a, map_b;
+    ActivationMaps map_a;
+    CUtensorMap map_b;
     const std::uint64_t w_rows = static_cast<std::uint64_t>(num_experts) * (swiglu ? 2 : 1) * n;
-    if (!make_map(&map_a, a, static_cast<std::uint64_t>(rows_capacity), static_cast<std::uint64_t>(k), kBlockM, fp8) ||
+    bool encoded = true;
+    for (int i = 0; i < kBoxesA; ++i)
+        encoded = encoded && make_map(&map_a.box[i], a, static_cast<std::uint64_t>(rows_capacity), static_cast<std::uint64_t>(k), box_rows_a(i), fp8);
+    if (!encoded ||
         !make_map(&map_b, w, w_rows, static_cast<std::uint64_t>(k), kBlockN, fp8))
         return "cuTensorMapEncodeTiled failed";
     GroupedGemmParams p{};
