@@ -486,18 +486,22 @@ class Runtime {
         return p;
     }
 
-    // `stream` = raw cudaStream_t to launch on; 0 means the current PyTorch stream of the device.
+    // `stream` = raw cudaStream_t to launch on; 0 means the current PyTorch stream of the device.  `beside_compute`: the stream
+    // is not the caller's, whose kernels may want the other SMs.
     std::shared_ptr<DispatchResult> dispatch(const at::Tensor& x, const at::Tensor& topk_idx,
                                              const std::optional<at::Tensor>& topk_weights, int alignment, bool expand,
                                              bool zero_padding, const std::shared_ptr<Layout>& cached, bool graph_pool,
-                                             std::int64_t stream) {
+                                             std::int64_t stream, bool beside_compute = false) {
         c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device_));
         PreparedDispatch p = prepare_dispatch(x, topk_idx, topk_weights, alignment, expand, zero_padding, cached, graph_pool);
         cudaStream_t launch_stream = stream != 0 ? reinterpret_cast<cudaStream_t>(stream)
                                                  : at::cuda::getCurrentCUDAStream(device_).stream();
-        if (dispatch_is_local()) {
+        // A launch that runs beside the compute stream keeps to as many SMs as the buffer has channels, as it always has.
+        const int max_ctas = beside_compute ? options_.channels : local_sms_;
+        if (dispatch_is_local() && (p.args.num_tokens + max_ctas - 1) / std::max(1, max_ctas) < local_plan_.token_cap) {
             cuda_check(launch_dispatch_local(p.args, rc_, local_plan_, block_hist_.data_ptr<int>() + kLocalCounterInts,
-                                             reinterpret_cast<unsigned long long*>(block_hist_.data_ptr<int>()), local_sms_, launch_stream),
+                                             reinterpret_cast<unsigned long long*>(block_hist_.data_ptr<int>()), local_sms_, max_ctas,
+                                             launch_stream),
                        "dispatch launch");
             return p.result;
         }

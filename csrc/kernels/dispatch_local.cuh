@@ -27,6 +27,7 @@ constexpr int kLocalWarps = kLocalThreads / 32;
 constexpr int kLocalMaxStages = 3;      // row buffers per warp
 constexpr int kLocalMinWarps = 4;       // fewer row buffers than this: rows too long, dispatch.cuh takes the call
 constexpr int kLocalMaxPairBytes = 64 * 1024;
+constexpr int kLocalSmallPairBytes = 16 * 1024;  // fits beside fourteen row buffers of hidden 7168
 
 struct LocalDispatchArgs {
     DispatchArgs a;
@@ -55,8 +56,11 @@ struct LocalShared {
 // header | base[E] | total[E] | eoff[E + 1] | chan_base[C] | pair_e[cap*K] | pair_ord[cap*K] | unique[cap] | row buffers
 inline LocalPlan make_local_plan(int experts, int channels, int topk, int hidden, int max_tokens, int sms, std::size_t smem_limit) {
     LocalPlan p;
-    p.token_cap = (max_tokens + sms - 1) / sms + 1;
-    const std::size_t pair_bytes = static_cast<std::size_t>(p.token_cap) * (8 * topk + 4);
+    // tokens per CTA: for a grid of `channels` CTAs (launches beside other work) if their tables stay small, else for all SMs
+    const auto cap = [max_tokens](int ctas) { return (max_tokens + ctas - 1) / ctas + 1; };
+    const int token_bytes = 8 * topk + 4, few = channels < sms ? channels : sms;
+    p.token_cap = cap(few) <= kLocalSmallPairBytes / token_bytes ? cap(few) : cap(sms);
+    const std::size_t pair_bytes = static_cast<std::size_t>(p.token_cap) * token_bytes;
     std::size_t bytes = align_up(sizeof(LocalShared), 16) + static_cast<std::size_t>(experts) * 12 + 4 + static_cast<std::size_t>(channels) * 4;
     bytes = align_up(bytes + pair_bytes, 128);
     p.rows_off = bytes;

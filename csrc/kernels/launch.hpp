@@ -30,10 +30,11 @@ cudaError_t launch_dispatch(const DispatchLaunch& launch, int ctas, int threads,
 cudaError_t launch_combine(const CombineLaunch& launch, int channels, std::size_t crow_stride, cudaStream_t stream);
 
 // A group of one rank: how the local dispatch kernel cuts up shared memory, the ints of its scratch, and the two launches.
-// `rc` is the host's copy of the rank's constants, `sms` bounds the dispatch's CTAs; `counters` and `hist` belong to one buffer, whose launches are stream-ordered.
+// `rc` is the host's copy of the rank's constants, `sms` is what the scratch was made for, `max_ctas` bounds the CTAs; `counters` and `hist` belong to one buffer, whose launches are stream-ordered.
 LocalPlan plan_dispatch_local(const SegmentLayout& lay, int sms, std::size_t smem_limit);
 std::size_t dispatch_local_hist_ints(const SegmentLayout& lay, int ctas);
-cudaError_t launch_dispatch_local(const DispatchArgs& a, const RankConst& rc, const LocalPlan& plan, int* hist, unsigned long long* counters, int sms, cudaStream_t stream);
+cudaError_t launch_dispatch_local(const DispatchArgs& a, const RankConst& rc, const LocalPlan& plan, int* hist, unsigned long long* counters, int sms, int max_ctas,
+                                  cudaStream_t stream);
 cudaError_t launch_combine_local(const CombineLocalArgs& args, cudaStream_t stream);
 
 // Ordinary launches of the combine paths: expert-side gather-reduce-push, owner-side sum.  Any grid size works.

@@ -191,7 +191,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         .def(py::init<int, int, int, int, int, int, const py::dict&, const std::vector<std::int64_t>&, int>())
         .def("dispatch", &Runtime::dispatch, py::arg("x"), py::arg("topk_idx"), py::arg("topk_weights"),
              py::arg("alignment"), py::arg("expand"), py::arg("zero_padding"), py::arg("cached"), py::arg("graph_pool"),
-             py::arg("stream") = 0)
+             py::arg("stream") = 0, py::arg("beside_compute") = false)
         .def("combine", &Runtime::combine, py::arg("y"), py::arg("dispatch_result"), py::arg("weighted"), py::arg("out"),
              py::arg("stream") = 0, py::arg("num_sms") = 0)
         .def("fused_scatter_gemm", &Runtime::fused_scatter_gemm, py::arg("hidden_rows"), py::arg("w_down"),

@@ -102,6 +102,25 @@ def test_local_dispatch_and_combine(one_rank, tokens, capacity, experts, topk, h
         del local, general, cached, result, got
 
 
+@pytest.mark.parametrize("tokens,capacity,channels", [(300, 300, 7), (40, 300, 32), (30000, 30000, 1)])
+def test_dispatch_beside_the_compute_stream_keeps_to_its_channels(one_rank, tokens, capacity, channels):
+    """On the communication stream: as many CTAs as channels (or the general kernel where their tables would not fit)."""
+    from pcie_ep_b200 import HostStagedConfig, HostStagedEPBuffer
+
+    with HostStagedEPBuffer(one_rank, capacity, 64, 4, 16, HostStagedConfig(channels=channels)) as buffer:
+        x = torch.randn(tokens, 64).to(torch.bfloat16).cuda()
+        idx = torch.rand(tokens, 16).topk(4, dim=1).indices.cuda()
+        here = buffer.dispatch(x, idx, do_expand=True)
+        there = buffer.dispatch(x, idx, do_expand=True, async_with_compute_stream=True)
+        there[4].wait()
+        buffer.check_errors(there[3])
+        rows = tokens * 4
+        assert torch.equal(here[0][:rows], there[0][:rows]) and torch.equal(here[3].source_meta[:rows], there[3].source_meta[:rows])
+        assert torch.equal(here[3]._result["comb_map"], there[3]._result["comb_map"])
+        assert torch.equal(here[0][:rows], x[here[3].source_meta[:rows, 1]])
+        del here, there
+
+
 @pytest.mark.parametrize("inference", [False, True])
 def test_results_are_ordinary_tensors_over_the_pool(one_rank, inference):
     """What a dispatch and a combine hand out shares the pool's memory and version counter, also in inference mode."""
