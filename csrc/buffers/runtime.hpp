@@ -560,6 +560,7 @@ class Runtime {
         p.inline_kernel = combine_is_inline();
         if (p.inline_kernel) return p;
         unsigned long long* counters = reinterpret_cast<unsigned long long*>(fused_counters_.data_ptr<std::int64_t>());
+        // with a single rank two kernels can do all of it, and which one does is chosen at the launch
         if (combine_is_local()) {
             CombineLocalArgs& local = p.local;
             local.rc = a.rc;
@@ -580,25 +581,28 @@ class Runtime {
             local.num_topk = lay_.num_topk;
             local.hidden = lay_.hidden;
             p.max_rows = expand ? std::min(lay_.num_topk, lay_.num_local_experts) : 1;
-            return p;
         }
         CombinePushArgs& push = p.push;
         push.rc = a.rc;
         push.y = a.y;
         push.comb_map = a.comb_map;
         push.recv_chan_counts = a.recv_chan_counts;
+        push.plan_mask = a.plan_mask;
+        push.num_tokens = T;
         push.weighted = a.weighted;
+        push.out = a.out;
         push.error = a.error;
         push.stats = a.stats;
         push.cta_done = counters + 3;
         push.stat_scratch = counters + 4;
         push.next_unit = counters + 9;
         push.forwarder_sms = counters + 16;
-        push.forward_ctas = combine_forward_ctas_;
+        push.forward_ctas = lay_.num_ranks > 1 ? combine_forward_ctas_ : 0;
+        p.reduce_needed = lay_.num_ranks > 1;
+        if (!p.reduce_needed) return p;
         ensure_outbox();
         push.outbox = outbox_.data_ptr<std::uint8_t>();
         push.outbox_units = reinterpret_cast<unsigned long long*>(outbox_units_.data_ptr<std::int64_t>());
-        p.reduce_needed = true;
         FusedReduceArgs& r = p.reduce;
         r.rc = a.rc;
         r.expert_ord = nullptr;
@@ -630,9 +634,10 @@ class Runtime {
         return per_sm * std::max(1, sms);
     }
 
-    // the launch that reads the expert rows: everything with a single rank, else the expert side
+    // the launch that reads the expert rows: everything with a single rank (two kernels, each for the sizes it is the faster
+    // one at), else the expert side
     void launch_combine_push(PreparedCombine& prepared, cudaStream_t stream, int num_sms = 0) {
-        if (combine_is_local()) {
+        if (combine_is_local() && combine_local_pays(prepared.local.num_tokens, lay_.hidden, prepared.max_rows, combine_ctas(1, 0))) {
             prepared.local.shape = combine_local_shape(prepared.local.num_tokens, lay_.hidden, prepared.max_rows, combine_ctas(1, num_sms), max_smem_);
             cuda_check(launch_combine_local(prepared.local, stream), "combine launch");
             return;

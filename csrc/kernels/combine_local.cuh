@@ -1,4 +1,5 @@
-// Combine of a group of one rank: every token's expert rows, weighted, become its result row in one ordinary launch.
+// Combine of a group of one rank: every token's expert rows, weighted, become its result row in one ordinary launch.  (Large
+// batches of short rows: combine_push.cuh, see combine_local_pays.)
 //
 // What bounds it: reading the expert rows from HBM (4096 tokens, hidden 7168, top-8: 470 MB in, 59 MB out).  The rows of a
 // token lie far apart, so how they are asked for matters more than how many loads are in flight: pieces of 1 KB per row
@@ -85,6 +86,20 @@ inline CombineLocalShape combine_local_shape(int tokens, int hidden, int max_row
     s.ctas = units < 1 ? 1 : units < sms ? static_cast<int>(units) : sms;
     s.batch = s.stage_bytes <= kCombineLocalSmallStage && units >= 12ll * sms ? 4 : 1;
     return s;
+}
+
+// Which calls this kernel is for; the others keep the register loads of combine_push.cuh.  One producer warp hands out a unit
+// in 0.8 to 1.1 us (1.6 where units are claimed singly) however short its rows are, while the reducer warps there take an
+// entry each and so little time for short rows; they start 4 to 6 us later.  Measured on 148 SMs, us, registers / bulk copies:
+//   few tokens (up to 8 per SM): 128 tokens, 8 rows of 1 KB 15.6 / 8.3; 1024 tokens, 8 rows of 2 KB 17.7 / 16.5, one of
+//     14 KB 21.4 / 16.5; beyond: 1536 tokens, 2 rows of 1 KB 17.2 / 18.5, 65536 tokens, one of 2 KB 143 / 359;
+//   up to 14 per SM with rows of 3 KB and more: 2048 tokens, 8 rows of 4 KB 28.1 / 24.8, of 2 KB 21.6 / 23.7;
+//   rows of 10 KB and more: 8192 tokens, one row 69.5 / 58.3, 8 rows of 14 KB 205 / 160; one row of 8 KB 53.3 / 57.5;
+//   several rows of 7 KB and more: 8192 tokens, 4 rows of 7 KB 74.9 / 66.3, two 55.0 / 59.5, 8 rows of 5.6 KB 95.5 / 103.7.
+inline bool combine_local_pays(int tokens, int hidden, int max_rows, int sms) {
+    const int row_bytes = hidden * 2;
+    if (tokens <= 8ll * sms || row_bytes >= 10 * 1024) return true;
+    return (row_bytes >= 7 * 1024 && max_rows >= 4) || (row_bytes >= 3 * 1024 && tokens <= 14ll * sms);
 }
 
 #ifdef __CUDACC__

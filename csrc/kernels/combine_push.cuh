@@ -4,7 +4,8 @@
 //   with the dispatch-time weights in FP32, round to BF16 and deliver the partial row to the token owner's landing
 //   area: reducer CTAs write it to a local outbox, a few forwarder CTAs of the same launch copy completed rows over
 //   NVLink with bulk copies.  The launch's last CTA publishes the epoch to every owner (whose fused_reduce_kernel,
-//   fused_reduce.cuh, then adds the ranks' rows).  A group of one rank takes combine_local.cuh instead.
+//   fused_reduce.cuh, then adds the ranks' rows).  With one rank the reduced rows are the result and go straight
+//   to `out`: the calls of a group of one rank that combine_local.cuh leaves to this kernel (combine_local_pays).
 #pragma once
 
 #include "fused_reduce.cuh"
@@ -16,7 +17,10 @@ struct CombinePushArgs {
     const __nv_bfloat16* y;        // expert outputs in the layout of the dispatch's recv_x
     const int* comb_map;           // [P][C][slots_full][2 + 2K]: token, n, then (row, weight bits) pairs
     const int* recv_chan_counts;   // [P][C] entries per (source, channel)
+    const std::uint32_t* plan_mask;  // [Tmax] destination mask of this rank's own tokens (0: routed nowhere)
+    int num_tokens;                // this rank's own token count at dispatch
     int weighted;
+    __nv_bfloat16* out;            // [T, H]; written here only with a single rank
     int* error;                    // [8]
     std::int64_t* stats;           // [8]: rows pushed, of which to other ranks, ns until the last reducer CTA / the last
                                    // forwarder CTA had finished (from the first CTA's start)
@@ -26,7 +30,7 @@ struct CombinePushArgs {
     // rows whose owner is another rank are reduced into a local outbox and forwarded by dedicated CTAs
     std::uint8_t* outbox;              // [P*C*slots_full][crow_stride], local memory
     unsigned long long* outbox_units;  // [P*C*slots_full] finished units of the row in the outbox; zero between launches
-    int forward_ctas;                  // the first CTAs of the grid only forward
+    int forward_ctas;                  // the first CTAs of the grid only forward; 0 with a single rank
     unsigned long long* next_unit;     // next entry to hand out to a reducer warp; zero between launches
     unsigned long long* forwarder_sms; // [kMaxSmTable] combine epoch in which SM i hosts a forwarder CTA
 };
@@ -53,6 +57,7 @@ inline std::size_t combine_push_smem_bytes(const SegmentLayout& lay, int forward
 // numbering order.
 //
 // Where the reduced row goes:
+//   * one rank: straight to `out`;
 //   * owner = this rank: straight into this rank's own landing area (a local store);
 //   * owner = another rank: into a local outbox row.  The first `forward_ctas` CTAs of the grid do nothing but
 //     copy completed outbox rows to their owners (bulk load into shared memory, bulk store to the peer).  A few SMs
@@ -114,7 +119,7 @@ __global__ void __launch_bounds__(kFusedReduceThreads, 2) combine_push_kernel(co
             if (blockIdx.x == 0) atomicCAS(&a.error[0], 0, kErrAlreadyAborted);
             s_failed = 1;
         }
-    } else if (static_cast<int>(threadIdx.x) < P) {
+    } else if (P > 1 && static_cast<int>(threadIdx.x) < P) {
         // reuse guard: an owner must have finished adding the previous combine's rows before new ones land
         Health health(rc, a.error);
         const std::uint64_t* done = flag_ptr(rc->seg[me], lay.cdone_off, threadIdx.x);
@@ -276,6 +281,7 @@ __global__ void __launch_bounds__(kFusedReduceThreads, 2) combine_push_kernel(co
     } else if (!s_failed) {
         // ---- reduce ----------------------------------------------------------------------------------------
         const long long total_warps = static_cast<long long>(gridDim.x - F) * warps;
+        const long long wid = static_cast<long long>(blockIdx.x - F) * warps + warp;
         const std::uint8_t* y = reinterpret_cast<const std::uint8_t*>(a.y);
         const std::size_t row_bytes = static_cast<std::size_t>(H) * 2;
         // Entries are handed out one at a time through a counter (a warp reduces all units of its entry), so that rows
@@ -294,7 +300,7 @@ __global__ void __launch_bounds__(kFusedReduceThreads, 2) combine_push_kernel(co
         int taken = 0, yields = 0;
         bool shares_sm = false;
         while (true) {
-            if (!shares_sm && (taken++ & 3) == 0 && my_sm < static_cast<unsigned>(kMaxSmTable))
+            if (F > 0 && !shares_sm && (taken++ & 3) == 0 && my_sm < static_cast<unsigned>(kMaxSmTable))
                 shares_sm = ptx::ld_relaxed_sys(reinterpret_cast<const std::uint64_t*>(a.forwarder_sms + my_sm)) == epoch;
             if (shares_sm && yields < 128) {
                 // stand aside (a few hundred microseconds at most, then help after all) and leave once every entry is taken
@@ -319,9 +325,10 @@ __global__ void __launch_bounds__(kFusedReduceThreads, 2) combine_push_kernel(co
                 row_of_lane = map[2 + 2 * lane];
                 weight_of_lane = a.weighted ? __int_as_float(map[3 + 2 * lane]) : 1.0f;
             }
-            const bool remote = e.s != me;
+            const bool remote = P > 1 && e.s != me;
             std::uint8_t* dst_row =
-                remote ? a.outbox + static_cast<std::size_t>(e.slot) * crow_stride
+                P == 1 ? reinterpret_cast<std::uint8_t*>(a.out + static_cast<std::size_t>(e.token) * H)
+                : remote ? a.outbox + static_cast<std::size_t>(e.slot) * crow_stride
                          : s_seg[me] + cstage_off + static_cast<std::size_t>(me) * rank_stride + static_cast<std::size_t>(e.token) * crow_stride;
             if (lane == 0 && part == 0) {
                 ++pushed;
@@ -403,6 +410,16 @@ __global__ void __launch_bounds__(kFusedReduceThreads, 2) combine_push_kernel(co
             __threadfence();
             atomicAdd(completed, 1ull);
         }
+        if (P == 1) {
+            // tokens that were routed nowhere have no map entry: their result is zero
+            const long long zero_units = static_cast<long long>(a.num_tokens) * groups;
+            for (long long u = wid; u < zero_units; u += total_warps) {
+                const int t = static_cast<int>(u / groups);
+                const int q = static_cast<int>(u % groups) * 32 + lane;
+                if (a.plan_mask[t] == 0 && q < chunks)
+                    reinterpret_cast<uint4*>(a.out + static_cast<std::size_t>(t) * H)[q] = make_uint4(0u, 0u, 0u, 0u);
+            }
+        }
         if (lane == 0 && pushed) {
             atomicAdd(&a.stat_scratch[0], pushed);
             atomicAdd(&a.stat_scratch[1], pushed_remote);
@@ -427,7 +444,8 @@ __global__ void __launch_bounds__(kFusedReduceThreads, 2) combine_push_kernel(co
             for (int i = 0; i < 5; ++i) a.stat_scratch[i] = i == 2 ? ~0ull : 0ull;
             *a.next_unit = 0ull;
             if (ptx::ld_volatile(&rc->sticky[0]) == 0) {
-                for (int p = 0; p < P; ++p) ptx::st_release_sys(flag_ptr(rc->seg[p], lay.csig_off, me), epoch);
+                if (P > 1)
+                    for (int p = 0; p < P; ++p) ptx::st_release_sys(flag_ptr(rc->seg[p], lay.csig_off, me), epoch);
                 rc->epochs[1] = epoch;
             }
         }

@@ -1,6 +1,7 @@
 """A group of one rank: the kernels without the exchange protocol against the general dispatch kernel, field by field, and
 the combine against a sum in 64 bits, where tiles, slices and chunks end."""
 
+import json
 import os
 import tempfile
 
@@ -145,3 +146,54 @@ def test_results_are_ordinary_tensors_over_the_pool(one_rank, inference):
             buffer.dispatch(x, [1])
         with pytest.raises(ValueError, match="contiguous"):
             buffer.combine(recv_x[:, :32], handle)
+
+
+def launches(call):
+    """The kernels that ``call`` launches, as a profiler saw them: name, CTAs, threads, shared memory and registers."""
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        call()
+        torch.cuda.synchronize()
+    with tempfile.NamedTemporaryFile(suffix=".json") as file:
+        prof.export_chrome_trace(file.name)
+        events = json.load(open(file.name))["traceEvents"]
+    kernels = sorted((e for e in events if e.get("cat") == "kernel"), key=lambda e: e["ts"])
+    return [dict(name=e["name"], ctas=e["args"]["grid"][0], threads=e["args"]["block"][0], shared=e["args"]["shared memory"],
+                 registers=e["args"]["registers per thread"]) for e in kernels]
+
+
+def weighted_sum(y, idx, w, topk):
+    """Expanded rows back to their tokens in 64 bits, and a bound on what 32-bit sums rounded to BF16 may differ by."""
+    order = torch.argsort(idx.reshape(-1), stable=True)
+    row_of = torch.empty_like(order)
+    row_of[order] = torch.arange(order.numel(), device=order.device)
+    terms = y[row_of].double().view(*idx.shape, -1) * w.double().unsqueeze(2)
+    want = terms.sum(1)
+    return want, want.abs() * 2.0 ** -8 + terms.abs().sum(1) * topk * 2.0 ** -23
+
+
+# tokens per SM, tokens on top, hidden, top-k, whether whole rows are copied in bulk (at the lines of combine_local_pays)
+KERNELS = [(8, 0, 512, 2, True), (8, 1, 512, 2, False), (14, 0, 1536, 2, True), (14, 0, 1528, 2, False), (14, 1, 1536, 2, False),
+           (14, 1, 3584, 4, True), (14, 1, 3576, 4, False), (14, 1, 3584, 3, False), (14, 1, 5120, 1, True), (14, 1, 5112, 1, False)]
+
+
+@pytest.mark.parametrize("per_sm,more,hidden,topk,bulk", KERNELS)
+def test_combine_takes_the_faster_kernel_for_its_rows(one_rank, per_sm, more, hidden, topk, bulk):
+    from pcie_ep_b200 import HostStagedConfig, HostStagedEPBuffer
+
+    tokens = torch.cuda.get_device_properties(0).multi_processor_count * per_sm + more
+    with HostStagedEPBuffer(one_rank, tokens, hidden, topk, 16, HostStagedConfig(channels=64)) as buffer:
+        gen = torch.Generator(device="cuda").manual_seed(hidden)
+        x = torch.randn(tokens, hidden, device="cuda", generator=gen).to(torch.bfloat16)
+        idx = torch.rand(tokens, 16, device="cuda", generator=gen).topk(topk, dim=1).indices
+        w = torch.rand(tokens, topk, device="cuda", generator=gen)
+        y = torch.randn(tokens * topk, hidden, device="cuda", generator=gen).to(torch.bfloat16)
+        handle = buffer.dispatch(x, idx, w, do_expand=True)[3]
+        got = []
+        seen = launches(lambda: got.append(buffer.combine(y, handle)[0]))
+        buffer.check_errors(handle)
+        assert [("local_combine" in k["name"]) for k in seen if "combine" in k["name"]] == [bulk]
+        want, bound = weighted_sum(y, idx, w, topk)
+        assert bool(((got[0].double() - want).abs() <= bound).all())
+        assert int(handle._result["combine_stats"][0]) == tokens
+        del got, handle
