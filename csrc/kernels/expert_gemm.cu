@@ -364,13 +364,17 @@ grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_a, const __grid_
             const std::uint32_t lane_base = tmem_base + (static_cast<std::uint32_t>(q * 32) << 16) + buf * kAccCols;
             const int tile_rows = p.expert_counts[cursor.expert] - m_tile * kBlockM;
             if (flips(box_of_rows(tile_rows))) {
-                // swapped tile: TMEM lane = output channel, column = row; a warp stores 32 channels of a row
+                // Swapped tile: TMEM lane = output channel, column = row; a warp stores 32 channels of a row.  The address of a row
+                // is only known once the row before has been stored: with all 32 addresses computed ahead the BF16 build took 166
+                // registers instead of 112, and a quarter of an SM had none left for two warps of a combine reducer
+                // (combine_push.cuh) beside two of these.
                 const long long row0 = static_cast<long long>(p.expert_offsets[cursor.expert]) + m_tile * kBlockM;
                 const int channel = q * 32 + lane;
                 const float w_gate = kFp8 ? __ldg(w_scale + channel) : 1.0f, w_up = kFp8 ? __ldg(w_scale + p.n + channel) : 1.0f;
 #pragma unroll 1
                 for (int c0 = 0; c0 < tile_rows; c0 += 32) {
                     const float a_scale_of_lane = (kFp8 && c0 + lane < tile_rows) ? p.a_scales[row0 + c0 + lane] : 1.0f;
+                    __nv_bfloat16* dst = p.out + (row0 + c0) * p.n + n_tile * kOutN + channel;
                     std::uint32_t g[32], u[32];
                     tmem_ld_32x32(lane_base + c0, g);
                     tmem_ld_32x32(lane_base + kBlockN + c0, u);
@@ -384,7 +388,9 @@ grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_a, const __grid_
                             up *= a_scale_i * w_up;
                         }
                         const float v = gate / (1.0f + __expf(-gate)) * up;
-                        if (c0 + i < tile_rows) p.out[(row0 + c0 + i) * p.n + n_tile * kOutN + channel] = __float2bfloat16_rn(v);
+                        if (c0 + i < tile_rows) *dst = __float2bfloat16_rn(v);
+                        dst += p.n;
+                        asm volatile("" : "+l"(dst));
                     }
                 }
                 tc_fence_before();

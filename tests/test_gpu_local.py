@@ -197,3 +197,42 @@ def test_combine_takes_the_faster_kernel_for_its_rows(one_rank, per_sm, more, hi
         assert bool(((got[0].double() - want).abs() <= bound).all())
         assert int(handle._result["combine_stats"][0]) == tokens
         del got, handle
+
+
+def room_beside(*kernels):
+    """Whether one CTA of each of these launches fits on one SM (a CTA's warps go round the four quarters of the SM, each with
+    a quarter of the registers; 1 KB of shared memory per CTA is the system's)."""
+    device = torch.cuda.get_device_properties(0)
+    shared = sum(k["shared"] + 1024 for k in kernels)
+    registers = sum(-(-k["threads"] // 128) * 32 * (-(-k["registers"] // 8) * 8) for k in kernels)
+    return shared <= device.shared_memory_per_multiprocessor and registers <= device.regs_per_multiprocessor // 4
+
+
+@pytest.mark.parametrize("swiglu,fp8", [(False, False), (True, False), (True, True)])
+def test_expert_gemm_leaves_room_for_a_combine_reducer(one_rank, swiglu, fp8):
+    """The reducers of the combine use no shared memory so that they can run on SMs which a persistent expert GEMM holds."""
+    from pcie_ep_b200 import HostStagedConfig, HostStagedEPBuffer
+    from pcie_ep_b200.ops.grouped_ffn import grouped_gemm
+
+    tokens = torch.cuda.get_device_properties(0).multi_processor_count * 8 + 1  # of short rows: the reducers take the call
+    with HostStagedEPBuffer(one_rank, tokens, 512, 2, 16, HostStagedConfig(channels=64)) as buffer:
+        x = torch.randn(tokens, 512).to(torch.bfloat16).cuda()
+        idx = torch.rand(tokens, 16).topk(2, dim=1).indices.cuda()
+        recv_x, _, _, handle, _ = buffer.dispatch(x, idx, do_expand=True)
+        dtype = torch.float8_e4m3fn if fp8 else torch.bfloat16
+        weights = torch.randn(16, 512 if swiglu else 256, 512).to(torch.bfloat16).cuda().to(dtype)
+        scales = dict(a_scales=torch.ones(recv_x.shape[0], device="cuda"), w_scales=torch.ones(16, 512, device="cuda")) if fp8 else {}
+        out = torch.empty(recv_x.shape[0], 256, dtype=torch.bfloat16, device="cuda")
+        rows, got = recv_x.to(dtype), []
+
+        def call():
+            grouped_gemm(rows, weights, handle.expert_offsets, handle.expert_counts, swiglu=swiglu, out=out, **scales)
+            got.append(buffer.combine(recv_x, handle)[0])
+
+        seen = launches(call)
+        buffer.check_errors(handle)
+        gemm, = (k for k in seen if "gemm" in k["name"])
+        combine, = (k for k in seen if "combine" in k["name"])
+        assert "local_combine" not in combine["name"] and room_beside(gemm, combine)
+        assert torch.equal(got[0], 2 * x)
+        del recv_x, handle, got
