@@ -634,11 +634,17 @@ class Runtime {
         return per_sm * std::max(1, sms);
     }
 
-    // the launch that reads the expert rows: everything with a single rank (two kernels, each for the sizes it is the faster
-    // one at), else the expert side
+    // The launch that reads the expert rows: everything with a single rank, else the expert side.  With a single rank two
+    // kernels can do it.  combine_local.cuh wants the shared memory of every SM to itself and gets it on the device's default
+    // stream; a launch that is limited to `num_sms`, or that another stream (the communication stream, a caller's own) runs
+    // beside something else, takes the reducers without shared memory, which fit on an SM beside a CTA of the expert GEMM.
+    // Behind the start of a gate/up GEMM of 8 x 1024 rows (334 us) a combine on the communication stream was done after, us,
+    // bulk copies / reducers: 256 tokens 342 / 45, 4096 tokens 410 / 233 (and both kernels 410 / 371).  The price: alone on
+    // such a stream 92 / 116 for 4096 tokens, beside library GEMMs, whose CTAs come and go, 218 / 257.
     void launch_combine_push(PreparedCombine& prepared, cudaStream_t stream, int num_sms = 0) {
-        if (combine_is_local() && combine_local_pays(prepared.local.num_tokens, lay_.hidden, prepared.max_rows, combine_ctas(1, 0))) {
-            prepared.local.shape = combine_local_shape(prepared.local.num_tokens, lay_.hidden, prepared.max_rows, combine_ctas(1, num_sms), max_smem_);
+        const bool shares_sms = num_sms > 0 || stream != nullptr;
+        if (combine_is_local() && !shares_sms && combine_local_pays(prepared.local.num_tokens, lay_.hidden, prepared.max_rows, combine_ctas(1, 0))) {
+            prepared.local.shape = combine_local_shape(prepared.local.num_tokens, lay_.hidden, prepared.max_rows, combine_ctas(1, 0), max_smem_);
             cuda_check(launch_combine_local(prepared.local, stream), "combine launch");
             return;
         }

@@ -1,5 +1,6 @@
 // Combine of a group of one rank: every token's expert rows, weighted, become its result row in one ordinary launch.  (Large
-// batches of short rows: combine_push.cuh, see combine_local_pays.)
+// batches of short rows: combine_push.cuh, see combine_local_pays.  Launches that share the SMs with other work, too: a CTA
+// of this kernel takes nearly all of an SM's shared memory.)
 //
 // What bounds it: reading the expert rows from HBM (4096 tokens, hidden 7168, top-8: 470 MB in, 59 MB out).  The rows of a
 // token lie far apart, so how they are asked for matters more than how many loads are in flight: pieces of 1 KB per row

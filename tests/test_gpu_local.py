@@ -236,3 +236,45 @@ def test_expert_gemm_leaves_room_for_a_combine_reducer(one_rank, swiglu, fp8):
         assert "local_combine" not in combine["name"] and room_beside(gemm, combine)
         assert torch.equal(got[0], 2 * x)
         del recv_x, handle, got
+
+
+@pytest.mark.parametrize("how", ["async", "event", "side stream", "num_sms", "default"])
+@pytest.mark.parametrize("tokens", [40, 600])
+def test_combine_beside_other_work_fits_next_to_the_expert_gemm(one_rank, how, tokens):
+    """On the communication stream, on a stream of the caller's own or limited to some SMs, a CTA of the combine finds room on
+    an SM that a CTA of the persistent expert GEMM holds."""
+    from pcie_ep_b200 import HostStagedConfig, HostStagedEPBuffer
+    from pcie_ep_b200.ops.grouped_ffn import grouped_gemm
+
+    with HostStagedEPBuffer(one_rank, tokens, 1024, 2, 16, HostStagedConfig(channels=8)) as buffer:
+        x = torch.randn(tokens, 1024).to(torch.bfloat16).cuda()
+        idx = torch.rand(tokens, 16).topk(2, dim=1).indices.cuda()
+        w = torch.rand(tokens, 2).cuda()
+        y = torch.randn(2 * tokens, 1024).to(torch.bfloat16).cuda()
+        handle = buffer.dispatch(x, idx, w, do_expand=True)[3]
+        weights = torch.randn(16, 512, 1024).to(torch.bfloat16).cuda()
+        gemm_out = torch.empty(2 * tokens, 256, dtype=torch.bfloat16, device="cuda")
+        got = []
+
+        def call():
+            grouped_gemm(y, weights, handle.expert_offsets, handle.expert_counts, swiglu=True, out=gemm_out)
+            if how == "side stream":
+                side = torch.cuda.Stream()
+                side.wait_stream(torch.cuda.current_stream())
+                with torch.cuda.stream(side):
+                    got.append(buffer.combine(y, handle)[0])
+            elif how == "event":
+                got.append(buffer.combine(y, handle, previous_event=buffer.capture(), allocate_on_comm_stream=True)[0])
+            else:
+                got.append(buffer.combine(y, handle, async_with_compute_stream=how == "async", num_sms=5 if how == "num_sms" else 0)[0])
+
+        seen = launches(call)
+        buffer.check_errors(handle)
+        gemm, = (k for k in seen if "gemm" in k["name"])
+        combine, = (k for k in seen if "combine" in k["name"])
+        assert ("local_combine" in combine["name"]) == (how == "default")
+        assert how == "default" or room_beside(gemm, combine)
+        assert how != "num_sms" or combine["ctas"] <= 2 * 5
+        want, bound = weighted_sum(y, idx, w, 2)
+        assert bool(((got[0].double() - want).abs() <= bound).all())
+        del got, handle
