@@ -520,6 +520,9 @@ class Runtime {
                rc_.test_withhold_counts == 0 && rc_.test_corrupt_sequence == 0 && rc_.test_abort_after_ns == 0;
     }
 
+    // Whether a dispatch of `tokens` tokens is another launch beside the compute stream than on it.
+    bool dispatch_differs_beside_compute(int tokens) const { return dispatch_is_local() && options_.channels < std::min(local_sms_, tokens); }
+
     // ---- combine --------------------------------------------------------------------------------
     PreparedCombine prepare_combine(const at::Tensor& y, const DispatchResult& dispatch_result, bool weighted,
                                     const std::optional<at::Tensor>& out_opt) {

@@ -63,6 +63,10 @@ class StreamPolicy:
             stream = self._known[raw] = torch.cuda.current_stream(self.device)
         return stream
 
+    def is_comm(self, stream: Any) -> bool:
+        """Also true for a caller that has made the communication stream its current one."""
+        return stream is self.comm or stream.cuda_stream == self.comm.cuda_stream
+
     # -- readers of result pools ---------------------------------------------------------------
     def add_consumer(self, stream: Any) -> None:
         """Remember a stream that reads results; it outlives the Python tensors it reads."""

@@ -278,3 +278,44 @@ def test_combine_beside_other_work_fits_next_to_the_expert_gemm(one_rank, how, t
         want, bound = weighted_sum(y, idx, w, 2)
         assert bool(((got[0].double() - want).abs() <= bound).all())
         del got, handle
+
+
+@pytest.mark.parametrize("cached", [False, True])
+@pytest.mark.parametrize("tokens,channels", [(300, 7), (40, 300 // 4), (5, 32), (30000, 1)])
+def test_dispatch_and_replay_launch_what_their_stream_allows(one_rank, tokens, channels, cached):
+    """On the caller's stream every SM, on the communication stream as many CTAs as channels (the general kernel where the
+    tables of so few CTAs would not fit); a captured dispatch follows the stream of the replay, not that of the capture."""
+    from pcie_ep_b200 import HostStagedConfig, HostStagedEPBuffer
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    with HostStagedEPBuffer(one_rank, tokens, 64, 4, 16, HostStagedConfig(channels=channels, enable_graph=True)) as buffer:
+        x = torch.randn(tokens, 64).to(torch.bfloat16).cuda()
+        idx = torch.rand(tokens, 16).topk(4, dim=1).indices.cuda()
+        plan = buffer.cache_layout(buffer.dispatch(x, idx, do_expand=True)[3])
+        routes = dict(handle=plan) if cached else dict(topk_idx=idx)
+        graph = buffer.capture_dispatch(x, do_expand=True, **routes)
+        beside = dict(async_with_compute_stream=True)
+
+        def on_comm_stream(call):
+            buffer.get_comm_stream().wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(buffer.get_comm_stream()):
+                return call()
+
+        def eager(**how):
+            return buffer.dispatch(x, do_expand=True, **routes, **how)
+
+        calls = [(eager, False), (lambda: eager(**beside), True), (lambda: on_comm_stream(eager), True), (graph.replay, False),
+                 (lambda: graph.replay(**beside), True), (lambda: graph.replay(previous_event=buffer.capture()), True),
+                 (lambda: on_comm_stream(graph.replay), True), (graph.replay, False)]
+        for number, (call, few) in enumerate(calls):
+            got = []
+            seen, = launches(lambda: got.append(call()))
+            buffer.check_errors(got[0][3])
+            fits = not (few and tokens == 30000)
+            assert ("local_dispatch" in seen["name"]) == fits, number
+            assert seen["ctas"] == (min(channels if few else sms, sms, tokens) if fits else channels), number
+            rows = tokens * 4
+            meta = got[0][3].source_meta[:rows]
+            assert torch.equal(got[0][0][:rows], x[meta[:, 1]]) and torch.equal(got[0][3].expert_counts.long(), torch.bincount(idx.reshape(-1), minlength=16))
+            del got, meta
+        graph.close()
