@@ -541,9 +541,7 @@ class Runtime {
         // No allocation on the hot path: without `out`, the result comes from a small ring of
         // preallocated [Tmax, hidden] tensors with the same "busy while referenced" rule as dispatch.
         at::Tensor out = out_opt.has_value() ? *out_opt : select_combine_output(T);
-        if (!out.is_cuda() || out.scalar_type() != at::kBFloat16 || !out.is_contiguous() || out.dim() != 2 ||
-            out.size(0) != T || out.size(1) != lay_.hidden)
-            throw std::invalid_argument("combine output must be contiguous CUDA BF16 [T, hidden]");
+        check_combine_output(out, T, rc_.vec_ok != 0);
         PreparedCombine p;
         p.out = out;
         CombineArgs& a = p.args;
@@ -740,9 +738,7 @@ class Runtime {
         if (!layout || !layout->valid) throw std::invalid_argument("dispatch result carries no routing plan");
         const int T = layout->num_tokens;
         at::Tensor out = out_opt.has_value() ? *out_opt : select_combine_output(T);
-        if (!out.is_cuda() || out.scalar_type() != at::kBFloat16 || !out.is_contiguous() || out.dim() != 2 ||
-            out.size(0) != T || out.size(1) != lay_.hidden)
-            throw std::invalid_argument("combine output must be contiguous CUDA BF16 [T, hidden]");
+        check_combine_output(out, T, true);
         FusedReduceArgs a{};
         a.rc = reinterpret_cast<const RankConst*>(rank_const_.data_ptr<std::uint8_t>());
         a.expert_ord = layout->expert_ord.data_ptr<int>();
@@ -766,6 +762,11 @@ class Runtime {
         return out;
     }
     at::Tensor fused_status() const { return fused_status_; }
+    // an output that fused_reduce would refuse, refused before the GEMM is launched (each GEMM needs its reduction)
+    void check_fused_output(const at::Tensor& out, const DispatchResult& dispatch_result) const {
+        check_open();
+        check_combine_output(out, dispatch_result.num_tokens(), true);
+    }
 
     // ---- diagnostics / test hooks --------------------------------------------------------------
     py::dict pool_debug() const {
@@ -841,6 +842,15 @@ class Runtime {
     bool matches(const at::Tensor& t, at::ScalarType dtype, std::int64_t rows, std::int64_t columns) const {
         return t.defined() && t.layout() == at::kStrided && t.is_cuda() && t.get_device() == device_ && t.scalar_type() == dtype && t.dim() == 2 &&
                t.is_contiguous() && (rows < 0 || t.size(0) == rows) && t.size(1) == columns;
+    }
+
+    // `wide`: the kernel stores 16 bytes at a time
+    void check_combine_output(const at::Tensor& out, int tokens, bool wide) const {
+        if (!out.is_cuda() || out.get_device() != device_ || out.scalar_type() != at::kBFloat16 || !out.is_contiguous() || out.dim() != 2 ||
+            out.size(0) != tokens || out.size(1) != lay_.hidden)
+            throw std::invalid_argument("combine output must be contiguous CUDA BF16 [T, hidden] on the buffer's device");
+        if (wide && reinterpret_cast<std::uintptr_t>(out.data_ptr()) % 16 != 0)
+            throw std::invalid_argument("combine output must start on a 16-byte boundary");
     }
 
     void validate_inputs(const at::Tensor& x, const at::Tensor& idx, const std::optional<at::Tensor>& w, int alignment,

@@ -197,6 +197,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         .def("fused_scatter_gemm", &Runtime::fused_scatter_gemm, py::arg("hidden_rows"), py::arg("w_down"),
              py::arg("dispatch_result"), py::arg("stream") = 0)
         .def("fused_reduce", &Runtime::fused_reduce, py::arg("dispatch_result"), py::arg("out"), py::arg("stream") = 0)
+        .def("check_fused_output", &Runtime::check_fused_output, py::arg("out"), py::arg("dispatch_result"))
         .def("fused_status", &Runtime::fused_status)
         .def("accepts_inputs", &Runtime::accepts_inputs, py::arg("x"), py::arg("topk_idx"), py::arg("topk_weights"))
         .def("accepts_rows", &Runtime::accepts_rows, py::arg("y"), py::arg("dispatch_result"))

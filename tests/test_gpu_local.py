@@ -319,3 +319,29 @@ def test_dispatch_and_replay_launch_what_their_stream_allows(one_rank, tokens, c
             assert torch.equal(got[0][0][:rows], x[meta[:, 1]]) and torch.equal(got[0][3].expert_counts.long(), torch.bincount(idx.reshape(-1), minlength=16))
             del got, meta
         graph.close()
+
+
+def test_combine_refuses_outputs_that_its_stores_do_not_fit(one_rank):
+    """An output off the 16-byte boundary is an error of the call, and the buffer goes on after it, fused calls included."""
+    from pcie_ep_b200 import HostStagedConfig, HostStagedEPBuffer
+
+    tokens, hidden, inter = 24, 256, 128
+    with HostStagedEPBuffer(one_rank, tokens, hidden, 2, 4, HostStagedConfig(channels=4, fused_expert_combine=True)) as buffer:
+        x = torch.randn(tokens, hidden).to(torch.bfloat16).cuda()
+        idx = torch.rand(tokens, 4).topk(2, dim=1).indices.cuda()
+        w = torch.rand(tokens, 2).cuda()
+        recv_x, _, _, handle, _ = buffer.dispatch(x, idx, w, do_expand=True)
+        hidden_rows = torch.randn(recv_x.shape[0], inter).to(torch.bfloat16).cuda()
+        w_down = torch.randn(4, hidden, inter).to(torch.bfloat16).cuda()
+        room = torch.empty(tokens * hidden + 8, dtype=torch.bfloat16, device="cuda")
+        calls = [lambda out: buffer.combine(recv_x, handle, out=out), lambda out: buffer.fused_expert_combine(hidden_rows, w_down, handle, out=out)]
+        for call in calls:
+            for offset in (1, 4, 7):
+                with pytest.raises(ValueError, match="16-byte boundary"):
+                    call(room[offset:offset + tokens * hidden].view(tokens, hidden))
+            with pytest.raises(ValueError, match=r"\[T, hidden\]"):
+                call(room[:hidden].view(1, hidden))
+            want = call(None)[0].clone()
+            assert torch.equal(call(room[8:].view(tokens, hidden))[0], want) and float(want.float().abs().max()) > 0
+        buffer.check_errors(handle)
+        del recv_x, handle
