@@ -520,8 +520,10 @@ class Runtime {
                rc_.test_withhold_counts == 0 && rc_.test_corrupt_sequence == 0 && rc_.test_abort_after_ns == 0;
     }
 
-    // Whether a dispatch of `tokens` tokens is another launch beside the compute stream than on it.
-    bool dispatch_differs_beside_compute(int tokens) const { return dispatch_is_local() && options_.channels < std::min(local_sms_, tokens); }
+    // Whether a dispatch of `tokens` tokens (`padding`: that zeroes rows) is another launch beside the compute stream than on it.
+    bool dispatch_differs_beside_compute(int tokens, bool padding) const {
+        return dispatch_is_local() && options_.channels < std::min(local_sms_, dispatch_local_width(lay_, tokens, padding));
+    }
 
     // ---- combine --------------------------------------------------------------------------------
     PreparedCombine prepare_combine(const at::Tensor& y, const DispatchResult& dispatch_result, bool weighted,

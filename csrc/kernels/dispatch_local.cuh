@@ -2,9 +2,11 @@
 // the expansion are left: no counts message, no READY flags, no send role, no control warp.  Results, routing plan and
 // combine map are the ones dispatch.cuh leaves behind, bit for bit; the two kernels may alternate on one buffer.
 //
-// Grid: one CTA per SM, or one per token where there are fewer tokens; CTA b owns the tokens [T*b/G, T*(b+1)/G).  (The
-// channels of the configuration only number the combine map here: few CTAs would keep a barrier between ranks short, but
-// the SMs that write the rows are what sets the pace.)
+// Grid: one CTA per SM, or one per token where there are fewer tokens (and as many as experts where rows between their
+// segments are zeroed); CTA b owns the tokens [T*b/G, T*(b+1)/G).  A launch beside the compute stream has no more CTAs than the
+// configuration has channels; where the tables of so many tokens per CTA do not fit, dispatch.cuh takes the call.  (Otherwise the
+// channels only number the combine map here: few CTAs would keep a barrier between ranks short, but the SMs that write the
+// rows are what sets the pace.)
 //   1. token rows are on their way into shared memory before anything about the layout is known;
 //   2. expert ids -> histogram and stable ordinals inside the CTA's tokens, 32 tokens at a time, one thread per (token, k);
 //   3. one grid barrier; then a prefix over the CTAs before this one and a scan over experts, one thread per bin.  A cached
@@ -558,9 +560,12 @@ __global__ void __launch_bounds__(kLocalThreads, 1) local_dispatch_kernel(const 
                 ptx::nanosleep(64);
     }
     if (!failed) {
-        if (expand && a.zero_padding) {  // rows between the experts' segments
-            for (int el = b * kLocalWarps + warp; el < E; el += G * kLocalWarps) {
-                for (int row = eoff[el] + total[el]; row < eoff[el + 1]; ++row) {
+        // Rows between the experts' segments: experts go round the CTAs, their rows round the warps.  (A warp per expert, CTA after
+        // CTA, left them to a few SMs: 64 tokens, 32 experts, top-8, hidden 7168, padded to multiples of 256 907 us, now 76;
+        // the general kernel, a warp per channel, 148.)
+        if (expand && a.zero_padding) {
+            for (int el = b; el < E; el += G) {
+                for (int row = eoff[el] + total[el] + warp; row < eoff[el + 1]; row += kLocalWarps) {
                     if (recv_fp8) {
                         for (int x = lane; x < H; x += 32) recv_bytes[static_cast<std::size_t>(row) * H + x] = 0;
                         if (lane == 0) a.recv_scale[row] = 0.0f;

@@ -93,6 +93,10 @@ LocalPlan plan_dispatch_local(const SegmentLayout& lay, int sms, std::size_t sme
 
 std::size_t dispatch_local_hist_ints(const SegmentLayout& lay, int ctas) { return local_hist_ints(ctas, lay.num_experts, lay.num_channels); }
 
+int dispatch_local_width(const SegmentLayout& lay, int tokens, bool padding) {
+    return padding && tokens > 0 ? std::max(tokens, lay.num_experts) : tokens;
+}
+
 cudaError_t launch_dispatch_local(const DispatchArgs& a, const RankConst& rc, const LocalPlan& plan, int* hist, unsigned long long* counters, int sms, int max_ctas, cudaStream_t stream) {
     static std::mutex mutex;
     static std::size_t configured[64] = {0};
@@ -110,7 +114,7 @@ cudaError_t launch_dispatch_local(const DispatchArgs& a, const RankConst& rc, co
     }
     LocalDispatchArgs args{a, plan, hist, counters, sms, rc.lay.num_experts, rc.lay.num_channels, rc.lay.num_topk, rc.lay.hidden,
                            rc.lay.slots_full, rc.expanded_cap, rc.unique_cap, rc.recv_fp8};
-    const int ctas = std::max(1, std::min(std::min(sms, max_ctas), a.num_tokens));
+    const int ctas = std::max(1, std::min(std::min(sms, max_ctas), dispatch_local_width(rc.lay, a.num_tokens, a.do_expand && a.zero_padding && a.alignment > 1)));
     // a fresh layout has a grid barrier and needs every CTA resident; with a cached one no CTA waits for another
     if (!a.cached) return cooperative_launch(local_dispatch_kernel, args, dim3(ctas), kLocalThreads, plan.bytes, stream);
     local_dispatch_kernel<<<ctas, kLocalThreads, plan.bytes, stream>>>(args);

@@ -203,7 +203,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         .def("accepts_rows", &Runtime::accepts_rows, py::arg("y"), py::arg("dispatch_result"))
         .def("combine_is_split", &Runtime::combine_is_split)
         .def("combine_is_local", &Runtime::combine_is_local)
-        .def("dispatch_differs_beside_compute", &Runtime::dispatch_differs_beside_compute, py::arg("tokens"))
+        .def("dispatch_differs_beside_compute", &Runtime::dispatch_differs_beside_compute, py::arg("tokens"), py::arg("padding"))
         .def("dispatch_is_local", &Runtime::dispatch_is_local)
         .def("combine_is_inline", &Runtime::combine_is_inline)
         .def("send_stages", &Runtime::send_stages)

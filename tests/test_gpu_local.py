@@ -345,3 +345,49 @@ def test_combine_refuses_outputs_that_its_stores_do_not_fit(one_rank):
             assert torch.equal(call(room[8:].view(tokens, hidden))[0], want) and float(want.float().abs().max()) > 0
         buffer.check_errors(handle)
         del recv_x, handle
+
+
+def median_us(call, repeats=7, calls=5):
+    times = []
+    for _ in range(repeats):
+        begin, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        torch.cuda._sleep(2_000_000)  # the launches are queued behind it
+        begin.record()
+        for _ in range(calls):
+            call()
+        end.record()
+        torch.cuda.synchronize()
+        times.append(begin.elapsed_time(end) * 1000 / calls)
+    return sorted(times)[repeats // 2]
+
+
+@pytest.mark.parametrize("cached", [False, True])
+@pytest.mark.parametrize("tokens,alignment,fp8", [(3, 256, False), (64, 256, False), (1000, 128, True)])
+def test_zeroing_padding_rows_is_spread_over_the_sms(one_rank, tokens, alignment, fp8, cached):
+    """The rows between the experts' segments are zero, and zeroing them takes no longer than in the general kernel (a third
+    on top for the spread between measurements; a few SMs doing it take three to six times as long)."""
+    from pcie_ep_b200 import HostStagedConfig, HostStagedEPBuffer
+
+    wire = "fp8_e4m3" if fp8 else "bf16"
+    config = HostStagedConfig(stage=7 if fp8 else 6, channels=32, wire_dtype=wire, recv_dtype=wire)
+    with HostStagedEPBuffer(one_rank, tokens, 7168, 8, 32, config) as buffer:
+        x = torch.randn(tokens, 7168).to(torch.bfloat16).cuda()
+        idx = torch.rand(tokens, 32).topk(8, dim=1).indices.cuda()
+        routes = dict(handle=buffer.cache_layout(buffer.dispatch(x, idx, do_expand=True, expert_alignment=alignment)[3])) if cached else dict(topk_idx=idx)
+
+        def dispatch():
+            return buffer.dispatch(x, do_expand=True, expert_alignment=alignment, do_zero_padding=True, **routes)
+
+        for _ in range(config.output_pool_size):  # whatever set of results comes next holds no zeros
+            dispatch()[0].view(torch.uint8).fill_(7)
+        got = dispatch()
+        buffer.check_errors(got[3])
+        rows = int(got[3].expert_offsets[-1])
+        padding = got[3].source_meta[:rows, 1] < 0
+        assert int(padding.sum()) == rows - tokens * 8 and int(got[0][:rows][padding].view(torch.uint8).max()) == 0
+        assert bool((got[1][:rows][padding] == -1).all()) and float(got[3]._result["recv_topk_weights"][:rows][padding].abs().max()) == 0.0
+        del got
+        local = median_us(dispatch)
+        buffer.runtime.set_test_prefix_delay_ns(1)  # the general kernel takes the call
+        general = median_us(dispatch)
+        assert local <= general * 4 / 3, (local, general)
