@@ -51,7 +51,11 @@ struct CombineLocalArgs {
 constexpr int kCombineLocalMaxStages = 8;
 constexpr int kCombineLocalConsumers = 14;  // warps that add, behind the producer warp: 448 threads, half a row of 7168
 constexpr int kCombineLocalThreads = 32 * (1 + kCombineLocalConsumers);
-constexpr int kCombineLocalSmallStage = 32 * 1024;  // stages up to this size: units are claimed four at a time, given a dozen per CTA
+// Units whose stage is at most this large are claimed four at a time, given a dozen per CTA: a claim and the map entries behind
+// it are a latency that four units share, 8192 tokens with six rows each 0.9 us a unit at 30 KB (hidden 2560, 68 us) and 1.6
+// claimed singly at 34 KB (hidden 2880, 95 us).  Larger units take that long to read anyway (7 stages of 32 KB are in flight),
+// and four of them in one CTA would be an uneven end.
+constexpr int kCombineLocalSmallStage = 32 * 1024;
 
 struct CombineLocalHeader {
     int token, n, first_chunk, chunks;  // n < 0: no more units

@@ -19,7 +19,7 @@ UNSUPPORTED_DISPATCH_KEYWORDS = (
     ("do_cpu_sync", "dispatch never waits on the CPU; sizes stay on the device (do_cpu_sync must be False)"),
     ("do_handle_copy", "handles are not copied; cache_layout() detaches a routing plan instead"),
     ("num_qps", "there are no queue pairs on this transport"),
-    ("num_sms", "the dispatch grid is fixed by the buffer's channel count; num_sms cannot override it"),
+    ("num_sms", "the dispatch grid follows from the buffer's channels (with one rank, on the caller's stream: from the GPU's SMs); num_sms cannot override it"),
     ("use_tma_aligned_col_major_sf", "scale factors are one FP32 per row; no column-major layout exists"),
 )
 
