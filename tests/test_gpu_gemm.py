@@ -86,3 +86,47 @@ def test_grouped_gemm_fp8_matches_dequantised_reference(ext, swiglu):
     scale = float(want[valid].abs().max())
     assert torch.allclose(got[valid], want[valid], rtol=2e-2, atol=1e-2 * scale), (got[valid] - want[valid]).abs().max()
     assert (got[~valid] == 7.0).all()
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("swiglu,n", [(True, 256), (False, 256), (False, 128)])
+def test_last_tiles_at_the_box_heights(ext, fp8, swiglu, n):
+    """Experts whose last tile ends at, before and behind the heights of the activation boxes (32, 64, 128 rows).  The rows
+    around an expert's own hold NaN: what shares a box with it must not reach its results, nor be written."""
+    counts = [31, 32, 33, 0, 63, 64, 65, 127, 128, 1, 128 + 32, 128 + 33, 128 + 64, 128 + 65]
+    k, experts = 384, len(counts)
+    offsets = torch.zeros(experts + 1, dtype=torch.int32)
+    for e, c in enumerate(counts):
+        offsets[e + 1] = offsets[e] + c + (1, 40, 0, 7)[e % 4]  # rows between the experts: none, few, more than a box
+    rows = int(offsets[-1]) + 5
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    a = torch.randn(rows, k, device="cuda", generator=gen).to(torch.bfloat16)
+    own = torch.zeros(rows, dtype=torch.bool, device="cuda")
+    for e, c in enumerate(counts):
+        own[int(offsets[e]):int(offsets[e]) + c] = True
+    a[~own] = float("nan")
+    w = (torch.randn(experts, (2 if swiglu else 1) * n, k, device="cuda", generator=gen) * 0.1).to(torch.bfloat16)
+    scales = {}
+    if fp8:
+        a, w = a.to(torch.float8_e4m3fn), w.to(torch.float8_e4m3fn)
+        scales = dict(a_scales=torch.rand(rows, device="cuda", generator=gen) + 0.5, w_scales=torch.rand(w.shape[:2], device="cuda", generator=gen) + 0.5)
+    out = torch.full((rows, n), 7.0, dtype=torch.bfloat16, device="cuda")
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    grouped_gemm(a, w, offsets.cuda(), torch.tensor(counts, dtype=torch.int32, device="cuda"), swiglu=swiglu, out=out, status=status, **scales)
+    torch.cuda.synchronize()
+    assert status.tolist() == [0, 0, 0, 0] and bool((out[~own] == 7.0).all())
+    for e, c in enumerate(counts):
+        at = slice(int(offsets[e]), int(offsets[e]) + c)
+        x, m = a[at].double(), w[e].double()
+        if fp8:
+            x, m = x * scales["a_scales"][at].double().unsqueeze(1), m * scales["w_scales"][e].double().unsqueeze(1)
+        want = x @ m.t()
+        # K products summed in 32 bits (and two scale factors): relative to the sum of their magnitudes
+        error = (x.abs() @ m.abs().t()) * (k + 4) * 2.0 ** -24
+        if swiglu:
+            gate, up = want[:, :n], want[:, n:]
+            silu = torch.nn.functional.silu(gate)
+            # |silu'| < 1.1; the fast exponential is good to 2 + 1.2 |gate| units in the last of 24 bits
+            error = 1.1 * error[:, :n] * up.abs() + silu.abs() * error[:, n:] + (silu * up).abs() * (8 + 2 * gate.abs()) * 2.0 ** -24
+            want = silu * up
+        assert bool(((out[at].double() - want).abs() <= error + (want.abs() + error) * 2.0 ** -8).all()), counts[e]

@@ -391,3 +391,52 @@ def test_zeroing_padding_rows_is_spread_over_the_sms(one_rank, tokens, alignment
         buffer.runtime.set_test_prefix_delay_ns(1)  # the general kernel takes the call
         general = median_us(dispatch)
         assert local <= general * 4 / 3, (local, general)
+
+
+def assert_same_result(got, want, rows, channels, fp8):
+    """Every field, the rows in use and the combine map's entries of two dispatch results."""
+    for field in FIELDS:
+        assert torch.equal(got[3]._result[field], want[3]._result[field]), field
+    for mine, theirs in zip(got[:3], want[:3]):
+        assert torch.equal(mine[:rows].view(torch.uint8), theirs[:rows].view(torch.uint8))
+    assert torch.equal(got[3].source_meta[:rows], want[3].source_meta[:rows])
+    if fp8:
+        assert torch.equal(got[3]._result["recv_x_scales"][:rows], want[3]._result["recv_x_scales"][:rows])
+    mine, theirs = (r[3]._result["comb_map"].view(channels, -1, r[3]._result["comb_map"].shape[1]) for r in (got, want))
+    exists = torch.arange(theirs.shape[1], device="cuda") < want[3]._result["recv_chan_counts"].view(-1, 1)
+    words = torch.arange(theirs.shape[2], device="cuda") < 2 + 2 * theirs[:, :, 1:2]
+    assert torch.equal(mine[exists.unsqueeze(2) & words], theirs[exists.unsqueeze(2) & words])
+
+
+@pytest.mark.parametrize("tokens,capacity,experts,topk,hidden,channels,fp8,expand,alignment", CASES)
+def test_plans_of_both_kernels_are_the_same(one_rank, tokens, capacity, experts, topk, hidden, channels, fp8, expand, alignment):
+    """A plan that either kernel has written gives the same results in either kernel when it is used again."""
+    from pcie_ep_b200 import HostStagedConfig, HostStagedEPBuffer
+
+    gen = torch.Generator(device="cuda").manual_seed(tokens + topk)
+    x = torch.randn(tokens, hidden, device="cuda", generator=gen).to(torch.bfloat16)
+    idx = torch.rand(tokens, experts, device="cuda", generator=gen).topk(topk, dim=1).indices
+    idx[torch.rand(tokens, topk, device="cuda", generator=gen) < 0.2] = -1
+    w = torch.rand(tokens, topk, device="cuda", generator=gen)
+    wire = "fp8_e4m3" if fp8 else "bf16"
+    config = HostStagedConfig(stage=7 if fp8 else 6, channels=channels, wire_dtype=wire, recv_dtype=wire, output_pool_size=5)
+    options = dict(do_expand=expand, expert_alignment=alignment, do_zero_padding=expand)
+    with HostStagedEPBuffer(one_rank, capacity, hidden, topk, experts, config) as buffer:
+        def dispatch(general, *args, **more):
+            buffer.runtime.set_test_prefix_delay_ns(1 if general else 0)  # a hook of the protocol: the general kernel takes the call
+            assert buffer.runtime.dispatch_is_local() != general
+            return buffer.dispatch(x, *args, topk_weights=w, **options, **more)
+
+        want = dispatch(True, idx)
+        buffer.check_errors(want[3])
+        rows = int(want[3].expert_offsets[-1]) if expand else int(want[3].unique_count[0])
+        for written_by_general in (False, True):
+            fresh = dispatch(written_by_general, idx)
+            plan = buffer.cache_layout(fresh[3])
+            for used_by_general in (False, True):
+                got = dispatch(used_by_general, handle=plan)
+                buffer.check_errors(got[3])
+                assert_same_result(got, want, rows, channels, fp8)
+                del got
+            del fresh, plan
+        del want
