@@ -2,7 +2,6 @@
 #include "expert_gemm.cuh"
 
 #include <mutex>
-#include <type_traits>
 
 #include "expert_gemm.hpp"
 #include "ptx.cuh"
@@ -18,9 +17,6 @@ __device__ __forceinline__ std::uint32_t smem_addr(const void* p) {
 }
 __device__ __forceinline__ void mbar_init(std::uint64_t* bar, unsigned count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(std::uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
 __device__ __forceinline__ void mbar_expect_tx(std::uint64_t* bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
@@ -46,49 +42,74 @@ __device__ __forceinline__ bool mbar_wait(std::uint64_t* bar, unsigned parity, v
     return false;
 }
 
-// 2-D tiled TMA load, no multicast: box lands in shared memory with the tensor map's swizzle
-__device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, int x, int y, std::uint64_t* bar) {
+// address of the same shared-memory location in CTA `rank` of the cluster
+__device__ __forceinline__ std::uint32_t cluster_addr(const void* p, unsigned rank) {
+    std::uint32_t remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_addr(p)), "r"(rank));
+    return remote;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(std::uint32_t bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Tiled TMA loads, no multicast: the box lands in this CTA's shared memory with the tensor map's swizzle, its bytes are
+// counted on `bar`, which may be the other CTA's of the pair.
+__device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, int x, int y, std::uint32_t bar) {
     asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-        ::"r"(smem_addr(smem_dst)), "l"(reinterpret_cast<std::uint64_t>(map)), "r"(x), "r"(y), "r"(smem_addr(bar))
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+        ::"r"(smem_addr(smem_dst)), "l"(reinterpret_cast<std::uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_5d(void* smem_dst, const CUtensorMap* map, int x, int group, int expert, std::uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %3, %4, %5}], [%6];"
+        ::"r"(smem_addr(smem_dst)), "l"(reinterpret_cast<std::uint64_t>(map)), "r"(x), "r"(0), "r"(group), "r"(expert), "r"(bar)
         : "memory");
 }
 
 __device__ __forceinline__ void tmem_alloc(std::uint32_t* smem_result, unsigned columns) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(smem_result)), "r"(columns)
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(smem_result)), "r"(columns)
                  : "memory");
 }
 __device__ __forceinline__ void tmem_relinquish() {
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tmem_dealloc(std::uint32_t taddr, unsigned columns) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(columns) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(columns) : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// D[tmem] (+)= A[smem desc] * B[smem desc]; one thread issues for the CTA
-__device__ __forceinline__ void umma_f16(std::uint32_t tmem_d, std::uint64_t desc_a, std::uint64_t desc_b,
-                                         std::uint32_t idesc, std::uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-        : "memory");
+// D[tmem of both CTAs] (+)= A[smem desc] * B[smem desc]; one thread of the leading CTA issues for the pair
+template <bool kFp8>
+__device__ __forceinline__ void umma(std::uint32_t tmem_d, std::uint64_t desc_a, std::uint64_t desc_b, std::uint32_t idesc, std::uint32_t accumulate) {
+    if constexpr (kFp8)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
+            ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+            ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+            : "memory");
 }
-__device__ __forceinline__ void umma_f8(std::uint32_t tmem_d, std::uint64_t desc_a, std::uint64_t desc_b,
-                                        std::uint32_t idesc, std::uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// all MMAs issued so far by this thread arrive on `bar` when they have completed
-__device__ __forceinline__ void umma_commit(std::uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar))
+// all MMAs issued so far by this thread arrive on `bar` of both CTAs when they have completed
+__device__ __forceinline__ void umma_commit_pair(std::uint64_t* bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_addr(bar)),
+                 "h"(static_cast<std::uint16_t>(3))
                  : "memory");
 }
 // 32 lanes x 32 columns of FP32 out of TMEM: thread i gets columns [c, c+32) of lane (base lane + i)
@@ -103,7 +124,40 @@ __device__ __forceinline__ void tmem_ld_32x32(std::uint32_t taddr, std::uint32_t
         : "r"(taddr)
         : "memory");
 }
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// (the registers pass through, so that nothing reads or copies them before the loads have arrived)
+__device__ __forceinline__ void tmem_ld_wait(std::uint32_t (&r)[32]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]),
+                   "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]), "+r"(r[16]),
+                   "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), "+r"(r[24]),
+                   "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])::"memory");
+}
+
+// a / b for b >= 1 (or infinite): one correction of a * (1 / b) by its remainder (Markstein, "Computation of elementary functions on
+// the IBM RISC System/6000 processor", 1990).  Where the remainder is no number (an infinite operand) the product is the answer.
+// No branch, so that the quotients of a chunk overlap: with the operator a warp took them one after the other and the epilogue of a
+// tile longer than its MMAs where K is 2048 (2000 tokens, intermediate 768: 118 -> 95 us) or the operands are E4M3 (849 -> 749).
+__device__ __forceinline__ float quotient(float a, float b) {
+    float r;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(b));
+    const float q = a * r, remainder = fmaf(-q, b, a);
+    return remainder == remainder ? fmaf(remainder, r, q) : q;
+}
+
+// barrier among the four epilogue warps; true when `ok` held in all of them
+__device__ __forceinline__ bool epilogue_all(bool ok) {
+    std::uint32_t all;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "barrier.cta.red.and.pred.aligned q, 1, 128, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(all)
+        : "r"(static_cast<std::uint32_t>(ok))
+        : "memory");
+    return all != 0;
+}
+__device__ __forceinline__ void epilogue_sync() { asm volatile("barrier.cta.sync.aligned 1, 128;" ::: "memory"); }
 
 // Shared-memory matrix descriptor of a K-major tile whose rows are 128 bytes (64 bf16) wide, stored
 // with the 128-byte swizzle TMA applied: 8-row groups are 1024 bytes apart (stride byte offset), the
@@ -120,210 +174,188 @@ __device__ __forceinline__ std::uint64_t make_smem_desc(const void* tile) {
     return desc;
 }
 
-// Instruction descriptor, kind::f16: D = F32, A = B = BF16, both K-major, N and M encoded /8 and /16.
-__host__ __device__ constexpr std::uint32_t make_idesc_bf16(int m, int n) {
+// Instruction descriptor, D = F32, both operands K-major, N and M encoded /8 and /16; kind::f16 with A = B = BF16, or
+// kind::f8f6f4 with E4M3 operands (format code 0 for both).
+template <bool kFp8>
+__host__ __device__ constexpr std::uint32_t make_idesc(int m, int n) {
     return (1u << 4)                                   // D format: F32
-           | (1u << 7)                                 // A format: BF16
-           | (1u << 10)                                // B format: BF16
+           | (kFp8 ? 0u : (1u << 7) | (1u << 10))      // A and B format: BF16
            | (static_cast<std::uint32_t>(n >> 3) << 17)
            | (static_cast<std::uint32_t>(m >> 4) << 24);
 }
 
-// kind::f8f6f4 with E4M3 operands (format code 0 for both), FP32 accumulation
-__host__ __device__ constexpr std::uint32_t make_idesc_e4m3(int m, int n) {
-    return (1u << 4) | (static_cast<std::uint32_t>(n >> 3) << 17) | (static_cast<std::uint32_t>(m >> 4) << 24);
-}
+// Walks every pairs-th tile in the order expert, channel tile, row chunk, so that tiles which run at the same time share a weight tile.
+struct TileWalk {
+    int tile, pairs, m_tiles;
+    int next_expert = 0, rows = 0, first_row = 0, first_tile = 0, end_tile = 0;  // of the present expert
+    RowChunks chunks{0, 0};
+    // the present tile: channel tile, row chunk, first row of the activations, valid rows
+    int expert = 0, m_tile = 0, chunk = 0, row0 = 0, tile_rows = 0;
 
-struct TileCursor {
-    // walks tiles in (expert, n-tile, m-tile) order: consecutive tiles share the weight tile
-    int expert = 0;
-    int first_tile = 0;  // index of the expert's first tile
-    int m_tiles = 0;
+    __device__ __forceinline__ explicit TileWalk(int m_tiles_) : tile(blockIdx.x >> 1), pairs(gridDim.x >> 1), m_tiles(m_tiles_) {}
 
-    __device__ __forceinline__ bool locate(int tile, const GroupedGemmParams& p, int n_tiles, int& m_tile, int& n_tile) {
-        while (expert < p.num_experts) {
-            m_tiles = (p.expert_counts[expert] + kBlockM - 1) / kBlockM;
-            const int tiles_here = m_tiles * n_tiles;
-            if (tile < first_tile + tiles_here) {
-                const int local = tile - first_tile;
-                n_tile = local / m_tiles;
-                m_tile = local % m_tiles;
-                return true;
-            }
-            first_tile += tiles_here;
-            ++expert;
+    __device__ __forceinline__ bool next(const GroupedGemmParams& p) {
+        while (tile >= end_tile) {
+            if (next_expert >= p.num_experts) return false;
+            expert = next_expert++;
+            rows = p.expert_counts[expert];
+            chunks = row_chunks(rows);
+            first_tile = end_tile;
+            end_tile += chunks.count * m_tiles;
+            first_row = p.expert_offsets[expert];
         }
-        return false;
+        const int local = tile - first_tile;
+        m_tile = local / chunks.count;
+        chunk = local - m_tile * chunks.count;
+        row0 = first_row + chunk * chunks.rows;
+        tile_rows = min(chunks.rows, rows - chunk * chunks.rows);
+        tile += pairs;
+        return true;
     }
 };
 
 }  // namespace
 
-// kBoxesB: 128-row weight boxes per stage.  Two boxes land back to back in shared memory and feed ONE
-// tcgen05.mma of N = 256 (A is read from shared memory once per 256 output columns): for SwiGLU they are
-// the gate and the up rows of the same 128 output columns, for the plain GEMM 256 adjacent output columns.
-template <bool kSwiGLU, bool kFp8, int kBoxesB, bool kScatter>
-__global__ void __launch_bounds__(kThreads, 1)
-grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_a, const __grid_constant__ CUtensorMap map_b,
+// Launch bounds: at most 128 registers, so that a reducer CTA of the combine (combine_push.cuh) finds room on this CTA's SM.
+template <bool kSwiGLU, bool kFp8, bool kScatter>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 2)
+grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_rows, const __grid_constant__ CUtensorMap map_w,
                     const GroupedGemmParams p) {
-    static_assert(kBoxesB == 2 || !kSwiGLU, "SwiGLU stages carry the gate and the up box");
-    static_assert(!kScatter || (kBoxesB == 2 && !kSwiGLU && !kFp8), "the scatter epilogue exists for the plain BF16 256-column tile");
-    using Plan = SmemPlan<kBoxesB>;
-    constexpr int kStages = Plan::kStages;
-    constexpr int kAccCols = kBoxesB * kBlockN;   // TMEM columns of one accumulator set = N of one MMA
-    constexpr int kTmemCols = 2 * kAccCols;       // double buffered: 256 or 512 (powers of two)
-    constexpr int kOutN = kSwiGLU ? kBlockN : kAccCols;  // output columns of one tile
+    static_assert(!kScatter || (!kSwiGLU && !kFp8), "the scatter epilogue exists for the plain BF16 GEMM");
+    constexpr int kElemBytes = kFp8 ? 1 : 2;
+    constexpr int kBlockK = kBlockKBytes / kElemBytes;  // elements of K per stage
+    constexpr int kChannels = kSwiGLU ? kCtaM / 2 : kCtaM;  // output channels of one CTA in a tile
+    constexpr int kPitch = staging_pitch(kSwiGLU);
 
     extern __shared__ __align__(1024) unsigned char smem_unaligned[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<std::uintptr_t>(smem_unaligned) + 1023) & ~std::uintptr_t(1023));
-    if (kScatter) {
-        // the scatter variant asks for less alignment slack than the worst case: refuse (uniformly) instead of overrunning
-        std::uint32_t dynamic_bytes;
-        asm volatile("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dynamic_bytes));
-        const std::uint32_t needed = static_cast<std::uint32_t>(smem - smem_unaligned) + kStages * Plan::kStageBytes + 256 + kScatterStagingBytes;
-        if (needed > dynamic_bytes) {
-            if (threadIdx.x == 0) atomicExch(&p.status[0], 2);
-            return;
-        }
-    }
-    unsigned char* staging = smem + kStages * Plan::kStageBytes + 256;
     unsigned char* tiles = smem;
-    std::uint64_t* full_bar = reinterpret_cast<std::uint64_t*>(smem + kStages * Plan::kStageBytes);
-    std::uint64_t* empty_bar = full_bar + kStages;
-    std::uint64_t* tmem_full = empty_bar + kStages;
-    std::uint64_t* tmem_empty = tmem_full + 2;
-    std::uint32_t* tmem_ptr = reinterpret_cast<std::uint32_t*>(tmem_empty + 2);
-    volatile int* abort = reinterpret_cast<volatile int*>(tmem_ptr + 1);
+    unsigned char* staging = smem + kRingBytes;
+    auto* sh = reinterpret_cast<GemmShared*>(staging + 2 * kChunkRows * kPitch);
+    volatile int* abort = &sh->abort;
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    constexpr int kElemBytes = kFp8 ? 1 : 2;
-    constexpr int kBlockK = kBlockKBytes / kElemBytes;  // elements of K per stage
-    const int n_tiles = p.n / kOutN;
+    const unsigned rank = cluster_rank();
     const int k_blocks = p.k / kBlockK;
-    const int w_rows_per_expert = kSwiGLU ? 2 * p.n : p.n;
-    // gate/up tiles with few rows swap the operands (see ActivationMaps)
-    auto flips = [](int box) { return kSwiGLU && box != kBoxesA - 1; };
+    const int m_tiles = (p.n + 2 * kChannels - 1) / (2 * kChannels);
 
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < kStages; ++s) {
-            mbar_init(&full_bar[s], 1);
-            mbar_init(&empty_bar[s], 1);
+    if (warp == 0 && lane < kBoxes + 1) {
+        const CUtensorMap* map = lane < kBoxes ? &maps_rows.box[lane] : &map_w;
+        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<std::uint64_t>(map)) : "memory");
+    }
+    if (threadIdx.x == 64) {
+        for (int s = 0; s < kMaxStages; ++s) {
+            mbar_init(&sh->full[s], 1);
+            mbar_init(&sh->empty[s], 1);
         }
         for (int b = 0; b < 2; ++b) {
-            mbar_init(&tmem_full[b], 1);
-            mbar_init(&tmem_empty[b], 4);
+            mbar_init(&sh->tmem_full[b], 1);
+            mbar_init(&sh->tmem_empty[b], 8);
         }
         *abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
-        tmem_alloc(tmem_ptr, kTmemCols);
+        tmem_alloc(&sh->tmem_base, kTmemCols);
         tmem_relinquish();
     }
+    int most_rows = 1;  // of any expert
+    for (int e = threadIdx.x; e < p.num_experts; e += kThreads) most_rows = max(most_rows, p.expert_counts[e]);
+    most_rows = __reduce_max_sync(0xffffffffu, most_rows);
+    if (lane == 0) sh->most_rows[warp] = most_rows;
     tc_fence_before();
     __syncthreads();
+    cluster_sync();  // barriers of both CTAs are ready before either names the other's
     tc_fence_after();
-    const std::uint32_t tmem_base = *tmem_ptr;
+    const std::uint32_t tmem_base = sh->tmem_base;
+    for (int w = 0; w < kThreads / 32; ++w) most_rows = max(most_rows, sh->most_rows[w]);
+    const int stage_bytes = kTileW + box_rows(box_of_rows(min(most_rows, kMaxRows))) * kBlockKBytes;
+    const int stages = min(kMaxStages, kRingBytes / stage_bytes);
+    TileWalk walk(m_tiles);
 
     if (warp == 0) {
-        // ===== TMA producer =====
+        // ===== TMA producer: this CTA's 128 weight rows and its half of the activation rows =====
         if (lane == 0) {
-            TileCursor cursor;
             int stage = 0;
             unsigned phase = 0;
             bool ok = true;
-            for (int tile = blockIdx.x; ok; tile += gridDim.x) {
-                int m_tile, n_tile;
-                if (!cursor.locate(tile, p, n_tiles, m_tile, n_tile)) break;
-                const int row0 = p.expert_offsets[cursor.expert] + m_tile * kBlockM;
-                const int wrow0 = cursor.expert * w_rows_per_expert + n_tile * kOutN;
-                const int wrow1 = wrow0 + (kSwiGLU ? p.n : kBlockN);
-                // a tile with few valid rows loads only those (rows of the box beyond them are never written out)
-                const int box = box_of_rows(p.expert_counts[cursor.expert] - m_tile * kBlockM);
-                const CUtensorMap* map_a = &maps_a.box[box];
-                const unsigned stage_bytes = static_cast<unsigned>(Plan::kStageBytes - Plan::kTileA + box_rows_a(box) * kBlockKBytes);
+            while (ok && walk.next(p)) {
+                const int box = box_of_rows(walk.tile_rows);
+                const int half = box_rows(box);
+                const CUtensorMap* map_rows = &maps_rows.box[box];
+                const int row = walk.row0 + static_cast<int>(rank) * half;
+                const unsigned pair_bytes = 2u * static_cast<unsigned>(kTileW + half * kBlockKBytes);
+                const int group = (walk.m_tile * 2 + static_cast<int>(rank)) * (kChannels / 16);
+                const int wrow = walk.expert * p.n + (walk.m_tile * 2 + static_cast<int>(rank)) * kCtaM;
                 for (int kb = 0; kb < k_blocks; ++kb) {
-                    if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort)) {
+                    if (!mbar_wait(&sh->empty[stage], phase ^ 1u, abort)) {
                         ok = false;
                         break;
                     }
-                    unsigned char* stage_base = tiles + stage * Plan::kStageBytes;
-                    mbar_expect_tx(&full_bar[stage], stage_bytes);
-                    tma_load_2d(stage_base, map_a, kb * kBlockK, row0, &full_bar[stage]);
-                    tma_load_2d(stage_base + Plan::kTileA, &map_b, kb * kBlockK, wrow0, &full_bar[stage]);
-                    if (kBoxesB == 2)
-                        tma_load_2d(stage_base + Plan::kTileA + Plan::kTileB, &map_b, kb * kBlockK, wrow1, &full_bar[stage]);
-                    if (++stage == kStages) {
+                    unsigned char* stage_base = tiles + stage * stage_bytes;
+                    if (rank == 0) mbar_expect_tx(&sh->full[stage], pair_bytes);
+                    const std::uint32_t bar = cluster_addr(&sh->full[stage], 0);
+                    if (kSwiGLU) tma_load_5d(stage_base, &map_w, kb * kBlockK, group, walk.expert, bar);
+                    else tma_load_2d(stage_base, &map_w, kb * kBlockK, wrow, bar);
+                    tma_load_2d(stage_base + kTileW, map_rows, kb * kBlockK, row, bar);
+                    if (++stage == stages) {
                         stage = 0;
                         phase ^= 1u;
                     }
                 }
             }
+            // the other roles have taken every stage (and the leading CTA's commits have arrived here) before this CTA ends
+            for (int i = 0; ok && i < stages; ++i) {
+                ok = mbar_wait(&sh->empty[stage], phase ^ 1u, abort);
+                if (++stage == stages) {
+                    stage = 0;
+                    phase ^= 1u;
+                }
+            }
+            // gave up: what is still on its way gets time to land before shared memory goes away
+            if (!ok)
+                for (int i = 0; i < 1000; ++i) ptx::nanosleep(1000);
         }
     } else if (warp == 1) {
-        // ===== MMA issuer =====
-        if (lane == 0) {
-            TileCursor cursor;
+        // ===== MMA issuer of the pair =====
+        if (lane == 0 && rank == 0) {
             int stage = 0;
             unsigned phase = 0;
             bool ok = true;
             int it = 0;
-            // The K loop exists once per box height: with the operand order and the instruction descriptor chosen at run time
-            // inside it, every tile was 28 % slower.  kBox = kBoxesA - 1: not swapped.
-            auto multiply = [&](auto box, std::uint32_t acc) {
-                constexpr int kBox = decltype(box)::value;
-                constexpr bool kFlip = kBox != kBoxesA - 1;
-                constexpr int kM = kFlip ? kBlockN : kBlockM, kN = kFlip ? box_rows_a(kBox) : kAccCols;
-                constexpr std::uint32_t idesc = kFp8 ? make_idesc_e4m3(kM, kN) : make_idesc_bf16(kM, kN);
+            for (; ok && walk.next(p); ++it) {
+                const int buf = it & 1;
+                const unsigned acc_phase = (it >> 1) & 1u;
+                if (!mbar_wait(&sh->tmem_empty[buf], acc_phase ^ 1u, abort)) break;
+                tc_fence_after();
+                const std::uint32_t acc = tmem_base + buf * kAccCols;
+                const std::uint32_t idesc = make_idesc<kFp8>(2 * kCtaM, 2 * box_rows(box_of_rows(walk.tile_rows)));
                 for (int kb = 0; kb < k_blocks; ++kb) {
-                    if (!mbar_wait(&full_bar[stage], phase, abort)) {
+                    if (!mbar_wait(&sh->full[stage], phase, abort)) {
                         ok = false;
-                        return;
+                        break;
                     }
                     tc_fence_after();
-                    unsigned char* stage_base = tiles + stage * Plan::kStageBytes;
-                    const std::uint64_t desc_a = make_smem_desc(stage_base);
-                    // the B boxes are contiguous: 8-row groups stay 1024 bytes apart across the box boundary
-                    const std::uint64_t desc_b = make_smem_desc(stage_base + Plan::kTileA);
+                    const std::uint64_t desc_w = make_smem_desc(tiles + stage * stage_bytes);
+                    const std::uint64_t desc_rows = make_smem_desc(tiles + stage * stage_bytes + kTileW);
 #pragma unroll
                     for (int k = 0; k < kBlockKBytes / kUmmaKBytes; ++k) {
                         // 32 bytes further along K inside the swizzle atom: +2 in the address field
                         const std::uint64_t step = static_cast<std::uint64_t>(k * kUmmaKBytes) >> 4;
-                        const std::uint32_t accumulate = (kb | k) != 0 ? 1u : 0u;
-#pragma unroll
-                        for (int bx = 0; bx < (kFlip ? kBoxesB : 1); ++bx) {
-                            const std::uint64_t first = kFlip ? desc_b + step + (static_cast<std::uint64_t>(bx * Plan::kTileB) >> 4) : desc_a + step;
-                            const std::uint64_t second = kFlip ? desc_a + step : desc_b + step;
-                            if (kFp8) umma_f8(acc + bx * kBlockN, first, second, idesc, accumulate);
-                            else umma_f16(acc + bx * kBlockN, first, second, idesc, accumulate);
-                        }
+                        umma<kFp8>(acc, desc_w + step, desc_rows + step, idesc, (kb | k) != 0 ? 1u : 0u);
                     }
-                    umma_commit(&empty_bar[stage]);  // the stage is free once these MMAs have read it
-                    if (++stage == kStages) {
+                    umma_commit_pair(&sh->empty[stage]);  // the stage is free in both CTAs once these MMAs have read it
+                    if (++stage == stages) {
                         stage = 0;
                         phase ^= 1u;
                     }
                 }
-            };
-            for (int tile = blockIdx.x; ok; tile += gridDim.x, ++it) {
-                int m_tile, n_tile;
-                if (!cursor.locate(tile, p, n_tiles, m_tile, n_tile)) break;
-                const int buf = it & 1;
-                const unsigned acc_phase = (it >> 1) & 1u;
-                if (!mbar_wait(&tmem_empty[buf], acc_phase ^ 1u, abort)) break;
-                tc_fence_after();
-                const std::uint32_t acc = tmem_base + buf * kAccCols;
-                const int box = box_of_rows(p.expert_counts[cursor.expert] - m_tile * kBlockM);
-                if constexpr (!kSwiGLU) multiply(std::integral_constant<int, kBoxesA - 1>{}, acc);
-                else if (!flips(box)) multiply(std::integral_constant<int, kBoxesA - 1>{}, acc);
-                else if (box == 0) multiply(std::integral_constant<int, 0>{}, acc);
-                else multiply(std::integral_constant<int, 1>{}, acc);
-                if (ok) umma_commit(&tmem_full[buf]);
+                if (ok) umma_commit_pair(&sh->tmem_full[buf]);
             }
         }
     } else {
-        // ===== epilogue: 4 warps, warp q owns TMEM lanes [32q, 32q+32) =====
+        // ===== epilogue: 4 warps, warp q owns TMEM lanes [32q, 32q+32); lane = weight row, column = activation row =====
         const int q = warp & 3;
         const ScatterTarget& sc = p.scatter;
         if (kScatter) {
@@ -344,159 +376,101 @@ grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_a, const __grid_
             }
             __syncwarp();
         }
-        unsigned char* my_stage = staging + (q * 32 + lane) * kScatterRowPitch;
-        TileCursor cursor;
-        int it = 0;
-        for (int tile = blockIdx.x;; tile += gridDim.x, ++it) {
-            int m_tile, n_tile;
-            if (!cursor.locate(tile, p, n_tiles, m_tile, n_tile)) break;
+        const std::uint32_t empty_addr = cluster_addr(&sh->tmem_empty[0], 0);  // in the leading CTA
+        // this lane's channel inside the CTA's part of the tile; for SwiGLU lanes 0..15 hold gate rows, 16..31 up rows of the same channels
+        const int channel = kSwiGLU ? q * 16 + (lane & 15) : q * 32 + lane;
+        const bool upper = lane >= 16;
+        constexpr int kLanesPerRow = kChannels / 8;             // 16-byte pieces of a row
+        constexpr int kRowsPerStore = 32 / kLanesPerRow;
+        const int piece = lane % kLanesPerRow, store_row = q * (kChunkRows / 4) + lane / kLanesPerRow;
+        int it = 0, half = 0;
+        for (; walk.next(p); ++it) {
             const int buf = it & 1;
             const unsigned acc_phase = (it >> 1) & 1u;
-            if (!mbar_wait(&tmem_full[buf], acc_phase, abort)) break;
+            // all four warps go on or none: they meet at the barriers below
+            if (!epilogue_all(mbar_wait(&sh->tmem_full[buf], acc_phase, abort))) break;
             tc_fence_after();
-            const int row = m_tile * kBlockM + q * 32 + lane;
-            const bool valid = row < p.expert_counts[cursor.expert];
-            const long long out_row = static_cast<long long>(p.expert_offsets[cursor.expert]) + row;
-            __nv_bfloat16* out = p.out + out_row * p.n + n_tile * kOutN;
-            // FP8: the per-row activation scale and the per-output-channel weight scale factor out of the K sum
-            const float a_scale = (kFp8 && valid) ? p.a_scales[out_row] : 1.0f;
-            const float* w_scale = kFp8 ? p.w_scales + static_cast<long long>(cursor.expert) * w_rows_per_expert + n_tile * kOutN : nullptr;
-            const std::uint32_t lane_base = tmem_base + (static_cast<std::uint32_t>(q * 32) << 16) + buf * kAccCols;
-            const int tile_rows = p.expert_counts[cursor.expert] - m_tile * kBlockM;
-            if (flips(box_of_rows(tile_rows))) {
-                // Swapped tile: TMEM lane = output channel, column = row; a warp stores 32 channels of a row.  The address of a row
-                // is only known once the row before has been stored: with all 32 addresses computed ahead the BF16 build took 166
-                // registers instead of 112, and a quarter of an SM had none left for two warps of a combine reducer
-                // (combine_push.cuh) beside two of these.
-                const long long row0 = static_cast<long long>(p.expert_offsets[cursor.expert]) + m_tile * kBlockM;
-                const int channel = q * 32 + lane;
-                const float w_gate = kFp8 ? __ldg(w_scale + channel) : 1.0f, w_up = kFp8 ? __ldg(w_scale + p.n + channel) : 1.0f;
-#pragma unroll 1
-                for (int c0 = 0; c0 < tile_rows; c0 += 32) {
-                    const float a_scale_of_lane = (kFp8 && c0 + lane < tile_rows) ? p.a_scales[row0 + c0 + lane] : 1.0f;
-                    __nv_bfloat16* dst = p.out + (row0 + c0) * p.n + n_tile * kOutN + channel;
-                    std::uint32_t g[32], u[32];
-                    tmem_ld_32x32(lane_base + c0, g);
-                    tmem_ld_32x32(lane_base + kBlockN + c0, u);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        float gate = __uint_as_float(g[i]), up = __uint_as_float(u[i]);
-                        if (kFp8) {
-                            const float a_scale_i = __shfl_sync(0xffffffffu, a_scale_of_lane, i);
-                            gate *= a_scale_i * w_gate;
-                            up *= a_scale_i * w_up;
-                        }
-                        const float v = gate / (1.0f + __expf(-gate)) * up;
-                        if (c0 + i < tile_rows) *dst = __float2bfloat16_rn(v);
-                        dst += p.n;
-                        asm volatile("" : "+l"(dst));
-                    }
-                }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&tmem_empty[buf]);
-                continue;
+            const int first_channel = (walk.m_tile * 2 + static_cast<int>(rank)) * kChannels;
+            const bool inside = first_channel < p.n;  // n an odd multiple of 128: the last tile has one CTA's channels only
+            float w_first = 1.0f, w_up = 1.0f;  // FP8: scale of the weight row(s) of this lane's channel
+            if (kFp8 && inside) {
+                const float* w_scale = p.w_scales + static_cast<long long>(walk.expert) * (kSwiGLU ? 2 : 1) * p.n + first_channel + channel;
+                w_first = __ldg(w_scale);
+                if (kSwiGLU) w_up = __ldg(w_scale + p.n);
             }
-            if (kScatter) {
-                int owner = -1, token = 0, slot = -1;
-                float weight = 1.0f;
-                if (valid) {
-                    const long long* meta = sc.source_meta + out_row * 3;
-                    owner = static_cast<int>(meta[0]);
-                    token = static_cast<int>(meta[1]);
-                    slot = static_cast<int>(meta[2]);
-                    if (sc.row_weights != nullptr) weight = sc.row_weights[out_row];
+            const std::uint32_t acc = tmem_base + (static_cast<std::uint32_t>(q * 32) << 16) + buf * kAccCols;
+            // (2) of a chunk, see below: a few lanes = one row, its channels of this CTA leave as contiguous 16-byte pieces
+            unsigned long long dst_bits = 0;  // where the row of this lane goes, 0: nowhere
+            auto store_chunk = [&]() {
+                epilogue_sync();
+#pragma unroll
+                for (int i = 0; i < kChunkRows / 4; i += kRowsPerStore) {
+                    const int r = store_row + i;
+                    const unsigned long long dst = __shfl_sync(0xffffffffu, dst_bits, r);
+                    const uint4 packed = *reinterpret_cast<const uint4*>(staging + (half * kChunkRows + r) * kPitch + piece * 16);
+                    if (dst != 0ull) ptx::st_v4(reinterpret_cast<unsigned char*>(dst) + piece * 16, packed);
                 }
-                const bool send = valid && owner >= 0 && owner < sc.num_ranks && slot >= 0 && slot < sc.num_topk && token >= 0;
-                unsigned char* dst = nullptr;
-                if (send)
-                    dst = sc.seg[owner] + sc.stage_off +
-                          (static_cast<std::size_t>(token) * sc.num_topk + slot) * static_cast<std::size_t>(sc.row_stride) +
-                          static_cast<std::size_t>(n_tile) * kOutN * 2;
-                const unsigned long long dst_bits = reinterpret_cast<unsigned long long>(dst);
-                const unsigned char* warp_stage = staging + q * 32 * kScatterRowPitch;
-                const int sub = lane & 15;  // 16-byte piece of a 256-byte row segment
+                half ^= 1;  // the other half was read before the barrier above
+            };
 #pragma unroll 1
-                for (int half = 0; half < kOutN / kBlockN; ++half) {
-                    // (1) lane = row: accumulator columns -> weighted BF16 -> this lane's staging row
-#pragma unroll 1
-                    for (int c0 = 0; c0 < kBlockN; c0 += 32) {
-                        std::uint32_t g[32];
-                        tmem_ld_32x32(lane_base + half * kBlockN + c0, g);
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int i = 0; i < 32; i += 8) {
-                            uint4 packed;
-                            __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&packed);
-#pragma unroll
-                            for (int j = 0; j < 4; ++j)
-                                h[j] = __floats2bfloat162_rn(__uint_as_float(g[i + 2 * j]) * weight, __uint_as_float(g[i + 2 * j + 1]) * weight);
-                            *reinterpret_cast<uint4*>(my_stage + (c0 + i) * 2) = packed;
-                        }
-                    }
-                    if (half == kOutN / kBlockN - 1) {
-                        // the accumulator has been read completely: the MMA warp may start the tile after next
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(&tmem_empty[buf]);
+            for (int c0 = 0; c0 < walk.tile_rows; c0 += kChunkRows) {
+                std::uint32_t v[32];
+                tmem_ld_32x32(acc + c0, v);
+                // what belongs to the chunk's rows, one row per lane
+                float row_factor = 1.0f;
+                unsigned long long dst_next = 0;
+                if (c0 + lane < walk.tile_rows && inside) {
+                    const long long r = static_cast<long long>(walk.row0) + c0 + lane;
+                    if (kFp8) row_factor = p.a_scales[r];
+                    if (kScatter) {
+                        const long long* meta = sc.source_meta + r * 3;
+                        const int owner = static_cast<int>(meta[0]), token = static_cast<int>(meta[1]), slot = static_cast<int>(meta[2]);
+                        if (sc.row_weights != nullptr) row_factor = sc.row_weights[r];
+                        if (owner >= 0 && owner < sc.num_ranks && slot >= 0 && slot < sc.num_topk && token >= 0)
+                            dst_next = reinterpret_cast<unsigned long long>(sc.seg[owner] + sc.stage_off +
+                                                                            (static_cast<std::size_t>(token) * sc.num_topk + slot) * static_cast<std::size_t>(sc.row_stride) +
+                                                                            static_cast<std::size_t>(first_channel) * 2);
                     } else {
-                        __syncwarp();
+                        dst_next = reinterpret_cast<unsigned long long>(p.out + r * p.n + first_channel);
                     }
-                    // (2) half a warp = one row: 16 lanes store 256 contiguous bytes into the owner's slot, so a
-                    //     peer receives full 128-byte write packets instead of 32 scattered 16-byte pieces
-#pragma unroll 4
-                    for (int r = 0; r < 32; r += 2) {
-                        const int row_lane = r + (lane >> 4);
-                        const unsigned long long to = __shfl_sync(0xffffffffu, dst_bits, row_lane);
-                        const uint4 v = *reinterpret_cast<const uint4*>(warp_stage + row_lane * kScatterRowPitch + sub * 16);
-                        if (to != 0ull) ptx::st_v4(reinterpret_cast<unsigned char*>(to) + half * kBlockN * 2 + sub * 16, v);
-                    }
-                    __syncwarp();  // the staging rows are rewritten by the next half / tile
                 }
-                continue;
-            }
-#pragma unroll 1
-            for (int c0 = 0; c0 < kOutN; c0 += 32) {
-                std::uint32_t g[32];
-                tmem_ld_32x32(lane_base + c0, g);
-                float v[32];
+                if (c0 > 0) store_chunk();  // the chunk before leaves while this one's values are on their way
+                dst_bits = dst_next;
+                tmem_ld_wait(v);
+                if (c0 + kChunkRows >= walk.tile_rows) {
+                    // the accumulator has been read completely: the MMA warp may start the tile after next
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster(empty_addr + buf * 8);
+                }
+                // (1) transpose through shared memory: lane = channel -> staging[row][channel]
+                unsigned char* to = staging + half * (kChunkRows * kPitch) + channel * 2;
                 if (kSwiGLU) {
-                    std::uint32_t u[32];
-                    tmem_ld_32x32(lane_base + kBlockN + c0, u);
-                    tmem_ld_wait();
+                    // gate and up of a channel lie in lanes 16 apart: the lower lane takes the even rows of both, the upper one the odd ones
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        float gate = __uint_as_float(g[i]);
-                        float up = __uint_as_float(u[i]);
+                    for (int i = 0; i < 16; ++i) {
+                        const float even = __uint_as_float(v[2 * i]), odd = __uint_as_float(v[2 * i + 1]);
+                        const float other = __shfl_xor_sync(0xffffffffu, upper ? even : odd, 16);
+                        float gate = upper ? other : even, up = upper ? odd : other;
                         if (kFp8) {
-                            gate *= a_scale * __ldg(w_scale + c0 + i);
-                            up *= a_scale * __ldg(w_scale + p.n + c0 + i);
+                            const float a_scale = __shfl_sync(0xffffffffu, row_factor, 2 * i + (upper ? 1 : 0));
+                            gate *= a_scale * w_first;
+                            up *= a_scale * w_up;
                         }
-                        v[i] = gate / (1.0f + __expf(-gate)) * up;
+                        const float silu = quotient(gate, 1.0f + __expf(-gate)) * up;
+                        *reinterpret_cast<__nv_bfloat16*>(to + (2 * i + (upper ? 1 : 0)) * kPitch) = __float2bfloat16_rn(silu);
                     }
                 } else {
-                    tmem_ld_wait();
 #pragma unroll
                     for (int i = 0; i < 32; ++i) {
-                        v[i] = __uint_as_float(g[i]);
-                        if (kFp8) v[i] *= a_scale * __ldg(w_scale + c0 + i);
-                    }
-                }
-                if (valid) {
-#pragma unroll
-                    for (int i = 0; i < 32; i += 8) {
-                        uint4 packed;
-                        __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&packed);
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) h[j] = __floats2bfloat162_rn(v[i + 2 * j], v[i + 2 * j + 1]);
-                        *reinterpret_cast<uint4*>(out + c0 + i) = packed;
+                        float value = __uint_as_float(v[i]);
+                        if (kFp8) value *= __shfl_sync(0xffffffffu, row_factor, i) * w_first;
+                        if (kScatter) value *= __shfl_sync(0xffffffffu, row_factor, i);
+                        *reinterpret_cast<__nv_bfloat16*>(to + i * kPitch) = __float2bfloat16_rn(value);
                     }
                 }
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&tmem_empty[buf]);
+            store_chunk();
         }
         if (kScatter) ptx::fence_sys();  // this thread's rows before the CTA is counted as finished
     }
@@ -504,6 +478,7 @@ grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_a, const __grid_
     // ---- teardown: every role has left its loop (normally or through the abort latch)
     tc_fence_before();
     __syncthreads();
+    cluster_sync();  // nothing of the other CTA names this one's shared memory any more
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem_base, kTmemCols);
@@ -548,35 +523,47 @@ EncodeTiled encode_tiled() {
     return fn;
 }
 
-// [rows, k] row-major (bf16 or 1-byte fp8), box = 128 bytes of K x box_rows rows, 128-byte swizzle
-bool make_map(CUtensorMap* map, const void* base, std::uint64_t rows, std::uint64_t k, std::uint32_t box_rows, bool fp8) {
+template <int kDims>
+bool make_map(CUtensorMap* map, const void* base, const cuuint64_t (&dims)[kDims], const cuuint64_t (&strides)[kDims - 1], const cuuint32_t (&box)[kDims], bool fp8) {
     EncodeTiled encode = encode_tiled();
     if (encode == nullptr) return false;
-    const std::uint64_t elem_bytes = fp8 ? 1 : 2;
-    const cuuint64_t dims[2] = {k, rows};
-    const cuuint64_t strides[1] = {k * elem_bytes};
-    const cuuint32_t box[2] = {static_cast<cuuint32_t>(kBlockKBytes / elem_bytes), box_rows};
-    const cuuint32_t elem[2] = {1, 1};
-    return encode(map, fp8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,
+    cuuint32_t elem[kDims];
+    for (cuuint32_t& e : elem) e = 1;
+    return encode(map, fp8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, kDims, const_cast<void*>(base), dims, strides, box, elem,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <bool kSwiGLU, bool kFp8, int kBoxesB, bool kScatter = false>
-cudaError_t launch(const ActivationMaps& map_a, const CUtensorMap& map_b, const GroupedGemmParams& p, int ctas, cudaStream_t stream) {
+// [rows, k] row-major (bf16 or 1-byte fp8), box = 128 bytes of K x box_rows rows, 128-byte swizzle
+bool make_row_map(CUtensorMap* map, const void* base, std::uint64_t rows, std::uint64_t k, std::uint32_t box_rows, bool fp8) {
+    const std::uint64_t elem_bytes = fp8 ? 1 : 2;
+    const cuuint64_t dims[2] = {k, rows}, strides[1] = {k * elem_bytes};
+    const cuuint32_t box[2] = {static_cast<cuuint32_t>(kBlockKBytes / elem_bytes), box_rows};
+    return make_map<2>(map, base, dims, strides, box, fp8);
+}
+
+// gate/up weights [experts, 2n, k] seen as [experts][n / 16][gate, up][16][k]: a box of 128 rows alternates sixteen gate and the
+// matching sixteen up rows
+bool make_gate_up_map(CUtensorMap* map, const void* base, std::uint64_t experts, std::uint64_t n, std::uint64_t k, bool fp8) {
+    const std::uint64_t row = k * (fp8 ? 1 : 2);
+    const cuuint64_t dims[5] = {k, 16, 2, n / 16, experts}, strides[4] = {row, n * row, 16 * row, 2 * n * row};
+    const cuuint32_t box[5] = {static_cast<cuuint32_t>(kBlockKBytes / (fp8 ? 1 : 2)), 16, 2, kCtaM / 32, 1};
+    return make_map<5>(map, base, dims, strides, box, fp8);
+}
+
+template <bool kSwiGLU, bool kFp8, bool kScatter = false>
+cudaError_t launch(const ActivationMaps& maps_rows, const CUtensorMap& map_w, const GroupedGemmParams& p, int sms, cudaStream_t stream) {
     static bool configured[64] = {false};
     int device = 0;
     cudaError_t status = cudaGetDevice(&device);
     if (status != cudaSuccess) return status;
-    // the scatter variant adds its staging rows and keeps 512 bytes of alignment slack (checked in the kernel)
-    constexpr int smem = kScatter ? SmemPlan<kBoxesB>::kStages * SmemPlan<kBoxesB>::kStageBytes + 256 + kScatterStagingBytes + 512
-                                  : SmemPlan<kBoxesB>::kBytes;
+    constexpr int smem = gemm_smem_bytes(kSwiGLU);
     if (device >= 0 && device < 64 && !configured[device]) {
-        status = cudaFuncSetAttribute(grouped_gemm_kernel<kSwiGLU, kFp8, kBoxesB, kScatter>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        status = cudaFuncSetAttribute(grouped_gemm_kernel<kSwiGLU, kFp8, kScatter>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (status != cudaSuccess) return status;
         configured[device] = true;
     }
-    grouped_gemm_kernel<kSwiGLU, kFp8, kBoxesB, kScatter><<<ctas, kThreads, smem, stream>>>(map_a, map_b, p);
+    grouped_gemm_kernel<kSwiGLU, kFp8, kScatter><<<sms / 2 * 2, kThreads, smem, stream>>>(maps_rows, map_w, p);
     return cudaGetLastError();
 }
 
@@ -591,13 +578,13 @@ const char* run_grouped_gemm(const void* a, const void* w, void* out, const floa
                              cudaStream_t stream) {
     using namespace gemm;
     const int block_k = kBlockKBytes / (fp8 ? 1 : 2);
-    if (n % kBlockN != 0 || k % block_k != 0 || n <= 0 || k <= 0)
+    if (n % 128 != 0 || k % block_k != 0 || n <= 0 || k <= 0)
         return "n must be a multiple of 128 and k a multiple of 64 (bf16) / 128 (fp8)";
     if (reinterpret_cast<std::uintptr_t>(a) % 16 || reinterpret_cast<std::uintptr_t>(w) % 16 ||
         reinterpret_cast<std::uintptr_t>(out) % 16)
         return "operands must be 16-byte aligned";
     if (target != nullptr) {
-        if (swiglu || fp8 || n % (2 * kBlockN) != 0) return "the scatter epilogue needs a plain BF16 GEMM with n a multiple of 256";
+        if (swiglu || fp8 || n % 256 != 0) return "the scatter epilogue needs a plain BF16 GEMM with n a multiple of 256";
         if (target->num_ranks < 1 || target->num_ranks > kScatterMaxRanks || target->rank < 0 || target->rank >= target->num_ranks)
             return "scatter target: bad rank table";
         if (target->row_stride % 16 != 0 || target->row_stride < 2 * n || target->stage_off % 16 != 0 || target->epoch == 0 ||
@@ -605,15 +592,12 @@ const char* run_grouped_gemm(const void* a, const void* w, void* out, const floa
             return "scatter target: bad landing-area description";
     }
     if (fp8 && (a_scales == nullptr || w_scales == nullptr)) return "fp8 operands need their scales";
-    ActivationMaps map_a;
-    CUtensorMap map_b;
-    const std::uint64_t w_rows = static_cast<std::uint64_t>(num_experts) * (swiglu ? 2 : 1) * n;
-    bool encoded = true;
-    for (int i = 0; i < kBoxesA; ++i)
-        encoded = encoded && make_map(&map_a.box[i], a, static_cast<std::uint64_t>(rows_capacity), static_cast<std::uint64_t>(k), box_rows_a(i), fp8);
-    if (!encoded ||
-        !make_map(&map_b, w, w_rows, static_cast<std::uint64_t>(k), kBlockN, fp8))
-        return "cuTensorMapEncodeTiled failed";
+    ActivationMaps maps_rows;
+    CUtensorMap map_w;
+    bool encoded = swiglu ? make_gate_up_map(&map_w, w, num_experts, n, k, fp8)
+                          : make_row_map(&map_w, w, static_cast<std::uint64_t>(num_experts) * n, k, kCtaM, fp8);
+    for (int i = 0; i < kBoxes; ++i) encoded = encoded && make_row_map(&maps_rows.box[i], a, rows_capacity, k, box_rows(i), fp8);
+    if (!encoded) return "cuTensorMapEncodeTiled failed";
     GroupedGemmParams p{};
     p.expert_offsets = expert_offsets;
     p.expert_counts = expert_counts;
@@ -630,18 +614,9 @@ const char* run_grouped_gemm(const void* a, const void* w, void* out, const floa
     if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
         return "cannot query the device";
     cudaError_t err;
-    const bool wide = n % (2 * kBlockN) == 0;  // plain GEMM: 256-column tiles whenever n allows
-    if (target != nullptr) {
-        err = launch<false, false, 2, true>(map_a, map_b, p, sms, stream);
-    } else if (fp8) {
-        err = swiglu ? launch<true, true, 2>(map_a, map_b, p, sms, stream)
-              : wide ? launch<false, true, 2>(map_a, map_b, p, sms, stream)
-                     : launch<false, true, 1>(map_a, map_b, p, sms, stream);
-    } else {
-        err = swiglu ? launch<true, false, 2>(map_a, map_b, p, sms, stream)
-              : wide ? launch<false, false, 2>(map_a, map_b, p, sms, stream)
-                     : launch<false, false, 1>(map_a, map_b, p, sms, stream);
-    }
+    if (target != nullptr) err = launch<false, false, true>(maps_rows, map_w, p, sms, stream);
+    else if (swiglu) err = fp8 ? launch<true, true>(maps_rows, map_w, p, sms, stream) : launch<true, false>(maps_rows, map_w, p, sms, stream);
+    else err = fp8 ? launch<false, true>(maps_rows, map_w, p, sms, stream) : launch<false, false>(maps_rows, map_w, p, sms, stream);
     return err == cudaSuccess ? nullptr : cudaGetErrorString(err);
 }
 }  // namespace

@@ -8,15 +8,25 @@
 //   plain  : out[row, n]        = sum_k A[row, k] * W[e, n, k]
 //   SwiGLU : out[row, n]        = silu(sum_k A[row,k] * W[e, n, k]) * (sum_k A[row,k] * W[e, N + n, k])
 //
-// One tcgen05.mma covers 128 rows x 256 columns (two 128-row weight boxes back to back in shared memory:
-// gate + up rows for SwiGLU, 256 adjacent output columns for the plain GEMM when n allows), so A is read
-// from shared memory once per 256 accumulator columns.
+// A pair of CTAs (a cluster, cta_group::2) multiplies one tile: 256 weight rows x up to 256 activation rows.  The weight rows are
+// the M operand (128 per CTA), the activation rows the N operand (half per CTA), so that a tile is as wide as its rows in steps
+// of 32: an expert's rows are cut into equal chunks, and nothing is multiplied for rows that are not there beyond those 32.
+// For SwiGLU the 256 weight rows are 128 gate and the matching 128 up rows, interleaved in sixteens by the weight's tensor map.
 //
-// Work decomposition: persistent CTAs walk a tile list (expert, n-tile, m-tile) computed on the
-// device from the counts -- the host never reads a count.  Per CTA: warp 0 = TMA producer,
-// warp 1 = MMA issuer (and TMEM owner), warps 2..5 = epilogue.  Shared-memory stages are handed over
-// with mbarriers (TMA complete_tx -> MMA; tcgen05.commit -> producer), accumulators are double
-// buffered in TMEM (tcgen05.commit -> epilogue; epilogue arrive -> MMA).
+// What bounds it.  Few rows per expert: the weights from HBM.  64 tokens, top-8 of 32 experts, 7168 x 2048: gate/up 299 -> 283 us
+// (6.6 TB/s), down 154 -> 154, against tiles of 128 rows x 256 weight rows by single CTAs.  Many: tensor cores under the power
+// limit.  4096 tokens (1024 rows per expert), back to back: gate/up 1709 -> 1718 us in BF16 (1,120 TFLOP/s; with exactly 1024
+// rows everywhere 1595 -> 1593) and 1050 -> 913 in E4M3, down 935 -> 872.  Between them, and with a short K, the epilogue: 2000
+// tokens of hidden 2048 and intermediate 768 gate/up 117 -> 95 us, 300 tokens in E4M3 192 -> 161.  Slower than before where a few
+// experts have many rows and the others about a hundred (1024 tokens, a fifth of the experts popular: gate/up 442 -> 468 us):
+// stages as long as the widest tile needs leave 96 KB of weights on their way per SM instead of 128.  (Stages of each tile's own
+// length in a circle were 20 % slower everywhere; asking weights into L2 ahead of the stages 2 to 80 %.)
+//
+// Work decomposition: persistent pairs walk a tile list (expert, channel tile, row chunk) computed on the device from the
+// counts -- the host never reads a count.  Per CTA: warp 0 = TMA producer (this CTA's weight rows and its half of the
+// activation rows), warp 1 of the leading CTA = MMA issuer for both, warps 2..5 = epilogue.  Shared-memory stages are handed
+// over with mbarriers (TMA complete_tx of both CTAs -> the leading CTA's MMA; tcgen05.commit -> both producers), accumulators
+// are double buffered in TMEM (tcgen05.commit -> both epilogues; epilogue arrive -> MMA).
 //
 // Every mbarrier wait is bounded: on expiry the thread latches an abort flag, all roles drain, TMEM
 // is released and the kernel returns with status[0] != 0.
@@ -31,11 +41,12 @@
 namespace bep {
 namespace gemm {
 
-constexpr int kBlockM = 128;
-constexpr int kBlockN = 128;
+constexpr int kCtaM = 128;         // weight rows per CTA and tile
+constexpr int kMaxRows = 256;      // activation rows per tile
+constexpr int kRowStep = 32;       // a tile has a multiple of this many (padded) rows
 constexpr int kBlockKBytes = 128;  // one 128B-swizzle atom row: 64 bf16 or 128 fp8 elements of K
 constexpr int kUmmaKBytes = 32;    // K extent of one tcgen05.mma: 16 bf16 or 32 fp8
-constexpr int kThreads = 192;  // 6 warps
+constexpr int kThreads = 192;      // 6 warps
 constexpr std::uint32_t kWaitLimit = 20u * 1000u * 1000u;  // try_wait probes before giving up (seconds at most)
 
 // Fused down-projection + combine send: instead of writing `out`, the epilogue multiplies every valid row by
@@ -43,8 +54,6 @@ constexpr std::uint32_t kWaitLimit = 20u * 1000u * 1000u;  // try_wait probes be
 // a peer's, through the segment table -- so the NVLink transfer of a tile overlaps the MMAs of the next ones.
 // When the last CTA of the launch has drained its stores it publishes `epoch` to every rank.
 constexpr int kScatterMaxRanks = 16;
-constexpr int kScatterRowPitch = kBlockN * 2 + 16;  // one 128-column BF16 row segment + 16 B: conflict-free column writes
-constexpr int kScatterStagingBytes = 4 * 32 * kScatterRowPitch;
 struct ScatterTarget {
     unsigned char* seg[kScatterMaxRanks];  // segment of every rank as addressed from this one
     const long long* source_meta;          // [rows][3]: owner rank, token, slot k (-1: padding row)
@@ -63,7 +72,7 @@ struct GroupedGemmParams {
     __nv_bfloat16* out;         // [rows, N]
     const float* a_scales;      // FP8 only: one scale per row of A
     const float* w_scales;      // FP8 only: one scale per weight row [E, (2)N]
-    int* status;                // [4]: 0 = ok, 1 = a wait expired, 2 = shared memory misaligned, 3 = a peer never freed its area
+    int* status;                // [4]: 0 = ok, 1 = a wait expired, 3 = a peer never freed its area
     int num_experts;
     int n;                      // output columns
     int k;                      // reduction length in elements
@@ -71,29 +80,45 @@ struct GroupedGemmParams {
     ScatterTarget scatter;      // only read by the scatter variant
 };
 
-// Activation rows are loaded in boxes of one of three heights: a 128-row box for a handful of valid rows would be a third of
-// the traffic into shared memory.  A gate/up tile that fits one of the lower two also swaps the MMA's operands: each 128-row
-// weight box becomes the M = 128 operand and the rows the N = 32 or 64 one, so the tensor core reads the few rows once per
-// box instead of multiplying 128 of them.  The accumulator then holds channels in its lanes and rows in its columns, and the
-// epilogue stores 32 channels of a row per warp.  64 tokens, top-8 of 32 experts (16 rows per expert), gate/up 7168 -> 2 x
-// 2048: 324 us with full boxes, 319 with low ones, 303 swapped as well; 1024 rows per expert 1447 -> 1444 us, E4M3 768 -> 758.
-// The plain GEMM is not swapped: it lost 2 % at both sizes (2-byte stores of 256 columns), low boxes alone gain it 1 %.
-constexpr int kBoxesA = 3;
-__host__ __device__ constexpr int box_rows_a(int box) { return box == 0 ? 32 : box == 1 ? 64 : kBlockM; }
-__host__ __device__ constexpr int box_of_rows(int rows) { return rows <= box_rows_a(0) ? 0 : rows <= box_rows_a(1) ? 1 : 2; }
+// How an expert's rows are cut into tiles: as few as possible, equal but for the last.  (256 each and the rest in one more: the same
+// within 1 %, 4096 tokens gate/up 1800 and 1785 us, down 898 and 908.)
+struct RowChunks {
+    int count, rows;
+};
+__host__ __device__ constexpr RowChunks row_chunks(int rows) {
+    const int count = (rows + kMaxRows - 1) / kMaxRows;
+    return {count, count == 0 ? 0 : ((rows + count - 1) / count + kRowStep - 1) / kRowStep * kRowStep};
+}
+// Each CTA of a pair loads half of a tile's rows: boxes of 16, 32, ... 128 rows, one tensor map each.
+constexpr int kBoxes = kMaxRows / kRowStep;
+__host__ __device__ constexpr int box_rows(int box) { return (box + 1) * (kRowStep / 2); }
+__host__ __device__ constexpr int box_of_rows(int tile_rows) { return (tile_rows + kRowStep - 1) / kRowStep - 1; }
 struct ActivationMaps {
-    CUtensorMap box[kBoxesA];
+    CUtensorMap box[kBoxes];
 };
 
-// stages of (A tile + B boxes) that fit; a stage carries one or two 128-row weight boxes
-template <int kBoxesB>
-struct SmemPlan {
-    static constexpr int kTileA = kBlockM * kBlockKBytes;
-    static constexpr int kTileB = kBlockN * kBlockKBytes;
-    static constexpr int kStageBytes = kTileA + kBoxesB * kTileB;
-    static constexpr int kStages = kBoxesB == 2 ? 4 : 6;
-    static constexpr int kBytes = kStages * kStageBytes + 1024 /* alignment slack */ + 256 /* barriers */;
+constexpr int kTileW = kCtaM * kBlockKBytes;
+// Stages are as long as the widest tile of the launch needs: where all experts have few rows, more of them keep weights on their way.
+constexpr int kRingBytes = 6 * (kTileW + kMaxRows / 2 * kBlockKBytes);  // six stages of the widest tiles, more of narrower ones
+constexpr int kMaxStages = 10;
+constexpr int kAccCols = kMaxRows;       // TMEM columns of one accumulator set
+constexpr int kTmemCols = 2 * kAccCols;  // double buffered
+// The epilogue turns the accumulator (lane = channel) round in shared memory, kChunkRows rows at a time in two alternating halves.
+// Row pitch: 16 bytes more than a row keep the 2-byte column writes of a warp apart; for SwiGLU, where a warp writes sixteen
+// channels of two rows at once, 32.
+constexpr int kChunkRows = 32;
+__host__ __device__ constexpr int staging_pitch(bool swiglu) { return swiglu ? kCtaM / 2 * 2 + 32 : kCtaM * 2 + 16; }
+struct GemmShared {
+    std::uint64_t full[kMaxStages], empty[kMaxStages], tmem_full[2], tmem_empty[2];
+    std::uint32_t tmem_base;
+    int abort;
+    int most_rows[kThreads / 32];  // of any expert, per warp
 };
+__host__ __device__ constexpr int gemm_smem_bytes(bool swiglu) {
+    return 1024 /* alignment slack */ + kRingBytes + 2 * kChunkRows * staging_pitch(swiglu) + static_cast<int>(sizeof(GemmShared));
+}
+static_assert(2 * kChunkRows * staging_pitch(true) % 16 == 0 && 2 * kChunkRows * staging_pitch(false) % 16 == 0, "barriers follow the staging");
+static_assert(gemm_smem_bytes(false) <= 227 * 1024, "one CTA per SM");
 
 }  // namespace gemm
 }  // namespace bep

@@ -130,3 +130,60 @@ def test_last_tiles_at_the_box_heights(ext, fp8, swiglu, n):
             error = 1.1 * error[:, :n] * up.abs() + silu.abs() * error[:, n:] + (silu * up).abs() * (8 + 2 * gate.abs()) * 2.0 ** -24
             want = silu * up
         assert bool(((out[at].double() - want).abs() <= error + (want.abs() + error) * 2.0 ** -8).all()), counts[e]
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("swiglu", [True, False])
+@pytest.mark.parametrize("k", [128, 1152])
+def test_tiles_of_every_width(ext, fp8, swiglu, k):
+    """Tiles of 32 to 256 rows (one expert each, and several chunks per expert), K shorter and longer than the ring of stages, and
+    output columns that leave the second CTA of the last pair without channels."""
+    counts = [1, 33, 95, 97, 129, 161, 193, 225, 256, 257, 0, 289, 511, 513, 770, 1025]
+    n, experts = 384, len(counts)
+    offsets, cnts = _layout(counts)
+    rows = int(offsets[-1])
+    gen = torch.Generator(device="cuda").manual_seed(k)
+    x = torch.randn(rows, k, device="cuda", generator=gen).to(torch.bfloat16)
+    w = (torch.randn(experts, (2 if swiglu else 1) * n, k, device="cuda", generator=gen) * 0.1).to(torch.bfloat16)
+    scales = {}
+    if fp8:
+        x, w = x.to(torch.float8_e4m3fn), w.to(torch.float8_e4m3fn)
+        scales = dict(a_scales=torch.rand(rows, device="cuda", generator=gen) + 0.5, w_scales=torch.rand(w.shape[:2], device="cuda", generator=gen) + 0.5)
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    out = grouped_gemm(x, w, offsets.cuda(), cnts.cuda(), swiglu=swiglu, status=status, **scales)
+    torch.cuda.synchronize()
+    assert status.tolist() == [0, 0, 0, 0]
+    for e, c in enumerate(counts):
+        at = slice(int(offsets[e]), int(offsets[e]) + c)
+        a, m = x[at].double(), w[e].double()
+        if fp8:
+            a, m = a * scales["a_scales"][at].double().unsqueeze(1), m * scales["w_scales"][e].double().unsqueeze(1)
+        want = a @ m.t()
+        # as in test_last_tiles_at_the_box_heights: K products summed in 32 bits, the fast exponential, one rounding to BF16
+        error = (a.abs() @ m.abs().t()) * (k + 4) * 2.0 ** -24
+        if swiglu:
+            gate, up = want[:, :n], want[:, n:]
+            silu = torch.nn.functional.silu(gate)
+            error = 1.1 * error[:, :n] * up.abs() + silu.abs() * error[:, n:] + (silu * up).abs() * (8 + 2 * gate.abs()) * 2.0 ** -24
+            want = silu * up
+        assert bool(((out[at].double() - want).abs() <= error + (want.abs() + error) * 2.0 ** -8).all()), c
+
+
+def test_swiglu_of_extreme_gates(ext):
+    """gate / (1 + exp(-gate)) where the exponential over- or underflows, and of values that are no numbers."""
+    gates = torch.tensor([0.0, -0.0, 1e-30, -1e-30, 20.0, -20.0, 80.0, -80.0, -87.0, -88.0, -88.5, -89.0, 89.0, -104.0, 3e38, -3e38, float("inf"),
+                          -float("inf"), float("nan")] + [0.5 * i - 27.0 for i in range(109)]).to(torch.bfloat16)
+    n, k = 128, 128
+    assert gates.numel() == n
+    w = torch.zeros(1, 2 * n, k, dtype=torch.bfloat16)
+    w[0, :n, 0], w[0, n:, 0] = gates, 1.0
+    x = torch.zeros(1, k, dtype=torch.bfloat16)
+    x[0, 0] = 1.0
+    got = grouped_gemm(x.cuda(), w.cuda(), torch.tensor([0, 1], dtype=torch.int32).cuda(), torch.tensor([1], dtype=torch.int32).cuda(), swiglu=True).cpu()[0]
+    g = gates.float()
+    want = (g.double() / (1.0 + torch.exp(-g.double()))).float()
+    want[g == -float("inf")] = float("nan")
+    assert torch.equal(got.isnan(), want.isnan())
+    same = ~want.isnan()
+    # a rounding to BF16; below -88 the 32-bit exponential is infinite and the quotient zero
+    assert bool(((got.float() - want)[same].abs() <= want[same].abs() * 2.0 ** -8 + 1e-36).logical_or(got.float()[same] == want[same]).all())
