@@ -9,8 +9,9 @@
 // rows are what sets the pace.)
 //   1. token rows are on their way into shared memory before anything about the layout is known;
 //   2. expert ids -> histogram and stable ordinals inside the CTA's tokens, 32 tokens at a time, one thread per (token, k);
-//   3. one grid barrier; then a prefix over the CTAs before this one and a scan over experts, one thread per bin.  A cached
-//      layout skips 2 and the barrier, and its launch is an ordinary one;
+//   3. one grid barrier; then a prefix over the CTAs before this one and a scan over experts, one thread per bin.  A small batch
+//      (kLocalWholePairs) is counted as a whole by every CTA instead, a cached layout skips 2 as well: without the barrier the
+//      launch is an ordinary one;
 //   4. a warp per token: every lane k < K whose expert is valid starts the bulk store of the row to its expert's segment.
 //
 // What bounds it.  Large batches: writing the expanded rows to HBM.  4096 tokens, hidden 7168, top-8 move 528 MB.
@@ -33,6 +34,15 @@ constexpr int kLocalMaxPairBytes = 64 * 1024;
 // can have this kernel too; beyond it they would cost row buffers (at hidden 7168 fourteen of them leave 26 KB), which large
 // batches need more: fourteen on all SMs instead of eight on 128 are 71 instead of 106 us for 4096 E4M3 rows.
 constexpr int kLocalSmallPairBytes = 16 * 1024;
+
+// How a launch lays out its batch.  A kernel each: a launch mostly finds its code driven out of L2 by the rows of the one before
+// and fetches it line by line (all three in one kernel: the scan alone 1.5 -> 3.1 us).
+enum LocalMode { kLocalTogether, kLocalWhole, kLocalCached };
+// Batches of up to this many (token, k) are counted by every CTA by itself, without a barrier: no CTA waits for another one, and
+// where none claims tokens the launch needs no cooperative grid and nobody has to be the last.  Together / by itself, top-8: 16 tokens
+// 17.2 / 10.7 us, 128 tokens 17.3 / 10.9, 2048 (at the line) 26.3 / 22.1, 4096 99.7 / 103.4; 777 tokens top-4 20.9 / 14.0.
+constexpr int kLocalWholePairs = 16 * 1024;
+constexpr int kLocalFewExperts = 64;  // counted with ballots, without atomics (a warp's 32 pairs meet few counters again and again)
 
 struct LocalDispatchArgs {
     DispatchArgs a;
@@ -76,7 +86,19 @@ inline LocalPlan make_local_plan(int experts, int channels, int topk, int hidden
     p.stages = slots / kLocalWarps < 1 ? 1 : slots / kLocalWarps < kLocalMaxStages ? slots / kLocalWarps : kLocalMaxStages;
     p.bytes = bytes + static_cast<std::size_t>(p.warps) * p.stages * p.slot_bytes;
     p.usable = p.warps >= kLocalMinWarps;
+    // what is left over holds the tables of a batch that every CTA counts by itself
+    p.whole_off = align_up(p.bytes, 16);
+    p.whole_bytes = smem_limit > p.whole_off ? static_cast<int>(smem_limit - p.whole_off) : 0;
     return p;
+}
+
+// Those tables: a bit per (token, k), a bit per token, routed tokens before each 32.
+__host__ __device__ inline std::size_t local_whole_bytes(int tokens, int topk) {
+    const std::size_t pair_words = (static_cast<std::size_t>(tokens) * topk + 31) / 32 + 1, token_words = static_cast<std::size_t>(tokens + 31) / 32;
+    return 4 * (pair_words + 2 * token_words + 1);
+}
+inline bool local_counts_whole(int tokens, int topk, const LocalPlan& plan) {
+    return tokens > 0 && static_cast<long long>(tokens) * topk <= kLocalWholePairs && local_whole_bytes(tokens, topk) <= static_cast<std::size_t>(plan.whole_bytes);
 }
 
 #ifdef __CUDACC__
@@ -91,6 +113,7 @@ __device__ __forceinline__ void local_wait_read(int groups_left) {
 
 }  // namespace detail
 
+template <LocalMode kMode>
 __global__ void __launch_bounds__(kLocalThreads, 1) local_dispatch_kernel(const __grid_constant__ LocalDispatchArgs args) {
     using namespace detail;
     const DispatchArgs& a = args.a;
@@ -102,7 +125,8 @@ __global__ void __launch_bounds__(kLocalThreads, 1) local_dispatch_kernel(const 
     const int nt = t1 - t0;
     const int tid = threadIdx.x, warp = tid >> 5;
     const unsigned lane = ptx::lane_id(), full = 0xffffffffu, lt_mask = (1u << lane) - 1u;
-    const bool recv_fp8 = args.recv_fp8 != 0, expand = a.do_expand != 0, cached = a.cached != 0;
+    const bool recv_fp8 = args.recv_fp8 != 0, expand = a.do_expand != 0;
+    constexpr bool cached = kMode == kLocalCached, whole = kMode == kLocalWhole;
     const int row_warps = args.plan.warps, stages = args.plan.stages, slot_bytes = args.plan.slot_bytes;
     const unsigned in_bytes = static_cast<unsigned>(H) * 2u;
 
@@ -121,7 +145,9 @@ __global__ void __launch_bounds__(kLocalThreads, 1) local_dispatch_kernel(const 
     const int sticky_before = tid == 0 ? ptx::ld_volatile(&rc->sticky[0]) : 0;
     const std::uint64_t epoch_before = tid == 0 ? __ldcg(rc->epochs) : 0;
     const unsigned long long t_start = ptx::globaltimer_ns();
-    if (tid == 0) atomicMax(&args.counters[2], ~t_start);
+    // where no CTA needs another one's counts or claims its tokens, nothing has to be settled by the last one
+    const bool alone = (cached || whole) && (T + G - 1) / G <= row_warps * stages;
+    if (tid == 0 && !alone) atomicMax(&args.counters[2], ~t_start);
     // profile rows are per channel: CTA b fills the rows b, b + G, ...
 #define BEP_PROF(point)                                                                                          \
     do {                                                                                                         \
@@ -147,7 +173,8 @@ __global__ void __launch_bounds__(kLocalThreads, 1) local_dispatch_kernel(const 
     const int groups = (args.hist_ctas + kHistGroup - 1) / kHistGroup;
     int* const sums_base = args.hist + static_cast<std::size_t>(args.hist_ctas) * W;
     int* const generation_at = sums_base + static_cast<std::size_t>(2) * groups * S;
-    const int generation = cached ? 0 : __ldcg(generation_at);
+    const int generation = cached || whole ? 0 : __ldcg(generation_at);
+    auto* const counts = reinterpret_cast<unsigned*>(eoff);  // whole: pairs of the expert, those of earlier CTAs in the upper half
     if (tid == 0) {
         sh->flag = 0;
         sh->routed = 0;
@@ -156,8 +183,9 @@ __global__ void __launch_bounds__(kLocalThreads, 1) local_dispatch_kernel(const 
     for (int i = tid; i < E; i += kLocalThreads) {
         base[i] = 0;
         total[i] = 0;
+        counts[i] = 0;
     }
-    if (!cached) {
+    if (!cached && !whole) {
         // the sums this CTA will add to have been driven out of L2 by the rows of the last launch: fetch both copies' lines
         for (int i = tid * 32; i < S; i += kLocalThreads * 32)
             for (int copy = 0; copy < 2; ++copy)
@@ -190,12 +218,63 @@ __global__ void __launch_bounds__(kLocalThreads, 1) local_dispatch_kernel(const 
             if (b == 0) atomicCAS(&a.error[0], 0, kErrAlreadyAborted);
             return true;
         }
+        if (alone && b != G - 1) return false;  // (the last CTA may have advanced the epoch already)
         if (epoch_before + 1 >= (1ull << 32)) record_error(rc, a.error, kErrEpochExhausted, 0, 0);
         return epoch_before + 1 >= (1ull << 32);
     };
 
     // ---- 2. ordinals inside the CTA ------------------------------------------------------------------------------
-    if (!cached) {
+    const int all_pairs = T * K, pair_words = (all_pairs + 31) / 32 + 1, token_words = (T + 31) / 32;
+    auto* const pair_bits = reinterpret_cast<unsigned*>(local_smem + args.plan.whole_off);  // whole: which pairs name an expert,
+    unsigned* const token_bits = pair_bits + pair_words;                                    // which tokens are routed,
+    int* const routed_words = reinterpret_cast<int*>(token_bits + token_words);             // [token_words + 1] routed tokens before word w
+    if constexpr (whole) {
+        // The pairs of the whole batch: 32 per warp and step, the ids of four steps on their way at once.  Few experts meet in
+        // a step again and again: there a lane counts two of them from ballots of the ids' bits.
+        const int own_first = t0 * K;
+        const bool few = E <= kLocalFewExperts;
+        unsigned mine[2] = {0u, 0u};  // few: pairs of the experts lane and lane + 32, those of earlier CTAs in the upper half
+        bool bad = false;
+        for (int p0 = warp * 32; p0 < all_pairs; p0 += kLocalThreads * 4) {
+            std::int64_t id[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int p = p0 + u * kLocalThreads + static_cast<int>(lane);
+                id[u] = p < all_pairs ? __ldg(a.topk_idx + p) : -1;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int first = p0 + u * kLocalThreads;
+                if (first >= all_pairs) break;
+                const bool named = id[u] >= 0 && id[u] < E;
+                bad = bad || id[u] < -1 || id[u] >= E;
+                const unsigned bits = __ballot_sync(full, named);
+                if (lane == 0) pair_bits[first >> 5] = bits;
+                if (few) {
+                    unsigned same = bits;
+#pragma unroll
+                    for (int i = 0; i < 5; ++i) {
+                        const unsigned plane = __ballot_sync(full, id[u] >> i & 1);
+                        same &= lane >> i & 1u ? plane : ~plane;
+                    }
+                    const unsigned high = __ballot_sync(full, id[u] >> 5 & 1);
+                    const int before = own_first - first;  // pairs of the step that belong to earlier CTAs
+                    const unsigned earlier = before >= 32 ? full : before <= 0 ? 0u : (1u << before) - 1u;
+                    mine[0] += __popc(same & ~high) + (__popc(same & ~high & earlier) << 16);
+                    mine[1] += __popc(same & high) + (__popc(same & high & earlier) << 16);
+                } else if (named) {
+                    atomicAdd(&counts[id[u]], first + static_cast<int>(lane) < own_first ? 0x10001u : 1u);
+                }
+            }
+        }
+        if (few)
+            for (int i = 0; i < 2; ++i)
+                if (mine[i] != 0) atomicAdd(&counts[lane + 32 * i], mine[i]);
+        if (tid == 0) pair_bits[pair_words - 1] = 0;
+        if (bad) sh->flag = 1;  // (the CTA that owns the token says so)
+        start_first_loads();
+    }
+    if constexpr (!cached) {
         unsigned* bits = reinterpret_cast<unsigned*>(total);
         constexpr int kLastFlag = 1 << 30;  // the pair of the chunk's last token in its expert carries the count forward
         int routed_before = 0;              // (last warp) routed tokens of earlier chunks
@@ -249,6 +328,57 @@ __global__ void __launch_bounds__(kLocalThreads, 1) local_dispatch_kernel(const 
             }
             __syncthreads();
         }
+    }
+    if constexpr (whole) {
+        __syncthreads();
+        for (int i = tid; i < E; i += kLocalThreads) {
+            base[i] = static_cast<int>(counts[i] >> 16);
+            total[i] = static_cast<int>(counts[i] & 0xffffu);
+        }
+        const unsigned k_mask = K == 32 ? full : (1u << K) - 1u;
+        for (int w = warp; w < token_words; w += kLocalWarps) {
+            const int t = w * 32 + static_cast<int>(lane), at = t * K;
+            bool routed = false;
+            if (t < T) routed = (__funnelshift_r(pair_bits[at >> 5], pair_bits[(at >> 5) + 1], at & 31) & k_mask) != 0;
+            const unsigned bits = __ballot_sync(full, routed);
+            if (lane == 0) token_bits[w] = bits;
+        }
+        if (tid == 0 && (leaves() || health.failed())) sh->flag = 1;
+        __syncthreads();
+        if (warp == kLocalWarps - 1) {
+            int before = 0;
+            for (int w0 = 0; w0 < token_words; w0 += 32) {
+                const int w = w0 + static_cast<int>(lane), n = w < token_words ? __popc(token_bits[w]) : 0;
+                int incl = n;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int up = __shfl_up_sync(full, incl, o);
+                    if (lane >= static_cast<unsigned>(o)) incl += up;
+                }
+                if (w < token_words) routed_words[w] = before + incl - n;
+                before += __shfl_sync(full, incl, 31);
+            }
+            if (lane == 0) {
+                routed_words[token_words] = before;
+                sh->first_unique = 0;
+                sh->unique_total = before;
+            }
+        }
+        __syncthreads();
+        auto routed_before = [&](int t) {  // t <= T
+            const int w = t >> 5;
+            return routed_words[w] + (t & 31 ? __popc(token_bits[w] & ((1u << (t & 31)) - 1u)) : 0);
+        };
+        for (int c = tid; c < C; c += kLocalThreads) chan_base[c] = routed_before(min(T, (c + 1) * Tc)) - routed_before(min(T, c * Tc));
+        for (int i = tid; i < nt; i += kLocalThreads) {
+            const int t = t0 + i, r = routed_before(t);
+            unique[i] = token_bits[t >> 5] >> (t & 31) & 1u ? r : ~r;
+        }
+        if (tid == 0) {
+            BEP_PROF(kProfHistDone);
+            BEP_PROF(kProfBarrierDone);
+        }
+    } else if constexpr (!cached) {
         // ---- 3. prefix over the CTAs before this one.  Two levels (groups of kHistGroup CTAs, then the CTAs of the group),
         // as in dispatch.cuh: a CTA reads G / kHistGroup + kHistGroup rows, all at once, instead of G.
         int* const sums = sums_base + static_cast<std::size_t>(generation & 1) * groups * S;
@@ -609,6 +739,19 @@ __global__ void __launch_bounds__(kLocalThreads, 1) local_dispatch_kernel(const 
         BEP_PROF(kProfRxDone);
         BEP_PROF(kProfEnd);
         if (any_failed) return;  // the rank has failed: nothing of it is used again
+        if (alone) {
+            // launches of a buffer are stream-ordered: the next one sees all of this, whichever CTA wrote it when
+            atomicMax(reinterpret_cast<unsigned long long*>(&a.timestamps[1]), static_cast<unsigned long long>(ptx::globaltimer_ns()));
+            if (b == 0) a.timestamps[0] = static_cast<std::int64_t>(t_start);
+            if (b == G - 1) {
+                for (int i = 0; i < 8; ++i) a.stats[i] = i == kStatLocalRows ? sh->unique_total : 0;
+                if (ptx::ld_volatile(&rc->sticky[0]) == 0) {
+                    ptx::st_relaxed_sys(flag_ptr(rc->seg[rc->rank], rc->lay.done_off, rc->rank), epoch_before + 1);
+                    rc->epochs[0] = epoch_before + 1;
+                }
+            }
+            return;
+        }
         __threadfence();
         if (atomicAdd(&args.counters[1], 1ull) + 1ull == static_cast<unsigned long long>(G)) {
             __threadfence();
@@ -620,7 +763,7 @@ __global__ void __launch_bounds__(kLocalThreads, 1) local_dispatch_kernel(const 
                 const std::uint64_t epoch = epoch_before + 1;
                 ptx::st_release_sys(flag_ptr(rc->seg[rc->rank], rc->lay.done_off, rc->rank), epoch);
                 rc->epochs[0] = epoch;
-                if (!cached) *generation_at = generation + 1;
+                if (!cached && !whole) *generation_at = generation + 1;
             }
         }
     }

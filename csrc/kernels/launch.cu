@@ -98,26 +98,32 @@ int dispatch_local_width(const SegmentLayout& lay, int tokens, bool padding) {
 }
 
 cudaError_t launch_dispatch_local(const DispatchArgs& a, const RankConst& rc, const LocalPlan& plan, int* hist, unsigned long long* counters, int sms, int max_ctas, cudaStream_t stream) {
+    const int ctas = std::max(1, std::min(std::min(sms, max_ctas), dispatch_local_width(rc.lay, a.num_tokens, a.do_expand && a.zero_padding && a.alignment > 1)));
+    const bool whole = !a.cached && local_counts_whole(a.num_tokens, rc.lay.num_topk, plan);
+    const LocalMode mode = a.cached ? kLocalCached : whole ? kLocalWhole : kLocalTogether;
+    const auto kernel = mode == kLocalCached ? local_dispatch_kernel<kLocalCached> : mode == kLocalWhole ? local_dispatch_kernel<kLocalWhole> : local_dispatch_kernel<kLocalTogether>;
+    const std::size_t bytes = whole ? plan.whole_off + local_whole_bytes(a.num_tokens, rc.lay.num_topk) : plan.bytes;
     static std::mutex mutex;
-    static std::size_t configured[64] = {0};
+    static std::size_t configured[3][64] = {{0}};
     {
         std::lock_guard<std::mutex> guard(mutex);
         int device = 0;
         cudaError_t status = cudaGetDevice(&device);
         if (status != cudaSuccess) return status;
         if (device < 0 || device >= 64) return cudaErrorInvalidDevice;
-        if (plan.bytes > configured[device]) {
-            status = cudaFuncSetAttribute(local_dispatch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(plan.bytes));
+        if (bytes > configured[mode][device]) {
+            status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
             if (status != cudaSuccess) return status;
-            configured[device] = plan.bytes;
+            configured[mode][device] = bytes;
         }
     }
     LocalDispatchArgs args{a, plan, hist, counters, sms, rc.lay.num_experts, rc.lay.num_channels, rc.lay.num_topk, rc.lay.hidden,
                            rc.lay.slots_full, rc.expanded_cap, rc.unique_cap, rc.recv_fp8};
-    const int ctas = std::max(1, std::min(std::min(sms, max_ctas), dispatch_local_width(rc.lay, a.num_tokens, a.do_expand && a.zero_padding && a.alignment > 1)));
-    // a fresh layout has a grid barrier and needs every CTA resident; with a cached one no CTA waits for another
-    if (!a.cached) return cooperative_launch(local_dispatch_kernel, args, dim3(ctas), kLocalThreads, plan.bytes, stream);
-    local_dispatch_kernel<<<ctas, kLocalThreads, plan.bytes, stream>>>(args);
+    // A CTA waits for others at the barrier of a layout that they count together, and for their plans where tokens are claimed:
+    // then every CTA has to be resident.  With a cached layout (whose plan is there) and with a small batch no CTA waits.
+    const bool claims = (a.num_tokens + ctas - 1) / ctas > plan.warps * plan.stages;
+    if (!a.cached && (!whole || claims)) return cooperative_launch(kernel, args, dim3(ctas), kLocalThreads, bytes, stream);
+    kernel<<<ctas, kLocalThreads, bytes, stream>>>(args);
     return cudaGetLastError();
 }
 

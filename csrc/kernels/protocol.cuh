@@ -290,6 +290,8 @@ struct LocalPlan {
     int stages = 0;      // row buffers per such warp
     int slot_bytes = 0;  // bytes of a row buffer
     std::size_t rows_off = 0, bytes = 0;
+    std::size_t whole_off = 0;  // tables of a batch that every CTA counts by itself, in what is left over
+    int whole_bytes = 0;
     bool usable = false;
 };
 

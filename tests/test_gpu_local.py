@@ -266,3 +266,60 @@ def test_plans_of_both_kernels_are_the_same(one_rank, tokens, capacity, experts,
                 del got
             del fresh, plan
         del want
+
+
+# at the most pairs that every CTA counts by itself and one token beyond, pairs across words, the widest and the narrowest top-k,
+# experts up to and beyond those that are counted with ballots
+@pytest.mark.parametrize("tokens,topk,experts,channels", [(1, 1, 1, 1), (33, 3, 7, 4), (1003, 3, 9, 32), (2048, 8, 64, 128), (2049, 8, 64, 128), (700, 4, 65, 16),
+                                                          (512, 32, 600, 20), (513, 32, 600, 20), (16384, 1, 5, 64), (16385, 1, 5, 64), (149, 32, 33, 3)])
+@pytest.mark.parametrize("routes", ["some", "one expert", "none"])
+def test_small_and_large_batches_lay_out_alike(one_rank, tokens, topk, experts, channels, routes):
+    """Every CTA counts a small batch by itself, a large one is counted together behind a barrier: both as the general kernel,
+    on the caller's stream and with fewer CTAs beside it, several times in a row."""
+    from pcie_ep_b200 import HostStagedConfig, HostStagedEPBuffer
+
+    gen = torch.Generator(device="cuda").manual_seed(tokens + topk)
+    x = torch.randn(tokens, 64, device="cuda", generator=gen).to(torch.bfloat16)
+    idx = torch.rand(tokens, experts, device="cuda", generator=gen).topk(topk, dim=1).indices
+    if routes == "some":
+        idx[torch.rand(tokens, topk, device="cuda", generator=gen) < 0.3] = -1
+    else:
+        idx[:, 1:] = -1
+        idx[:, 0] = experts - 1 if routes == "one expert" else -1
+    w = torch.rand(tokens, topk, device="cuda", generator=gen)
+    with HostStagedEPBuffer(one_rank, tokens, 64, topk, experts, HostStagedConfig(channels=channels, output_pool_size=4)) as buffer:
+        def dispatch(general, **how):
+            buffer.runtime.set_test_prefix_delay_ns(1 if general else 0)  # a hook of the protocol: the general kernel takes the call
+            return buffer.dispatch(x, idx, w, do_expand=True, expert_alignment=4, do_zero_padding=True, **how)
+
+        want = dispatch(True)
+        buffer.check_errors(want[3])
+        rows, epoch = int(want[3].expert_offsets[-1]), int(buffer.runtime.epochs()[0])
+        for number, how in enumerate([{}, dict(async_with_compute_stream=True), {}]):
+            got = dispatch(False, **how)
+            got[4].wait()
+            buffer.check_errors(got[3])
+            assert_same_result(got, want, rows, channels, False)
+            assert int(got[3].stats[6]) == int((idx >= 0).any(1).sum()) and int(buffer.runtime.epochs()[0]) == epoch + number + 1
+            begin, end = got[3].transport_timestamps_ns.tolist()
+            assert 0 < begin < end
+            del got
+        again = dispatch(True)  # the general kernel finds the epoch that the others left
+        buffer.check_errors(again[3])
+        assert_same_result(again, want, rows, channels, False)
+        del again, want
+
+
+@pytest.mark.parametrize("tokens,bad", [(40, 99), (40, -2), (5000, 99)])
+def test_invalid_routes_are_an_error_whoever_counts_them(one_rank, tokens, bad):
+    from pcie_ep_b200 import HostStagedConfig, HostStagedEPBuffer
+
+    with HostStagedEPBuffer(one_rank, tokens, 64, 8, 16, HostStagedConfig(channels=8)) as buffer:
+        x = torch.randn(tokens, 64).to(torch.bfloat16).cuda()
+        idx = torch.rand(tokens, 16).topk(8, dim=1).indices
+        idx[tokens - 3, 5] = bad
+        handle = buffer.dispatch(x, idx.cuda(), do_expand=True)[3]
+        with pytest.raises(RuntimeError, match="EP dispatch GPU error"):
+            buffer.check_errors(handle)
+        assert handle.error.tolist()[1:3] == [tokens - 3, 5]
+        del handle
