@@ -71,7 +71,7 @@ def resolve_alignment(requested: Any, inherited: Optional[int], upper: Optional[
     return value
 
 
-@dataclass
+@dataclass(slots=True)
 class DispatchRequest:
     """A dispatch call after validation: what the native runtime needs, nothing else."""
 
@@ -102,11 +102,13 @@ def build_dispatch_request(owner: Any, x: Any, topk_idx: Any, topk_weights: Any,
         topk_idx = handle.topk_idx
     if do_zero_padding and not do_expand:
         raise ValueError("do_zero_padding pads expert segments, which exist only with do_expand=True")
-    alignment = resolve_alignment(expert_alignment, getattr(handle, "expert_alignment", None), alignment_limit)
-    for name, given, prepared in (("num_experts", num_experts, owner.num_experts),
-                                  ("num_max_tokens_per_rank", num_max_tokens_per_rank, owner.num_max_tokens_per_rank)):
-        if given is not None and given != prepared:
-            raise ValueError(f"{name}={given} contradicts the buffer, which was built for {prepared}")
+    alignment = 1 if expert_alignment is None and handle is None else resolve_alignment(
+        expert_alignment, getattr(handle, "expert_alignment", None), alignment_limit)
+    if num_experts is not None or num_max_tokens_per_rank is not None:
+        for name, given, prepared in (("num_experts", num_experts, owner.num_experts),
+                                      ("num_max_tokens_per_rank", num_max_tokens_per_rank, owner.num_max_tokens_per_rank)):
+            if given is not None and given != prepared:
+                raise ValueError(f"{name}={given} contradicts the buffer, which was built for {prepared}")
     device, on_gpu = owner.device, owner.on_gpu
     # the runtime answers "all as the rules below want it" in one call; the rules say what is wrong if it is not
     if not (on_gpu and owner.runtime.accepts_inputs(x, topk_idx, topk_weights)):

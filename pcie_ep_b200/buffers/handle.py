@@ -19,7 +19,7 @@ if TYPE_CHECKING:  # pragma: no cover
 
 def _fingerprint(tensor: torch.Tensor) -> tuple:
     """Everything that makes a tensor 'the same memory seen the same way' (not its contents)."""
-    return (id(tensor), tensor.data_ptr(), tuple(tensor.shape), tuple(tensor.stride()), tensor.dtype, tensor.device)
+    return (id(tensor), tensor.data_ptr(), tensor.shape, tensor.stride(), tensor.dtype, tensor.device)
 
 
 class RouteBinding:
@@ -119,18 +119,18 @@ class HostStagedEPHandle(_Routed):
     time on fields nobody reads.
     """
 
+    num_sms = 0
+    num_recv_tokens_per_expert_list = None
+
     def __init__(self, owner: "HostStagedEPBuffer", topk_idx: torch.Tensor, result: Dict[str, Any], do_expand: bool,
                  expert_alignment: int, event: EventOverlap) -> None:
         self._owner = owner
         self._route = RouteBinding(topk_idx)
         self._result = result
-        self._layout = result.get("_layout")
         self.buffer_id, self.generation = owner.buffer_id, owner._generation
         self.group, self.global_ranks = owner.group, owner.global_ranks
         self.num_experts, self.num_max_tokens_per_rank = owner.num_experts, owner.num_max_tokens_per_rank
         self.do_expand, self.expert_alignment = do_expand, expert_alignment
-        self.num_sms = 0
-        self.num_recv_tokens_per_expert_list = None
         self.completion = event
         self._completion_event = event.event
 
@@ -138,6 +138,8 @@ class HostStagedEPHandle(_Routed):
         # reached only for names that __init__ did not set: resolve against the native result and remember
         if name == "psum_num_recv_tokens_per_scaleup_rank":
             value = self._result["source_offsets"][1:]
+        elif name == "_layout":  # the native routing plan, or None
+            value = self._result.get("_layout")
         else:
             key = _RESULT_FIELDS.get(name)
             if key is None:

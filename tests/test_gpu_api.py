@@ -253,3 +253,16 @@ def test_large_and_small_buffers_alive_together(world1):
     finally:
         small.close()
         large.close()
+
+
+def test_events_are_recorded_again_only_when_nobody_holds_them(ext):
+    """Events come from a pool; one that a token, a handle or a caller still refers to is left alone."""
+    from pcie_ep_b200.buffers.streams import StreamPolicy
+
+    policy = StreamPolicy(torch.cuda.current_device(), True)
+    held = [policy.event() for _ in range(20)]
+    assert len({id(e) for e in held}) == 20 and len(policy._events) == 16
+    kept, query = held[3], held[5].query
+    del held
+    seen = {id(policy.event()) for _ in range(40)}
+    assert len(seen) == 14 and id(kept) not in seen and id(query.__self__) not in seen
