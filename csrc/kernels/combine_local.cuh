@@ -133,6 +133,7 @@ __global__ void __launch_bounds__(kCombineLocalThreads, 1) local_combine_push_ke
     const int Tc = max(1, (T + C - 1) / C);  // tokens per channel: no channel has more entries
     const long long units = static_cast<long long>((T + Tc - 1) / Tc) * Tc * a.shape.slices;
     const bool fixed = units <= static_cast<long long>(kCombineLocalFixedRounds) * kBatch * gridDim.x;
+    ptx::wait_for_launch_before();  // (the expert GEMM, usually)
     const std::uint64_t t_start = threadIdx.x == 0 ? ptx::globaltimer_ns() : 0;
     if (threadIdx.x == 0 && !fixed) atomicMin(a.first_start, static_cast<unsigned long long>(t_start));
     const bool aborted = ptx::ld_volatile(&rc->sticky[0]) != 0;

@@ -260,8 +260,15 @@ grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_rows, const __gr
         tmem_alloc(&sh->tmem_base, kTmemCols);
         tmem_relinquish();
     }
+    // Up to here nothing was read that an earlier launch writes: the launch behind another kernel of the layer gets this far while
+    // the last CTAs of that one are still at work (a layer of 64 tokens 459 -> 454 us, of which two launches gain).
+    ptx::wait_for_launch_before();
+    ptx::let_next_launch_start();
     int most_rows = 1;  // of any expert
-    for (int e = threadIdx.x; e < p.num_experts; e += kThreads) most_rows = max(most_rows, p.expert_counts[e]);
+    for (int e = threadIdx.x; e < p.num_experts; e += kThreads) {
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(p.expert_offsets + e));  // asked for again at the first tile
+        most_rows = max(most_rows, p.expert_counts[e]);
+    }
     most_rows = __reduce_max_sync(0xffffffffu, most_rows);
     if (lane == 0) sh->most_rows[warp] = most_rows;
     tc_fence_before();
@@ -563,8 +570,17 @@ cudaError_t launch(const ActivationMaps& maps_rows, const CUtensorMap& map_w, co
         if (status != cudaSuccess) return status;
         configured[device] = true;
     }
-    grouped_gemm_kernel<kSwiGLU, kFp8, kScatter><<<sms / 2 * 2, kThreads, smem, stream>>>(maps_rows, map_w, p);
-    return cudaGetLastError();
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(static_cast<unsigned>(sms / 2 * 2));
+    config.blockDim = dim3(kThreads);
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    cudaLaunchAttribute attribute[1];
+    attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute[0].val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = attribute;
+    config.numAttrs = 1;
+    return cudaLaunchKernelEx(&config, grouped_gemm_kernel<kSwiGLU, kFp8, kScatter>, maps_rows, map_w, p);
 }
 
 }  // namespace

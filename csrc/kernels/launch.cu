@@ -145,8 +145,17 @@ cudaError_t launch_combine_local(const CombineLocalArgs& args, cudaStream_t stre
             configured[device] = args.shape.bytes;
         }
     }
-    kernel<<<args.shape.ctas, kCombineLocalThreads, args.shape.bytes, stream>>>(args);
-    return cudaGetLastError();
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(static_cast<unsigned>(args.shape.ctas));
+    config.blockDim = dim3(kCombineLocalThreads);
+    config.dynamicSmemBytes = args.shape.bytes;
+    config.stream = stream;
+    cudaLaunchAttribute attribute[1];
+    attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // its CTAs come where those of the expert GEMM have ended
+    attribute[0].val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = attribute;
+    config.numAttrs = 1;
+    return cudaLaunchKernelEx(&config, kernel, args);
 }
 
 cudaError_t launch_combine(const CombineLaunch& launch, int channels, std::size_t crow_stride, cudaStream_t stream) {

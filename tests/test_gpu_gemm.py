@@ -187,3 +187,48 @@ def test_swiglu_of_extreme_gates(ext):
     same = ~want.isnan()
     # a rounding to BF16; below -88 the 32-bit exponential is infinite and the quotient zero
     assert bool(((got.float() - want)[same].abs() <= want[same].abs() * 2.0 ** -8 + 1e-36).logical_or(got.float()[same] == want[same]).all())
+
+
+@pytest.mark.parametrize("side_stream", [False, True])
+def test_launches_that_start_early_see_what_the_ones_before_wrote(ext, side_stream):
+    """The GEMM's CTAs come where those of the launch before have ended: its operands, counts and offsets are written by kernels
+    directly in front of it and overwritten directly behind it, on the default stream and on another, eagerly and in a graph."""
+    experts, rows, k, n = 8, 40, 1024, 512
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    base = torch.randn(experts * rows, k, device="cuda", generator=gen).to(torch.bfloat16)
+    up = (torch.randn(experts, n, k, device="cuda", generator=gen) * 0.05).to(torch.bfloat16)
+    down = (torch.randn(experts, k, n, device="cuda", generator=gen) * 0.05).to(torch.bfloat16)
+    offsets, counts = torch.arange(experts + 1, dtype=torch.int32, device="cuda") * rows, torch.full((experts,), rows, dtype=torch.int32, device="cuda")
+    x, at, count = torch.zeros_like(base), torch.zeros_like(offsets), torch.zeros_like(counts)
+    h = torch.zeros(experts * rows, n, dtype=torch.bfloat16, device="cuda")
+    y, status = torch.zeros_like(base), torch.zeros(4, dtype=torch.int32, device="cuda")
+
+    def layer(scale):
+        at.copy_(offsets)
+        count.copy_(counts)
+        torch.mul(base, scale, out=x)
+        grouped_gemm(x, up, at, count, out=h, status=status)
+        grouped_gemm(h, down, at, count, out=y, status=status)
+        got = y.clone()
+        for t in (x, h, y, at, count):
+            t.zero_()
+        return got
+
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream() if side_stream else torch.cuda.current_stream()
+    with torch.cuda.stream(stream):
+        results = [layer(2.0 ** (i % 3)) for i in range(60)]
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        replayed = layer(2.0)
+    for _ in range(20):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert status.tolist() == [0, 0, 0, 0]
+    # scaling by two is exact all the way
+    want = torch.cat([(base[e * rows:(e + 1) * rows].double() @ up[e].double().t()).to(torch.bfloat16).double() @ down[e].double().t() for e in range(experts)])
+    assert float((results[0].double() - want).norm() / want.norm()) < 2.0 ** -8
+    for i, got in enumerate(results):
+        assert torch.equal(got, results[0] * 2.0 ** (i % 3)), i
+    assert torch.equal(replayed, results[1])
