@@ -16,6 +16,22 @@ import torch
 _POOLED_EVENTS = 16
 
 
+def _references(objects: List[Any], index: int) -> int:
+    """References to ``objects[index]`` as the interpreter counts them from here, the list's and the call's own among them."""
+    return sys.getrefcount(objects[index])
+
+
+def _references_of_list_only() -> Optional[int]:
+    """What ``_references`` says of an object that nothing but the list holds.  How many references a call adds is the
+    interpreter's affair, so it is counted, not assumed; None where one more holder does not count as exactly one more."""
+    objects = [object()]
+    alone = _references(objects, 0)
+    holder = objects[0]
+    counted = _references(objects, 0) == alone + 1
+    del holder
+    return alone if counted and _references(objects, 0) == alone else None
+
+
 class NullStream:
     """Stands in for a CUDA stream on the CPU transport: every operation is already ordered."""
 
@@ -54,6 +70,7 @@ class StreamPolicy:
         # reader is the stream itself" is a comparison of identities
         self._known: Dict[int, Any] = {}
         self._events: List[Any] = []
+        self._unheld = _references_of_list_only()
         self._next_event = 0
         # work was queued on the communication stream that the compute stream has not waited for yet
         self._comm_ahead = False
@@ -75,11 +92,10 @@ class StreamPolicy:
         events = self._events
         for _ in range(len(events)):
             self._next_event = (self._next_event + 1) % len(events)
-            event = events[self._next_event]
-            if sys.getrefcount(event) == 3:  # the list, this name and the call's argument
-                return event
+            if _references(events, self._next_event) == self._unheld:
+                return events[self._next_event]
         event = torch.cuda.Event()
-        if len(events) < _POOLED_EVENTS:
+        if self._unheld is not None and len(events) < _POOLED_EVENTS:
             events.append(event)
         return event
 
