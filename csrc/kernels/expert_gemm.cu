@@ -124,6 +124,19 @@ __device__ __forceinline__ void tmem_ld_32x32(std::uint32_t taddr, std::uint32_t
         : "r"(taddr)
         : "memory");
 }
+// 16 lanes x 32 columns: thread t gets, for j = 0..3, columns 8j + 2(t % 4) + {0, 1} of lane t / 4 in r[4j], r[4j + 1] and of lane
+// t / 4 + 8 in r[4j + 2], r[4j + 3]: the fragments that stmatrix stores
+__device__ __forceinline__ void tmem_ld_16x32(std::uint32_t taddr, std::uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+                   "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr)
+                 : "memory");
+}
+// four transposed 8 x 8 matrices of 16-bit values: lane l gives the address of row l % 8 of matrix l / 8
+__device__ __forceinline__ void stmatrix_transposed(std::uint32_t addr, std::uint32_t m0, std::uint32_t m1, std::uint32_t m2, std::uint32_t m3) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(m0), "r"(m1), "r"(m2), "r"(m3) : "memory");
+}
 // (the registers pass through, so that nothing reads or copies them before the loads have arrived)
 __device__ __forceinline__ void tmem_ld_wait(std::uint32_t (&r)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;"
@@ -232,6 +245,7 @@ grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_rows, const __gr
     unsigned char* tiles = smem;
     unsigned char* staging = smem + kRingBytes;
     auto* sh = reinterpret_cast<GemmShared*>(staging + 2 * kChunkRows * kPitch);
+    auto* targets = reinterpret_cast<RowTargets*>(sh + 1);  // scatter only
     volatile int* abort = &sh->abort;
 
     const int warp = threadIdx.x >> 5;
@@ -390,15 +404,55 @@ grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_rows, const __gr
         constexpr int kLanesPerRow = kChannels / 8;             // 16-byte pieces of a row
         constexpr int kRowsPerStore = 32 / kLanesPerRow;
         const int piece = lane % kLanesPerRow, store_row = q * (kChunkRows / 4) + lane / kLanesPerRow;
+        // Scatter: where the rows of a tile go and their weights, two rows per thread, asked for a tile ahead.  Asked for in their own
+        // chunk, every 32 rows waited for L2, and with a short K the epilogue was longer than the MMAs of its tile: 2000 tokens,
+        // top-8 of 32 experts, 768 -> 2048, GEMM and sum 107 -> 91 us.
+        TileWalk ahead = walk;
+        int owner[2], token[2], slot[2];
+        float weight[2];
+        auto ask_targets = [&]() {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int in_tile = static_cast<int>(threadIdx.x) - 64 + 128 * i;
+                owner[i] = -1;
+                if (in_tile >= ahead.tile_rows) continue;
+                const long long r = static_cast<long long>(ahead.row0) + in_tile;
+                const long long* meta = sc.source_meta + r * 3;
+                owner[i] = static_cast<int>(meta[0]);
+                token[i] = static_cast<int>(meta[1]);
+                slot[i] = static_cast<int>(meta[2]);
+                weight[i] = sc.row_weights != nullptr ? sc.row_weights[r] : 1.0f;
+            }
+        };
+        // into shared memory: what was there was read two tiles ago, and all warps have met since then (epilogue_all)
+        auto store_targets = [&](int rows, int buf, int first_channel) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int in_tile = static_cast<int>(threadIdx.x) - 64 + 128 * i;
+                if (in_tile >= rows) continue;
+                unsigned long long dst = 0;
+                if (owner[i] >= 0 && owner[i] < sc.num_ranks && slot[i] >= 0 && slot[i] < sc.num_topk && token[i] >= 0)
+                    dst = reinterpret_cast<unsigned long long>(sc.seg[owner[i]] + sc.stage_off +
+                                                               (static_cast<std::size_t>(token[i]) * sc.num_topk + slot[i]) * static_cast<std::size_t>(sc.row_stride) +
+                                                               static_cast<std::size_t>(first_channel) * 2);
+                targets->dst[buf][in_tile] = dst;
+                targets->weight[buf][in_tile] = weight[i];
+            }
+        };
+        if (kScatter && ahead.next(p)) ask_targets();
         int it = 0, half = 0;
         for (; walk.next(p); ++it) {
             const int buf = it & 1;
             const unsigned acc_phase = (it >> 1) & 1u;
+            const int first_channel = (walk.m_tile * 2 + static_cast<int>(rank)) * kChannels;
+            const bool inside = first_channel < p.n;  // n an odd multiple of 128: the last tile has one CTA's channels only
+            if (kScatter) {
+                store_targets(walk.tile_rows, buf, first_channel);
+                if (ahead.next(p)) ask_targets();
+            }
             // all four warps go on or none: they meet at the barriers below
             if (!epilogue_all(mbar_wait(&sh->tmem_full[buf], acc_phase, abort))) break;
             tc_fence_after();
-            const int first_channel = (walk.m_tile * 2 + static_cast<int>(rank)) * kChannels;
-            const bool inside = first_channel < p.n;  // n an odd multiple of 128: the last tile has one CTA's channels only
             float w_first = 1.0f, w_up = 1.0f;  // FP8: scale of the weight row(s) of this lane's channel
             if (kFp8 && inside) {
                 const float* w_scale = p.w_scales + static_cast<long long>(walk.expert) * (kSwiGLU ? 2 : 1) * p.n + first_channel + channel;
@@ -422,7 +476,15 @@ grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_rows, const __gr
 #pragma unroll 1
             for (int c0 = 0; c0 < walk.tile_rows; c0 += kChunkRows) {
                 std::uint32_t v[32];
-                tmem_ld_32x32(acc + c0, v);
+                float2 weights[4];  // scatter: of the rows that this thread's registers hold
+                if constexpr (kScatter) {
+                    tmem_ld_16x32(acc + c0, v);
+                    tmem_ld_16x32(acc + (16u << 16) + c0, v + 16);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) weights[j] = *reinterpret_cast<const float2*>(&targets->weight[buf][c0 + 8 * j + 2 * (lane & 3)]);
+                } else {
+                    tmem_ld_32x32(acc + c0, v);
+                }
                 // what belongs to the chunk's rows, one row per lane
                 float row_factor = 1.0f;
                 unsigned long long dst_next = 0;
@@ -430,13 +492,7 @@ grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_rows, const __gr
                     const long long r = static_cast<long long>(walk.row0) + c0 + lane;
                     if (kFp8) row_factor = p.a_scales[r];
                     if (kScatter) {
-                        const long long* meta = sc.source_meta + r * 3;
-                        const int owner = static_cast<int>(meta[0]), token = static_cast<int>(meta[1]), slot = static_cast<int>(meta[2]);
-                        if (sc.row_weights != nullptr) row_factor = sc.row_weights[r];
-                        if (owner >= 0 && owner < sc.num_ranks && slot >= 0 && slot < sc.num_topk && token >= 0)
-                            dst_next = reinterpret_cast<unsigned long long>(sc.seg[owner] + sc.stage_off +
-                                                                            (static_cast<std::size_t>(token) * sc.num_topk + slot) * static_cast<std::size_t>(sc.row_stride) +
-                                                                            static_cast<std::size_t>(first_channel) * 2);
+                        dst_next = targets->dst[buf][c0 + lane];
                     } else {
                         dst_next = reinterpret_cast<unsigned long long>(p.out + r * p.n + first_channel);
                     }
@@ -467,12 +523,26 @@ grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_rows, const __gr
                         const float silu = quotient(gate, 1.0f + __expf(-gate)) * up;
                         *reinterpret_cast<__nv_bfloat16*>(to + (2 * i + (upper ? 1 : 0)) * kPitch) = __float2bfloat16_rn(silu);
                     }
+                } else if constexpr (kScatter) {
+                    // 8 rows x 32 channels at a time, turned round by the matrix stores: 4 of them instead of 32 stores of 2 bytes and
+                    // 32 shuffles of the weights (the same tokens 91 -> 86 us; 4096 tokens, 2048 -> 7168, inside a layer 800 -> 780)
+                    const std::uint32_t at = smem_addr(staging + (half * kChunkRows + (lane & 7)) * kPitch + (q * 32 + (lane >> 3) * 8) * 2);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        std::uint32_t m[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const int first = (i >> 1) * 16 + 4 * j + (i & 1) * 2;
+                            const __nv_bfloat162 packed = __floats2bfloat162_rn(__uint_as_float(v[first]) * weights[j].x, __uint_as_float(v[first + 1]) * weights[j].y);
+                            m[i] = *reinterpret_cast<const std::uint32_t*>(&packed);
+                        }
+                        stmatrix_transposed(at + 8 * j * kPitch, m[0], m[1], m[2], m[3]);
+                    }
                 } else {
 #pragma unroll
                     for (int i = 0; i < 32; ++i) {
                         float value = __uint_as_float(v[i]);
                         if (kFp8) value *= __shfl_sync(0xffffffffu, row_factor, i) * w_first;
-                        if (kScatter) value *= __shfl_sync(0xffffffffu, row_factor, i);
                         *reinterpret_cast<__nv_bfloat16*>(to + i * kPitch) = __float2bfloat16_rn(value);
                     }
                 }
@@ -564,7 +634,7 @@ cudaError_t launch(const ActivationMaps& maps_rows, const CUtensorMap& map_w, co
     int device = 0;
     cudaError_t status = cudaGetDevice(&device);
     if (status != cudaSuccess) return status;
-    constexpr int smem = gemm_smem_bytes(kSwiGLU);
+    constexpr int smem = gemm_smem_bytes(kSwiGLU, kScatter);
     if (device >= 0 && device < 64 && !configured[device]) {
         status = cudaFuncSetAttribute(grouped_gemm_kernel<kSwiGLU, kFp8, kScatter>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (status != cudaSuccess) return status;

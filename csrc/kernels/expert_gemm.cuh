@@ -60,7 +60,7 @@ struct ScatterTarget {
     const float* row_weights;              // [rows] routing weight of the row; nullptr: 1
     unsigned long long stage_off, sig_off, done_off;  // landing area, "rows are here" flags, "area consumed" flags
     unsigned long long epoch;              // number of this fused call (1, 2, ...), the same on every rank
-    unsigned long long* cta_done;          // local monotonic count of finished CTAs over all launches
+    unsigned long long* cta_done;          // CTAs of this launch that have finished; the last one puts it back to zero
     unsigned long long timeout_ns;
     int row_stride;                        // bytes between landing slots
     int num_topk, num_ranks, rank, flag_stride;
@@ -108,17 +108,24 @@ constexpr int kTmemCols = 2 * kAccCols;  // double buffered
 // channels of two rows at once, 32.
 constexpr int kChunkRows = 32;
 __host__ __device__ constexpr int staging_pitch(bool swiglu) { return swiglu ? kCtaM / 2 * 2 + 32 : kCtaM * 2 + 16; }
-struct GemmShared {
+struct alignas(16) GemmShared {
     std::uint64_t full[kMaxStages], empty[kMaxStages], tmem_full[2], tmem_empty[2];
     std::uint32_t tmem_base;
     int abort;
     int most_rows[kThreads / 32];  // of any expert, per warp
 };
-__host__ __device__ constexpr int gemm_smem_bytes(bool swiglu) {
-    return 1024 /* alignment slack */ + kRingBytes + 2 * kChunkRows * staging_pitch(swiglu) + static_cast<int>(sizeof(GemmShared));
+// Scatter: where the rows of a tile go (0: nowhere) and their weights, for two tiles in turn.  Behind the tile's rows lies what was
+// there; what is made of it goes nowhere.
+struct alignas(16) RowTargets {
+    unsigned long long dst[2][kMaxRows];
+    float weight[2][kMaxRows];
+};
+__host__ __device__ constexpr int gemm_smem_bytes(bool swiglu, bool scatter) {
+    return 1024 /* alignment slack */ + kRingBytes + 2 * kChunkRows * staging_pitch(swiglu) + static_cast<int>(sizeof(GemmShared)) +
+           (scatter ? static_cast<int>(sizeof(RowTargets)) : 0);
 }
 static_assert(2 * kChunkRows * staging_pitch(true) % 16 == 0 && 2 * kChunkRows * staging_pitch(false) % 16 == 0, "barriers follow the staging");
-static_assert(gemm_smem_bytes(false) <= 227 * 1024, "one CTA per SM");
+static_assert(gemm_smem_bytes(false, true) <= 227 * 1024, "one CTA per SM");
 
 }  // namespace gemm
 }  // namespace bep

@@ -19,8 +19,7 @@ const char* grouped_gemm(const void* a, const void* w, void* out, const float* a
 
 // Plain BF16 GEMM (n a multiple of 256) whose epilogue, instead of writing an output matrix, multiplies each row
 // by its routing weight and stores it into the token owner's landing slot (see gemm::ScatterTarget); the launch's
-// last CTA publishes target.epoch to every rank.  Every launch on a device must use the same CTA count
-// (grouped_gemm_ctas()) and consecutive epochs, because completion is detected with a monotonic counter.
+// last CTA publishes target.epoch to every rank.  Epochs are consecutive; launches that share target.cta_done are stream-ordered.
 const char* grouped_gemm_scatter(const void* a, const void* w, const int* expert_offsets, const int* expert_counts,
                                  int* status, int rows_capacity, int num_experts, int n, int k,
                                  const gemm::ScatterTarget& target, cudaStream_t stream);

@@ -77,6 +77,47 @@ def test_fused_expert_combine_matches_two_step_path_and_dense_reference(ext, ali
             del results, two_step
 
 
+@pytest.mark.parametrize("counts,hidden,inter", [
+    ([1, 15, 16, 17, 31, 32, 33, 63, 65, 127, 128, 129, 255, 256, 257, 0, 513], 4096, 1600),  # edges of tiles and of chunks, six stages
+    ([1, 7, 8, 9, 15, 16, 2, 0, 3, 12, 16, 5, 11, 6, 16, 1], 7168, 1600),  # one chunk at most, ten stages
+    ([40, 0, 3, 130], 256, 64),  # one block of K, one tile per pair
+])
+@pytest.mark.parametrize("weighted", [True, False])
+def test_scattered_tiles_at_their_edges(ext, counts, hidden, inter, weighted):
+    """Every row of every tile in its token's slot, with its weight, and nothing else: one route per token, some unused slots."""
+    from pcie_ep_b200.parallel.virtual import VirtualEPGroup
+
+    experts, tokens = len(counts), sum(counts)
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    expert = torch.repeat_interleave(torch.arange(experts), torch.tensor(counts))[torch.randperm(tokens, generator=torch.Generator().manual_seed(1))]
+    idx = torch.full((tokens, 2), -1, dtype=torch.int64)
+    idx[torch.arange(tokens), torch.arange(tokens) % 2] = expert  # in the first or the second slot
+    idx = idx.cuda()
+    weights = torch.rand(tokens, 2, device="cuda", generator=gen) + 0.5 if weighted else torch.ones(tokens, 2, device="cuda")
+    x = torch.randn(tokens, hidden, device="cuda", generator=gen).to(torch.bfloat16)
+    h = torch.randn(tokens, inter, device="cuda", generator=gen).to(torch.bfloat16)
+    w2 = (torch.randn(experts, hidden, inter, device="cuda", generator=gen) * 0.05).to(torch.bfloat16)
+    config = HostStagedConfig(channels=4, timeout_ms=5000, fused_expert_combine=True)
+    with VirtualEPGroup(1, tokens, hidden, 2, experts, config) as group:
+        results = group.dispatch([x], [idx], [weights], do_expand=True)
+        for _ in range(2):
+            out = group.fused_expert_combine([h], [w2], results)[0].clone()
+        torch.cuda.synchronize()
+        assert int(group.runtimes[0].fused_status()[0]) == 0 and results[0]["combine_error"].tolist()[0] == 0
+        token = results[0]["source_meta"][:tokens, 1]
+        offsets = results[0]["expert_offsets"].tolist()
+        for e, count in enumerate(counts):
+            rows = slice(offsets[e], offsets[e] + count)
+            of = token[rows]
+            assert torch.equal(torch.sort(of).values.cpu(), torch.nonzero(expert == e).flatten())
+            a, m, w = h[rows].double(), w2[e].double(), weights[of, of % 2].double().unsqueeze(1)
+            want = a @ m.t() * w
+            # K products summed in 32 bits, one factor, one rounding to BF16 (the sum over the slots has a single term)
+            error = (a.abs() @ m.abs().t()) * w * (inter + 4) * 2.0 ** -24
+            assert bool(((out[of].double() - want).abs() <= error + (want.abs() + error) * 2.0 ** -8).all()), count
+        del results, out
+
+
 def test_fused_reduce_gives_up_when_a_rank_never_signals(ext):
     from pcie_ep_b200.parallel.virtual import VirtualEPGroup
 

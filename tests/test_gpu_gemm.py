@@ -91,8 +91,8 @@ def test_grouped_gemm_fp8_matches_dequantised_reference(ext, swiglu):
 @pytest.mark.parametrize("fp8", [False, True])
 @pytest.mark.parametrize("swiglu,n", [(True, 256), (False, 256), (False, 128)])
 def test_last_tiles_at_the_box_heights(ext, fp8, swiglu, n):
-    """Experts whose last tile ends at, before and behind the heights of the activation boxes (32, 64, 128 rows).  The rows
-    around an expert's own hold NaN: what shares a box with it must not reach its results, nor be written."""
+    """Experts whose last tile ends at, before and behind steps of a tile's width (two activation boxes of 8 to 128 rows).  The
+    rows around an expert's own hold NaN: what shares a box with it must not reach its results, nor be written."""
     counts = [31, 32, 33, 0, 63, 64, 65, 127, 128, 1, 128 + 32, 128 + 33, 128 + 64, 128 + 65]
     k, experts = 384, len(counts)
     offsets = torch.zeros(experts + 1, dtype=torch.int32)
@@ -136,10 +136,22 @@ def test_last_tiles_at_the_box_heights(ext, fp8, swiglu, n):
 @pytest.mark.parametrize("swiglu", [True, False])
 @pytest.mark.parametrize("k", [128, 1152])
 def test_tiles_of_every_width(ext, fp8, swiglu, k):
-    """Tiles of 32 to 256 rows (one expert each, and several chunks per expert), K shorter and longer than the ring of stages, and
-    output columns that leave the second CTA of the last pair without channels."""
-    counts = [1, 33, 95, 97, 129, 161, 193, 225, 256, 257, 0, 289, 511, 513, 770, 1025]
-    n, experts = 384, len(counts)
+    """Tiles of 16 to 256 rows in steps of 16 (one expert each, and several chunks per expert), K shorter and longer than the ring
+    of stages, and output columns that leave the second CTA of the last pair without channels."""
+    _check_tiles([1, 17, 33, 49, 65, 81, 97, 113, 129, 145, 161, 177, 193, 209, 225, 256, 257, 0, 289, 511, 513, 770, 1025], 384, k, fp8, swiglu)
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("swiglu", [True, False])
+@pytest.mark.parametrize("widest", [16, 48, 80, 112, 144, 176, 224])
+def test_rings_of_every_depth(ext, fp8, swiglu, widest):
+    """The ring has as many stages as fit for the widest tile of the launch (ten for 16 rows, six for 224).  Twenty-five K blocks a
+    tile and several tiles per pair of CTAs: the ring turns over many times, at another stage in every tile."""
+    _check_tiles([widest if e % 5 == 0 else max(1, widest - 7 * (e % 9)) for e in range(24)], 2048, 25 * (128 if fp8 else 64), fp8, swiglu)
+
+
+def _check_tiles(counts, n, k, fp8, swiglu):
+    experts = len(counts)
     offsets, cnts = _layout(counts)
     rows = int(offsets[-1])
     gen = torch.Generator(device="cuda").manual_seed(k)
