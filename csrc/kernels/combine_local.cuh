@@ -133,7 +133,9 @@ __global__ void __launch_bounds__(kCombineLocalThreads, 1) local_combine_push_ke
     const int Tc = max(1, (T + C - 1) / C);  // tokens per channel: no channel has more entries
     const long long units = static_cast<long long>((T + Tc - 1) / Tc) * Tc * a.shape.slices;
     const bool fixed = units <= static_cast<long long>(kCombineLocalFixedRounds) * kBatch * gridDim.x;
-    ptx::wait_for_launch_before();  // (the expert GEMM, usually)
+    // The launch before is the expert GEMM, usually, or the dispatch whose map is read below.  Reads of what it may have written are
+    // ordinary loads: one that counts on memory staying as it is for the whole kernel (ld.global.nc) may be moved in front of the wait.
+    ptx::wait_for_launch_before();
     const std::uint64_t t_start = threadIdx.x == 0 ? ptx::globaltimer_ns() : 0;
     if (threadIdx.x == 0 && !fixed) atomicMin(a.first_start, static_cast<unsigned long long>(t_start));
     const bool aborted = ptx::ld_volatile(&rc->sticky[0]) != 0;
@@ -164,9 +166,9 @@ __global__ void __launch_bounds__(kCombineLocalThreads, 1) local_combine_push_ke
             e.j = entry % Tc;
             // (entries beyond the channel's count hold what an earlier dispatch left: read, not used)
             const int* map = a.comb_map + (static_cast<std::size_t>(c) * a.slots_full + e.j) * map_stride;
-            e.count = __ldg(a.recv_chan_counts + c);
-            e.head = __ldg(reinterpret_cast<const int2*>(map));
-            if (lane < K) e.pair = __ldg(reinterpret_cast<const int2*>(map) + 1 + lane);
+            e.count = a.recv_chan_counts[c];
+            e.head = *reinterpret_cast<const int2*>(map);
+            if (lane < K) e.pair = reinterpret_cast<const int2*>(map)[1 + lane];
             return e;
         };
         auto claim = [&]() {
@@ -234,7 +236,7 @@ __global__ void __launch_bounds__(kCombineLocalThreads, 1) local_combine_push_ke
         // ---- consumers ---------------------------------------------------------------------------------------------
         const int consumer = warp - 1, rank = consumer * 32 + lane;  // first chunk of this thread in a slice
         const int first_zero = blockIdx.x * kCombineLocalConsumers + consumer, zero_step = gridDim.x * kCombineLocalConsumers;
-        const std::uint32_t first_mask = first_zero < T ? __ldg(a.plan_mask + first_zero) : 1u;  // needed at the end
+        const std::uint32_t first_mask = first_zero < T ? a.plan_mask[first_zero] : 1u;  // needed at the end
         for (int f = 0;; ++f) {
             const int stage = f % stages;
             ok = __all_sync(0xffffffffu, wait(&sh->full[stage], static_cast<unsigned>(f / stages) & 1u)) != 0;
@@ -269,7 +271,7 @@ __global__ void __launch_bounds__(kCombineLocalThreads, 1) local_combine_push_ke
         }
         // tokens that were routed nowhere have no entry: their result is zero
         for (int t = first_zero; ok && t < T; t += zero_step) {
-            if ((t == first_zero ? first_mask : __ldg(a.plan_mask + t)) != 0) continue;
+            if ((t == first_zero ? first_mask : a.plan_mask[t]) != 0) continue;
             for (int q = lane; q < chunks; q += 32)
                 ptx::st_v4(reinterpret_cast<std::uint8_t*>(a.out) + static_cast<std::size_t>(t) * row_bytes + static_cast<std::size_t>(q) * 16, make_uint4(0u, 0u, 0u, 0u));
         }
@@ -286,7 +288,7 @@ __global__ void __launch_bounds__(kCombineLocalThreads, 1) local_combine_push_ke
             // launches that share these counters are stream-ordered
             int rows = 0;
             if (!aborted)
-                for (int c = lane; c < C; c += 32) rows += __ldg(a.recv_chan_counts + c);
+                for (int c = lane; c < C; c += 32) rows += a.recv_chan_counts[c];
             rows = __reduce_add_sync(0xffffffffu, rows);
             if (lane == 0) {
                 std::uint64_t first = t_start;

@@ -275,7 +275,8 @@ grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_rows, const __gr
         tmem_relinquish();
     }
     // Up to here nothing was read that an earlier launch writes: the launch behind another kernel of the layer gets this far while
-    // the last CTAs of that one are still at work (a layer of 64 tokens 459 -> 454 us, of which two launches gain).
+    // the last CTAs of that one are still at work (a layer of 64 tokens 459 -> 454 us, of which two launches gain).  What is read from
+    // here on is read by ordinary loads, which stay behind the wait (ld.global.nc need not).
     ptx::wait_for_launch_before();
     ptx::let_next_launch_start();
     int most_rows = 1;  // of any expert
@@ -456,8 +457,8 @@ grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_rows, const __gr
             float w_first = 1.0f, w_up = 1.0f;  // FP8: scale of the weight row(s) of this lane's channel
             if (kFp8 && inside) {
                 const float* w_scale = p.w_scales + static_cast<long long>(walk.expert) * (kSwiGLU ? 2 : 1) * p.n + first_channel + channel;
-                w_first = __ldg(w_scale);
-                if (kSwiGLU) w_up = __ldg(w_scale + p.n);
+                w_first = *w_scale;
+                if (kSwiGLU) w_up = w_scale[p.n];
             }
             const std::uint32_t acc = tmem_base + (static_cast<std::uint32_t>(q * 32) << 16) + buf * kAccCols;
             // (2) of a chunk, see below: a few lanes = one row, its channels of this CTA leave as contiguous 16-byte pieces

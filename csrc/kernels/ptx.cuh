@@ -129,7 +129,8 @@ __device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bu
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 // ---- launches that may start before the one in front of them on the stream has ended ---------
-// everything that launch wrote is visible after this (at once, if there is no such launch)
+// everything that launch wrote is visible after this (at once, if there is no such launch) to loads that stay behind it: not to
+// ld.global.nc (__ldg), which promises that nobody writes while the kernel runs, and this kernel runs beside that launch
 __device__ __forceinline__ void wait_for_launch_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // the next launch may put its CTAs where this one's have ended
 __device__ __forceinline__ void let_next_launch_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
