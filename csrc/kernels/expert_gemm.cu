@@ -146,17 +146,6 @@ __device__ __forceinline__ void tmem_ld_wait(std::uint32_t (&r)[32]) {
                    "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])::"memory");
 }
 
-// a / b for b >= 1 (or infinite): one correction of a * (1 / b) by its remainder (Markstein, "Computation of elementary functions on
-// the IBM RISC System/6000 processor", 1990).  Where the remainder is no number (an infinite operand) the product is the answer.
-// No branch, so that the quotients of a chunk overlap: with the operator a warp took them one after the other and the epilogue of a
-// tile longer than its MMAs where K is 2048 (2000 tokens, intermediate 768: 118 -> 95 us) or the operands are E4M3 (849 -> 749).
-__device__ __forceinline__ float quotient(float a, float b) {
-    float r;
-    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(b));
-    const float q = a * r, remainder = fmaf(-q, b, a);
-    return remainder == remainder ? fmaf(remainder, r, q) : q;
-}
-
 // barrier among the four epilogue warps; true when `ok` held in all of them
 __device__ __forceinline__ bool epilogue_all(bool ok) {
     std::uint32_t all;
@@ -521,7 +510,7 @@ grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_rows, const __gr
                             gate *= a_scale * w_first;
                             up *= a_scale * w_up;
                         }
-                        const float silu = quotient(gate, 1.0f + __expf(-gate)) * up;
+                        const float silu = ptx::quotient(gate, 1.0f + __expf(-gate)) * up;
                         *reinterpret_cast<__nv_bfloat16*>(to + (2 * i + (upper ? 1 : 0)) * kPitch) = __float2bfloat16_rn(silu);
                     }
                 } else if constexpr (kScatter) {

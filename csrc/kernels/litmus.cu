@@ -140,7 +140,19 @@ __global__ void litmus_kernel(std::uint8_t* mine, std::uint8_t* theirs, int role
     }
 }
 
+__global__ void quotients_kernel(const float* a, const float* b, float* out, int n) {
+    const int i = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
+    if (i < n) out[i] = ptx::quotient(a[i], b[i]);
+}
+
 }  // namespace
+
+const char* litmus_quotients(const float* a, const float* b, float* out, int n, cudaStream_t stream) {
+    if (n < 1) return "no values";
+    quotients_kernel<<<(n + 255) / 256, 256, 0, stream>>>(a, b, out, n);
+    const cudaError_t err = cudaGetLastError();
+    return err == cudaSuccess ? nullptr : cudaGetErrorString(err);
+}
 
 const char* litmus_pingpong(void* mine, void* theirs, int role, int rounds, int words, long long* status,
                             unsigned long long timeout_ns, cudaStream_t stream, int method) {

@@ -11,4 +11,7 @@ namespace bep {
 const char* litmus_pingpong(void* mine, void* theirs, int role, int rounds, int words, long long* status,
                             unsigned long long timeout_ns, cudaStream_t stream, int method = 0);
 
+// out[i] = ptx::quotient(a[i], b[i]), the division of the expert GEMM's SwiGLU, in 32 bits
+const char* litmus_quotients(const float* a, const float* b, float* out, int n, cudaStream_t stream);
+
 }  // namespace bep

@@ -276,6 +276,18 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     }, py::arg("a"), py::arg("w"), py::arg("out"), py::arg("expert_offsets"), py::arg("expert_counts"), py::arg("status"),
        py::arg("swiglu"), py::arg("a_scales") = py::none(), py::arg("w_scales") = py::none(), py::arg("stream") = 0);
 
+    m.def("litmus_quotients", [](const at::Tensor& a, const at::Tensor& b) {
+        for (const at::Tensor* t : {&a, &b})
+            if (!t->is_cuda() || t->scalar_type() != at::kFloat || !t->is_contiguous() || t->numel() != a.numel() || t->get_device() != a.get_device() ||
+                t->numel() < 1 || t->numel() > (1 << 30))
+                throw std::invalid_argument("litmus_quotients: two contiguous CUDA FP32 tensors of one size");
+        c10::cuda::CUDAGuard guard(a.device());
+        at::Tensor out = at::empty_like(a);
+        const char* error = litmus_quotients(a.data_ptr<float>(), b.data_ptr<float>(), out.data_ptr<float>(), static_cast<int>(a.numel()),
+                                             at::cuda::getCurrentCUDAStream().stream());
+        if (error != nullptr) throw std::runtime_error(std::string("litmus_quotients: ") + error);
+        return out;
+    }, py::arg("a"), py::arg("b"), "the SwiGLU division of the expert GEMM, element by element");
     m.def("litmus", [](std::int64_t mine, std::int64_t theirs, int role, int rounds, int words, at::Tensor& status,
                        int timeout_ms, int device, int method) {
         if (!status.is_cuda() || status.scalar_type() != at::kLong || status.numel() < (role < 0 ? 8 : 4))

@@ -201,6 +201,31 @@ def test_swiglu_of_extreme_gates(ext):
     assert bool(((got.float() - want)[same].abs() <= want[same].abs() * 2.0 ** -8 + 1e-36).logical_or(got.float()[same] == want[same]).all())
 
 
+def test_swiglu_division_in_32_bits(ext):
+    """gate / (1 + exp(-gate)) before anything rounds it to BF16, and the division alone over all exponents, against 64 bits.  The
+    bound: half a unit in the last place and 2^-20 of one, two units of the subnormal numbers (the remainder may be one), and |a| of
+    them where the reciprocal of b is."""
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    gate = torch.cat([torch.randn(1 << 20, device="cuda", generator=gen) * 4, torch.linspace(-89, 89, 1 << 20, device="cuda"),
+                      torch.linspace(-1e-3, 1e-3, 1 << 16, device="cuda")])
+    mantissa = torch.rand(1 << 20, device="cuda", generator=gen) + 1.0
+    exponent = torch.randint(0, 128, (1 << 20,), device="cuda", generator=gen)
+    wide = torch.ldexp(torch.rand(1 << 20, device="cuda", generator=gen) * 2 - 1, torch.randint(-100, 127, (1 << 20,), device="cuda", generator=gen))
+    a = torch.cat([gate, wide])
+    b = torch.cat([1.0 + torch.exp(-gate), torch.ldexp(mantissa, exponent)])
+    got, finite = ext.litmus_quotients(a, b), b.isfinite()
+    want = a.double() / b.double()
+    error = (got.double() - want).abs()
+    bound = want.abs() * 2.0 ** -24 * (1 + 2.0 ** -20) + torch.where(b >= 2.0 ** 126, a.abs().double() + 2, 2.0) * 2.0 ** -149
+    assert bool((error <= bound)[finite].all()), (error / bound)[finite].max()
+    # an infinite sum, and operands that are no numbers: as the operator has it
+    inf, nan = float("inf"), float("nan")
+    a = torch.tensor([-88.9, -inf, inf, 0.0, -0.0, nan, 1.0, inf, 3e38, -3e38], device="cuda")
+    b = torch.tensor([inf, inf, 1.0, 2.0, 2.0, inf, nan, inf, 1.0, inf], device="cuda")
+    got, want = ext.litmus_quotients(a, b), a / b
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got[~want.isnan()], want[~want.isnan()])
+
+
 @pytest.mark.parametrize("side_stream", [False, True])
 def test_launches_that_start_early_see_what_the_ones_before_wrote(ext, side_stream):
     """The GEMM's CTAs come where those of the launch before have ended: its operands, counts and offsets are written by kernels
