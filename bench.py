@@ -485,11 +485,11 @@ def run_ours(args, rank, world, local_rank):
         stamps = res[3].transport_timestamps_ns.cpu().tolist()
         kernel_us = (stamps[1] - stamps[0]) / 1000.0
         del res
-        kernels = ["dispatch_kernel"]
+        kernels = ["local_dispatch_kernel" if buffer.runtime.dispatch_is_local() else "dispatch_kernel"]
         if buffer.runtime.combine_is_inline():
             kernels.append("combine_kernel")
         else:
-            kernels.append("combine_push_kernel")
+            kernels.append("local_combine_push_kernel" if buffer.runtime.combine_is_local() else "combine_push_kernel")
             if buffer.runtime.combine_is_split():
                 kernels.append("fused_reduce_kernel")
         result = {

@@ -8,11 +8,11 @@
 // two stages in shared memory allow -- a whole row of 7168 with top-8 -- and one bulk copy: 95 us, and 104 us with half rows.
 //
 // Work unit = (entry of the combine map, slice of its rows).  A CTA's first units are its own, the others come from a
-// counter: SMs do not all get the same share of HBM, and equal shares waited for the slowest (125 us).  The producer warp
+// counter (launches of a few units per CTA: in a fixed order, kCombineLocalFixedRounds): SMs do not all get the same share of HBM, and equal shares waited for the slowest (125 us).  The producer warp
 // keeps the claim after next and the map entries of the next units on their way while it starts the copies of the present
 // ones; a round of that takes 1.4 us, so small units are claimed four at a time (2048 tokens, a row each: 25.5 -> 21.9 us).
 // Before, through the multi-rank reducers (combine_push.cuh): 111 us, 139 us for 8192 tokens top-4 (now 103), 22 us for 128
-// tokens (now 11).  The other warps add the rows out of shared memory in the order of the entry, in FP32, a thread per 16-byte chunk.
+// tokens (now 8.4).  The other warps add the rows out of shared memory in the order of the entry, in FP32, a thread per 16-byte chunk.
 #pragma once
 
 #include "protocol.cuh"
@@ -40,7 +40,7 @@ struct CombineLocalArgs {
     int weighted;
     __nv_bfloat16* out;              // [T, H]
     int* error;                      // [8]
-    std::int64_t* stats;             // [8]: rows written, 0, ns from the first CTA's start to the last one's end (without claims: of CTA 0)
+    std::int64_t* stats;             // [8]: rows written, 0, ns from the first CTA's start to the last one's end (without claims: of CTA 0 alone)
     unsigned long long* cta_done;    // CTAs of this launch that have finished; the last one puts it back to zero
     unsigned long long* first_start; // earliest start; all ones between launches
     unsigned long long* next_unit;   // units handed out beyond every CTA's first; zero between launches
@@ -58,7 +58,8 @@ constexpr int kCombineLocalThreads = 32 * (1 + kCombineLocalConsumers);
 constexpr int kCombineLocalSmallStage = 32 * 1024;
 // Launches with at most this many claims per CTA don't claim: CTA b takes the units b, b + grid, ...  There is nothing to even out
 // yet, and without counters no CTA has to find out whether it is the last one: 16 tokens, 8 rows of 14 KB 7.0 -> 5.2 us, 128 tokens
-// 11.3 -> 8.3, 256 tokens 14.7 -> 12.2, 2048 tokens of one row 21.7 -> 18.8.
+// 11.3 -> 8.3, 256 tokens 14.7 -> 12.2, 2048 tokens of one row 21.7 -> 18.8.  Nobody is the last one then, so the duration in `stats` is that
+// of CTA 0 (3.0 us of such a launch of 16 tokens, 16.3 of 2048): counting the CTAs for the sake of that number cost 0.3 to 0.6 us a launch.
 constexpr int kCombineLocalFixedRounds = 4;
 
 struct CombineLocalHeader {

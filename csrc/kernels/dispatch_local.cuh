@@ -15,9 +15,9 @@
 //   4. a warp per token: every lane k < K whose expert is valid starts the bulk store of the row to its expert's segment.
 //
 // What bounds it.  Large batches: writing the expanded rows to HBM.  4096 tokens, hidden 7168, top-8 move 528 MB.
-// Small ones: the chain launch -> ids -> barrier -> prefix -> rows.  Launch to end with a cold L2, general kernel -> this
-// one: 128 tokens 46 -> 19 us (no flags to wait for, no prefix by a single warp), 4096 tokens 131 ->
-// 104 us, the same with E4M3 rows 106 -> 71 us (fourteen row buffers per SM on all SMs instead of eight on 128), 256 tokens
+// Small ones: the chain launch -> ids -> counts -> scan -> rows; between them, from kLocalWholePairs on, a barrier and a prefix.
+// Launch to end with a cold L2, general kernel -> this one: 128 tokens 46 -> 10.9 us (no flags to wait for, no prefix by a single
+// warp, no barrier), 4096 tokens 131 -> 104 us, the same with E4M3 rows 106 -> 71 us (fourteen row buffers per SM on all SMs instead of eight on 128), 256 tokens
 // with a cached layout 45 -> 17 us.
 #pragma once
 
@@ -740,7 +740,8 @@ __global__ void __launch_bounds__(kLocalThreads, 1) local_dispatch_kernel(const 
         BEP_PROF(kProfEnd);
         if (any_failed) return;  // the rank has failed: nothing of it is used again
         if (alone) {
-            // launches of a buffer are stream-ordered: the next one sees all of this, whichever CTA wrote it when
+            // launches of a buffer are stream-ordered: the next one sees all of this, whichever CTA wrote it when.  (The end needs no
+            // reset: what an earlier launch left in the tensor, or its zeroes, is before any time of this one.)
             atomicMax(reinterpret_cast<unsigned long long*>(&a.timestamps[1]), static_cast<unsigned long long>(ptx::globaltimer_ns()));
             if (b == 0) a.timestamps[0] = static_cast<std::int64_t>(t_start);
             if (b == G - 1) {

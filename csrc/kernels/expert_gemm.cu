@@ -684,7 +684,6 @@ const char* run_grouped_gemm(const void* a, const void* w, void* out, const floa
     p.num_experts = num_experts;
     p.n = n;
     p.k = k;
-    p.rows_capacity = rows_capacity;
     if (target != nullptr) p.scatter = *target;
     int device = 0, sms = 0;
     if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)

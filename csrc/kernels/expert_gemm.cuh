@@ -76,7 +76,6 @@ struct GroupedGemmParams {
     int num_experts;
     int n;                      // output columns
     int k;                      // reduction length in elements
-    int rows_capacity;          // rows of A / out
     ScatterTarget scatter;      // only read by the scatter variant
 };
 

@@ -252,7 +252,8 @@ struct DispatchArgs {
     int* source_expert_prefix;     // [P][El]
     int* error;                    // [8]
     std::int64_t* stats;           // [8]
-    std::int64_t* timestamps;      // [2] transport start / end (globaltimer ns)
+    std::int64_t* timestamps;      // [2] transport start / end (globaltimer ns), zero when allocated; the start is the earliest of all CTAs,
+                                   //     in one-rank launches without a last CTA that of CTA 0 (the first to be placed)
     std::int64_t* prefix_tx_ts;    // [C+1][2]
     std::int64_t* profile;         // [C][16] per-channel phase timestamps (globaltimer ns), see ProfilePoint
     std::int64_t* role_profile;    // [C][kMaxWarps][16] per-warp role counters (profiling builds only), or nullptr
