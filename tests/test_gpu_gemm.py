@@ -1,5 +1,5 @@
 """tcgen05 grouped expert GEMM against a PyTorch FP32 reference: ragged expert sizes (including empty
-experts, sizes that are not multiples of the 128-row tile, aligned gaps), plain and SwiGLU epilogues."""
+experts, sizes that are no multiple of a tile's rows, aligned gaps), plain and SwiGLU epilogues."""
 
 import pytest
 import torch
@@ -19,7 +19,7 @@ def _layout(counts, alignment=1):
 
 
 @pytest.mark.parametrize("swiglu", [False, True])
-@pytest.mark.parametrize("n", [384, 512])  # plain GEMM: 128-column tiles / 256-column tiles
+@pytest.mark.parametrize("n", [384, 512])  # plain GEMM: a last tile with the channels of one CTA / whole tiles
 @pytest.mark.parametrize("counts,alignment", [([128], 1), ([5, 0, 300, 129, 1, 0, 77, 256], 1), ([40, 130, 0, 9], 16)])
 def test_grouped_gemm_matches_reference(ext, swiglu, n, counts, alignment):
     torch.manual_seed(0)
