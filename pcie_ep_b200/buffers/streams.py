@@ -16,20 +16,16 @@ import torch
 _POOLED_EVENTS = 16
 
 
-def _references(objects: List[Any], index: int) -> int:
-    """References to ``objects[index]`` as the interpreter counts them from here, the list's and the call's own among them."""
-    return sys.getrefcount(objects[index])
-
-
 def _references_of_list_only() -> Optional[int]:
-    """What ``_references`` says of an object that nothing but the list holds.  How many references a call adds is the
-    interpreter's affair, so it is counted, not assumed; None where one more holder does not count as exactly one more."""
-    objects = [object()]
-    alone = _references(objects, 0)
-    holder = objects[0]
-    counted = _references(objects, 0) == alone + 1
+    """What ``sys.getrefcount(objects[index])`` says of an object that nothing but the list holds.  How many references the
+    expression adds is the interpreter's affair, so it is counted, not assumed; None where one more holder does not count as
+    exactly one more."""
+    objects, index = [object()], 0
+    alone = sys.getrefcount(objects[index])
+    holder = objects[index]
+    counted = sys.getrefcount(objects[index]) == alone + 1
     del holder
-    return alone if counted and _references(objects, 0) == alone else None
+    return alone if counted and sys.getrefcount(objects[index]) == alone else None
 
 
 class NullStream:
@@ -92,7 +88,7 @@ class StreamPolicy:
         events = self._events
         for _ in range(len(events)):
             self._next_event = (self._next_event + 1) % len(events)
-            if _references(events, self._next_event) == self._unheld:
+            if sys.getrefcount(events[self._next_event]) == self._unheld:
                 return events[self._next_event]
         event = torch.cuda.Event()
         if self._unheld is not None and len(events) < _POOLED_EVENTS:
