@@ -56,6 +56,21 @@ __device__ __forceinline__ unsigned cluster_rank() {
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
 }
+// True in one lane of a converged warp.  Behind a branch on it the compiler knows that tcgen05 and TMA instructions, whose operands are
+// uniform registers, are issued once; behind `lane == 0` it does not, and an MMA of a pair took 145 cycles to issue, longer than one of
+// 256 x 256 x 16 takes to execute (127).  One pair alone, per K block of 64: 16 to 128 rows 285 -> 131 to 138 ns (weights into an SM at 57 ->
+// 125 GB/s), 192 rows 282 -> 207.  64 tokens, top-8 of 32 experts, 7168 x 2048: layer 467 -> 449 us; 555 tokens in E4M3, popular experts,
+// 495 -> 458; 4096 tokens in E4M3 1935 -> 1845.  Under the power limit 32 experts of 1024 rows, 7168 -> 4096: 1,205 -> 1,255 TFLOP/s at 1,080
+// instead of 1,100 MHz (torch.bmm 1,305 at 1,170).
+__device__ __forceinline__ bool elect_one() {
+    std::uint32_t elected;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(elected)::"memory");
+    return elected != 0;
+}
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -287,7 +302,7 @@ grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_rows, const __gr
 
     if (warp == 0) {
         // ===== TMA producer: this CTA's 128 weight rows and its half of the activation rows =====
-        if (lane == 0) {
+        if (elect_one()) {
             int stage = 0;
             unsigned phase = 0;
             bool ok = true;
@@ -330,7 +345,7 @@ grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_rows, const __gr
         }
     } else if (warp == 1) {
         // ===== MMA issuer of the pair =====
-        if (lane == 0 && rank == 0) {
+        if (rank == 0 && elect_one()) {
             int stage = 0;
             unsigned phase = 0;
             bool ok = true;

@@ -17,12 +17,9 @@
 // (6.6 TB/s), down 154 -> 154, against tiles of 128 rows x 256 weight rows by single CTAs.  Many: tensor cores under the power
 // limit.  4096 tokens (1024 rows per expert), back to back: gate/up 1709 -> 1718 us in BF16 (1,120 TFLOP/s; with exactly 1024
 // rows everywhere 1595 -> 1593) and 1050 -> 913 in E4M3, down 935 -> 872.  Between them, and with a short K, the epilogue: 2000
-// tokens of hidden 2048 and intermediate 768 gate/up 117 -> 95 us, 300 tokens in E4M3 192 -> 161.  Slower than before: where a few
-// experts have many rows and the others about a hundred (1024 tokens, a fifth of the experts popular: gate/up 528 -> 538 us, on another
-// box 442 -> 468): stages as long as the widest tile needs leave 96 KB of weights on their way per SM instead of 128; and where few
-// rows fill the pairs one time and a bit (8 experts of 40 rows, 96 tiles: 70 -> 81 us): a pair's MMA takes about 140 cycles with 16 rows
-// as with 256, so its weights come at 57 GB/s per SM however few pairs are at work.  (Stages of each tile's own
-// length in a circle were 20 % slower everywhere; asking weights into L2 ahead of the stages 2 to 80 %.)
+// tokens of hidden 2048 and intermediate 768 gate/up 117 -> 95 us, 300 tokens in E4M3 192 -> 161.  Stages are
+// as long as the widest tile of the launch needs.  (Stages of each tile's own length in a circle were 20 % slower everywhere; asking weights
+// into L2 ahead of the stages 2 to 80 %.)  Both roles of one thread are entered through elect.sync, see elect_one.
 //
 // Work decomposition: persistent pairs walk a tile list (expert, channel tile, row chunk) computed on the device from the
 // counts -- the host never reads a count.  Per CTA: warp 0 = TMA producer (this CTA's weight rows and its half of the
