@@ -143,6 +143,13 @@ def test_tiles_of_every_width(ext, fp8, swiglu, k):
 
 @pytest.mark.parametrize("fp8", [False, True])
 @pytest.mark.parametrize("swiglu", [True, False])
+def test_more_row_chunks_than_a_group(ext, fp8, swiglu):
+    """Tiles go by groups of eight row chunks: experts with exactly one group, one and two chunks more, two full groups and a part."""
+    _check_tiles([2048, 2049, 3, 2304 + 1, 4096, 0, 4625], 640, 128, fp8, swiglu)
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("swiglu", [True, False])
 @pytest.mark.parametrize("widest", [16, 48, 80, 112, 144, 176, 224])
 def test_rings_of_every_depth(ext, fp8, swiglu, widest):
     """The ring has as many stages as fit for the widest tile of the launch (ten for 16 rows, six for 224).  Twenty-five K blocks a
