@@ -127,18 +127,6 @@ __device__ __forceinline__ void umma_commit_pair(std::uint64_t* bar) {
                  "h"(static_cast<std::uint16_t>(3))
                  : "memory");
 }
-// 32 lanes x 32 columns of FP32 out of TMEM: thread i gets columns [c, c+32) of lane (base lane + i)
-__device__ __forceinline__ void tmem_ld_32x32(std::uint32_t taddr, std::uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr)
-        : "memory");
-}
 // 16 lanes x 32 columns: thread t gets, for j = 0..3, columns 8j + 2(t % 4) + {0, 1} of lane t / 4 in r[4j], r[4j + 1] and of lane
 // t / 4 + 8 in r[4j + 2], r[4j + 3]: the fragments that stmatrix stores
 __device__ __forceinline__ void tmem_ld_16x32(std::uint32_t taddr, std::uint32_t* r) {
@@ -256,7 +244,8 @@ grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_rows, const __gr
     unsigned char* tiles = smem;
     unsigned char* staging = smem + kRingBytes;
     auto* sh = reinterpret_cast<GemmShared*>(staging + 2 * kChunkRows * kPitch);
-    auto* targets = reinterpret_cast<RowTargets*>(sh + 1);  // scatter only
+    auto* row_factors = reinterpret_cast<float*>(sh + 1);                                        // [2][kMaxRows] scatter and E4M3
+    auto* row_targets = reinterpret_cast<unsigned long long*>(row_factors + 2 * kMaxRows);       // [2][kMaxRows] scatter
     volatile int* abort = &sh->abort;
 
     const int warp = threadIdx.x >> 5;
@@ -410,107 +399,100 @@ grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_rows, const __gr
             __syncwarp();
         }
         const std::uint32_t empty_addr = cluster_addr(&sh->tmem_empty[0], 0);  // in the leading CTA
-        // this lane's channel inside the CTA's part of the tile; for SwiGLU lanes 0..15 hold gate rows, 16..31 up rows of the same channels
-        const int channel = kSwiGLU ? q * 16 + (lane & 15) : q * 32 + lane;
-        const bool upper = lane >= 16;
         constexpr int kLanesPerRow = kChannels / 8;             // 16-byte pieces of a row
         constexpr int kRowsPerStore = 32 / kLanesPerRow;
         const int piece = lane % kLanesPerRow, store_row = q * (kChunkRows / 4) + lane / kLanesPerRow;
-        // Scatter: where the rows of a tile go and their weights, two rows per thread, asked for a tile ahead.  Asked for in their own
-        // chunk, every 32 rows waited for L2, and with a short K the epilogue was longer than the MMAs of its tile: 2000 tokens,
-        // top-8 of 32 experts, 768 -> 2048, GEMM and sum 107 -> 91 us.
+        // What belongs to the rows of a tile (scatter: where they go and their weights; E4M3: their scales), two rows per thread, is asked
+        // for a tile ahead.  Asked for in their own chunk, every 32 rows waited for L2, and the epilogue was longer than the MMAs of its
+        // tile: 2000 tokens, top-8 of 32 experts, 768 -> 2048, scattered down projection and sum 107 -> 91 us.
+        constexpr bool kRowFactors = kScatter || kFp8;
         TileWalk ahead = walk;
         int owner[2], token[2], slot[2];
-        float weight[2];
-        auto ask_targets = [&]() {
+        float factor[2];
+        auto ask_rows = [&]() {
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const int in_tile = static_cast<int>(threadIdx.x) - 64 + 128 * i;
                 owner[i] = -1;
                 if (in_tile >= ahead.tile_rows) continue;
                 const long long r = static_cast<long long>(ahead.row0) + in_tile;
-                const long long* meta = sc.source_meta + r * 3;
-                owner[i] = static_cast<int>(meta[0]);
-                token[i] = static_cast<int>(meta[1]);
-                slot[i] = static_cast<int>(meta[2]);
-                weight[i] = sc.row_weights != nullptr ? sc.row_weights[r] : 1.0f;
+                if constexpr (kScatter) {
+                    const long long* meta = sc.source_meta + r * 3;
+                    owner[i] = static_cast<int>(meta[0]);
+                    token[i] = static_cast<int>(meta[1]);
+                    slot[i] = static_cast<int>(meta[2]);
+                    factor[i] = sc.row_weights != nullptr ? sc.row_weights[r] : 1.0f;
+                } else {
+                    factor[i] = p.a_scales[r];
+                }
             }
         };
         // into shared memory: what was there was read two tiles ago, and all warps have met since then (epilogue_all)
-        auto store_targets = [&](int rows, int buf, int first_channel) {
+        auto store_rows = [&](int rows, int buf, int first_channel) {
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const int in_tile = static_cast<int>(threadIdx.x) - 64 + 128 * i;
                 if (in_tile >= rows) continue;
-                unsigned long long dst = 0;
-                if (owner[i] >= 0 && owner[i] < sc.num_ranks && slot[i] >= 0 && slot[i] < sc.num_topk && token[i] >= 0)
-                    dst = reinterpret_cast<unsigned long long>(sc.seg[owner[i]] + sc.stage_off +
-                                                               (static_cast<std::size_t>(token[i]) * sc.num_topk + slot[i]) * static_cast<std::size_t>(sc.row_stride) +
-                                                               static_cast<std::size_t>(first_channel) * 2);
-                targets->dst[buf][in_tile] = dst;
-                targets->weight[buf][in_tile] = weight[i];
+                row_factors[buf * kMaxRows + in_tile] = factor[i];
+                if constexpr (kScatter) {
+                    unsigned long long dst = 0;
+                    if (owner[i] >= 0 && owner[i] < sc.num_ranks && slot[i] >= 0 && slot[i] < sc.num_topk && token[i] >= 0)
+                        dst = reinterpret_cast<unsigned long long>(sc.seg[owner[i]] + sc.stage_off +
+                                                                   (static_cast<std::size_t>(token[i]) * sc.num_topk + slot[i]) * static_cast<std::size_t>(sc.row_stride) +
+                                                                   static_cast<std::size_t>(first_channel) * 2);
+                    row_targets[buf * kMaxRows + in_tile] = dst;
+                }
             }
         };
-        if (kScatter && ahead.next(p)) ask_targets();
+        if (kRowFactors && ahead.next(p)) ask_rows();
         int it = 0, half = 0;
         for (; walk.next(p); ++it) {
             const int buf = it & 1;
             const unsigned acc_phase = (it >> 1) & 1u;
             const int first_channel = (walk.m_tile * 2 + static_cast<int>(rank)) * kChannels;
             const bool inside = first_channel < p.n;  // n an odd multiple of 128: the last tile has one CTA's channels only
-            if (kScatter) {
-                store_targets(walk.tile_rows, buf, first_channel);
-                if (ahead.next(p)) ask_targets();
+            // E4M3: scales of the weight rows of this thread's channels, lane / 4 + 8 i of its warp's (SwiGLU: two gate, then two up rows)
+            float w_scale[4] = {1.0f, 1.0f, 1.0f, 1.0f};
+            if (kFp8 && inside) {
+                const float* at = p.w_scales + static_cast<long long>(walk.expert) * (kSwiGLU ? 2 : 1) * p.n + first_channel + q * (kChannels / 4) + (lane >> 2);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) w_scale[i] = kSwiGLU ? at[(i >> 1) * p.n + (i & 1) * 8] : at[i * 8];
+            }
+            if (kRowFactors) {
+                store_rows(walk.tile_rows, buf, first_channel);
+                if (ahead.next(p)) ask_rows();
             }
             // all four warps go on or none: they meet at the barriers below
             if (!epilogue_all(mbar_wait(&sh->tmem_full[buf], acc_phase, abort))) break;
             tc_fence_after();
-            float w_first = 1.0f, w_up = 1.0f;  // FP8: scale of the weight row(s) of this lane's channel
-            if (kFp8 && inside) {
-                const float* w_scale = p.w_scales + static_cast<long long>(walk.expert) * (kSwiGLU ? 2 : 1) * p.n + first_channel + channel;
-                w_first = *w_scale;
-                if (kSwiGLU) w_up = w_scale[p.n];
-            }
             const std::uint32_t acc = tmem_base + (static_cast<std::uint32_t>(q * 32) << 16) + buf * kAccCols;
             // (2) of a chunk, see below: a few lanes = one row, its channels of this CTA leave as contiguous 16-byte pieces
-            unsigned long long dst_bits = 0;  // where the row of this lane goes, 0: nowhere
-            auto store_chunk = [&]() {
+            auto store_chunk = [&](int c0) {
                 epilogue_sync();
 #pragma unroll
                 for (int i = 0; i < kChunkRows / 4; i += kRowsPerStore) {
                     const int r = store_row + i;
-                    const unsigned long long dst = __shfl_sync(0xffffffffu, dst_bits, r);
+                    unsigned char* dst = nullptr;
+                    if (c0 + r < walk.tile_rows && inside) {
+                        if constexpr (kScatter) dst = reinterpret_cast<unsigned char*>(row_targets[buf * kMaxRows + c0 + r]);
+                        else dst = reinterpret_cast<unsigned char*>(p.out + static_cast<long long>(walk.row0 + c0 + r) * p.n + first_channel);
+                    }
                     const uint4 packed = *reinterpret_cast<const uint4*>(staging + (half * kChunkRows + r) * kPitch + piece * 16);
-                    if (dst != 0ull) ptx::st_v4(reinterpret_cast<unsigned char*>(dst) + piece * 16, packed);
+                    if (dst != nullptr) ptx::st_v4(dst + piece * 16, packed);
                 }
                 half ^= 1;  // the other half was read before the barrier above
             };
 #pragma unroll 1
             for (int c0 = 0; c0 < walk.tile_rows; c0 += kChunkRows) {
+                // v[16 h + 4 j + 2 i + x]: weight row 16 h + 8 i + lane / 4 of the warp's 32, activation row c0 + 8 j + 2 (lane % 4) + x
                 std::uint32_t v[32];
-                float2 weights[4];  // scatter: of the rows that this thread's registers hold
-                if constexpr (kScatter) {
-                    tmem_ld_16x32(acc + c0, v);
-                    tmem_ld_16x32(acc + (16u << 16) + c0, v + 16);
+                tmem_ld_16x32(acc + c0, v);
+                tmem_ld_16x32(acc + (16u << 16) + c0, v + 16);
+                float2 factors[4];  // of the rows that this thread's registers hold
+                if constexpr (kRowFactors)
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) weights[j] = *reinterpret_cast<const float2*>(&targets->weight[buf][c0 + 8 * j + 2 * (lane & 3)]);
-                } else {
-                    tmem_ld_32x32(acc + c0, v);
-                }
-                // what belongs to the chunk's rows, one row per lane
-                float row_factor = 1.0f;
-                unsigned long long dst_next = 0;
-                if (c0 + lane < walk.tile_rows && inside) {
-                    const long long r = static_cast<long long>(walk.row0) + c0 + lane;
-                    if (kFp8) row_factor = p.a_scales[r];
-                    if (kScatter) {
-                        dst_next = targets->dst[buf][c0 + lane];
-                    } else {
-                        dst_next = reinterpret_cast<unsigned long long>(p.out + r * p.n + first_channel);
-                    }
-                }
-                if (c0 > 0) store_chunk();  // the chunk before leaves while this one's values are on their way
-                dst_bits = dst_next;
+                    for (int j = 0; j < 4; ++j) factors[j] = *reinterpret_cast<const float2*>(&row_factors[buf * kMaxRows + c0 + 8 * j + 2 * (lane & 3)]);
+                if (c0 > 0) store_chunk(c0 - kChunkRows);  // the chunk before leaves while this one's values are on their way
                 tmem_ld_wait(v);
                 if (c0 + kChunkRows >= walk.tile_rows) {
                     // the accumulator has been read completely: the MMA warp may start the tile after next
@@ -518,26 +500,35 @@ grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_rows, const __gr
                     __syncwarp();
                     if (lane == 0) mbar_arrive_cluster(empty_addr + buf * 8);
                 }
-                // (1) transpose through shared memory: lane = channel -> staging[row][channel]
-                unsigned char* to = staging + half * (kChunkRows * kPitch) + channel * 2;
-                if (kSwiGLU) {
-                    // gate and up of a channel lie in lanes 16 apart: the lower lane takes the even rows of both, the upper one the odd ones
+                // (1) 8 rows x 8 channels at a time turned round through shared memory by matrix stores: lane = channel -> staging[row][channel].
+                // (A lane per channel with 32 stores of 2 bytes, and as many shuffles of the rows' factors or between gate and up, was slower
+                // where K is short: 32 experts of 500 rows, 768 -> 2048 69.9 -> 61.9 us, gate/up 2048 -> 768 97.7 -> 91.5, in E4M3 81.9 -> 76.4.)
+                if constexpr (kSwiGLU) {
+                    // gate (h = 0) and up (h = 1) of a channel are in one thread
+                    const std::uint32_t at = smem_addr(staging + (half * kChunkRows + (lane >> 4) * 8 + (lane & 7)) * kPitch + (q * 16 + (lane >> 3 & 1) * 8) * 2);
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        const float even = __uint_as_float(v[2 * i]), odd = __uint_as_float(v[2 * i + 1]);
-                        const float other = __shfl_xor_sync(0xffffffffu, upper ? even : odd, 16);
-                        float gate = upper ? other : even, up = upper ? odd : other;
-                        if (kFp8) {
-                            const float a_scale = __shfl_sync(0xffffffffu, row_factor, 2 * i + (upper ? 1 : 0));
-                            gate *= a_scale * w_first;
-                            up *= a_scale * w_up;
+                    for (int j0 = 0; j0 < 4; j0 += 2) {
+                        std::uint32_t m[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const int j = j0 + (i >> 1), first = 4 * j + (i & 1) * 2;
+                            float silu[2];
+#pragma unroll
+                            for (int x = 0; x < 2; ++x) {
+                                float gate = __uint_as_float(v[first + x]), up = __uint_as_float(v[16 + first + x]);
+                                if (kFp8) {
+                                    const float a_scale = x == 0 ? factors[j].x : factors[j].y;
+                                    gate *= a_scale * w_scale[i & 1];
+                                    up *= a_scale * w_scale[2 + (i & 1)];
+                                }
+                                silu[x] = ptx::quotient(gate, 1.0f + __expf(-gate)) * up;
+                            }
+                            const __nv_bfloat162 packed = __floats2bfloat162_rn(silu[0], silu[1]);
+                            m[i] = *reinterpret_cast<const std::uint32_t*>(&packed);
                         }
-                        const float silu = ptx::quotient(gate, 1.0f + __expf(-gate)) * up;
-                        *reinterpret_cast<__nv_bfloat16*>(to + (2 * i + (upper ? 1 : 0)) * kPitch) = __float2bfloat16_rn(silu);
+                        stmatrix_transposed(at + 8 * j0 * kPitch, m[0], m[1], m[2], m[3]);
                     }
-                } else if constexpr (kScatter) {
-                    // 8 rows x 32 channels at a time, turned round by the matrix stores: 4 of them instead of 32 stores of 2 bytes and
-                    // 32 shuffles of the weights (the same tokens 91 -> 86 us; 4096 tokens, 2048 -> 7168, inside a layer 800 -> 780)
+                } else {
                     const std::uint32_t at = smem_addr(staging + (half * kChunkRows + (lane & 7)) * kPitch + (q * 32 + (lane >> 3) * 8) * 2);
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
@@ -545,21 +536,22 @@ grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_rows, const __gr
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
                             const int first = (i >> 1) * 16 + 4 * j + (i & 1) * 2;
-                            const __nv_bfloat162 packed = __floats2bfloat162_rn(__uint_as_float(v[first]) * weights[j].x, __uint_as_float(v[first + 1]) * weights[j].y);
+                            float a = __uint_as_float(v[first]), b = __uint_as_float(v[first + 1]);
+                            if (kScatter) {
+                                a *= factors[j].x;
+                                b *= factors[j].y;
+                            } else if (kFp8) {
+                                a *= factors[j].x * w_scale[i];
+                                b *= factors[j].y * w_scale[i];
+                            }
+                            const __nv_bfloat162 packed = __floats2bfloat162_rn(a, b);
                             m[i] = *reinterpret_cast<const std::uint32_t*>(&packed);
                         }
                         stmatrix_transposed(at + 8 * j * kPitch, m[0], m[1], m[2], m[3]);
                     }
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        float value = __uint_as_float(v[i]);
-                        if (kFp8) value *= __shfl_sync(0xffffffffu, row_factor, i) * w_first;
-                        *reinterpret_cast<__nv_bfloat16*>(to + i * kPitch) = __float2bfloat16_rn(value);
-                    }
                 }
             }
-            store_chunk();
+            store_chunk((walk.tile_rows - 1) / kChunkRows * kChunkRows);
         }
         if (kScatter) ptx::fence_sys();  // this thread's rows before the CTA is counted as finished
     }
@@ -646,7 +638,7 @@ cudaError_t launch(const ActivationMaps& maps_rows, const CUtensorMap& map_w, co
     int device = 0;
     cudaError_t status = cudaGetDevice(&device);
     if (status != cudaSuccess) return status;
-    constexpr int smem = gemm_smem_bytes(kSwiGLU, kScatter);
+    constexpr int smem = gemm_smem_bytes(kSwiGLU, kFp8, kScatter);
     if (device >= 0 && device < 64 && !configured[device]) {
         status = cudaFuncSetAttribute(grouped_gemm_kernel<kSwiGLU, kFp8, kScatter>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (status != cudaSuccess) return status;

@@ -102,28 +102,23 @@ constexpr int kMaxStages = 10;
 constexpr int kAccCols = kMaxRows;       // TMEM columns of one accumulator set
 constexpr int kTmemCols = 2 * kAccCols;  // double buffered
 // The epilogue turns the accumulator (lane = channel) round in shared memory, kChunkRows rows at a time in two alternating halves.
-// Row pitch: 16 bytes more than a row keep the 2-byte column writes of a warp apart; for SwiGLU, where a warp writes sixteen
-// channels of two rows at once, 32.
+// Row pitch: 16 bytes more than a row (a multiple of 128) put the eight rows of a matrix into different banks.
 constexpr int kChunkRows = 32;
-__host__ __device__ constexpr int staging_pitch(bool swiglu) { return swiglu ? kCtaM / 2 * 2 + 32 : kCtaM * 2 + 16; }
+__host__ __device__ constexpr int staging_pitch(bool swiglu) { return (swiglu ? kCtaM / 2 : kCtaM) * 2 + 16; }
 struct alignas(16) GemmShared {
     std::uint64_t full[kMaxStages], empty[kMaxStages], tmem_full[2], tmem_empty[2];
     std::uint32_t tmem_base;
     int abort;
     int most_rows[kThreads / 32];  // of any expert, per warp
 };
-// Scatter: where the rows of a tile go (0: nowhere) and their weights, for two tiles in turn.  Behind the tile's rows lies what was
-// there; what is made of it goes nowhere.
-struct alignas(16) RowTargets {
-    unsigned long long dst[2][kMaxRows];
-    float weight[2][kMaxRows];
-};
-__host__ __device__ constexpr int gemm_smem_bytes(bool swiglu, bool scatter) {
+// Behind it, for two tiles in turn: a factor per row (scatter: the routing weight; E4M3: the row's scale) and, for scatter, where the
+// row goes (0: nowhere).  Behind the tile's rows lies what was there; what is made of it goes nowhere.
+__host__ __device__ constexpr int gemm_smem_bytes(bool swiglu, bool fp8, bool scatter) {
     return 1024 /* alignment slack */ + kRingBytes + 2 * kChunkRows * staging_pitch(swiglu) + static_cast<int>(sizeof(GemmShared)) +
-           (scatter ? static_cast<int>(sizeof(RowTargets)) : 0);
+           (fp8 || scatter ? 2 * kMaxRows * 4 : 0) + (scatter ? 2 * kMaxRows * 8 : 0);
 }
 static_assert(2 * kChunkRows * staging_pitch(true) % 16 == 0 && 2 * kChunkRows * staging_pitch(false) % 16 == 0, "barriers follow the staging");
-static_assert(gemm_smem_bytes(false, true) <= 227 * 1024, "one CTA per SM");
+static_assert(gemm_smem_bytes(false, false, true) <= 227 * 1024 && gemm_smem_bytes(false, true, false) <= 227 * 1024, "one CTA per SM");
 
 }  // namespace gemm
 }  // namespace bep
