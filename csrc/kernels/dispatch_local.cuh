@@ -40,7 +40,8 @@ constexpr int kLocalSmallPairBytes = 16 * 1024;
 enum LocalMode { kLocalTogether, kLocalWhole, kLocalCached };
 // Batches of up to this many (token, k) are counted by every CTA by itself, without a barrier: no CTA waits for another one, and
 // where none claims tokens the launch needs no cooperative grid and nobody has to be the last.  Together / by itself, top-8: 16 tokens
-// 17.2 / 10.7 us, 128 tokens 17.3 / 10.9, 2048 (at the line) 26.3 / 22.1, 4096 99.7 / 103.4; 777 tokens top-4 20.9 / 14.0.
+// 17.2 / 10.7 us, 128 tokens 17.3 / 10.9, 4096 97.5 / 101 (layout done after 12.6 / 15.8); 777 tokens top-4 20.9 / 13.6.  At the line, 2048
+// tokens, the layout is done after 9.2 us (12.5 before ids came eight steps at a time and nothing was read behind the row loads).
 constexpr int kLocalWholePairs = 16 * 1024;
 constexpr int kLocalFewExperts = 64;  // counted with ballots, without atomics (a warp's 32 pairs meet few counters again and again)
 
@@ -229,21 +230,21 @@ __global__ void __launch_bounds__(kLocalThreads, 1) local_dispatch_kernel(const 
     unsigned* const token_bits = pair_bits + pair_words;                                    // which tokens are routed,
     int* const routed_words = reinterpret_cast<int*>(token_bits + token_words);             // [token_words + 1] routed tokens before word w
     if constexpr (whole) {
-        // The pairs of the whole batch: 32 per warp and step, the ids of four steps on their way at once.  Few experts meet in
+        // The pairs of the whole batch: 32 per warp and step, the ids of eight steps on their way at once (of four: 2048 tokens top-8 0.8 us more).  Few experts meet in
         // a step again and again: there a lane counts two of them from ballots of the ids' bits.
         const int own_first = t0 * K;
         const bool few = E <= kLocalFewExperts;
         unsigned mine[2] = {0u, 0u};  // few: pairs of the experts lane and lane + 32, those of earlier CTAs in the upper half
         bool bad = false;
-        for (int p0 = warp * 32; p0 < all_pairs; p0 += kLocalThreads * 4) {
-            std::int64_t id[4];
+        for (int p0 = warp * 32; p0 < all_pairs; p0 += kLocalThreads * 8) {
+            std::int64_t id[8];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
+            for (int u = 0; u < 8; ++u) {
                 const int p = p0 + u * kLocalThreads + static_cast<int>(lane);
                 id[u] = p < all_pairs ? __ldg(a.topk_idx + p) : -1;
             }
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
+            for (int u = 0; u < 8; ++u) {
                 const int first = p0 + u * kLocalThreads;
                 if (first >= all_pairs) break;
                 const bool named = id[u] >= 0 && id[u] < E;
@@ -286,12 +287,14 @@ __global__ void __launch_bounds__(kLocalThreads, 1) local_dispatch_kernel(const 
                 int mine = -1;
                 if (e < -1 || e >= E) {
                     record_error(rc, a.error, kErrInvalidRouting, t0 + c0 + tl, k);
+                    sh->flag = 1;
                 } else if (e >= 0) {
                     if (atomicOr(&bits[e], 1u << tl) >> tl & 1u) {  // the token names this expert twice
                         int at = k;
                         for (int k2 = k + 1; k2 < K; ++k2)
                             if (a.topk_idx[static_cast<std::size_t>(t0 + c0 + tl) * K + k2] == e) at = k2;
                         record_error(rc, a.error, kErrInvalidRouting, t0 + c0 + tl, at);
+                        sh->flag = 1;
                     } else {
                         mine = static_cast<int>(e);
                     }
@@ -343,7 +346,9 @@ __global__ void __launch_bounds__(kLocalThreads, 1) local_dispatch_kernel(const 
             const unsigned bits = __ballot_sync(full, routed);
             if (lane == 0) token_bits[w] = bits;
         }
-        if (tid == 0 && (leaves() || health.failed())) sh->flag = 1;
+        // (no look at the rank's error word here: a read behind the row loads waits for them, 2048 tokens 2 us.  What this CTA itself
+        // has found wrong is in the flag, and so is what was wrong before the launch.)
+        if (tid == 0 && leaves()) sh->flag = 1;
         __syncthreads();
         if (warp == kLocalWarps - 1) {
             int before = 0;
