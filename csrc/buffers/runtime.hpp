@@ -8,6 +8,7 @@
 // instead of waiting or allocating.  Routing plans come from a pool of the same size (+1 for graphs).
 #pragma once
 
+#include <array>
 #include <cstdint>
 #include <cstdlib>
 #include <memory>
@@ -59,6 +60,23 @@ inline TensorRefs tensor_refs(const at::Tensor& t) {
     return {static_cast<std::int64_t>(t.use_count()),
             static_cast<std::int64_t>(t.unsafeGetTensorImpl()->unsafe_storage().use_count())};
 }
+
+// Where a tensor lives and how it is laid out, and its version counter (none: inference tensors), as of now.
+struct TensorBinding {
+    explicit TensorBinding(const at::Tensor& t)
+        : data(t.data_ptr()), sizes(t.sizes()), strides(t.strides()), dtype(t.scalar_type()), device(t.device()) {
+        if (!t.is_inference()) version = t._version();
+    }
+    bool same_memory(const at::Tensor& t) const {
+        return t.data_ptr() == data && t.sizes() == at::IntArrayRef(sizes) && t.strides() == at::IntArrayRef(strides) && t.scalar_type() == dtype &&
+               t.device() == device;
+    }
+    void* data;
+    c10::SmallVector<std::int64_t, 4> sizes, strides;
+    at::ScalarType dtype;
+    at::Device device;
+    std::optional<std::int64_t> version;
+};
 
 struct RuntimeOptions {
     int channels = 32;
@@ -135,7 +153,7 @@ struct OutputSet {
     at::Tensor source_expert_prefix, error, stats, timestamps, prefix_tx_ts;
     at::Tensor combine_error, combine_stats, profile, combine_profile, role_profile;
 
-    std::vector<const at::Tensor*> all() const {
+    std::array<const at::Tensor*, 23> all() const {
         return {&recv_x, &recv_idx, &recv_w, &recv_scale, &source_meta, &comb_map, &recv_chan_counts, &unique_count,
                 &expanded_count, &expert_counts, &expert_offsets, &expert_prefix, &source_offsets,
                 &source_expert_prefix, &error, &stats, &timestamps, &prefix_tx_ts, &combine_error, &combine_stats, &profile, &combine_profile,
@@ -159,33 +177,44 @@ class DispatchResult {
         : set_(std::move(set)), layout_(std::move(layout)), expand_(expand), num_tokens_(num_tokens),
           unique_cap_(unique_cap), expanded_cap_(expanded_cap), topk_(topk), recv_fp8_(recv_fp8) {}
 
-    static const std::vector<std::string>& tensor_keys() {
-        static const std::vector<std::string> keys = {
+    static constexpr int kFields = 23;
+    static const std::array<std::string, kFields>& tensor_keys() {
+        static const std::array<std::string, kFields> keys = {
             "recv_x", "recv_topk_idx", "recv_topk_weights", "source_meta", "comb_map", "recv_chan_counts",
             "unique_count", "expanded_count", "expert_counts", "expert_offsets", "expert_prefix", "source_offsets",
             "source_expert_prefix", "error", "stats", "transport_timestamps_ns", "prefix_tx_timestamps_ns",
             "combine_error", "combine_stats", "profiling", "combine_profiling", "recv_x_scales", "role_profiling"};
         return keys;
     }
+    static int field(const std::string& key) {  // -1: no tensor of that name
+        static const std::unordered_map<std::string, int> fields = [] {
+            std::unordered_map<std::string, int> m;
+            for (int i = 0; i < kFields; ++i) m.emplace(tensor_keys()[i], i);
+            return m;
+        }();
+        const auto hit = fields.find(key);
+        return hit == fields.end() ? -1 : hit->second;
+    }
 
     bool contains(const std::string& key) const {
         if (!overrides_.empty() && overrides_.contains(key.c_str())) return true;
-        if (key == "_layout" || key == "_expand" || key == "_num_tokens") return true;
-        for (const auto& k : tensor_keys())
-            if (k == key) return true;
-        return false;
+        return key == "_layout" || key == "_expand" || key == "_num_tokens" || field(key) >= 0;
     }
 
-    py::object get(const std::string& key) {
+    // a null object: no such key
+    py::object find(const std::string& key) {
         if (!overrides_.empty() && overrides_.contains(key.c_str())) return overrides_[key.c_str()];
+        const int i = field(key);
+        if (i >= 0) return py::cast(tensor(i));
         if (key == "_layout") return py::cast(layout_);
         if (key == "_expand") return py::cast(expand_);
         if (key == "_num_tokens") return py::cast(num_tokens_);
-        auto hit = cache_.find(key);
-        if (hit != cache_.end()) return py::cast(hit->second);
-        at::Tensor t = make(key);
-        cache_.emplace(key, t);
-        return py::cast(t);
+        return py::object();
+    }
+    py::object get(const std::string& key) {
+        py::object value = find(key);
+        if (!value) throw py::key_error(key);
+        return value;
     }
     void set(const std::string& key, py::object value) { overrides_[key.c_str()] = std::move(value); }
     py::list keys() const {
@@ -199,7 +228,9 @@ class DispatchResult {
 
     // recv_x, recv_topk_idx and (with weights) recv_topk_weights in one go: what every dispatch returns
     py::tuple received(bool with_weights) {
-        return py::make_tuple(get("recv_x"), get("recv_topk_idx"), with_weights ? get("recv_topk_weights") : py::object(py::none()));
+        if (!overrides_.empty())
+            return py::make_tuple(get("recv_x"), get("recv_topk_idx"), with_weights ? get("recv_topk_weights") : py::object(py::none()));
+        return py::make_tuple(tensor(0), tensor(1), with_weights ? py::cast(tensor(2)) : py::object(py::none()));
     }
 
     const OutputSet& set_ref() const { return *set_; }
@@ -209,6 +240,10 @@ class DispatchResult {
     int num_tokens() const { return num_tokens_; }
 
    private:
+    const at::Tensor& tensor(int field) {
+        if (!cache_[field].defined()) cache_[field] = make(tensor_keys()[field]);
+        return cache_[field];
+    }
     at::Tensor make(const std::string& key) const {
         const OutputSet& s = *set_;
         const std::int64_t K = topk_;
@@ -251,7 +286,7 @@ class DispatchResult {
     bool expand_;
     int num_tokens_, unique_cap_, expanded_cap_, topk_;
     bool recv_fp8_ = false;
-    std::unordered_map<std::string, at::Tensor> cache_;
+    std::array<at::Tensor, kFields> cache_;
     py::dict overrides_;
 };
 
@@ -510,6 +545,31 @@ class Runtime {
         launch.r[0] = p.args;
         cuda_check(launch_dispatch(launch, grid_ctas_, threads_, smem_, launch_stream), "dispatch launch");
         return p.result;
+    }
+
+    void record_behind(std::int64_t stream, std::int64_t event) const {
+        c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device_));
+        cuda_check(cudaEventRecord(reinterpret_cast<cudaEvent_t>(event), reinterpret_cast<cudaStream_t>(stream)), "event record");
+    }
+
+    // The usual calls of the Python layer in one: argument check, launch on `stream` and record of `event` behind it.  None where the
+    // arguments are not what the layer's rules ask for, or the stream is being captured: the layer then goes step by step and says so.
+    py::object enqueue_dispatch(const py::handle& x, const py::handle& idx, const py::handle& w, bool expand, bool zero_padding, std::int64_t stream,
+                                std::int64_t event) {
+        if (closed_ || !accepts_inputs(x, idx, w) || capturing(stream)) return py::none();
+        const at::Tensor& routes = THPVariable_Unpack(idx.ptr());
+        std::optional<at::Tensor> weights;
+        if (!w.is_none()) weights = THPVariable_Unpack(w.ptr());
+        std::shared_ptr<DispatchResult> result = dispatch(THPVariable_Unpack(x.ptr()), routes, weights, 1, expand, zero_padding, nullptr, false, stream);
+        record_behind(stream, event);
+        return py::make_tuple(result, result->received(weights.has_value()), TensorBinding(routes));
+    }
+    py::object enqueue_combine(const py::handle& y, const std::shared_ptr<DispatchResult>& result, bool weighted, const std::optional<at::Tensor>& out,
+                               std::int64_t stream, std::int64_t event) {
+        if (closed_ || !accepts_rows(y, *result) || capturing(stream)) return py::none();
+        at::Tensor combined = combine(THPVariable_Unpack(y.ptr()), *result, weighted, out, stream);
+        record_behind(stream, event);
+        return py::cast(combined);
     }
 
     // A single rank whose rows move with bulk copies takes the kernel without the protocol (dispatch_local.cuh), unless a
@@ -839,6 +899,11 @@ class Runtime {
                                    at::cuda::getCurrentCUDAStream(device_)),
                    "upload rank constants");
         cuda_check(cudaStreamSynchronize(at::cuda::getCurrentCUDAStream(device_)), "upload rank constants");
+    }
+
+    static bool capturing(std::int64_t stream) {
+        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+        return cudaStreamIsCapturing(reinterpret_cast<cudaStream_t>(stream), &status) != cudaSuccess || status != cudaStreamCaptureStatusNone;
     }
 
     bool matches(const at::Tensor& t, at::ScalarType dtype, std::int64_t rows, std::int64_t columns) const {

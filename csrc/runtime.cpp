@@ -184,8 +184,14 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         .def("keys", &DispatchResult::keys)
         .def("received", &DispatchResult::received, py::arg("with_weights"))
         .def("get", [](DispatchResult& r, const std::string& key, py::object fallback) {
-            return r.contains(key) ? r.get(key) : fallback;
+            py::object value = r.find(key);
+            return value ? value : fallback;
         }, py::arg("key"), py::arg("default") = py::none());
+
+    py::class_<TensorBinding>(m, "TensorBinding")
+        .def(py::init<const at::Tensor&>())
+        .def("same_memory", &TensorBinding::same_memory)
+        .def_readonly("version", &TensorBinding::version);
 
     py::class_<Runtime, std::shared_ptr<Runtime>>(m, "Runtime")
         .def(py::init<int, int, int, int, int, int, const py::dict&, const std::vector<std::int64_t>&, int>())
@@ -194,6 +200,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
              py::arg("stream") = 0, py::arg("beside_compute") = false)
         .def("combine", &Runtime::combine, py::arg("y"), py::arg("dispatch_result"), py::arg("weighted"), py::arg("out"),
              py::arg("stream") = 0, py::arg("num_sms") = 0)
+        .def("enqueue_dispatch", &Runtime::enqueue_dispatch, py::arg("x"), py::arg("topk_idx"), py::arg("topk_weights"), py::arg("expand"),
+             py::arg("zero_padding"), py::arg("stream"), py::arg("event"))
+        .def("record_event", &Runtime::record_behind, py::arg("stream"), py::arg("event"))
+        .def("enqueue_combine", &Runtime::enqueue_combine, py::arg("y"), py::arg("dispatch_result"), py::arg("weighted"), py::arg("out"),
+             py::arg("stream"), py::arg("event"))
         .def("fused_scatter_gemm", &Runtime::fused_scatter_gemm, py::arg("hidden_rows"), py::arg("w_down"),
              py::arg("dispatch_result"), py::arg("stream") = 0)
         .def("fused_reduce", &Runtime::fused_reduce, py::arg("dispatch_result"), py::arg("out"), py::arg("stream") = 0)

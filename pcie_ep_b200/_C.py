@@ -142,6 +142,7 @@ first_touch_host_segment = _module.first_touch_host_segment
 dispatch_group = _module.dispatch_group
 combine_group = _module.combine_group
 tensor_refs = _module.tensor_refs
+TensorBinding = _module.TensorBinding
 
 
 def __getattr__(name: str):

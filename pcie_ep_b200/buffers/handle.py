@@ -17,9 +17,22 @@ if TYPE_CHECKING:  # pragma: no cover
     from .ep import HostStagedEPBuffer
 
 
-def _fingerprint(tensor: torch.Tensor) -> tuple:
-    """Everything that makes a tensor 'the same memory seen the same way' (not its contents)."""
-    return (id(tensor), tensor.data_ptr(), tensor.shape, tensor.stride(), tensor.dtype, tensor.device)
+class TensorBinding:
+    """Everything that makes a tensor 'the same memory seen the same way' (not its contents), and its version counter.  GPU
+    buffers use the native class of the same name."""
+
+    __slots__ = ("version", "_layout")
+
+    def __init__(self, tensor: torch.Tensor) -> None:
+        self.version: Optional[int] = None if tensor.is_inference() else tensor._version
+        self._layout = self._of(tensor)
+
+    @staticmethod
+    def _of(tensor: torch.Tensor) -> tuple:
+        return (tensor.data_ptr(), tensor.shape, tensor.stride(), tensor.dtype, tensor.device)
+
+    def same_memory(self, tensor: torch.Tensor) -> bool:
+        return self._of(tensor) == self._layout
 
 
 class RouteBinding:
@@ -29,12 +42,12 @@ class RouteBinding:
     which is why they can be dispatched but not cached.
     """
 
-    __slots__ = ("tensor", "version", "fingerprint")
+    __slots__ = ("tensor", "version", "binding")
 
-    def __init__(self, tensor: torch.Tensor) -> None:
+    def __init__(self, tensor: torch.Tensor, binding: Any = None) -> None:
         self.tensor = tensor
-        self.version: Optional[int] = None if tensor.is_inference() else tensor._version
-        self.fingerprint = _fingerprint(tensor)
+        self.binding = TensorBinding(tensor) if binding is None else binding
+        self.version: Optional[int] = self.binding.version
 
     @property
     def cacheable(self) -> bool:
@@ -46,7 +59,7 @@ class RouteBinding:
         return self.tensor
 
     def same_memory(self) -> bool:
-        return _fingerprint(self.tensor) == self.fingerprint
+        return self.binding.same_memory(self.tensor)
 
 
 class _Routed:
@@ -112,6 +125,10 @@ _RESULT_FIELDS = {
 }
 
 
+# what a handle shares with its buffer, fixed for the buffer's life
+_BUFFER_FIELDS = ("buffer_id", "group", "global_ranks", "num_experts", "num_max_tokens_per_rank")
+
+
 class HostStagedEPHandle(_Routed):
     """Device-side description of one capacity-shaped dispatch result.
 
@@ -123,28 +140,28 @@ class HostStagedEPHandle(_Routed):
     num_recv_tokens_per_expert_list = None
 
     def __init__(self, owner: "HostStagedEPBuffer", topk_idx: torch.Tensor, result: Dict[str, Any], do_expand: bool,
-                 expert_alignment: int, event: EventOverlap) -> None:
+                 expert_alignment: int, event: EventOverlap, binding: Any = None) -> None:
         self._owner = owner
-        self._route = RouteBinding(topk_idx)
+        self._route = RouteBinding(topk_idx, binding)
         self._result = result
-        self.buffer_id, self.generation = owner.buffer_id, owner._generation
-        self.group, self.global_ranks = owner.group, owner.global_ranks
-        self.num_experts, self.num_max_tokens_per_rank = owner.num_experts, owner.num_max_tokens_per_rank
+        self.generation = owner._generation
         self.do_expand, self.expert_alignment = do_expand, expert_alignment
         self.completion = event
         self._completion_event = event.event
 
     def __getattr__(self, name: str) -> Any:
-        # reached only for names that __init__ did not set: resolve against the native result and remember
-        if name == "psum_num_recv_tokens_per_scaleup_rank":
+        # reached only for names that __init__ did not set: resolve against the native result (or the buffer) and remember
+        key = _RESULT_FIELDS.get(name)
+        if key is not None:
+            value = self._result.get(key)
+        elif name == "psum_num_recv_tokens_per_scaleup_rank":
             value = self._result["source_offsets"][1:]
         elif name == "_layout":  # the native routing plan, or None
             value = self._result.get("_layout")
+        elif name in _BUFFER_FIELDS:
+            value = getattr(self._owner, name)
         else:
-            key = _RESULT_FIELDS.get(name)
-            if key is None:
-                raise AttributeError(name)
-            value = self._result.get(key)
+            raise AttributeError(name)
         self.__dict__[name] = value
         return value
 

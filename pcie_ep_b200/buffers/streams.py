@@ -62,6 +62,8 @@ class StreamPolicy:
         self.device = device
         self.comm = torch.cuda.Stream(device=device) if on_gpu else NullStream()
         self.consumers: Dict[Tuple[int, int], Any] = {}
+        self._reader: Any = None  # the last stream of the callers' that a synchronous call ran on
+        self._reader_raw, self._reader_key = -1, None
         # stream objects by raw handle: torch builds a new one per query (1.3 us), and with one object per stream "the only
         # reader is the stream itself" is a comparison of identities
         self._known: Dict[int, Any] = {}
@@ -118,6 +120,16 @@ class StreamPolicy:
             if key not in done:
                 target.wait_stream(reader)
 
+    def sole(self) -> Any:
+        """The caller's current stream if a synchronous launch on it has nothing to be ordered with: it alone reads results, and the
+        communication stream is not ahead of it.  Else None."""
+        if self._comm_ahead or torch._C._cuda_getCurrentRawStream(self.device) != self._reader_raw:
+            return None
+        return self._reader if len(self.consumers) == 1 and self._reader_key in self.consumers else None
+
+    def raw(self, stream: Any) -> int:
+        return self._reader_raw if stream is self._reader else int(stream.cuda_stream)
+
     # -- one launch ------------------------------------------------------------------------------
     def begin(self, compute: Any, previous_event: Any, run_async: bool) -> Any:
         """Return the stream the next kernel is launched on, with its input dependencies in place."""
@@ -157,6 +169,8 @@ class StreamPolicy:
             self._comm_ahead = False
         if not (len(self.consumers) == 1 and compute in self.consumers.values()):
             self.add_consumer(compute)
+        if compute is not self._reader and not self.is_comm(compute):
+            self._reader, self._reader_raw, self._reader_key = compute, int(compute.cuda_stream), stream_key(compute)
 
     def drain(self, last_event: Optional[Any]) -> None:
         """Blocking: used by ``close`` only."""

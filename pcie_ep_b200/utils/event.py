@@ -41,14 +41,15 @@ class EventOverlap:
     ``on_wait``        callback ``f(stream)`` invoked with each waiting stream.
     """
 
+    _epilogue: Optional[Callable[[], Any]] = None
+    _release_on_exit = False
+    _spent = False
+
     def __init__(self, event: Any = None, extra_tensors: Any = None,
                  on_wait: Optional[Callable[[Any], None]] = None) -> None:
         self.event = event
         self.extra_tensors = extra_tensors
         self._notify = on_wait
-        self._epilogue: Optional[Callable[[], Any]] = None
-        self._release_on_exit = False
-        self._spent = False
 
     # -- waiting ---------------------------------------------------------------------------------
     def current_stream_wait(self, release_handle: bool = False) -> Any:

@@ -186,6 +186,57 @@ def test_cumulative_stats_and_invalid_routes(world1):
                 buffer.dispatch(x, idx, w)
 
 
+class _CountingWatchdog:
+    launches = 0
+
+    def watch(self, label, query):
+        self.launches += 1
+
+
+@pytest.mark.parametrize("expand", [True, False])
+@pytest.mark.parametrize("with_weights", [True, False])
+def test_usual_calls_are_the_general_ones(world1, expand, with_weights):
+    """A call on the stream that alone reads results goes down in one native call: same results and tokens as step by step (with a
+    watchdog), same refusals, cacheable until the routing tensor is written to; another reader or stream ends it."""
+    with _buffer() as buffer:
+        cpu, (x, idx, w) = _dev_inputs(pattern="partial")
+        weights = w if with_weights else None
+        assert buffer._streams.sole() is None  # nothing was launched yet
+        buffer.dispatch(x, idx, weights, do_expand=expand)
+        results = []
+        for watchdog in (None, _CountingWatchdog()):
+            buffer.attach_watchdog(watchdog)
+            recv_x, recv_idx, recv_w, handle, token = buffer.dispatch(x, idx, weights, do_expand=expand)
+            rows = int(handle.num_expanded_tokens if expand else handle.num_recv_tokens)
+            combined, _, done = buffer.combine(recv_x, handle)
+            done.event.synchronize()
+            assert token.event.query() and done.event.query() and (recv_w is None) == (weights is None)
+            results.append([recv_x[:rows].clone(), recv_idx[:rows].clone(), combined.clone(), handle.expert_counts.clone()])
+            del recv_x, recv_idx, recv_w, combined, token, done
+        assert watchdog.launches == 2 and all(torch.equal(a, b) for a, b in zip(*results))
+        buffer.attach_watchdog(None)
+        assert buffer._streams.sole() is not None
+        for bad in (lambda: buffer.dispatch(x.float(), idx, weights, do_expand=expand), lambda: buffer.dispatch(x[:, 1:], idx, weights, do_expand=expand),
+                    lambda: buffer.dispatch(x, idx[1:], weights, do_expand=expand), lambda: buffer.dispatch(x, idx, w.double(), do_expand=expand),
+                    lambda: buffer.combine(x.float(), handle), lambda: buffer.combine(x, handle, num_sms=-1)):
+            with pytest.raises(ValueError):
+                bad()
+        with pytest.raises(TypeError):
+            buffer.dispatch(None, idx, weights, do_expand=expand)
+        own = idx.clone()
+        fresh = buffer.dispatch(x, own, weights, do_expand=expand)[3]
+        buffer.cache_layout(fresh)
+        own.add_(0)
+        with pytest.raises(RuntimeError, match="changed"):
+            buffer.cache_layout(fresh)
+        with torch.cuda.stream(torch.cuda.Stream()):
+            assert buffer._streams.sole() is None
+            token = buffer.dispatch(x, idx, weights, do_expand=expand)[4]
+        token.wait()
+        assert buffer._streams.sole() is None  # two streams read results now
+        _check(buffer.dispatch(x, idx, w, do_expand=expand), cpu, expand)
+
+
 @pytest.mark.parametrize("mode", ["auto", "inline"])
 def test_combine_weighted_and_unique(world1, mode):
     """Single rank: "auto" is the one-launch gather-reduce, "inline" the cooperative kernel writing straight to out."""
