@@ -8,7 +8,7 @@
 // two stages in shared memory allow -- a whole row of 7168 with top-8 -- and one bulk copy: 95 us, and 104 us with half rows.
 //
 // Work unit = (entry of the combine map, slice of its rows).  A CTA's first units are its own, the others come from a
-// counter (launches of a few units per CTA: in a fixed order, kCombineLocalFixedRounds): SMs do not all get the same share of HBM, and equal shares waited for the slowest (125 us).  The producer warp
+// counter (launches of a few units per CTA: in a fixed order, kCombineLocalFixed): SMs do not all get the same share of HBM, and equal shares waited for the slowest (125 us).  The producer warp
 // keeps the claim after next and the map entries of the next units on their way while it starts the copies of the present
 // ones; a round of that takes 1.4 us, so small units are claimed four at a time (2048 tokens, a row each: 25.5 -> 21.9 us).
 // Before, through the multi-rank reducers (combine_push.cuh): 111 us, 139 us for 8192 tokens top-4 (now 103), 22 us for 128
@@ -27,6 +27,7 @@ struct CombineLocalShape {
     int stage_bytes = 0;   // rows of a unit, one slice each
     int ctas = 0;
     int batch = 1;         // consecutive units per claim: 1 or 4
+    bool fixed = false;    // nothing is claimed: CTA b takes the units b, b + ctas, ...
     std::size_t bytes = 0; // dynamic shared memory
 };
 
@@ -56,11 +57,15 @@ constexpr int kCombineLocalThreads = 32 * (1 + kCombineLocalConsumers);
 // claimed singly at 34 KB (hidden 2880, 95 us).  Larger units take that long to read anyway (7 stages of 32 KB are in flight),
 // and four of them in one CTA would be an uneven end.
 constexpr int kCombineLocalSmallStage = 32 * 1024;
-// Launches with at most this many claims per CTA don't claim: CTA b takes the units b, b + grid, ...  There is nothing to even out
-// yet, and without counters no CTA has to find out whether it is the last one: 16 tokens, 8 rows of 14 KB 7.0 -> 5.2 us, 128 tokens
-// 11.3 -> 8.3, 256 tokens 14.7 -> 12.2, 2048 tokens of one row 21.7 -> 18.8.  Nobody is the last one then, so the duration in `stats` is that
-// of CTA 0 (3.0 us of such a launch of 16 tokens, 16.3 of 2048): counting the CTAs for the sake of that number cost 0.3 to 0.6 us a launch.
-constexpr int kCombineLocalFixedRounds = 4;
+// Launches with at most this many units per CTA (the second line: of stages up to kCombineLocalSmallStage) don't claim: CTA b takes the
+// units b, b + grid, ...  There is little to even out yet, the map entries of four units are asked for at once, and without counters no
+// CTA has to find out whether it is the last one: 16 tokens, 8 rows of 14 KB 7.0 -> 5.2 us, 128 tokens 11.3 -> 8.3.  From 4 units on, singly
+// claimed / in a fixed order: 777 tokens, 4 rows of 8 KB 14.7 / 12.5, 1000 tokens, 2 rows of 4 KB 14.6 / 9.5, 8 rows of 14 KB 30.9 / 28.7, 1800
+// tokens, 8 rows of 8 KB (12 units) 31.4 / 30.0; 2048 tokens, 8 rows of 14 KB (14 units) an exchange of 102.9 / 103.5.  Nobody is the last one
+// then, so the duration in `stats` is that of CTA 0 (3.0 us of such a launch of 16 tokens, 16.3 of 2048 single rows): counting the CTAs for the
+// sake of that number cost 0.3 to 0.6 us a launch.
+constexpr int kCombineLocalFixed = 12;
+constexpr int kCombineLocalFixedSmall = 16;
 
 struct CombineLocalHeader {
     int token, n, first_chunk, chunks;  // n < 0: no more units
@@ -95,6 +100,7 @@ inline CombineLocalShape combine_local_shape(int tokens, int hidden, int max_row
     const long long units = static_cast<long long>(tokens) * s.slices;
     s.ctas = units < 1 ? 1 : units < sms ? static_cast<int>(units) : sms;
     s.batch = s.stage_bytes <= kCombineLocalSmallStage && units >= 12ll * sms ? 4 : 1;
+    s.fixed = units <= static_cast<long long>(s.stage_bytes <= kCombineLocalSmallStage ? kCombineLocalFixedSmall : kCombineLocalFixed) * s.ctas;
     return s;
 }
 
@@ -114,7 +120,7 @@ inline bool combine_local_pays(int tokens, int hidden, int max_rows, int sms) {
 
 #ifdef __CUDACC__
 
-// kBatch: consecutive units per claim
+// kBatch: units whose map entries are asked for at once; consecutive ones, one claim, or in a fixed order `ctas` apart
 template <int kBatch>
 __global__ void __launch_bounds__(kCombineLocalThreads, 1) local_combine_push_kernel(const __grid_constant__ CombineLocalArgs a) {
     const RankConst* __restrict__ rc = a.rc;
@@ -133,7 +139,8 @@ __global__ void __launch_bounds__(kCombineLocalThreads, 1) local_combine_push_ke
     }
     const int Tc = max(1, (T + C - 1) / C);  // tokens per channel: no channel has more entries
     const long long units = static_cast<long long>((T + Tc - 1) / Tc) * Tc * a.shape.slices;
-    const bool fixed = units <= static_cast<long long>(kCombineLocalFixedRounds) * kBatch * gridDim.x;
+    const bool fixed = a.shape.fixed;
+    const int apart = fixed ? gridDim.x : 1;  // units of a batch
     // The launch before is the expert GEMM, usually, or the dispatch whose map is read below.  Reads of what it may have written are
     // ordinary loads: one that counts on memory staying as it is for the whole kernel (ld.global.nc) may be moved in front of the wait.
     ptx::wait_for_launch_before();
@@ -177,10 +184,10 @@ __global__ void __launch_bounds__(kCombineLocalThreads, 1) local_combine_push_ke
             if (lane == 0) got = atomicAdd(a.next_unit, 1ull);
             return got;  // lane 0's value counts
         };
-        long long u = static_cast<long long>(blockIdx.x) * kBatch;
+        long long u = static_cast<long long>(blockIdx.x) * (fixed ? 1 : kBatch);
         Entry e[kBatch];
 #pragma unroll
-        for (int i = 0; i < kBatch; ++i) e[i] = load_entry(u + i);
+        for (int i = 0; i < kBatch; ++i) e[i] = load_entry(u + i * apart);
         unsigned long long claimed = fixed ? 0 : claim();
         int filled = 0;  // stages handed to the consumers
         while (ok && u < units) {
@@ -188,7 +195,7 @@ __global__ void __launch_bounds__(kCombineLocalThreads, 1) local_combine_push_ke
                                            : (static_cast<long long>(gridDim.x) + static_cast<long long>(__shfl_sync(0xffffffffu, claimed, 0))) * kBatch;
             Entry next[kBatch];
 #pragma unroll
-            for (int i = 0; i < kBatch; ++i) next[i] = load_entry(next_u + i);
+            for (int i = 0; i < kBatch; ++i) next[i] = load_entry(next_u + i * apart);
             if (!fixed && next_u < units) claimed = claim();
 #pragma unroll
             for (int i = 0; i < kBatch; ++i) {
@@ -196,7 +203,7 @@ __global__ void __launch_bounds__(kCombineLocalThreads, 1) local_combine_push_ke
                 const int stage = filled % stages;
                 ok = __all_sync(0xffffffffu, wait(&sh->empty[stage], (static_cast<unsigned>(filled / stages) & 1u) ^ 1u)) != 0;
                 if (!ok) continue;
-                const int n = e[i].head.y, first = static_cast<int>((u + i) % a.shape.slices) * a.shape.slice_chunks;
+                const int n = e[i].head.y, first = static_cast<int>((u + i * apart) % a.shape.slices) * a.shape.slice_chunks;
                 const int len = min(a.shape.slice_chunks, chunks - first);
                 CombineLocalHeader& header = sh->header[stage];
                 if (lane < n) header.weight[lane] = a.weighted ? __int_as_float(e[i].pair.y) : 1.0f;

@@ -128,7 +128,7 @@ cudaError_t launch_dispatch_local(const DispatchArgs& a, const RankConst& rc, co
 }
 
 cudaError_t launch_combine_local(const CombineLocalArgs& args, cudaStream_t stream) {
-    const auto kernel = args.shape.batch == 1 ? local_combine_push_kernel<1> : local_combine_push_kernel<4>;
+    const auto kernel = args.shape.batch == 1 && !args.shape.fixed ? local_combine_push_kernel<1> : local_combine_push_kernel<4>;
     static std::mutex mutex;
     static std::size_t configured[64] = {0};
     {

@@ -198,7 +198,7 @@ class _CountingWatchdog:
 def test_usual_calls_are_the_general_ones(world1, expand, with_weights):
     """A call on the stream that alone reads results goes down in one native call: same results and tokens as step by step (with a
     watchdog), same refusals, cacheable until the routing tensor is written to; another reader or stream ends it."""
-    with _buffer() as buffer:
+    with _buffer(output_pool_size=6) as buffer:
         cpu, (x, idx, w) = _dev_inputs(pattern="partial")
         weights = w if with_weights else None
         assert buffer._streams.sole() is None  # nothing was launched yet

@@ -102,6 +102,34 @@ def test_local_dispatch_and_combine(one_rank, tokens, capacity, experts, topk, h
         del local, general, cached, result, got
 
 
+@pytest.mark.parametrize("tokens,topk,hidden", [(148 * 4 - 1, 8, 2880), (148 * 5 + 3, 8, 2880), (148 * 12, 8, 2880), (148 * 12 + 1, 8, 2880), (148 * 13, 8, 2880),
+                                                (148 * 11 + 5, 4, 3584), (148 * 16, 4, 3584), (148 * 16 + 1, 4, 3584), (148 * 17, 4, 3584)])
+def test_combine_at_the_line_between_fixed_order_and_claims(one_rank, tokens, topk, hidden):
+    """Units of more and of at most 32 KB, around 4, 12 and 16 of them per CTA, some entries missing: two passes (the counters of the
+    first are the second's) against the sum in 64 bits."""
+    from pcie_ep_b200 import HostStagedConfig, HostStagedEPBuffer
+
+    gen = torch.Generator().manual_seed(tokens)
+    x = torch.randn(tokens, hidden, generator=gen).to(torch.bfloat16).cuda()
+    idx = torch.rand(tokens, 16, generator=gen).topk(topk, dim=1).indices.to(torch.int64)
+    idx[torch.rand(tokens, generator=gen) < 0.1] = -1
+    w = torch.rand(tokens, topk, generator=gen).cuda()
+    with HostStagedEPBuffer(one_rank, tokens, hidden, topk, 16, HostStagedConfig(channels=16)) as buffer:
+        recv_x, _, _, handle, _ = buffer.dispatch(x, idx.cuda(), w, do_expand=True)
+        rows = int(handle.num_expanded_tokens)
+        y = torch.randn(rows, hidden, generator=gen).to(torch.bfloat16).cuda()
+        meta = handle.source_meta[:rows]
+        terms = y.double() * w[meta[:, 1], meta[:, 2]].double().unsqueeze(1)
+        want = torch.zeros(tokens, hidden, dtype=torch.float64, device="cuda").index_add_(0, meta[:, 1], terms)
+        size = torch.zeros(tokens, hidden, dtype=torch.float64, device="cuda").index_add_(0, meta[:, 1], terms.abs())
+        for _ in range(2):
+            out = buffer.combine(y, handle)[0].double()
+            # as above: one rounding to BF16, one FP32 rounding per added row
+            assert bool(((out - want).abs() <= want.abs() * 2.0 ** -8 + size * topk * 2.0 ** -23).all())
+        buffer.check_errors(handle)
+        del recv_x, handle
+
+
 @pytest.mark.parametrize("tokens,capacity,channels", [(300, 300, 7), (40, 300, 32), (30000, 30000, 1)])
 def test_dispatch_beside_the_compute_stream_keeps_to_its_channels(one_rank, tokens, capacity, channels):
     """On the communication stream: as many CTAs as channels (or the general kernel where their tables would not fit)."""
