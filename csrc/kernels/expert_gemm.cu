@@ -279,19 +279,29 @@ grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_rows, const __gr
     // here on is read by ordinary loads, which stay behind the wait (ld.global.nc need not).
     ptx::wait_for_launch_before();
     ptx::let_next_launch_start();
-    int most_rows = 1;  // of any expert
+    int most_rows = 1, all_rows = 0;  // of any expert, of all
     for (int e = threadIdx.x; e < p.num_experts; e += kThreads) {
         asm volatile("prefetch.global.L1 [%0];" ::"l"(p.expert_offsets + e));  // asked for again at the first tile
-        most_rows = max(most_rows, p.expert_counts[e]);
+        const int rows = p.expert_counts[e];
+        most_rows = max(most_rows, rows);
+        all_rows += rows;
     }
     most_rows = __reduce_max_sync(0xffffffffu, most_rows);
-    if (lane == 0) sh->most_rows[warp] = most_rows;
+    all_rows = __reduce_add_sync(0xffffffffu, all_rows);
+    if (lane == 0) {
+        sh->most_rows[warp] = most_rows;
+        sh->all_rows[warp] = all_rows;
+    }
     tc_fence_before();
     __syncthreads();
     cluster_sync();  // barriers of both CTAs are ready before either names the other's
     tc_fence_after();
     const std::uint32_t tmem_base = sh->tmem_base;
-    for (int w = 0; w < kThreads / 32; ++w) most_rows = max(most_rows, sh->most_rows[w]);
+    all_rows = 0;
+    for (int w = 0; w < kThreads / 32; ++w) {
+        most_rows = max(most_rows, sh->most_rows[w]);
+        all_rows += sh->all_rows[w];
+    }
     const int stage_bytes = kTileW + box_rows(box_of_rows(min(most_rows, kMaxRows))) * kBlockKBytes;
     const int stages = min(kMaxStages, kRingBytes / stage_bytes);
     TileWalk walk(m_tiles);
@@ -341,7 +351,7 @@ grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_rows, const __gr
         }
     } else if (warp == 1) {
         // ===== MMA issuer of the pair =====
-        if (rank == 0 && elect_one()) {
+        auto issue = [&]() {
             int stage = 0;
             unsigned phase = 0;
             bool ok = true;
@@ -374,6 +384,20 @@ grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_rows, const __gr
                     }
                 }
                 if (ok) umma_commit_pair(&sh->tmem_full[buf]);
+            }
+        };
+        // What the compiler makes of the branch sets the pace.  Behind elect_one MMAs follow each other without a gap.  A long BF16 launch
+        // then runs into the power limit: 4096 tokens, 7168 -> 2 x 2048 of 32 experts, 1.05 GHz instead of 1.3, no more MMAs a second than
+        // with a gap of 18 cycles behind each, which an undecided `lane == 0` leaves, and everything else at the lower clock, the memory-bound
+        // kernels of the layer too: layer 2745 us against 2635, dispatch 147 against 125, both at 1000 W.  2048 tokens 1500 / 1486, 1024 tokens
+        // with popular experts, half as long again, 878 / 915, 8 experts of 1024 rows, 4096 -> 2 x 1024, 224 / 228: the line lies at 2048
+        // tokens.  (Gaps between K blocks only, or longer ones, cost more than they gave.  E4M3 gains without any, 1936 -> 1822, the down
+        // projection of that layer included.)
+        if (rank == 0) {
+            if (!kFp8 && kSwiGLU && static_cast<long long>(all_rows) * p.n * p.k >= kLongLaunch) {
+                if (lane == 0) issue();
+            } else if (elect_one()) {
+                issue();
             }
         }
     } else {

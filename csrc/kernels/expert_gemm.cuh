@@ -99,6 +99,7 @@ constexpr int kTileW = kCtaM * kBlockKBytes;
 // Stages are as long as the widest tile of the launch needs: where all experts have few rows, more of them keep weights on their way.
 constexpr int kRingBytes = 6 * (kTileW + kMaxRows / 2 * kBlockKBytes);  // six stages of the widest tiles, more of narrower ones
 constexpr int kMaxStages = 10;
+constexpr long long kLongLaunch = 225ll * 1000 * 1000 * 1000;  // rows x channels x K of a SwiGLU launch of 0.7 ms (0.9 TFLOP), see the MMA issuer
 constexpr int kAccCols = kMaxRows;       // TMEM columns of one accumulator set
 constexpr int kTmemCols = 2 * kAccCols;  // double buffered
 // The epilogue turns the accumulator (lane = channel) round in shared memory, kChunkRows rows at a time in two alternating halves.
@@ -110,6 +111,7 @@ struct alignas(16) GemmShared {
     std::uint32_t tmem_base;
     int abort;
     int most_rows[kThreads / 32];  // of any expert, per warp
+    int all_rows[kThreads / 32];   // of all experts, per warp
 };
 // Behind it, for two tiles in turn: a factor per row (scatter: the routing weight; E4M3: the row's scale) and, for scatter, where the
 // row goes (0: nowhere).  Behind the tile's rows lies what was there; what is made of it goes nowhere.
