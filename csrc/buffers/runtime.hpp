@@ -78,6 +78,15 @@ struct TensorBinding {
     std::optional<std::int64_t> version;
 };
 
+// The link between two grouped GEMMs (gemm::Progress) over `progress`, int32 [experts + 1], zero before the first of them; `behind`: output
+// channels of the first launch, where this is the second, else 0.
+inline gemm::Progress linked(const std::optional<at::Tensor>& progress, int experts, int behind) {
+    if (!progress.has_value()) return {nullptr, 0};
+    if (!progress->is_cuda() || progress->scalar_type() != at::kInt || !progress->is_contiguous() || progress->numel() != experts + 1 || behind < 0)
+        throw std::invalid_argument("progress must be contiguous CUDA int32 [experts + 1]");
+    return {reinterpret_cast<unsigned*>(progress->data_ptr<int>()), behind > 0 ? grouped_gemm_tiles_per_chunk(behind) : 0};
+}
+
 struct RuntimeOptions {
     int channels = 32;
     int payload_slots = 0;
@@ -749,8 +758,9 @@ class Runtime {
     // the GEMM epilogue into the token owners' landing slots.  Step 2 (owner side): sum the K slots per token.
     // The two steps are separate calls so that several virtual ranks of one process can run all their GEMMs
     // before any reduction (a reduction waits for every rank's GEMM).
+    // `progress`, `behind`: see linked().
     void fused_scatter_gemm(const at::Tensor& hidden_rows, const at::Tensor& w_down, const DispatchResult& dispatch_result,
-                            std::int64_t stream) {
+                            std::int64_t stream, const std::optional<at::Tensor>& progress, int behind) {
         c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device_));
         check_open();
         if (!options_.enable_fused) throw std::runtime_error("this buffer was built with fused_expert_combine=False");
@@ -787,7 +797,7 @@ class Runtime {
         const char* message = grouped_gemm_scatter(hidden_rows.data_ptr(), w_down.data_ptr(), set.expert_offsets.data_ptr<int>(),
                                                    set.expert_counts.data_ptr<int>(), fused_status_.data_ptr<int>(),
                                                    static_cast<int>(hidden_rows.size(0)), lay_.num_local_experts, lay_.hidden,
-                                                   static_cast<int>(inter), target, launch_stream);
+                                                   static_cast<int>(inter), target, linked(progress, lay_.num_local_experts, behind), launch_stream);
         if (message != nullptr) throw std::runtime_error(std::string("fused scatter GEMM: ") + message);
         ++fused_gemm_epoch_;
     }

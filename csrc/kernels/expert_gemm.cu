@@ -228,6 +228,27 @@ struct TileWalk {
 
 }  // namespace
 
+namespace {
+// waits (bounded) until the launch before has written all rows of an expert
+__device__ __noinline__ bool rows_written(const GroupedGemmParams& p, int expert, unsigned tiles, volatile int* abort) {
+    const auto* counter = reinterpret_cast<const std::uint32_t*>(p.progress.counters + expert);
+    unsigned long long deadline = 0;
+    for (unsigned polls = 1; ptx::ld_acquire_gpu(counter) < tiles; ++polls) {
+        if (polls % 64 == 0) {
+            const unsigned long long now = ptx::globaltimer_ns();
+            if (deadline == 0) deadline = now + kProgressLimitNs;
+            if (*abort || now > deadline) {
+                *abort = 1;
+                return false;
+            }
+        }
+        ptx::nanosleep(100);
+    }
+    asm volatile("fence.proxy.async.global;" ::: "memory");
+    return true;
+}
+}  // namespace
+
 // Launch bounds: at most 128 registers, so that a reducer CTA of the combine (combine_push.cuh) finds room on this CTA's SM.
 template <bool kSwiGLU, bool kFp8, bool kScatter>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 2)
@@ -277,7 +298,8 @@ grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_rows, const __gr
     // Up to here nothing was read that an earlier launch writes: the launch behind another kernel of the layer gets this far while
     // the last CTAs of that one are still at work (a layer of 64 tokens 459 -> 454 us, of which two launches gain).  What is read from
     // here on is read by ordinary loads, which stay behind the wait (ld.global.nc need not).
-    ptx::wait_for_launch_before();
+    const bool second = p.progress.per_chunk != 0;  // of two linked launches: see Progress
+    if (!second) ptx::wait_for_launch_before();
     ptx::let_next_launch_start();
     int most_rows = 1, all_rows = 0;  // of any expert, of all
     for (int e = threadIdx.x; e < p.num_experts; e += kThreads) {
@@ -312,7 +334,13 @@ grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_rows, const __gr
             int stage = 0;
             unsigned phase = 0;
             bool ok = true;
+            int ready = -1;  // second launch: expert whose rows are known to be there
             while (ok && walk.next(p)) {
+                if (second && walk.expert != ready) {
+                    ok = rows_written(p, walk.expert, static_cast<unsigned>(walk.chunks.count * p.progress.per_chunk), abort);
+                    if (!ok) break;
+                    ready = walk.expert;
+                }
                 const int box = box_of_rows(walk.tile_rows);
                 const int half = box_rows(box);
                 const CUtensorMap* map_rows = &maps_rows.box[box];
@@ -576,6 +604,13 @@ grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_rows, const __gr
                 }
             }
             store_chunk((walk.tile_rows - 1) / kChunkRows * kChunkRows);
+            if (!kScatter && p.progress.counters != nullptr && !second) {
+                // this CTA's part of the tile, for the TMA loads of other SMs
+                asm volatile("fence.proxy.async.global;" ::: "memory");
+                __threadfence();
+                epilogue_sync();
+                if (threadIdx.x == 64) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p.progress.counters + walk.expert) : "memory");
+            }
         }
         if (kScatter) ptx::fence_sys();  // this thread's rows before the CTA is counted as finished
     }
@@ -589,6 +624,14 @@ grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_rows, const __gr
         tmem_dealloc(tmem_base, kTmemCols);
     }
     if (threadIdx.x == 0 && *abort) atomicCAS(&p.status[0], 0, 1);
+    if (second) {
+        ptx::wait_for_launch_before();  // whoever waits for this launch has waited for the first one, too
+        if (threadIdx.x == 0) {
+            __threadfence();
+            if (atomicAdd(p.progress.counters + p.num_experts, 1u) + 1u == gridDim.x)
+                for (int e = 0; e <= p.num_experts; ++e) p.progress.counters[e] = 0u;
+        }
+    }
     if (kScatter && threadIdx.x == 0) {
         const ScatterTarget& sc = p.scatter;
         ptx::fence_sys();
@@ -689,7 +732,7 @@ namespace {
 const char* run_grouped_gemm(const void* a, const void* w, void* out, const float* a_scales, const float* w_scales,
                              const int* expert_offsets, const int* expert_counts, int* status, int rows_capacity,
                              int num_experts, int n, int k, bool swiglu, bool fp8, const gemm::ScatterTarget* target,
-                             cudaStream_t stream) {
+                             const gemm::Progress& progress, cudaStream_t stream) {
     using namespace gemm;
     const int block_k = kBlockKBytes / (fp8 ? 1 : 2);
     if (n % 128 != 0 || k % block_k != 0 || n <= 0 || k <= 0)
@@ -722,6 +765,7 @@ const char* run_grouped_gemm(const void* a, const void* w, void* out, const floa
     p.num_experts = num_experts;
     p.n = n;
     p.k = k;
+    p.progress = progress;
     if (target != nullptr) p.scatter = *target;
     int device = 0, sms = 0;
     if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
@@ -736,18 +780,20 @@ const char* run_grouped_gemm(const void* a, const void* w, void* out, const floa
 
 const char* grouped_gemm(const void* a, const void* w, void* out, const float* a_scales, const float* w_scales,
                          const int* expert_offsets, const int* expert_counts, int* status, int rows_capacity,
-                         int num_experts, int n, int k, bool swiglu, bool fp8, cudaStream_t stream) {
+                         int num_experts, int n, int k, bool swiglu, bool fp8, const gemm::Progress& progress, cudaStream_t stream) {
     return run_grouped_gemm(a, w, out, a_scales, w_scales, expert_offsets, expert_counts, status, rows_capacity, num_experts,
-                            n, k, swiglu, fp8, nullptr, stream);
+                            n, k, swiglu, fp8, nullptr, progress, stream);
 }
 
 const char* grouped_gemm_scatter(const void* a, const void* w, const int* expert_offsets, const int* expert_counts,
                                  int* status, int rows_capacity, int num_experts, int n, int k,
-                                 const gemm::ScatterTarget& target, cudaStream_t stream) {
+                                 const gemm::ScatterTarget& target, const gemm::Progress& progress, cudaStream_t stream) {
     // `out` is never written by the scatter epilogue; the A pointer stands in to satisfy the alignment check
     return run_grouped_gemm(a, w, const_cast<void*>(a), nullptr, nullptr, expert_offsets, expert_counts, status, rows_capacity,
-                            num_experts, n, k, false, false, &target, stream);
+                            num_experts, n, k, false, false, &target, progress, stream);
 }
+
+int grouped_gemm_tiles_per_chunk(int n) { return 2 * ((n + gemm::kCtaM - 1) / gemm::kCtaM); }  // (a pair's tile has 2 x 64 channels)
 
 int grouped_gemm_ctas() {
     int device = 0, sms = 0;

@@ -46,6 +46,7 @@ constexpr int kRowStep = 16;       // a tile has a multiple of this many (padded
 constexpr int kBlockKBytes = 128;  // one 128B-swizzle atom row: 64 bf16 or 128 fp8 elements of K
 constexpr int kUmmaKBytes = 32;    // K extent of one tcgen05.mma: 16 bf16 or 32 fp8
 constexpr int kThreads = 192;      // 6 warps
+constexpr unsigned long long kProgressLimitNs = 2ull * 1000 * 1000 * 1000;  // for the rows of an expert, while the launch before is at work on them
 constexpr std::uint32_t kWaitLimit = 20u * 1000u * 1000u;  // try_wait probes before giving up (seconds at most)
 
 // Fused down-projection + combine send: instead of writing `out`, the epilogue multiplies every valid row by
@@ -65,6 +66,15 @@ struct ScatterTarget {
     int num_topk, num_ranks, rank, flag_stride;
 };
 
+// Two GEMMs of which the second reads what the first writes, launched one behind the other on one stream: the first counts the tiles that
+// are written, per expert, and the second starts without waiting for all of the first.  Its CTAs come onto the SMs where the first has ended
+// (its pairs do not end together: HBM does not serve all SMs alike), and go on as soon as their own expert is there.  The second finds
+// everything from before the first complete: the first has waited for that before it let the second start.
+struct Progress {
+    unsigned* counters;  // [E + 1]: CTAs' tiles written per expert, CTAs of the second launch that have ended; zero between the launches; nullptr: none
+    int per_chunk;       // second launch: what the first one counts for a row chunk (2 CTAs x its channel tiles); 0: this launch is the first
+};
+
 struct GroupedGemmParams {
     const int* expert_offsets;  // [E+1] first row of every expert in A / out
     const int* expert_counts;   // [E]   valid rows
@@ -75,6 +85,7 @@ struct GroupedGemmParams {
     int num_experts;
     int n;                      // output columns
     int k;                      // reduction length in elements
+    Progress progress;
     ScatterTarget scatter;      // only read by the scatter variant
 };
 

@@ -206,7 +206,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         .def("enqueue_combine", &Runtime::enqueue_combine, py::arg("y"), py::arg("dispatch_result"), py::arg("weighted"), py::arg("out"),
              py::arg("stream"), py::arg("event"))
         .def("fused_scatter_gemm", &Runtime::fused_scatter_gemm, py::arg("hidden_rows"), py::arg("w_down"),
-             py::arg("dispatch_result"), py::arg("stream") = 0)
+             py::arg("dispatch_result"), py::arg("stream") = 0, py::arg("progress") = py::none(), py::arg("behind") = 0)
         .def("fused_reduce", &Runtime::fused_reduce, py::arg("dispatch_result"), py::arg("out"), py::arg("stream") = 0)
         .def("check_fused_output", &Runtime::check_fused_output, py::arg("out"), py::arg("dispatch_result"))
         .def("fused_status", &Runtime::fused_status)
@@ -244,7 +244,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("grouped_gemm", [](const at::Tensor& a, const at::Tensor& w, at::Tensor& out, const at::Tensor& expert_offsets,
                              const at::Tensor& expert_counts, at::Tensor& status, bool swiglu,
                              const std::optional<at::Tensor>& a_scales, const std::optional<at::Tensor>& w_scales,
-                             std::int64_t stream) {
+                             std::int64_t stream, const std::optional<at::Tensor>& progress, int behind) {
         auto check = [](bool ok, const char* what) {
             if (!ok) throw std::invalid_argument(what);
         };
@@ -277,15 +277,18 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
             a_scale_ptr = a_scales->data_ptr<float>();
             w_scale_ptr = w_scales->data_ptr<float>();
         }
+        const gemm::Progress link = linked(progress, experts, behind);
+        check(behind != 0 || !progress.has_value() || swiglu, "the first of two linked launches has the SwiGLU epilogue");
         c10::cuda::CUDAGuard guard(a.device());
         cudaStream_t launch_stream = stream != 0 ? reinterpret_cast<cudaStream_t>(stream)
                                                  : at::cuda::getCurrentCUDAStream(a.get_device()).stream();
         const char* error = grouped_gemm(a.data_ptr(), w.data_ptr(), out.data_ptr(), a_scale_ptr, w_scale_ptr,
                                          expert_offsets.data_ptr<int>(), expert_counts.data_ptr<int>(), status.data_ptr<int>(),
-                                         static_cast<int>(a.size(0)), experts, n, k, swiglu, fp8, launch_stream);
+                                         static_cast<int>(a.size(0)), experts, n, k, swiglu, fp8, link, launch_stream);
         if (error != nullptr) throw std::runtime_error(std::string("grouped_gemm: ") + error);
     }, py::arg("a"), py::arg("w"), py::arg("out"), py::arg("expert_offsets"), py::arg("expert_counts"), py::arg("status"),
-       py::arg("swiglu"), py::arg("a_scales") = py::none(), py::arg("w_scales") = py::none(), py::arg("stream") = 0);
+       py::arg("swiglu"), py::arg("a_scales") = py::none(), py::arg("w_scales") = py::none(), py::arg("stream") = 0,
+       py::arg("progress") = py::none(), py::arg("behind") = 0);
 
     m.def("litmus_quotients", [](const at::Tensor& a, const at::Tensor& b) {
         for (const at::Tensor* t : {&a, &b})

@@ -21,6 +21,10 @@ from ..ops.grouped_ffn import grouped_gemm, quantize_weights_fp8
 from ..quantization import dequantize_fp8_reference, quantize_fp8_reference
 
 
+#: rows per expert, on average, up to which the two GEMMs of a layer are linked
+_LINKED_ROWS = 192
+
+
 class MoELayer:
     """Expert-parallel SwiGLU MoE layer bound to one ``EPBuffer``.
 
@@ -75,6 +79,7 @@ class MoELayer:
         self.fused_combine = bool(getattr(buffer.config, "fused_expert_combine", False))
         self._hidden_rows: Optional[torch.Tensor] = None
         self._out_rows: Optional[torch.Tensor] = None
+        self._progress: Optional[torch.Tensor] = None  # links the two GEMMs; zero between forward passes
         self.gemm_status = torch.zeros(4, dtype=torch.int32, device=self.device) if buffer.on_gpu else None
 
     @staticmethod
@@ -100,6 +105,18 @@ class MoELayer:
             self._out_rows = None if self.fused_combine else torch.empty(rows, self.hidden, dtype=self.dtype, device=self.device)
         return self._hidden_rows, self._out_rows
 
+    def _links(self, tokens: int) -> Tuple[tuple, tuple]:
+        """What joins the two GEMMs of a pass (``_link`` of ``grouped_gemm``).  With few rows per expert both read weights from HBM, and the
+        second starts where pairs of CTAs of the first have ended: 64 tokens, top-8 of 32 experts, layer 451 -> 444 us, 555 tokens, popular
+        experts, 463 -> 458.  With many the launches run into the power limit and gain nothing, and telling of every tile costs: 4096 tokens
+        2640 -> 2700."""
+        progress, self._progress = self._progress, None  # (a pass that fails between the launches leaves its counts behind)
+        if not self.buffer.on_gpu or tokens * self.num_topk * self.num_ranks > _LINKED_ROWS * self.num_experts:
+            return (None, 0), (None, 0)
+        if progress is None:
+            progress = torch.zeros(self.local_experts + 1, dtype=torch.int32, device=self.device)
+        return (progress, 0), (progress, self.intermediate)
+
     def forward(self, x: torch.Tensor, topk_idx: Optional[torch.Tensor] = None,
                 topk_weights: Optional[torch.Tensor] = None) -> torch.Tensor:
         """``y[t] = sum_k w[t,k] * FFN_{idx[t,k]}(x[t])`` for this rank's tokens ``x`` ``[T, hidden]``."""
@@ -108,16 +125,19 @@ class MoELayer:
         recv_x, _, _, handle, _ = self.buffer.dispatch(x, topk_idx, topk_weights, do_expand=True)
         hidden_rows, out_rows = self._buffers(recv_x.shape[0])
         offsets, counts = handle.expert_offsets, handle.expert_counts
+        first, second = self._links(x.shape[0])
         if self.fp8:
             grouped_gemm(recv_x, self.w_gate_up_fp8, offsets, counts, swiglu=True, out=hidden_rows, status=self.gemm_status,
-                         a_scales=handle._result["recv_x_scales"], w_scales=self.w_gate_up_scales)
+                         a_scales=handle._result["recv_x_scales"], w_scales=self.w_gate_up_scales, _link=first)
         else:
-            grouped_gemm(recv_x, self.w_gate_up, offsets, counts, swiglu=True, out=hidden_rows, status=self.gemm_status)
+            grouped_gemm(recv_x, self.w_gate_up, offsets, counts, swiglu=True, out=hidden_rows, status=self.gemm_status, _link=first)
         if self.fused_combine:
             # down projection and combine in one pass: the GEMM epilogue writes weighted rows into the owners' memory
-            combined, _, _ = self.buffer.fused_expert_combine(hidden_rows, self.w_down, handle)
+            combined, _, _ = self.buffer.fused_expert_combine(hidden_rows, self.w_down, handle, _link=second)
+            self._progress = first[0]
             return combined
-        grouped_gemm(hidden_rows, self.w_down, offsets, counts, swiglu=False, out=out_rows, status=self.gemm_status)
+        grouped_gemm(hidden_rows, self.w_down, offsets, counts, swiglu=False, out=out_rows, status=self.gemm_status, _link=second)
+        self._progress = first[0]
         combined, _, _ = self.buffer.combine(out_rows, handle)
         return combined
 

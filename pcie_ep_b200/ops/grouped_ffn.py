@@ -13,7 +13,7 @@ with the SwiGLU fused into the first GEMM's epilogue.  The reference project has
 
 from __future__ import annotations
 
-from typing import Optional
+from typing import Any, Optional
 
 import torch
 
@@ -60,7 +60,7 @@ def grouped_gemm_reference(a: torch.Tensor, w: torch.Tensor, expert_offsets: tor
 
 def grouped_gemm(a: torch.Tensor, w: torch.Tensor, expert_offsets: torch.Tensor, expert_counts: torch.Tensor, *,
                  swiglu: bool = False, out: Optional[torch.Tensor] = None, status: Optional[torch.Tensor] = None,
-                 a_scales: Optional[torch.Tensor] = None, w_scales: Optional[torch.Tensor] = None) -> torch.Tensor:
+                 a_scales: Optional[torch.Tensor] = None, w_scales: Optional[torch.Tensor] = None, _link: Any = (None, 0)) -> torch.Tensor:
     """``out[rows of e] = a[rows of e] @ w[e].T`` (with ``swiglu``: ``silu(gate) * up``, gate rows first in ``w[e]``).
 
     ``a`` is ``[rows, k]`` BF16, ``w`` ``[experts, n, k]`` (``[experts, 2n, k]`` with ``swiglu``); ``n`` must be a
@@ -69,6 +69,10 @@ def grouped_gemm(a: torch.Tensor, w: torch.Tensor, expert_offsets: torch.Tensor,
     With ``float8_e4m3fn`` operands (``kind::f8f6f4`` MMA, ``k`` a multiple of 128) ``a_scales`` ``[rows]`` and
     ``w_scales`` ``[experts, n]`` are applied in the epilogue: per-row and per-output-channel scales factor out
     of the reduction, so this is exact with respect to the quantised operands.
+
+    ``_link`` ``(progress, behind)`` joins two launches in a row on one stream, the second of which (``behind``: output channels of the
+    first) reads the first one's output: it starts an expert's tiles as soon as that expert is written.  ``progress`` is int32
+    ``[experts + 1]``, zero before the first launch and again after the second.
     """
     n = w.shape[1] // (2 if swiglu else 1)
     if not a.is_cuda:
@@ -84,7 +88,7 @@ def grouped_gemm(a: torch.Tensor, w: torch.Tensor, expert_offsets: torch.Tensor,
         out = torch.empty(a.shape[0], n, dtype=torch.bfloat16, device=a.device)
     if status is None:
         status = torch.zeros(4, dtype=torch.int32, device=a.device)
-    _C.grouped_gemm(a, w, out, expert_offsets, expert_counts, status, swiglu, a_scales, w_scales, 0)
+    _C.grouped_gemm(a, w, out, expert_offsets, expert_counts, status, swiglu, a_scales, w_scales, 0, *_link)
     return out
 
 

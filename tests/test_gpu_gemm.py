@@ -276,3 +276,55 @@ def test_launches_that_start_early_see_what_the_ones_before_wrote(ext, side_stre
     for i, got in enumerate(results):
         assert torch.equal(got, results[0] * 2.0 ** (i % 3)), i
     assert torch.equal(replayed, results[1])
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("counts", [[1], [0, 0, 0], [40] * 24, [700, 3, 0, 55, 513, 16, 2100, 9], [256] * 90])
+def test_linked_launches_are_the_unlinked_ones(ext, counts, fp8):
+    """Gate/up and down projection of which the second starts on its experts while the first is at work: the same bits as one after
+    the other, pass after pass on one set of counters, with other inputs in between, and the counters zero behind each pass."""
+    hidden, inter = 512, 384  # three channel tiles of the first, two of the second, the last with one CTA's channels in both
+    offsets, cnts = _layout(counts)
+    rows = int(offsets[-1])
+    gen = torch.Generator(device="cuda").manual_seed(len(counts))
+    w13 = (torch.randn(len(counts), 2 * inter, hidden, device="cuda", generator=gen) * 0.1).to(torch.bfloat16)
+    w2 = (torch.randn(len(counts), 128 * 3, inter, device="cuda", generator=gen) * 0.1).to(torch.bfloat16)
+    offsets, cnts = offsets.cuda(), cnts.cuda()
+    progress = torch.zeros(len(counts) + 1, dtype=torch.int32, device="cuda")
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    h = torch.zeros(max(1, rows), inter, dtype=torch.bfloat16, device="cuda")
+    for _ in range(4):
+        x = torch.randn(max(1, rows), hidden, device="cuda", generator=gen).to(torch.bfloat16)
+        scales = {}
+        if fp8:
+            scales = dict(a_scales=torch.rand(x.shape[0], device="cuda", generator=gen) + 0.5, w_scales=torch.rand(w13.shape[:2], device="cuda", generator=gen) + 0.5)
+        operands = (x.to(torch.float8_e4m3fn), w13.to(torch.float8_e4m3fn)) if fp8 else (x, w13)
+        outs = []
+        for first, second in (((None, 0), (None, 0)), ((progress, 0), (progress, inter))):
+            h.zero_()
+            out = torch.zeros(h.shape[0], w2.shape[1], dtype=torch.bfloat16, device="cuda")
+            grouped_gemm(*operands, offsets, cnts, swiglu=True, out=h, status=status, _link=first, **scales)
+            grouped_gemm(h, w2, offsets, cnts, out=out, status=status, _link=second)
+            outs.append(out)
+        assert torch.equal(outs[0], outs[1]) and (rows == 0 or float(outs[0].float().abs().max()) > 0)
+        assert int(progress.abs().max()) == 0
+    assert status.tolist() == [0, 0, 0, 0]
+
+
+def test_a_second_launch_whose_rows_never_come_gives_up(ext):
+    """Linked to a first launch that was never made: the bounded wait runs out, the status says so, nothing is written, and the counters
+    are as a pass leaves them."""
+    counts = torch.tensor([5, 7], dtype=torch.int32, device="cuda")
+    offsets = torch.tensor([0, 5, 12], dtype=torch.int32, device="cuda")
+    a, w = torch.ones(12, 64, dtype=torch.bfloat16, device="cuda"), torch.ones(2, 128, 64, dtype=torch.bfloat16, device="cuda")
+    out, status = torch.full((12, 128), 7.0, dtype=torch.bfloat16, device="cuda"), torch.zeros(4, dtype=torch.int32, device="cuda")
+    progress = torch.zeros(3, dtype=torch.int32, device="cuda")
+    grouped_gemm(a, w, offsets, counts, out=out, status=status, _link=(progress, 64))
+    torch.cuda.synchronize()
+    assert status.tolist()[0] == 1 and bool((out == 7.0).all()) and progress.tolist() == [0, 0, 0]
+    for bad in ((progress[:2], 64), (progress.float(), 64), (progress, -1), (progress, 0)):  # (the last: a plain GEMM is no first launch)
+        with pytest.raises(ValueError):
+            grouped_gemm(a, w, offsets, counts, out=out, status=status, _link=bad)
+    status.zero_()
+    grouped_gemm(a, w, offsets, counts, out=out, status=status)
+    assert bool((out == 64.0).all()) and status.tolist()[0] == 0
