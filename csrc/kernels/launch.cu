@@ -97,7 +97,7 @@ int dispatch_local_width(const SegmentLayout& lay, int tokens, bool padding) {
     return padding && tokens > 0 ? std::max(tokens, lay.num_experts) : tokens;
 }
 
-cudaError_t launch_dispatch_local(const DispatchArgs& a, const RankConst& rc, const LocalPlan& plan, int* hist, unsigned long long* counters, int sms, int max_ctas, cudaStream_t stream) {
+cudaError_t launch_dispatch_local(const DispatchArgs& a, const RankConst& rc, LocalPlan plan, int* hist, unsigned long long* counters, int sms, int max_ctas, cudaStream_t stream) {
     const int ctas = std::max(1, std::min(std::min(sms, max_ctas), dispatch_local_width(rc.lay, a.num_tokens, a.do_expand && a.zero_padding && a.alignment > 1)));
     const bool whole = !a.cached && local_counts_whole(a.num_tokens, rc.lay.num_topk, plan);
     const LocalMode mode = a.cached ? kLocalCached : whole ? kLocalWhole : kLocalTogether;

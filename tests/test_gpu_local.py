@@ -338,6 +338,34 @@ def test_small_and_large_batches_lay_out_alike(one_rank, tokens, topk, experts, 
         del again, want
 
 
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("tokens,hidden,experts", [(1, 7168, 32), (555, 7168, 32), (1184, 7168, 32), (2048, 7168, 32), (2000, 8192, 32), (700, 14336, 8)])
+def test_batches_whose_tables_take_a_row_buffer_lay_out_alike(one_rank, tokens, hidden, experts, fp8):
+    """Rows so long that the row buffers leave less than the counting tables need: with one of them given up as the general kernel,
+    and beside the compute stream, where CTAs have more tokens than row buffers."""
+    from pcie_ep_b200 import HostStagedConfig, HostStagedEPBuffer
+
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    x = torch.randn(tokens, hidden, device="cuda", generator=gen).to(torch.bfloat16)
+    idx = torch.rand(tokens, experts, device="cuda", generator=gen).topk(8, dim=1).indices
+    idx[torch.rand(tokens, 8, device="cuda", generator=gen) < 0.2] = -1
+    w = torch.rand(tokens, 8, device="cuda", generator=gen)
+    wire = "fp8_e4m3" if fp8 else "bf16"
+    config = HostStagedConfig(stage=7 if fp8 else 6, channels=128, wire_dtype=wire, recv_dtype=wire, output_pool_size=3)
+    with HostStagedEPBuffer(one_rank, tokens, hidden, 8, experts, config) as buffer:
+        buffer.runtime.set_test_prefix_delay_ns(1)  # a hook of the protocol: the general kernel takes the call
+        want = buffer.dispatch(x, idx, w, do_expand=True)
+        buffer.runtime.set_test_prefix_delay_ns(0)
+        rows = int((idx >= 0).sum())
+        for how in ({}, dict(async_with_compute_stream=True), {}):
+            got = buffer.dispatch(x, idx, w, do_expand=True, **how)
+            got[4].wait()
+            buffer.check_errors(got[3])
+            assert_same_result(got, want, rows, 128, fp8)
+            del got
+        del want
+
+
 @pytest.mark.parametrize("tokens,bad", [(40, 99), (40, -2), (5000, 99)])
 def test_invalid_routes_are_an_error_whoever_counts_them(one_rank, tokens, bad):
     from pcie_ep_b200 import HostStagedConfig, HostStagedEPBuffer
