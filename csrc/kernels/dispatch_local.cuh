@@ -51,7 +51,7 @@ struct LocalDispatchArgs {
     int* hist;                     // [G][E + 1] counts per CTA, then two copies of [groups][E + 1 + C] sums, then their generation
     unsigned long long* counters;  // barrier arrivals, finished CTAs, complement of the first start, CTAs whose plan is written, tokens claimed (zero between launches)
     int hist_ctas;                 // CTAs the scratch has room for
-    int num_experts, num_channels, num_topk, hidden, slots_full, expanded_cap, unique_cap, recv_fp8;  // as in the rank's constants
+    int num_experts, num_channels, num_topk, hidden, slots_full, expanded_cap, unique_cap;  // as in the rank's constants
 };
 
 inline std::size_t local_hist_ints(int ctas, int experts, int channels) {
@@ -130,7 +130,8 @@ __device__ __forceinline__ void local_wait_read(int groups_left) {
 
 }  // namespace detail
 
-template <LocalMode kMode>
+// kFp8: rows stay E4M3.  kPooled: a CTA has more tokens than row buffers.
+template <LocalMode kMode, bool kFp8, bool kPooled>
 __global__ void __launch_bounds__(kLocalThreads, 1) local_dispatch_kernel(const __grid_constant__ LocalDispatchArgs args) {
     using namespace detail;
     const DispatchArgs& a = args.a;
@@ -142,7 +143,8 @@ __global__ void __launch_bounds__(kLocalThreads, 1) local_dispatch_kernel(const 
     const int nt = t1 - t0;
     const int tid = threadIdx.x, warp = tid >> 5;
     const unsigned lane = ptx::lane_id(), full = 0xffffffffu, lt_mask = (1u << lane) - 1u;
-    const bool recv_fp8 = args.recv_fp8 != 0, expand = a.do_expand != 0;
+    constexpr bool recv_fp8 = kFp8;
+    const bool expand = a.do_expand != 0;
     constexpr bool cached = kMode == kLocalCached, whole = kMode == kLocalWhole;
     const int row_warps = args.plan.warps, stages = args.plan.stages, slot_bytes = args.plan.slot_bytes;
     const unsigned in_bytes = static_cast<unsigned>(H) * 2u;
@@ -163,7 +165,8 @@ __global__ void __launch_bounds__(kLocalThreads, 1) local_dispatch_kernel(const 
     const std::uint64_t epoch_before = tid == 0 ? __ldcg(rc->epochs) : 0;
     const unsigned long long t_start = ptx::globaltimer_ns();
     // where no CTA needs another one's counts or claims its tokens, nothing has to be settled by the last one
-    const bool alone = (cached || whole) && (T + G - 1) / G <= row_warps * stages;
+    constexpr bool pooled = kPooled;  // then every CTA has at least as many tokens as row buffers
+    constexpr bool alone = (cached || whole) && !pooled;
     if (tid == 0 && !alone) atomicMax(&args.counters[2], ~t_start);
     // profile rows are per channel: CTA b fills the rows b, b + G, ...
 #define BEP_PROF(point)                                                                                          \
@@ -229,7 +232,6 @@ __global__ void __launch_bounds__(kLocalThreads, 1) local_dispatch_kernel(const 
     // all CTAs (SMs do not all get the same share of HBM: with equal shares the slowest finished 17 us behind the others
     // at 4096 tokens: 110 -> 104 us, 8192 tokens top-4 122 -> 117, 4096 with E4M3 rows 73 -> 71).
     const int own_tokens = row_warps * stages, most_tokens = (T + G - 1) / G;
-    const bool pooled = most_tokens > own_tokens;  // then every CTA has at least own_tokens tokens
 
     // a rank that has failed, or has run out of epochs, leaves without rows
     auto leaves = [&]() {  // thread 0
@@ -588,7 +590,7 @@ __global__ void __launch_bounds__(kLocalThreads, 1) local_dispatch_kernel(const 
         for (int n = 0; n < started; ++n) {
             const int buffer = warp * stages + n % stages;
             const int t = sh->token[buffer], c = t / Tc, i = t - t0;
-            const bool own = n < stages;  // from this CTA's tables, else from the plan in global memory
+            const bool own = !pooled || n < stages;  // from this CTA's tables, else from the plan in global memory
             int e = -1, ord = -1, j = -1;
             float wgt = 1.0f;
             if (lane < static_cast<unsigned>(K)) {
