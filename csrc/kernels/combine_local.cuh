@@ -87,9 +87,15 @@ inline CombineLocalShape combine_local_shape(int tokens, int hidden, int max_row
     int slice = static_cast<int>((smem_limit - kCombineLocalTiles) / 2 - 128) / 16 / max_rows;
     if (slice > chunks) slice = chunks;
     int slices = slices_for(slice);
-    while (static_cast<long long>(tokens) * slices < 2ll * sms && slice >= 128) {
-        slice = (slice + 1) / 2;
-        slices = slices_for(slice);
+    // Few tokens: shorter slices, so that every SM has some.  A CTA takes rounds of one unit, each a slice's share of the row and about 0.3
+    // of a row's time on top, and the last round is as long as a full one.  Against "two units per SM or more": 128 tokens, 8 rows of
+    // 14 KB 8.8 -> 7.6 us (two rounds of halves instead of four of quarters), 64 tokens, 4 rows of 8 KB 7.3 -> 6.1, 230 of them 7.9 -> 6.8; 200
+    // tokens, 8 rows of 14 KB stay at three rounds of halves (10.3; two of whole rows 11.4).
+    const auto cost = [&](int cut) { return static_cast<double>((static_cast<long long>(tokens) * cut + sms - 1) / sms) * (1.0 / cut + 0.3); };
+    for (int shorter = slice, cut = slices; static_cast<long long>(tokens) * cut < 2ll * sms && shorter >= 128;) {
+        shorter = (shorter + 1) / 2;
+        cut = slices_for(shorter);
+        if (cost(cut) < cost(slices)) slices = cut;
     }
     s.slice_chunks = (chunks + slices - 1) / slices;  // equal slices
     s.slices = slices_for(s.slice_chunks);
