@@ -5,14 +5,15 @@
 // What bounds it: reading the expert rows from HBM (4096 tokens, hidden 7168, top-8: 470 MB in, 59 MB out).  The rows of a
 // token lie far apart, so how they are asked for matters more than how many loads are in flight: pieces of 1 KB per row
 // through 16-byte register loads read 4.3 TB/s however many of them were outstanding (110 us).  Here a piece is as long as
-// two stages in shared memory allow -- a whole row of 7168 with top-8 -- and one bulk copy: 95 us, and 104 us with half rows.
+// two stages in shared memory allow -- a whole row of 7168 with top-8 -- and one bulk copy: 95 us (91 since L2 gives up what was read first), and
+// 104 us with half rows.
 //
 // Work unit = (entry of the combine map, slice of its rows).  A CTA's first units are its own, the others come from a
 // counter (launches of a few units per CTA: in a fixed order, kCombineLocalFixed): SMs do not all get the same share of HBM, and equal shares waited for the slowest (125 us).  The producer warp
 // keeps the claim after next and the map entries of the next units on their way while it starts the copies of the present
 // ones; a round of that takes 1.4 us, so small units are claimed four at a time (2048 tokens, a row each: 25.5 -> 21.9 us).
 // Before, through the multi-rank reducers (combine_push.cuh): 111 us, 139 us for 8192 tokens top-4 (now 103), 22 us for 128
-// tokens (now 8.4).  The other warps add the rows out of shared memory in the order of the entry, in FP32, a thread per 16-byte chunk.
+// tokens (now 7.4).  The other warps add the rows out of shared memory in the order of the entry, in FP32, a thread per 16-byte chunk.
 #pragma once
 
 #include "protocol.cuh"

@@ -16,9 +16,9 @@
 //
 // What bounds it.  Large batches: writing the expanded rows to HBM.  4096 tokens, hidden 7168, top-8 move 528 MB.
 // Small ones: the chain launch -> ids -> counts -> scan -> rows; between them, from kLocalWholePairs on, a barrier and a prefix.
-// Launch to end with a cold L2, general kernel -> this one: 128 tokens 46 -> 10.9 us (no flags to wait for, no prefix by a single
-// warp, no barrier), 4096 tokens 131 -> 104 us, the same with E4M3 rows 106 -> 71 us (fourteen row buffers per SM on all SMs instead of eight on 128), 256 tokens
-// with a cached layout 45 -> 17 us.
+// Launch to end with a cold L2, general kernel -> this one: 128 tokens 46 -> 10.1 us (no flags to wait for, no prefix by a single
+// warp, no barrier), 4096 tokens 131 -> 99 us, the same with E4M3 rows 106 -> 67 us (fourteen row buffers per SM on all SMs instead of eight on 128), 256 tokens
+// with a cached layout 45 -> 10.1 us.
 #pragma once
 
 #include "dispatch_common.cuh"

@@ -13,13 +13,14 @@
 // of 16: an expert's rows are cut into equal chunks, and nothing is multiplied for rows that are not there beyond those 16.
 // For SwiGLU the 256 weight rows are 128 gate and the matching 128 up rows, interleaved in sixteens by the weight's tensor map.
 //
-// What bounds it.  Few rows per expert: the weights from HBM.  64 tokens, top-8 of 32 experts, 7168 x 2048: gate/up 299 -> 283 us
-// (6.6 TB/s), down 154 -> 154, against tiles of 128 rows x 256 weight rows by single CTAs.  Many: tensor cores under the power
-// limit.  4096 tokens (1024 rows per expert), back to back: gate/up 1709 -> 1718 us in BF16 (1,120 TFLOP/s; with exactly 1024
-// rows everywhere 1595 -> 1593) and 1050 -> 913 in E4M3, down 935 -> 872.  Between them, and with a short K, the epilogue: 2000
-// tokens of hidden 2048 and intermediate 768 gate/up 117 -> 95 us, 300 tokens in E4M3 192 -> 161.  Stages are
-// as long as the widest tile of the launch needs.  (Stages of each tile's own length in a circle were 20 % slower everywhere; asking weights
-// into L2 ahead of the stages 2 to 80 %.)  Both roles of one thread are entered through elect.sync, see elect_one.
+// What bounds it.  Few rows per expert: the weights from HBM.  64 tokens, top-8 of 32 experts, 7168 x 2048: gate/up 283 -> 268 us
+// (7.0 TB/s), down 154 -> 144.  Many: tensor cores, without a gap between MMAs, at the clock that the power limit leaves.  32 experts
+// of 1024 rows: gate/up 1373 -> 1345 us in BF16, for seconds 1574 -> 1512 (1,270 TFLOP/s), E4M3 inside a layer 910 -> 849, down 830 -> 771.  Between them, and with a
+// short K, the epilogue: 500 rows each, 768 -> 2048 69.9 -> 61.9 us.  Where a few experts have many rows and the others about fifty both share a
+// launch, half overlapped: 6 of 500 and 26 of 54 rows, in E4M3 199 -> 181 us (74 and 121 by themselves).  Where few rows fill the pairs one
+// time and a bit (8 experts of 40 rows, 96 tiles) the last round runs at 125 GB/s of weights per SM: 131 -> 72 us.  Stages are as long as the widest
+// tile of the launch needs.  (Stages of each tile's own length in a circle were slower; asking weights into L2 ahead of the stages 2 to
+// 80 %.)  Both roles of one thread are entered through elect.sync, see elect_one.
 //
 // Work decomposition: persistent pairs walk a tile list (expert, channel tile, row chunk) computed on the device from the
 // counts -- the host never reads a count.  Per CTA: warp 0 = TMA producer (this CTA's weight rows and its half of the
