@@ -278,6 +278,36 @@ def test_launches_that_start_early_see_what_the_ones_before_wrote(ext, side_stre
     assert torch.equal(replayed, results[1])
 
 
+@pytest.mark.parametrize("rows", [7663, 7664, 8192])
+def test_long_gate_up_launches_are_the_short_ones(ext, rows):
+    """Around the size from which MMAs keep a gap behind each (rows x channels x K of 225e9: 7663 rows are below it): the same bits as in
+    two launches of half as many rows, and a sample of rows against 64 bits."""
+    n, k = 4096, 7168
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn(rows, k, device="cuda", generator=gen).to(torch.bfloat16)
+    w = (torch.randn(1, 2 * n, k, device="cuda", generator=gen) * 0.02).to(torch.bfloat16)
+
+    def gemm(first, count):
+        out = torch.zeros(rows, n, dtype=torch.bfloat16, device="cuda")
+        status = torch.zeros(4, dtype=torch.int32, device="cuda")
+        grouped_gemm(x, w, torch.tensor([first, first + count], dtype=torch.int32, device="cuda"), torch.tensor([count], dtype=torch.int32, device="cuda"),
+                     swiglu=True, out=out, status=status)
+        assert status.tolist() == [0, 0, 0, 0]
+        return out
+
+    whole, half = gemm(0, rows), rows // 2
+    assert torch.equal(whole[:half], gemm(0, half)[:half]) and torch.equal(whole[half:], gemm(half, rows - half)[half:])
+    at = torch.tensor([0, 255, 256, rows // 2, rows - 1], device="cuda")
+    both = x[at].double() @ w[0].double().t()
+    size = (x[at].double().abs() @ w[0].double().abs().t()) * (k + 4) * 2.0 ** -24
+    gate, up = both[:, :n], both[:, n:]
+    silu = torch.nn.functional.silu(gate)
+    # as in test_last_tiles_at_the_box_heights
+    error = 1.1 * size[:, :n] * up.abs() + silu.abs() * size[:, n:] + (silu * up).abs() * (8 + 2 * gate.abs()) * 2.0 ** -24
+    want = silu * up
+    assert bool(((whole[at].double() - want).abs() <= error + (want.abs() + error) * 2.0 ** -8).all())
+
+
 @pytest.mark.parametrize("fp8", [False, True])
 @pytest.mark.parametrize("counts", [[1], [0, 0, 0], [40] * 24, [700, 3, 0, 55, 513, 16, 2100, 9], [256] * 90])
 def test_linked_launches_are_the_unlinked_ones(ext, counts, fp8):
