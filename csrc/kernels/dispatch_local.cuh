@@ -35,9 +35,6 @@ constexpr int kLocalMaxPairBytes = 64 * 1024;
 // batches need more: fourteen on all SMs instead of eight on 128 are 71 instead of 106 us for 4096 E4M3 rows.
 constexpr int kLocalSmallPairBytes = 16 * 1024;
 
-// How a launch lays out its batch.  A kernel each: a launch mostly finds its code driven out of L2 by the rows of the one before
-// and fetches it line by line (all three in one kernel: the scan alone 1.5 -> 3.1 us).
-enum LocalMode { kLocalTogether, kLocalWhole, kLocalCached };
 // Batches of up to this many (token, k) are counted by every CTA by itself, without a barrier: no CTA waits for another one, and
 // where none claims tokens the launch needs no cooperative grid and nobody has to be the last.  Together / by itself, top-8: 16 tokens
 // 17.2 / 10.7 us, 128 tokens 17.3 / 10.9, 4096 97.5 / 101 (layout done after 12.6 / 15.8); 777 tokens top-4 20.9 / 13.6.  At the line, 2048
@@ -98,24 +95,35 @@ __host__ __device__ inline std::size_t local_whole_bytes(int tokens, int topk) {
     const std::size_t pair_words = (static_cast<std::size_t>(tokens) * topk + 31) / 32 + 1, token_words = static_cast<std::size_t>(tokens + 31) / 32;
     return 4 * (pair_words + 2 * token_words + 1);
 }
-// Whether every CTA counts such a batch by itself.  Where the row buffers leave less than its tables need, `plan` gives one up (or one per
-// warp): 32 experts, rows of 14 KB, 555 tokens, the layout is done after 7.4 us instead of 8.9, and such a batch does not need them all.
-inline bool local_counts_whole(int tokens, int topk, LocalPlan& plan) {
+// Whether every CTA of `ctas` counts such a batch by itself.  Where the row buffers leave less than its tables need, `plan` gives up
+// the buffers of a warp, if the others still hold all tokens of a CTA: 32 experts, rows of 14 KB, 555 tokens, the layout is done after
+// 7.4 us instead of 8.9; 16 experts, rows of 7 KB, 4096 tokens top-2 (28 per CTA, 30 of 32 buffers) 27.6 -> 21.9 us.  Where tokens would
+// have to be claimed for it, the barrier is the better one, by itself / together: 2048 tokens top-8, rows of 16 KB in 16 experts (14
+// per CTA, 13 buffers) 68.5 / 63.1 us, top-4 in 32 experts 43.6 / 40.9.
+inline bool local_counts_whole(int tokens, int topk, int ctas, LocalPlan& plan) {
     if (tokens <= 0 || static_cast<long long>(tokens) * topk > kLocalWholePairs) return false;
     const std::size_t tables = local_whole_bytes(tokens, topk);
     LocalPlan fewer = plan;
-    if (tables > static_cast<std::size_t>(fewer.whole_bytes)) {
-        if (fewer.stages > 1) --fewer.stages;
-        else --fewer.warps;
-        if (fewer.warps < kLocalMinWarps) return false;
-        const std::size_t given = static_cast<std::size_t>(plan.warps * plan.stages - fewer.warps * fewer.stages) * plan.slot_bytes;
+    while (tables > static_cast<std::size_t>(fewer.whole_bytes)) {
+        if (--fewer.warps < kLocalMinWarps || (tokens + ctas - 1) / ctas > fewer.warps * fewer.stages) return false;
+        const std::size_t given = static_cast<std::size_t>(fewer.stages) * fewer.slot_bytes;
         fewer.bytes -= given;
         fewer.whole_off -= given;  // (a multiple of 128)
         fewer.whole_bytes += static_cast<int>(given);
     }
-    if (tables > static_cast<std::size_t>(fewer.whole_bytes)) return false;
     plan = fewer;
     return true;
+}
+
+// What a launch of `ctas` CTAs makes of a plan.  `pooled`: a CTA has more tokens than row buffers, the rest is claimed.
+inline LocalShape local_shape(LocalPlan plan, int tokens, int topk, int ctas, bool cached) {
+    LocalShape s;
+    const bool whole = !cached && local_counts_whole(tokens, topk, ctas, plan);
+    s.mode = cached ? kLocalCached : whole ? kLocalWhole : kLocalTogether;
+    s.pooled = (tokens + ctas - 1) / ctas > plan.warps * plan.stages;
+    s.bytes = whole ? plan.whole_off + local_whole_bytes(tokens, topk) : plan.bytes;
+    s.plan = plan;
+    return s;
 }
 
 #ifdef __CUDACC__

@@ -107,14 +107,13 @@ constexpr LocalKernel kernels[12] = {
     local_dispatch_kernel<kLocalCached, false, true>,    local_dispatch_kernel<kLocalCached, true, false>,   local_dispatch_kernel<kLocalCached, true, true>};
 }  // namespace
 
-cudaError_t launch_dispatch_local(const DispatchArgs& a, const RankConst& rc, LocalPlan plan, int* hist, unsigned long long* counters, int sms, int max_ctas, cudaStream_t stream) {
+LocalShape shape_dispatch_local(const LocalPlan& plan, int tokens, int topk, int ctas, bool cached) { return local_shape(plan, tokens, topk, ctas, cached); }
+
+cudaError_t launch_dispatch_local(const DispatchArgs& a, const RankConst& rc, const LocalPlan& plan, int* hist, unsigned long long* counters, int sms, int max_ctas, cudaStream_t stream) {
     const int ctas = std::max(1, std::min(std::min(sms, max_ctas), dispatch_local_width(rc.lay, a.num_tokens, a.do_expand && a.zero_padding && a.alignment > 1)));
-    const bool whole = !a.cached && local_counts_whole(a.num_tokens, rc.lay.num_topk, plan);
-    const LocalMode mode = a.cached ? kLocalCached : whole ? kLocalWhole : kLocalTogether;
-    const bool pooled = (a.num_tokens + ctas - 1) / ctas > plan.warps * plan.stages;
-    const int which = mode * 4 + (rc.recv_fp8 != 0 ? 2 : 0) + (pooled ? 1 : 0);
+    const LocalShape shape = local_shape(plan, a.num_tokens, rc.lay.num_topk, ctas, a.cached != 0);
+    const int which = shape.mode * 4 + (rc.recv_fp8 != 0 ? 2 : 0) + (shape.pooled ? 1 : 0);
     const auto kernel = kernels[which];
-    const std::size_t bytes = whole ? plan.whole_off + local_whole_bytes(a.num_tokens, rc.lay.num_topk) : plan.bytes;
     static std::mutex mutex;
     static std::size_t configured[12][64] = {{0}};
     {
@@ -123,18 +122,18 @@ cudaError_t launch_dispatch_local(const DispatchArgs& a, const RankConst& rc, Lo
         cudaError_t status = cudaGetDevice(&device);
         if (status != cudaSuccess) return status;
         if (device < 0 || device >= 64) return cudaErrorInvalidDevice;
-        if (bytes > configured[which][device]) {
-            status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+        if (shape.bytes > configured[which][device]) {
+            status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(shape.bytes));
             if (status != cudaSuccess) return status;
-            configured[which][device] = bytes;
+            configured[which][device] = shape.bytes;
         }
     }
-    LocalDispatchArgs args{a, plan, hist, counters, sms, rc.lay.num_experts, rc.lay.num_channels, rc.lay.num_topk, rc.lay.hidden,
+    LocalDispatchArgs args{a, shape.plan, hist, counters, sms, rc.lay.num_experts, rc.lay.num_channels, rc.lay.num_topk, rc.lay.hidden,
                            rc.lay.slots_full, rc.expanded_cap, rc.unique_cap};
     // A CTA waits for others at the barrier of a layout that they count together, and for their plans where tokens are claimed:
     // then every CTA has to be resident.  With a cached layout (whose plan is there) and with a small batch no CTA waits.
-    if (!a.cached && (!whole || pooled)) return cooperative_launch(kernel, args, dim3(ctas), kLocalThreads, bytes, stream);
-    kernel<<<ctas, kLocalThreads, bytes, stream>>>(args);
+    if (shape.mode != kLocalCached && (shape.mode == kLocalTogether || shape.pooled)) return cooperative_launch(kernel, args, dim3(ctas), kLocalThreads, shape.bytes, stream);
+    kernel<<<ctas, kLocalThreads, shape.bytes, stream>>>(args);
     return cudaGetLastError();
 }
 

@@ -35,7 +35,8 @@ LocalPlan plan_dispatch_local(const SegmentLayout& lay, int sms, std::size_t sme
 std::size_t dispatch_local_hist_ints(const SegmentLayout& lay, int ctas);
 // CTAs that a dispatch has work for: one per token, or one per expert where the rows between their segments are zeroed.
 int dispatch_local_width(const SegmentLayout& lay, int tokens, bool padding);
-cudaError_t launch_dispatch_local(const DispatchArgs& a, const RankConst& rc, LocalPlan plan, int* hist, unsigned long long* counters, int sms, int max_ctas,
+LocalShape shape_dispatch_local(const LocalPlan& plan, int tokens, int topk, int ctas, bool cached);
+cudaError_t launch_dispatch_local(const DispatchArgs& a, const RankConst& rc, const LocalPlan& plan, int* hist, unsigned long long* counters, int sms, int max_ctas,
                                   cudaStream_t stream);
 cudaError_t launch_combine_local(const CombineLocalArgs& args, cudaStream_t stream);
 

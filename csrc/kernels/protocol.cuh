@@ -295,6 +295,15 @@ struct LocalPlan {
     int whole_bytes = 0;
     bool usable = false;
 };
+// How a launch lays out its batch.  A kernel each: a launch mostly finds its code driven out of L2 by the rows of the one before
+// and fetches it line by line (all three in one kernel: the scan alone 1.5 -> 3.1 us).
+enum LocalMode { kLocalTogether, kLocalWhole, kLocalCached };
+struct LocalShape {
+    LocalMode mode = kLocalTogether;
+    bool pooled = false;
+    std::size_t bytes = 0;  // dynamic shared memory
+    LocalPlan plan;
+};
 
 // One combine of one (virtual) rank: the inverse of a finished dispatch.
 struct CombineArgs {

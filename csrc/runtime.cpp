@@ -91,6 +91,19 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                                      stages, send_ctas);
     }, py::arg("P"), py::arg("C"), py::arg("E"), py::arg("K"), py::arg("H"), py::arg("Tmax"), py::arg("payload_slots"),
        py::arg("tx_warps"), py::arg("rx_warps"), py::arg("bulk_engine"), py::arg("stages"), py::arg("send_ctas"));
+    // which kernel a dispatch of a group of one rank takes on `sms` SMs, and with how many row buffers (no GPU needed, too)
+    m.def("local_dispatch_shape", [](int C, int E, int K, int H, int Tmax, int tokens, int sms, std::size_t smem_limit) {
+        const LocalPlan plan = plan_dispatch_local(make_segment_layout(1, C, E, K, H, Tmax, 0, true, false), sms, smem_limit);
+        const LocalShape shape = shape_dispatch_local(plan, tokens, K, std::max(1, std::min(sms, tokens)), false);
+        py::dict out;
+        out["usable"] = plan.usable;
+        out["whole"] = shape.mode == kLocalWhole;
+        out["pooled"] = shape.pooled;
+        out["buffers"] = py::make_tuple(shape.plan.warps, shape.plan.stages);
+        out["most_buffers"] = py::make_tuple(plan.warps, plan.stages);
+        out["bytes"] = shape.bytes;
+        return out;
+    }, py::arg("C"), py::arg("E"), py::arg("K"), py::arg("H"), py::arg("Tmax"), py::arg("tokens"), py::arg("sms"), py::arg("smem_limit"));
     m.def("allocate_device_segment", [](std::size_t bytes, int device) {
         c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
         return reinterpret_cast<std::int64_t>(allocate_device_segment(bytes).ptr);

@@ -130,6 +130,7 @@ Runtime = _module.Runtime
 HostSegment = _module.HostSegment
 NumaRelay = _module.NumaRelay
 segment_layout = _module.segment_layout
+local_dispatch_shape = _module.local_dispatch_shape
 allocate_device_segment = _module.allocate_device_segment
 export_device_segment = _module.export_device_segment
 import_device_segment = _module.import_device_segment

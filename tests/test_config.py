@@ -119,3 +119,25 @@ def test_tuned_configurations_fit_the_shared_memory_of_one_cta(ext):
             assert cfg.channels + send_ctas <= 148, (ranks, tokens)
     # more row buffers than fit are reported as such (the runtime then reduces stages, send warps, receive warps)
     assert _C.dispatch_shared_bytes(8, 128, 256, 8, 7168, 4096, 0, 4, 8, True, 4, 0) > limit
+
+
+@pytest.mark.parametrize("channels,hidden,experts,topk,tokens,most,buffers", [
+    (128, 3584, 16, 2, 4096, (16, 2), (15, 2)), (128, 3584, 16, 8, 1024, (16, 2), (15, 2)),  # two buffers per warp
+    (32, 7168, 32, 8, 555, (16, 1), (15, 1)),                                                # one
+    (128, 3584, 16, 2, 148 * 30, (16, 2), (15, 2)), (128, 3584, 16, 2, 148 * 30 + 1, (16, 2), None),
+    (128, 8192, 16, 8, 148 * 13, (14, 1), (13, 1)), (128, 8192, 16, 8, 148 * 13 + 1, (14, 1), None),
+    (64, 7168, 8, 2, 4096, (16, 1), None)])
+def test_a_small_batch_gives_up_no_more_row_buffers_than_it_can_spare(ext, channels, hidden, experts, topk, tokens, most, buffers):
+    """Counting tables that do not fit beside the row buffers take those of one warp; where the others do not hold a CTA's tokens, the
+    CTAs keep them all and count together (None)."""
+    from pcie_ep_b200 import _C
+
+    limit, per_cta = 227 * 1024, -(-tokens // 148)
+    shape = _C.local_dispatch_shape(channels, experts, topk, hidden, tokens, tokens, 148, limit)
+    assert shape["usable"] and shape["bytes"] <= limit and shape["most_buffers"] == most
+    assert shape["whole"] == (buffers is not None) and shape["buffers"] == (buffers or most)
+    assert shape["pooled"] == (per_cta > shape["buffers"][0] * shape["buffers"][1])
+    assert not (shape["whole"] and shape["pooled"])
+    # with room for the tables on top nothing is given up, and every CTA counts by itself
+    roomy = _C.local_dispatch_shape(channels, experts, topk, hidden, tokens, tokens, 148, limit + 5 * 1024)
+    assert roomy["whole"] and roomy["buffers"] == roomy["most_buffers"]

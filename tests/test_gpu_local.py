@@ -343,16 +343,28 @@ def test_small_and_large_batches_lay_out_alike(one_rank, tokens, topk, experts, 
 def test_batches_whose_tables_take_a_row_buffer_lay_out_alike(one_rank, tokens, hidden, experts, fp8):
     """Rows so long that the row buffers leave less than the counting tables need: with one of them given up as the general kernel,
     and beside the compute stream, where CTAs have more tokens than row buffers."""
+    lay_out_alike(one_rank, tokens, 8, hidden, experts, fp8)
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("tokens,topk,hidden,experts", [(1024, 8, 3584, 16), (4096, 2, 3584, 16), (148 * 30, 2, 3584, 16), (148 * 30 + 1, 2, 3584, 16),
+                                                        (148 * 13, 8, 8192, 16), (148 * 13 + 1, 8, 8192, 16)])
+def test_batches_that_just_fit_or_miss_the_rest_of_the_row_buffers_lay_out_alike(one_rank, tokens, topk, hidden, experts, fp8):
+    """Two row buffers per warp, of which one warp's make room for the tables, and as many tokens as the other buffers hold or one more."""
+    lay_out_alike(one_rank, tokens, topk, hidden, experts, fp8)
+
+
+def lay_out_alike(one_rank, tokens, topk, hidden, experts, fp8):
     from pcie_ep_b200 import HostStagedConfig, HostStagedEPBuffer
 
     gen = torch.Generator(device="cuda").manual_seed(tokens)
     x = torch.randn(tokens, hidden, device="cuda", generator=gen).to(torch.bfloat16)
-    idx = torch.rand(tokens, experts, device="cuda", generator=gen).topk(8, dim=1).indices
-    idx[torch.rand(tokens, 8, device="cuda", generator=gen) < 0.2] = -1
-    w = torch.rand(tokens, 8, device="cuda", generator=gen)
+    idx = torch.rand(tokens, experts, device="cuda", generator=gen).topk(topk, dim=1).indices
+    idx[torch.rand(tokens, topk, device="cuda", generator=gen) < 0.2] = -1
+    w = torch.rand(tokens, topk, device="cuda", generator=gen)
     wire = "fp8_e4m3" if fp8 else "bf16"
     config = HostStagedConfig(stage=7 if fp8 else 6, channels=128, wire_dtype=wire, recv_dtype=wire, output_pool_size=3)
-    with HostStagedEPBuffer(one_rank, tokens, hidden, 8, experts, config) as buffer:
+    with HostStagedEPBuffer(one_rank, tokens, hidden, topk, experts, config) as buffer:
         buffer.runtime.set_test_prefix_delay_ns(1)  # a hook of the protocol: the general kernel takes the call
         want = buffer.dispatch(x, idx, w, do_expand=True)
         buffer.runtime.set_test_prefix_delay_ns(0)
