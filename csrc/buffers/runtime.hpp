@@ -371,7 +371,8 @@ class Runtime {
         // scratch of the layout phase; with a single rank the local kernel's counters and scratch lie in front of it
         if (num_ranks == 1) {
             cuda_check(cudaDeviceGetAttribute(&local_sms_, cudaDevAttrMultiProcessorCount, device), "query the device");
-            local_plan_ = plan_dispatch_local(lay_, local_sms_, max_smem_);
+            cuda_check(cudaDeviceGetAttribute(&l2_bytes_, cudaDevAttrL2CacheSize, device), "query the device");
+            local_plan_ = plan_dispatch_local(lay_, local_sms_, max_smem_, l2_bytes_);
             if (local_plan_.usable) local_ints_ = static_cast<std::int64_t>(align_up(kLocalCounterInts + dispatch_local_hist_ints(lay_, local_sms_), 32));
         }
         block_hist_ = at::zeros({local_ints_ + static_cast<std::int64_t>(hist_scratch_ints(C, E + P))}, i32);
@@ -716,7 +717,7 @@ class Runtime {
     void launch_combine_push(PreparedCombine& prepared, cudaStream_t stream, int num_sms = 0) {
         const bool shares_sms = num_sms > 0 || stream != nullptr;
         if (combine_is_local() && !shares_sms && combine_local_pays(prepared.local.num_tokens, lay_.hidden, prepared.max_rows, combine_ctas(1, 0))) {
-            prepared.local.shape = combine_local_shape(prepared.local.num_tokens, lay_.hidden, prepared.max_rows, combine_ctas(1, 0), max_smem_);
+            prepared.local.shape = combine_local_shape(prepared.local.num_tokens, lay_.hidden, prepared.max_rows, combine_ctas(1, 0), max_smem_, l2_bytes_);
             cuda_check(launch_combine_local(prepared.local, stream), "combine launch");
             return;
         }
@@ -1057,7 +1058,7 @@ class Runtime {
     int grid_ctas_ = 0;
     // single rank: shared-memory plan of the local dispatch kernel, CTAs it may use, ints of its counters and scratch
     LocalPlan local_plan_{};
-    int local_sms_ = 0;
+    int local_sms_ = 0, l2_bytes_ = 0;
     std::int64_t local_ints_ = 0;
     std::vector<std::shared_ptr<OutputSet>> pools_;
     std::vector<std::shared_ptr<Layout>> plans_;

@@ -49,6 +49,7 @@ struct LocalDispatchArgs {
     unsigned long long* counters;  // barrier arrivals, finished CTAs, complement of the first start, CTAs whose plan is written, tokens claimed (zero between launches)
     int hist_ctas;                 // CTAs the scratch has room for
     int num_experts, num_channels, num_topk, hidden, slots_full, expanded_cap, unique_cap;  // as in the rank's constants
+    bool once;                     // rows leave L2 first
 };
 
 inline std::size_t local_hist_ints(int ctas, int experts, int channels) {
@@ -115,9 +116,11 @@ inline bool local_counts_whole(int tokens, int topk, int ctas, LocalPlan& plan) 
     return true;
 }
 
-// What a launch of `ctas` CTAs makes of a plan.  `pooled`: a CTA has more tokens than row buffers, the rest is claimed.
-inline LocalShape local_shape(LocalPlan plan, int tokens, int topk, int ctas, bool cached) {
+// What a launch of `ctas` CTAs makes of a plan, for tokens of `token_bytes`, rows as received among them.  `pooled`: a CTA has more tokens
+// than row buffers, the rest is claimed.
+inline LocalShape local_shape(LocalPlan plan, int tokens, int topk, long long token_bytes, int ctas, bool cached) {
     LocalShape s;
+    s.once = outgrows_l2(tokens * token_bytes, plan.l2_bytes);
     const bool whole = !cached && local_counts_whole(tokens, topk, ctas, plan);
     s.mode = cached ? kLocalCached : whole ? kLocalWhole : kLocalTogether;
     s.pooled = (tokens + ctas - 1) / ctas > plan.warps * plan.stages;
@@ -222,12 +225,13 @@ __global__ void __launch_bounds__(kLocalThreads, 1) local_dispatch_kernel(const 
     __syncthreads();
 
     // ---- 1. the first rows of every warp start their way into shared memory ----------------------------------
+    const std::uint64_t policy = ptx::l2_policy(args.once);
     auto start_load = [&](int n, int t) {  // token t as the warp's n-th (lane 0 only)
         auto* bar = reinterpret_cast<std::uint64_t*>(&sh->mbar[warp * stages + n % stages]);
         ptx::mbar_expect_tx(bar, in_bytes);
-        // (read once: L2 keeps the rows that are written, and the tables.  Exchange of 2048 unique rows 39.1 -> 37.9 us, with the combine's loads.
-        // The stores of BF16 rows that way too: 4096 tokens 193 -> 196.5 us.)
-        ptx::bulk_g2s_once(rows_sm + static_cast<std::size_t>(warp * stages + n % stages) * slot_bytes, a.x + static_cast<std::size_t>(t) * H, in_bytes, bar);
+        std::uint8_t* const slot = rows_sm + static_cast<std::size_t>(warp * stages + n % stages) * slot_bytes;
+        // (The stores of BF16 rows as ones that leave L2 first, too: an exchange of 4096 tokens 193 -> 196.5 us.)
+        ptx::bulk_g2s(slot, a.x + static_cast<std::size_t>(t) * H, in_bytes, bar, policy);
         sh->token[warp * stages + n % stages] = t;
     };
     int started = 0;  // loads of this warp that are under way or done
@@ -638,10 +642,10 @@ __global__ void __launch_bounds__(kLocalThreads, 1) local_dispatch_kernel(const 
                 __syncwarp();
             }
             // every lane with a row starts its own copy: the bulk groups are the lanes' own
-            // (E4M3 rows leave L2 first: 4096 tokens 71.9 -> 69.1 us; layers that read them back at once are as fast, 555 tokens 456, 4096 1870.)
+            // (Layers that read E4M3 rows back at once are as fast where they leave L2 first: 555 tokens 456 us, 4096 1870.)
             if (row >= 0) {
                 std::uint8_t* const dst = recv_bytes + static_cast<std::size_t>(row) * out_row_bytes;
-                if (recv_fp8) ptx::bulk_s2g_once(dst, slot, static_cast<unsigned>(out_row_bytes));
+                if (recv_fp8) ptx::bulk_s2g(dst, slot, static_cast<unsigned>(out_row_bytes), policy);
                 else ptx::bulk_s2g(dst, slot, static_cast<unsigned>(out_row_bytes));
             }
             ptx::bulk_commit();

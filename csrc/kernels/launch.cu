@@ -87,8 +87,10 @@ cudaError_t launch_dispatch(const DispatchLaunch& launch, int ctas, int threads,
     return cooperative_launch(dispatch_kernel<kMaxWarps * 32>, launch, grid, threads, smem, stream);
 }
 
-LocalPlan plan_dispatch_local(const SegmentLayout& lay, int sms, std::size_t smem_limit) {
-    return make_local_plan(lay.num_experts, lay.num_channels, lay.num_topk, lay.hidden, lay.num_max_tokens, sms, smem_limit);
+LocalPlan plan_dispatch_local(const SegmentLayout& lay, int sms, std::size_t smem_limit, long long l2_bytes) {
+    LocalPlan plan = make_local_plan(lay.num_experts, lay.num_channels, lay.num_topk, lay.hidden, lay.num_max_tokens, sms, smem_limit);
+    plan.l2_bytes = l2_bytes;
+    return plan;
 }
 
 std::size_t dispatch_local_hist_ints(const SegmentLayout& lay, int ctas) { return local_hist_ints(ctas, lay.num_experts, lay.num_channels); }
@@ -107,11 +109,14 @@ constexpr LocalKernel kernels[12] = {
     local_dispatch_kernel<kLocalCached, false, true>,    local_dispatch_kernel<kLocalCached, true, false>,   local_dispatch_kernel<kLocalCached, true, true>};
 }  // namespace
 
-LocalShape shape_dispatch_local(const LocalPlan& plan, int tokens, int topk, int ctas, bool cached) { return local_shape(plan, tokens, topk, ctas, cached); }
+LocalShape shape_dispatch_local(const SegmentLayout& lay, const LocalPlan& plan, int tokens, bool expand, bool recv_fp8, int ctas, bool cached) {
+    const long long row_bytes = lay.hidden * (recv_fp8 ? 1ll : 2ll);
+    return local_shape(plan, tokens, lay.num_topk, lay.hidden * 2ll + (expand ? lay.num_topk : 1) * row_bytes, ctas, cached);
+}
 
 cudaError_t launch_dispatch_local(const DispatchArgs& a, const RankConst& rc, const LocalPlan& plan, int* hist, unsigned long long* counters, int sms, int max_ctas, cudaStream_t stream) {
     const int ctas = std::max(1, std::min(std::min(sms, max_ctas), dispatch_local_width(rc.lay, a.num_tokens, a.do_expand && a.zero_padding && a.alignment > 1)));
-    const LocalShape shape = local_shape(plan, a.num_tokens, rc.lay.num_topk, ctas, a.cached != 0);
+    const LocalShape shape = shape_dispatch_local(rc.lay, plan, a.num_tokens, a.do_expand != 0, rc.recv_fp8 != 0, ctas, a.cached != 0);
     const int which = shape.mode * 4 + (rc.recv_fp8 != 0 ? 2 : 0) + (shape.pooled ? 1 : 0);
     const auto kernel = kernels[which];
     static std::mutex mutex;
@@ -129,7 +134,7 @@ cudaError_t launch_dispatch_local(const DispatchArgs& a, const RankConst& rc, co
         }
     }
     LocalDispatchArgs args{a, shape.plan, hist, counters, sms, rc.lay.num_experts, rc.lay.num_channels, rc.lay.num_topk, rc.lay.hidden,
-                           rc.lay.slots_full, rc.expanded_cap, rc.unique_cap};
+                           rc.lay.slots_full, rc.expanded_cap, rc.unique_cap, shape.once};
     // A CTA waits for others at the barrier of a layout that they count together, and for their plans where tokens are claimed:
     // then every CTA has to be resident.  With a cached layout (whose plan is there) and with a small batch no CTA waits.
     if (shape.mode != kLocalCached && (shape.mode == kLocalTogether || shape.pooled)) return cooperative_launch(kernel, args, dim3(ctas), kLocalThreads, shape.bytes, stream);

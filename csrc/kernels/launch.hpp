@@ -31,11 +31,11 @@ cudaError_t launch_combine(const CombineLaunch& launch, int channels, std::size_
 
 // A group of one rank: how the local dispatch kernel cuts up shared memory, the ints of its scratch, and the two launches.
 // `rc` is the host's copy of the rank's constants, `sms` is what the scratch was made for, `max_ctas` bounds the CTAs; `counters` and `hist` belong to one buffer, whose launches are stream-ordered.
-LocalPlan plan_dispatch_local(const SegmentLayout& lay, int sms, std::size_t smem_limit);
+LocalPlan plan_dispatch_local(const SegmentLayout& lay, int sms, std::size_t smem_limit, long long l2_bytes);
 std::size_t dispatch_local_hist_ints(const SegmentLayout& lay, int ctas);
 // CTAs that a dispatch has work for: one per token, or one per expert where the rows between their segments are zeroed.
 int dispatch_local_width(const SegmentLayout& lay, int tokens, bool padding);
-LocalShape shape_dispatch_local(const LocalPlan& plan, int tokens, int topk, int ctas, bool cached);
+LocalShape shape_dispatch_local(const SegmentLayout& lay, const LocalPlan& plan, int tokens, bool expand, bool recv_fp8, int ctas, bool cached);
 cudaError_t launch_dispatch_local(const DispatchArgs& a, const RankConst& rc, const LocalPlan& plan, int* hist, unsigned long long* counters, int sms, int max_ctas,
                                   cudaStream_t stream);
 cudaError_t launch_combine_local(const CombineLocalArgs& args, cudaStream_t stream);

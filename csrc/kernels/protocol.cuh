@@ -283,6 +283,16 @@ struct DispatchLaunch {
     DispatchArgs r[kMaxVirtualRanks];
 };
 
+// One rank: whether L2 is to give up first what a launch that reads and writes `bytes` reads once (token rows, expert rows), and the
+// E4M3 rows it writes.  Between a dispatch and its combine more than twice as much goes by.  From 3/8 of L2 on (50 MB of 126) the hint
+// gains or is even; with it / without, us a pass over the data of the pass before: 512 tokens, 8 rows of 14 KB (66 MB) 36.9 / 38.2,
+// 2048 single rows of 14 KB (59 MB) 34.7 / 35.2, 4096 tokens, 2 rows of 4 KB (50 MB) 42.4 / 42.9, E4M3 dispatch of 2048 tokens
+// 35.2 / 36.8, of 4096 68.7 / 72.2.  Below, what is soon read again is lost: 256 tokens (33 MB) 25.6 / 22.6, 777 tokens, 4 rows of 8 KB
+// (32 MB) 26.7 / 24.7.  Another kernel that reads the tokens right behind the dispatch loses at any size, but less than the hint gains
+// above the line: 64 tokens 1.6 / 1.3 us, 256 3.1 / 2.5, 2048 single rows 10.0 / 9.6, 1024 tokens top-8 and more 7.0 / 7.0.  So does one
+// that reads the experts' rows again behind the combine: 1024 tokens 37.9 / 35.1 (combine 20.5 / 24.4), 4096 142 / 139 (82.6 / 93.0).
+constexpr bool outgrows_l2(long long bytes, long long l2_bytes) { return 8 * bytes >= 3 * l2_bytes; }
+
 // Dispatch of a group of one rank (dispatch_local.cuh): how a CTA's shared memory is cut up.
 constexpr int kLocalCounterInts = 32;  // its counters, in front of its scratch
 struct LocalPlan {
@@ -293,6 +303,7 @@ struct LocalPlan {
     std::size_t rows_off = 0, bytes = 0;
     std::size_t whole_off = 0;  // tables of a batch that every CTA counts by itself, in what is left over
     int whole_bytes = 0;
+    long long l2_bytes = 0;     // of the device
     bool usable = false;
 };
 // How a launch lays out its batch.  A kernel each: a launch mostly finds its code driven out of L2 by the rows of the one before
@@ -300,6 +311,7 @@ struct LocalPlan {
 enum LocalMode { kLocalTogether, kLocalWhole, kLocalCached };
 struct LocalShape {
     LocalMode mode = kLocalTogether;
+    bool once = false;      // rows leave L2 first, see outgrows_l2
     bool pooled = false;
     std::size_t bytes = 0;  // dynamic shared memory
     LocalPlan plan;

@@ -117,10 +117,14 @@ __device__ __forceinline__ void bulk_g2s(void* smem_dst, const void* gmem_src, u
                  "l"(gmem_src), "r"(bytes), "r"(smem_u32(bar))
                  : "memory");
 }
-// the same for what is hardly read again: its lines are the first to leave L2
-__device__ __forceinline__ void bulk_g2s_once(void* smem_dst, const void* gmem_src, unsigned bytes, std::uint64_t* bar) {
-    std::uint64_t policy;
-    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+// The same with a cache policy: `once`, for what is hardly read again: its lines are the first to leave L2; else as without one.
+__device__ __forceinline__ std::uint64_t l2_policy(bool once) {
+    std::uint64_t first, normal;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(first));
+    asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(normal));
+    return once ? first : normal;
+}
+__device__ __forceinline__ void bulk_g2s(void* smem_dst, const void* gmem_src, unsigned bytes, std::uint64_t* bar, std::uint64_t policy) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(
                      smem_u32(smem_dst)),
                  "l"(gmem_src), "r"(bytes), "r"(smem_u32(bar)), "l"(policy)
@@ -131,9 +135,7 @@ __device__ __forceinline__ void bulk_s2g(void* gmem_dst, const void* smem_src, u
                  "r"(smem_u32(smem_src)), "r"(bytes)
                  : "memory");
 }
-__device__ __forceinline__ void bulk_s2g_once(void* gmem_dst, const void* smem_src, unsigned bytes) {
-    std::uint64_t policy;
-    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+__device__ __forceinline__ void bulk_s2g(void* gmem_dst, const void* smem_src, unsigned bytes, std::uint64_t policy) {
     asm volatile("cp.async.bulk.global.shared::cta.bulk_group.L2::cache_hint [%0], [%1], %2, %3;" ::"l"(gmem_dst), "r"(smem_u32(smem_src)), "r"(bytes),
                  "l"(policy)
                  : "memory");

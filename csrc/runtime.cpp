@@ -92,9 +92,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     }, py::arg("P"), py::arg("C"), py::arg("E"), py::arg("K"), py::arg("H"), py::arg("Tmax"), py::arg("payload_slots"),
        py::arg("tx_warps"), py::arg("rx_warps"), py::arg("bulk_engine"), py::arg("stages"), py::arg("send_ctas"));
     // which kernel a dispatch of a group of one rank takes on `sms` SMs, and with how many row buffers (no GPU needed, too)
-    m.def("local_dispatch_shape", [](int C, int E, int K, int H, int Tmax, int tokens, int sms, std::size_t smem_limit) {
-        const LocalPlan plan = plan_dispatch_local(make_segment_layout(1, C, E, K, H, Tmax, 0, true, false), sms, smem_limit);
-        const LocalShape shape = shape_dispatch_local(plan, tokens, K, std::max(1, std::min(sms, tokens)), false);
+    m.def("local_dispatch_shape", [](int C, int E, int K, int H, int Tmax, int tokens, int sms, std::size_t smem_limit, long long l2_bytes, bool expand, bool recv_fp8) {
+        const SegmentLayout lay = make_segment_layout(1, C, E, K, H, Tmax, 0, true, false);
+        const LocalPlan plan = plan_dispatch_local(lay, sms, smem_limit, l2_bytes);
+        const LocalShape shape = shape_dispatch_local(lay, plan, tokens, expand, recv_fp8, std::max(1, std::min(sms, tokens)), false);
         py::dict out;
         out["usable"] = plan.usable;
         out["whole"] = shape.mode == kLocalWhole;
@@ -102,8 +103,22 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         out["buffers"] = py::make_tuple(shape.plan.warps, shape.plan.stages);
         out["most_buffers"] = py::make_tuple(plan.warps, plan.stages);
         out["bytes"] = shape.bytes;
+        out["once"] = shape.once;
         return out;
-    }, py::arg("C"), py::arg("E"), py::arg("K"), py::arg("H"), py::arg("Tmax"), py::arg("tokens"), py::arg("sms"), py::arg("smem_limit"));
+    }, py::arg("C"), py::arg("E"), py::arg("K"), py::arg("H"), py::arg("Tmax"), py::arg("tokens"), py::arg("sms"), py::arg("smem_limit"),
+       py::arg("l2_bytes") = 126 << 20, py::arg("expand") = true, py::arg("recv_fp8") = false);
+    // and how its combine cuts up the rows
+    m.def("local_combine_shape", [](int tokens, int H, int max_rows, int sms, std::size_t smem_limit, long long l2_bytes) {
+        const CombineLocalShape shape = combine_local_shape(tokens, H, max_rows, sms, smem_limit, l2_bytes);
+        py::dict out;
+        out["slices"] = shape.slices;
+        out["stages"] = shape.stages;
+        out["ctas"] = shape.ctas;
+        out["batch"] = shape.batch;
+        out["fixed"] = shape.fixed;
+        out["once"] = shape.once;
+        return out;
+    }, py::arg("tokens"), py::arg("H"), py::arg("max_rows"), py::arg("sms"), py::arg("smem_limit"), py::arg("l2_bytes") = 126 << 20);
     m.def("allocate_device_segment", [](std::size_t bytes, int device) {
         c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
         return reinterpret_cast<std::int64_t>(allocate_device_segment(bytes).ptr);

@@ -131,6 +131,7 @@ HostSegment = _module.HostSegment
 NumaRelay = _module.NumaRelay
 segment_layout = _module.segment_layout
 local_dispatch_shape = _module.local_dispatch_shape
+local_combine_shape = _module.local_combine_shape
 allocate_device_segment = _module.allocate_device_segment
 export_device_segment = _module.export_device_segment
 import_device_segment = _module.import_device_segment

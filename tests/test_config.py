@@ -141,3 +141,15 @@ def test_a_small_batch_gives_up_no_more_row_buffers_than_it_can_spare(ext, chann
     # with room for the tables on top nothing is given up, and every CTA counts by itself
     roomy = _C.local_dispatch_shape(channels, experts, topk, hidden, tokens, tokens, 148, limit + 5 * 1024)
     assert roomy["whole"] and roomy["buffers"] == roomy["most_buffers"]
+
+
+@pytest.mark.parametrize("tokens,expand,recv_fp8,once", [(383, True, False, False), (384, True, False, True), (1727, False, False, False), (1728, False, False, True),
+                                                         (691, True, True, False), (692, True, True, True), (1, True, False, False), (8192, True, True, True)])
+def test_rows_are_kept_in_l2_by_launches_that_move_less_than_it_holds(ext, tokens, expand, recv_fp8, once):
+    """From 3/8 of L2 on, token rows and received rows counted (and expert rows and results in the combine), what is read once leaves first."""
+    from pcie_ep_b200 import _C
+
+    l2, limit = 126 << 20, 227 * 1024
+    assert _C.local_dispatch_shape(128, 256, 8, 7168, 8192, tokens, 148, limit, l2, expand, recv_fp8)["once"] == once
+    if not recv_fp8:
+        assert _C.local_combine_shape(tokens, 7168, 8 if expand else 1, 148, limit, l2)["once"] == once
