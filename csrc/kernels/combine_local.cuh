@@ -80,8 +80,8 @@ struct CombineLocalShared {
 constexpr int kCombineLocalTiles = 2048;  // offset of the stages
 static_assert(sizeof(CombineLocalShared) <= kCombineLocalTiles, "the stages start behind the barriers and headers");
 
-// `max_rows`: most rows an entry can have.  Slices are as long as two stages allow, but short enough that a few tokens
-// reach every SM (units of at least 1 KB per row).
+// `max_rows`: most rows an entry can have.  Slices are as long as two stages allow, and with few tokens shorter (down to units of 1 KB
+// per row) where that spares time.
 inline CombineLocalShape combine_local_shape(int tokens, int hidden, int max_rows, int sms, std::size_t smem_limit, long long l2_bytes) {
     CombineLocalShape s;
     const int chunks = hidden / 8;
@@ -89,10 +89,11 @@ inline CombineLocalShape combine_local_shape(int tokens, int hidden, int max_row
     int slice = static_cast<int>((smem_limit - kCombineLocalTiles) / 2 - 128) / 16 / max_rows;
     if (slice > chunks) slice = chunks;
     int slices = slices_for(slice);
-    // Few tokens: shorter slices, so that every SM has some.  A CTA takes rounds of one unit, each a slice's share of the row and about 0.3
-    // of a row's time on top, and the last round is as long as a full one.  Against "two units per SM or more": 128 tokens, 8 rows of
-    // 14 KB 8.8 -> 7.6 us (two rounds of halves instead of four of quarters), 64 tokens, 4 rows of 8 KB 7.3 -> 6.1, 230 of them 7.9 -> 6.8; 200
-    // tokens, 8 rows of 14 KB stay at three rounds of halves (10.3; two of whole rows 11.4).
+    // Few tokens: a CTA takes rounds of one unit, each a slice's share of the row and about 0.3 of a row's time on top, and the last round is
+    // as long as a full one.  So 16 tokens are cut into eighths and 64 into halves (one round), 75 to 148 not at all (one round of whole
+    // rows; some SMs have none), 149 to 222 into halves (three rounds) and 223 to 296 not (two).  8 rows of 14 KB, us, whole / cut as before,
+    // into two units per SM or more: 75 tokens 7.0 / 7.7, 100 7.4 / 7.9, 128 7.4 / 8.8, 148 8.3 / 8.2; whole / halves: 149 tokens 9.6 / 9.2, 180
+    // 10.7 / 9.9, 200 11.7 / 10.6; 8 rows of 6 KB 75 tokens 6.0 / 7.3, 200 6.9 / 7.6, 4 rows of 8 KB 100 tokens 5.9 / 6.9, 180 6.8 / 7.1.
     const auto cost = [&](int cut) { return static_cast<double>((static_cast<long long>(tokens) * cut + sms - 1) / sms) * (1.0 / cut + 0.3); };
     for (int shorter = slice, cut = slices; static_cast<long long>(tokens) * cut < 2ll * sms && shorter >= 128;) {
         shorter = (shorter + 1) / 2;

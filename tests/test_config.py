@@ -153,3 +153,14 @@ def test_rows_are_kept_in_l2_by_launches_that_move_less_than_it_holds(ext, token
     assert _C.local_dispatch_shape(128, 256, 8, 7168, 8192, tokens, 148, limit, l2, expand, recv_fp8)["once"] == once
     if not recv_fp8:
         assert _C.local_combine_shape(tokens, 7168, 8 if expand else 1, 148, limit, l2)["once"] == once
+
+
+@pytest.mark.parametrize("rows,hidden", [(8, 7168), (4, 4096), (8, 2880)])
+def test_a_combine_of_few_tokens_cuts_rows_where_that_spares_a_round(ext, rows, hidden):
+    """Slices per row by the rounds that a CTA takes: eight or as many as the row has room for with few tokens, whole rows where the
+    tokens nearly fill the SMs once, halves from where a second round of whole rows would start, until two rounds are well filled."""
+    from pcie_ep_b200 import _C
+
+    slices = {tokens: _C.local_combine_shape(tokens, hidden, rows, 148, 227 * 1024)["slices"] for tokens in (16, 40, 64, 74, 75, 100, 128, 148, 149, 200, 222, 223, 256, 300)}
+    assert slices.pop(16) >= 4
+    assert slices == {40: 2, 64: 2, 74: 2, 75: 1, 100: 1, 128: 1, 148: 1, 149: 2, 200: 2, 222: 2, 223: 1, 256: 1, 300: 1}
