@@ -2,6 +2,7 @@
 #include "expert_gemm.cuh"
 
 #include <mutex>
+#include <type_traits>
 
 #include "expert_gemm.hpp"
 #include "ptx.cuh"
@@ -70,6 +71,15 @@ __device__ __forceinline__ bool elect_one() {
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(elected)::"memory");
     return elected != 0;
+}
+// kPauseLoads loads from shared memory, each at the address that the one before gives: `zero_at` holds a zero.
+__device__ __forceinline__ void pause(std::uint32_t& zero_at) {
+#pragma unroll
+    for (int i = 0; i < kPauseLoads; ++i) {
+        std::uint32_t zero;
+        asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(zero) : "r"(zero_at) : "memory");
+        zero_at += zero;
+    }
 }
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -289,6 +299,7 @@ grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_rows, const __gr
             mbar_init(&sh->tmem_empty[b], 8);
         }
         *abort = 0;
+        sh->zero = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -379,8 +390,9 @@ grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_rows, const __gr
         }
     } else if (warp == 1) {
         // ===== MMA issuer of the pair =====
-        auto issue = [&]() {
+        auto issue = [&](auto paced) {
             int stage = 0;
+            std::uint32_t zero_at = smem_addr(&sh->zero);
             unsigned phase = 0;
             bool ok = true;
             int it = 0;
@@ -403,6 +415,7 @@ grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_rows, const __gr
                     for (int k = 0; k < kBlockKBytes / kUmmaKBytes; ++k) {
                         // 32 bytes further along K inside the swizzle atom: +2 in the address field
                         const std::uint64_t step = static_cast<std::uint64_t>(k * kUmmaKBytes) >> 4;
+                        if (decltype(paced)::value && k % 2 == 0) pause(zero_at);
                         umma<kFp8>(acc, desc_w + step, desc_rows + step, idesc, (kb | k) != 0 ? 1u : 0u);
                     }
                     umma_commit_pair(&sh->empty[stage]);  // the stage is free in both CTAs once these MMAs have read it
@@ -414,18 +427,20 @@ grouped_gemm_kernel(const __grid_constant__ ActivationMaps maps_rows, const __gr
                 if (ok) umma_commit_pair(&sh->tmem_full[buf]);
             }
         };
-        // What the compiler makes of the branch sets the pace.  Behind elect_one MMAs follow each other without a gap.  A long BF16 launch
-        // then runs into the power limit: 4096 tokens, 7168 -> 2 x 2048 of 32 experts, 1.05 GHz instead of 1.3, no more MMAs a second than
-        // with a gap of 18 cycles behind each, which an undecided `lane == 0` leaves, and everything else at the lower clock, the memory-bound
-        // kernels of the layer too: layer 2745 us against 2635, dispatch 147 against 125, both at 1000 W.  2048 tokens 1500 / 1486, 1024 tokens
-        // with popular experts, half as long again, 878 / 915, 8 experts of 1024 rows, 4096 -> 2 x 1024, 224 / 228: the line lies at 2048
-        // tokens.  (Gaps between K blocks only, or longer ones, cost more than they gave.  E4M3 gains without any, 1936 -> 1822, the down
-        // projection of that layer included.)
+        // Long BF16 gate/up launches pause in front of every second MMA.  Without a gap the MMAs draw so much power that what follows runs at
+        // the lower clock it leaves behind.  4096 tokens, 32 experts, 7168 -> 2 x 2048, for seconds, us without / with the pause: gate/up 1722 /
+        // 1720 inside the layer, down projection 1025 / 842, dispatch 148 / 127, combine 162 / 133.  Layers, a few passes (and for seconds), by
+        // rows x channels x K of one matrix: 2.4e11 1240 / 1258 (1561 / 1499), 2.7e11 hidden 4096 1275 / 1300 (1551 / 1506), hidden 2048 1227 /
+        // 1261 (1429 / 1454), 2.9e11 1436 / 1475 (1787 / 1761), 3.5e11 1712 / 1688 (2119 / 2064), 16 experts with the fused down projection
+        // 1672 / 1630 (1995 / 1899), 4.0e11 hidden 4096 1835 / 1801 (2237 / 2094), 5.5e11 2431 / 2431 (2953 / 2828); 1.6e11 893 / 946.  The price
+        // is the launch by itself, 32 x 1024 rows 1296 / 1324 us, for seconds 1497 / 1550.  (One load in front of every MMA leaves half of the gain,
+        // two in front of each or three cost 5 to 15 %; a gap by the clock register, between K blocks or MMAs, 9 to 20 %.  E4M3 and the down
+        // projection gain without.)
         if (rank == 0) {
-            if (!kFp8 && kSwiGLU && static_cast<long long>(all_rows) * p.n * p.k >= kLongLaunch) {
-                if (lane == 0) issue();
+            if (!kFp8 && kSwiGLU && static_cast<long long>(all_rows) * p.n * p.k >= kLongLaunchPerSm * gridDim.x) {
+                if (elect_one()) issue(std::true_type());
             } else if (elect_one()) {
-                issue();
+                issue(std::false_type());
             }
         }
     } else {

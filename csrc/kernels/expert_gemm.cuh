@@ -14,13 +14,14 @@
 // For SwiGLU the 256 weight rows are 128 gate and the matching 128 up rows, interleaved in sixteens by the weight's tensor map.
 //
 // What bounds it.  Few rows per expert: the weights from HBM.  64 tokens, top-8 of 32 experts, 7168 x 2048: gate/up 283 -> 268 us
-// (7.0 TB/s), down 154 -> 144.  Many: tensor cores, without a gap between MMAs, at the clock that the power limit leaves.  32 experts
-// of 1024 rows: gate/up 1373 -> 1345 us in BF16, for seconds 1574 -> 1512 (1,270 TFLOP/s), E4M3 inside a layer 910 -> 849, down 830 -> 771.  Between them, and with a
-// short K, the epilogue: 500 rows each, 768 -> 2048 69.9 -> 61.9 us.  Where a few experts have many rows and the others about fifty both share a
-// launch, half overlapped: 6 of 500 and 26 of 54 rows, in E4M3 199 -> 181 us (74 and 121 by themselves).  Where few rows fill the pairs one
-// time and a bit (8 experts of 40 rows, 96 tiles) the last round runs at 125 GB/s of weights per SM: 131 -> 72 us.  Stages are as long as the widest
-// tile of the launch needs.  (Stages of each tile's own length in a circle were slower; asking weights into L2 ahead of the stages 2 to
-// 80 %.)  Both roles of one thread are entered through elect.sync, see elect_one.
+// (7.0 TB/s), down 154 -> 144.  Many: tensor cores, at the clock that the power limit leaves.  32 experts of 1024 rows, gate/up in BF16:
+// 1324 us (1,450 TFLOP/s) for eight launches in a row, 1550 (1,240) for seconds; 2 and 3.5 % of that are the pause between MMAs of such
+// launches, which the rest of a layer gets back (see the MMA issuer).  E4M3 inside a layer 910 -> 849 us, down 830 -> 771, without one.
+// Between them, and with a short K, the epilogue: 500 rows each, 768 -> 2048 69.9 -> 61.9 us.  Where a few experts have many rows and the
+// others about fifty both share a launch, half overlapped: 6 of 500 and 26 of 54 rows, in E4M3 199 -> 181 us (74 and 121 by themselves).
+// Where few rows fill the pairs one time and a bit (8 experts of 40 rows, 96 tiles) the last round runs at 125 GB/s of weights per SM:
+// 131 -> 72 us.  Stages are as long as the widest tile of the launch needs.  (Stages of each tile's own length in a circle were slower;
+// asking weights into L2 ahead of the stages 2 to 80 %.)  Both roles of one thread are entered through elect.sync, see elect_one.
 //
 // Work decomposition: persistent pairs walk a tile list (expert, channel tile, row chunk) computed on the device from the
 // counts -- the host never reads a count.  Per CTA: warp 0 = TMA producer (this CTA's weight rows and its half of the
@@ -111,7 +112,9 @@ constexpr int kTileW = kCtaM * kBlockKBytes;
 // Stages are as long as the widest tile of the launch needs: where all experts have few rows, more of them keep weights on their way.
 constexpr int kRingBytes = 6 * (kTileW + kMaxRows / 2 * kBlockKBytes);  // six stages of the widest tiles, more of narrower ones
 constexpr int kMaxStages = 10;
-constexpr long long kLongLaunch = 225ll * 1000 * 1000 * 1000;  // rows x channels x K of a SwiGLU launch of 0.7 ms (0.9 TFLOP), see the MMA issuer
+// From here on MMAs of a BF16 SwiGLU launch keep a gap, see the MMA issuer: rows x channels x K per SM (222e9 on 148: 0.9 TFLOP, 0.65 ms)
+constexpr long long kLongLaunchPerSm = 1500ll * 1000 * 1000;
+constexpr int kPauseLoads = 3;
 constexpr int kAccCols = kMaxRows;       // TMEM columns of one accumulator set
 constexpr int kTmemCols = 2 * kAccCols;  // double buffered
 // The epilogue turns the accumulator (lane = channel) round in shared memory, kChunkRows rows at a time in two alternating halves.
@@ -122,6 +125,7 @@ struct alignas(16) GemmShared {
     std::uint64_t full[kMaxStages], empty[kMaxStages], tmem_full[2], tmem_empty[2];
     std::uint32_t tmem_base;
     int abort;
+    std::uint32_t zero;
     int most_rows[kThreads / 32];  // of any expert, per warp
     int all_rows[kThreads / 32];   // of all experts, per warp
 };

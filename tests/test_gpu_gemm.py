@@ -278,11 +278,12 @@ def test_launches_that_start_early_see_what_the_ones_before_wrote(ext, side_stre
     assert torch.equal(replayed, results[1])
 
 
-@pytest.mark.parametrize("rows", [7663, 7664, 8192])
-def test_long_gate_up_launches_are_the_short_ones(ext, rows):
-    """Around the size from which MMAs keep a gap behind each (rows x channels x K of 225e9: 7663 rows are below it): the same bits as in
-    two launches of half as many rows, and a sample of rows against 64 bits."""
+@pytest.mark.parametrize("beyond", [-1, 0, 630])
+def test_long_gate_up_launches_are_the_short_ones(ext, beyond):
+    """Around the size from which MMAs keep a gap (rows x channels x K of 1.5e9 per SM): the same bits as in two launches of half as many
+    rows, and a sample of rows against 64 bits."""
     n, k = 4096, 7168
+    rows = -(-1500 * 10 ** 6 * (torch.cuda.get_device_properties(0).multi_processor_count // 2 * 2) // (n * k)) + beyond
     gen = torch.Generator(device="cuda").manual_seed(rows)
     x = torch.randn(rows, k, device="cuda", generator=gen).to(torch.bfloat16)
     w = (torch.randn(1, 2 * n, k, device="cuda", generator=gen) * 0.02).to(torch.bfloat16)
