@@ -79,8 +79,13 @@ class MoELayer:
         self.fused_combine = bool(getattr(buffer.config, "fused_expert_combine", False))
         self._hidden_rows: Optional[torch.Tensor] = None
         self._out_rows: Optional[torch.Tensor] = None
-        self._progress: Optional[torch.Tensor] = None  # links the two GEMMs; zero between forward passes
-        self.gemm_status = torch.zeros(4, dtype=torch.int32, device=self.device) if buffer.on_gpu else None
+        self.gemm_status = self._progress = self._zeroed = None
+        if buffer.on_gpu:
+            counters = torch.zeros(4 + self.local_experts + 1, dtype=torch.int32, device=self.device)
+            self.gemm_status = counters[:4]
+            self._progress: Optional[torch.Tensor] = counters[4:]  # links the two GEMMs; zero between forward passes
+            self._zeroed: Optional[torch.cuda.Event] = torch.cuda.Event()  # until a pass has waited for it
+            self._zeroed.record(torch.cuda.current_stream(self.device))
 
     @staticmethod
     def expert_weights(seed: int, expert: int, hidden: int, intermediate: int, weight_std: float = 0.02):
@@ -107,12 +112,16 @@ class MoELayer:
 
     def _links(self, tokens: int) -> Tuple[tuple, tuple]:
         """What joins the two GEMMs of a pass (``_link`` of ``grouped_gemm``).  With few rows per expert both read weights from HBM, and the
-        second starts where pairs of CTAs of the first have ended: 64 tokens, top-8 of 32 experts, layer 451 -> 444 us, 555 tokens, popular
-        experts, 463 -> 458.  With many the launches run into the power limit and gain nothing, and telling of every tile costs: 4096 tokens
-        2640 -> 2700."""
-        progress, self._progress = self._progress, None  # (a pass that fails between the launches leaves its counts behind)
+        second starts where pairs of CTAs of the first have ended; with many, telling of every tile costs more.  Linked against not, by rows
+        per expert, which say nothing of popular experts, so with uniform, hot-spot and Zipf routes: 32 experts, 7168 x 2048, 16 -1.5 %, 96
+        -0.8, -1.2, -1.5 %, 192 -0.5, -1.8, -1.2 % (E4M3 -1.7), 256 -1.1, -2.9, -0.2 % (E4M3 +0.1), 400 +1.5, -0.9, +0.3 %, 1024 +2 %; 8 experts,
+        4096 x 1536, fused, 96 -6.6 %, 192 -3.2 %.  At the line everything measured still gains."""
         if not self.buffer.on_gpu or tokens * self.num_topk * self.num_ranks > _LINKED_ROWS * self.num_experts:
             return (None, 0), (None, 0)
+        if self._zeroed is not None:
+            torch.cuda.current_stream(self.device).wait_event(self._zeroed)
+            self._zeroed = None
+        progress, self._progress = self._progress, None  # (a pass that fails between the launches leaves its counts behind)
         if progress is None:
             progress = torch.zeros(self.local_experts + 1, dtype=torch.int32, device=self.device)
         return (progress, 0), (progress, self.intermediate)
@@ -134,11 +143,11 @@ class MoELayer:
         if self.fused_combine:
             # down projection and combine in one pass: the GEMM epilogue writes weighted rows into the owners' memory
             combined, _, _ = self.buffer.fused_expert_combine(hidden_rows, self.w_down, handle, _link=second)
+        else:
+            grouped_gemm(hidden_rows, self.w_down, offsets, counts, swiglu=False, out=out_rows, status=self.gemm_status, _link=second)
+            combined, _, _ = self.buffer.combine(out_rows, handle)
+        if first[0] is not None:
             self._progress = first[0]
-            return combined
-        grouped_gemm(hidden_rows, self.w_down, offsets, counts, swiglu=False, out=out_rows, status=self.gemm_status, _link=second)
-        self._progress = first[0]
-        combined, _, _ = self.buffer.combine(out_rows, handle)
         return combined
 
     __call__ = forward

@@ -391,3 +391,58 @@ def test_invalid_routes_are_an_error_whoever_counts_them(one_rank, tokens, bad):
             buffer.check_errors(handle)
         assert handle.error.tolist()[1:3] == [tokens - 3, 5]
         del handle
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("fused", [False, True])
+def test_linked_layers_are_the_unlinked_ones_and_keep_their_counters(one_rank, fused, fp8, monkeypatch):
+    """Layers of which some passes link their GEMMs (the down projection scattered by its epilogue among them) and some do not, in turn:
+    the bits of unlinked passes, with stale activations gone between them, on one set of counters that ends at zero."""
+    from pcie_ep_b200 import HostStagedConfig, HostStagedEPBuffer
+    from pcie_ep_b200.models import moe_layer
+
+    experts, topk, hidden, inter, capacity = 16, 4, 2048, 384, 1024  # more tiles than pairs of CTAs in the second launch, three channel tiles in the first
+    line = moe_layer._LINKED_ROWS
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    weights = ((torch.randn(experts, 2 * inter, hidden, device="cuda", generator=gen) * 0.05).to(torch.bfloat16),
+               (torch.randn(experts, hidden, inter, device="cuda", generator=gen) * 0.05).to(torch.bfloat16))
+    wire = "fp8_e4m3" if fp8 else "bf16"
+    config = HostStagedConfig(stage=7 if fp8 else 6, channels=16, wire_dtype=wire, recv_dtype=wire, fused_expert_combine=fused)
+    with HostStagedEPBuffer(one_rank, capacity, hidden, topk, experts, config) as buffer:
+        layer = moe_layer.MoELayer(buffer, inter, with_router=False, weights=weights)
+        counters = layer._progress.data_ptr()
+        popularity = 1.0 / torch.arange(1, experts + 1, device="cuda") ** 2  # the last ones are often empty
+        for tokens in (300, capacity, 300, 1, 17, line * experts // topk, line * experts // topk + 1, 40):
+            x = torch.randn(tokens, hidden, device="cuda", generator=gen).to(torch.bfloat16)
+            scores = popularity.log() - (-torch.rand(tokens, experts, device="cuda", generator=gen).clamp(1e-6, 1 - 1e-6).log()).log()
+            idx, w = scores.topk(topk, dim=1).indices.contiguous(), torch.rand(tokens, topk, device="cuda", generator=gen)
+            outs = []
+            for linked_rows in (-1, line, line):
+                monkeypatch.setattr(moe_layer, "_LINKED_ROWS", linked_rows)
+                if layer._hidden_rows is not None:
+                    layer._hidden_rows.fill_(float("nan"))
+                outs.append(layer(x, idx, w).clone())
+                assert layer._progress is not None and layer._progress.data_ptr() == counters and int(layer._progress.abs().max()) == 0
+            assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2]) and float(outs[0].float().abs().max()) > 0
+        layer.check_errors()
+
+
+def test_a_layer_made_on_another_stream_waits_for_its_counters(one_rank):
+    """The counters are zeroed on the stream that built the layer; a first pass elsewhere waits for that."""
+    from pcie_ep_b200 import HostStagedConfig, HostStagedEPBuffer
+    from pcie_ep_b200.models.moe_layer import MoELayer
+
+    with HostStagedEPBuffer(one_rank, 32, 256, 2, 4, HostStagedConfig(channels=4)) as buffer:
+        x, idx, w = torch.randn(32, 256, device="cuda").to(torch.bfloat16), torch.rand(32, 4, device="cuda").topk(2, dim=1).indices, torch.rand(32, 2, device="cuda")
+        weights = tuple((torch.randn(4, *shape, device="cuda") * 0.05).to(torch.bfloat16) for shape in ((256, 256), (256, 128)))
+        want = MoELayer(buffer, 128, with_router=False, weights=weights)(x, idx, w).clone()
+        torch.cuda.synchronize()
+        junk = torch.full((4096,), 7, dtype=torch.int32, device="cuda")  # what the counters' memory may have held
+        del junk
+        torch.cuda._sleep(20_000_000)  # ten milliseconds, in front of the zeroing
+        layer = MoELayer(buffer, 128, with_router=False, weights=weights)
+        with torch.cuda.stream(torch.cuda.Stream()):
+            got = layer(x, idx, w).clone()
+        torch.cuda.synchronize()
+        layer.check_errors()
+        assert torch.equal(got, want) and int(layer._progress.abs().max()) == 0
