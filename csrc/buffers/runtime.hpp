@@ -79,12 +79,12 @@ struct TensorBinding {
 };
 
 // The link between two grouped GEMMs (gemm::Progress) over `progress`, int32 [experts + 1], zero before the first of them; `behind`: output
-// channels of the first launch, where this is the second, else 0.
-inline gemm::Progress linked(const std::optional<at::Tensor>& progress, int experts, int behind) {
-    if (!progress.has_value()) return {nullptr, 0};
+// channels of the first launch, where this is the second, else 0; `timeout_ns`: how long the second waits for an expert's rows.
+inline gemm::Progress linked(const std::optional<at::Tensor>& progress, int experts, int behind, unsigned long long timeout_ns) {
+    if (!progress.has_value()) return {};
     if (!progress->is_cuda() || progress->scalar_type() != at::kInt || !progress->is_contiguous() || progress->numel() != experts + 1 || behind < 0)
         throw std::invalid_argument("progress must be contiguous CUDA int32 [experts + 1]");
-    return {reinterpret_cast<unsigned*>(progress->data_ptr<int>()), behind > 0 ? grouped_gemm_tiles_per_chunk(behind) : 0};
+    return {reinterpret_cast<unsigned*>(progress->data_ptr<int>()), behind > 0 ? grouped_gemm_tiles_per_chunk(behind) : 0, timeout_ns};
 }
 
 struct RuntimeOptions {
@@ -798,7 +798,7 @@ class Runtime {
         const char* message = grouped_gemm_scatter(hidden_rows.data_ptr(), w_down.data_ptr(), set.expert_offsets.data_ptr<int>(),
                                                    set.expert_counts.data_ptr<int>(), fused_status_.data_ptr<int>(),
                                                    static_cast<int>(hidden_rows.size(0)), lay_.num_local_experts, lay_.hidden,
-                                                   static_cast<int>(inter), target, linked(progress, lay_.num_local_experts, behind), launch_stream);
+                                                   static_cast<int>(inter), target, linked(progress, lay_.num_local_experts, behind, rc_.timeout_ns), launch_stream);
         if (message != nullptr) throw std::runtime_error(std::string("fused scatter GEMM: ") + message);
         ++fused_gemm_epoch_;
     }

@@ -246,7 +246,7 @@ __device__ __noinline__ bool rows_written(const GroupedGemmParams& p, int expert
     for (unsigned polls = 1; ptx::ld_acquire_gpu(counter) < tiles; ++polls) {
         if (polls % 64 == 0) {
             const unsigned long long now = ptx::globaltimer_ns();
-            if (deadline == 0) deadline = now + kProgressLimitNs;
+            if (deadline == 0) deadline = now + p.progress.timeout_ns;
             if (*abort || now > deadline) {
                 *abort = 1;
                 return false;

@@ -48,7 +48,6 @@ constexpr int kRowStep = 16;       // a tile has a multiple of this many (padded
 constexpr int kBlockKBytes = 128;  // one 128B-swizzle atom row: 64 bf16 or 128 fp8 elements of K
 constexpr int kUmmaKBytes = 32;    // K extent of one tcgen05.mma: 16 bf16 or 32 fp8
 constexpr int kThreads = 192;      // 6 warps
-constexpr unsigned long long kProgressLimitNs = 2ull * 1000 * 1000 * 1000;  // for the rows of an expert, while the launch before is at work on them
 constexpr std::uint32_t kWaitLimit = 20u * 1000u * 1000u;  // try_wait probes before giving up (seconds at most)
 
 // Fused down-projection + combine send: instead of writing `out`, the epilogue multiplies every valid row by
@@ -75,6 +74,7 @@ struct ScatterTarget {
 struct Progress {
     unsigned* counters;  // [E + 1]: CTAs' tiles written per expert, CTAs of the second launch that have ended; zero between the launches; nullptr: none
     int per_chunk;       // second launch: what the first one counts for a row chunk (2 CTAs x its channel tiles); 0: this launch is the first
+    unsigned long long timeout_ns;  // second launch: for the rows of an expert at most, while the first is at work on them
 };
 
 struct GroupedGemmParams {

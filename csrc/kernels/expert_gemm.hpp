@@ -12,7 +12,7 @@ namespace bep {
 // both BF16 or both E4M3 (`fp8`; then a_scales [rows_capacity] and w_scales [num_experts, (2)n] are the
 // per-row / per-output-channel FP32 scales applied in the epilogue); out: [rows_capacity, n] BF16;
 // expert_offsets / expert_counts are device int32 arrays as a dispatch produces them.
-// `progress` links two launches, see there ({nullptr, 0}: none).  Returns nullptr on success, else a message.
+// `progress` links two launches, see there ({}: none).  Returns nullptr on success, else a message.
 const char* grouped_gemm(const void* a, const void* w, void* out, const float* a_scales, const float* w_scales,
                          const int* expert_offsets, const int* expert_counts, int* status, int rows_capacity,
                          int num_experts, int n, int k, bool swiglu, bool fp8, const gemm::Progress& progress, cudaStream_t stream);

@@ -272,7 +272,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("grouped_gemm", [](const at::Tensor& a, const at::Tensor& w, at::Tensor& out, const at::Tensor& expert_offsets,
                              const at::Tensor& expert_counts, at::Tensor& status, bool swiglu,
                              const std::optional<at::Tensor>& a_scales, const std::optional<at::Tensor>& w_scales,
-                             std::int64_t stream, const std::optional<at::Tensor>& progress, int behind) {
+                             std::int64_t stream, const std::optional<at::Tensor>& progress, int behind, int timeout_ms) {
         auto check = [](bool ok, const char* what) {
             if (!ok) throw std::invalid_argument(what);
         };
@@ -305,7 +305,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
             a_scale_ptr = a_scales->data_ptr<float>();
             w_scale_ptr = w_scales->data_ptr<float>();
         }
-        const gemm::Progress link = linked(progress, experts, behind);
+        check(timeout_ms > 0, "timeout_ms must be positive");
+        const gemm::Progress link = linked(progress, experts, behind, static_cast<unsigned long long>(timeout_ms) * 1000000ull);
         check(behind != 0 || !progress.has_value() || swiglu, "the first of two linked launches has the SwiGLU epilogue");
         c10::cuda::CUDAGuard guard(a.device());
         cudaStream_t launch_stream = stream != 0 ? reinterpret_cast<cudaStream_t>(stream)
@@ -316,7 +317,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         if (error != nullptr) throw std::runtime_error(std::string("grouped_gemm: ") + error);
     }, py::arg("a"), py::arg("w"), py::arg("out"), py::arg("expert_offsets"), py::arg("expert_counts"), py::arg("status"),
        py::arg("swiglu"), py::arg("a_scales") = py::none(), py::arg("w_scales") = py::none(), py::arg("stream") = 0,
-       py::arg("progress") = py::none(), py::arg("behind") = 0);
+       py::arg("progress") = py::none(), py::arg("behind") = 0, py::arg("timeout_ms") = 2000);
 
     m.def("litmus_quotients", [](const at::Tensor& a, const at::Tensor& b) {
         for (const at::Tensor* t : {&a, &b})

@@ -124,7 +124,7 @@ class MoELayer:
         progress, self._progress = self._progress, None  # (a pass that fails between the launches leaves its counts behind)
         if progress is None:
             progress = torch.zeros(self.local_experts + 1, dtype=torch.int32, device=self.device)
-        return (progress, 0), (progress, self.intermediate)
+        return (progress, 0), (progress, self.intermediate, self.buffer.config.timeout_ms)
 
     def forward(self, x: torch.Tensor, topk_idx: Optional[torch.Tensor] = None,
                 topk_weights: Optional[torch.Tensor] = None) -> torch.Tensor:

@@ -70,9 +70,10 @@ def grouped_gemm(a: torch.Tensor, w: torch.Tensor, expert_offsets: torch.Tensor,
     ``w_scales`` ``[experts, n]`` are applied in the epilogue: per-row and per-output-channel scales factor out
     of the reduction, so this is exact with respect to the quantised operands.
 
-    ``_link`` ``(progress, behind)`` joins two launches in a row on one stream, the second of which (``behind``: output channels of the
-    first) reads the first one's output: it starts an expert's tiles as soon as that expert is written.  ``progress`` is int32
-    ``[experts + 1]``, zero before the first launch and again after the second.
+    ``_link`` ``(progress, behind[, timeout_ms])`` joins two launches in a row on one stream, the second of which (``behind``: output channels of the
+    first) reads the first one's output: it starts an expert's tiles as soon as that expert is written (or gives up ``timeout_ms``
+    later, 2000 if not given, and says so in ``status``).  ``progress`` is int32 ``[experts + 1]``, zero before the first launch and again after
+    the second.
     """
     n = w.shape[1] // (2 if swiglu else 1)
     if not a.is_cuda:

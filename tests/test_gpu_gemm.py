@@ -342,16 +342,22 @@ def test_linked_launches_are_the_unlinked_ones(ext, counts, fp8):
     assert status.tolist() == [0, 0, 0, 0]
 
 
-def test_a_second_launch_whose_rows_never_come_gives_up(ext):
-    """Linked to a first launch that was never made: the bounded wait runs out, the status says so, nothing is written, and the counters
-    are as a pass leaves them."""
+@pytest.mark.parametrize("limit", [(), (300,)])
+def test_a_second_launch_whose_rows_never_come_gives_up(ext, limit):
+    """Linked to a first launch that was never made: the bounded wait runs out when it says, the status says so, nothing is written, and
+    the counters are as a pass leaves them."""
     counts = torch.tensor([5, 7], dtype=torch.int32, device="cuda")
     offsets = torch.tensor([0, 5, 12], dtype=torch.int32, device="cuda")
     a, w = torch.ones(12, 64, dtype=torch.bfloat16, device="cuda"), torch.ones(2, 128, 64, dtype=torch.bfloat16, device="cuda")
     out, status = torch.full((12, 128), 7.0, dtype=torch.bfloat16, device="cuda"), torch.zeros(4, dtype=torch.int32, device="cuda")
     progress = torch.zeros(3, dtype=torch.int32, device="cuda")
-    grouped_gemm(a, w, offsets, counts, out=out, status=status, _link=(progress, 64))
+    begin, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+    begin.record()
+    grouped_gemm(a, w, offsets, counts, out=out, status=status, _link=(progress, 64, *limit))
+    end.record()
     torch.cuda.synchronize()
+    # (three tenths of a second or two; not measured closer: the GPU's clock and its host are other things')
+    assert (begin.elapsed_time(end) < 1000) == bool(limit) and begin.elapsed_time(end) > 250
     assert status.tolist()[0] == 1 and bool((out == 7.0).all()) and progress.tolist() == [0, 0, 0]
     for bad in ((progress[:2], 64), (progress.float(), 64), (progress, -1), (progress, 0)):  # (the last: a plain GEMM is no first launch)
         with pytest.raises(ValueError):
