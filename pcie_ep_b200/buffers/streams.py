@@ -127,6 +127,14 @@ class StreamPolicy:
             return None
         return self._reader if len(self.consumers) == 1 and self._reader_key in self.consumers else None
 
+    def first(self) -> Any:
+        """The same for the first launch on a buffer: nobody reads results yet, and the caller's stream is about to."""
+        if self._reader is not None or self.consumers or self._comm_ahead:
+            return None
+        stream = self.current()
+        self.finish(stream, stream, None, False)
+        return self.sole()
+
     def raw(self, stream: Any) -> int:
         return self._reader_raw if stream is self._reader else int(stream.cuda_stream)
 

@@ -237,6 +237,36 @@ def test_usual_calls_are_the_general_ones(world1, expand, with_weights):
         _check(buffer.dispatch(x, idx, w, do_expand=expand), cpu, expand)
 
 
+def test_the_first_call_on_a_buffer_is_a_usual_one(world1, monkeypatch):
+    """On the caller's stream the first dispatch and combine go down in native calls as later ones do; on the communication stream, or with
+    a reader already there, step by step, and the results are the same."""
+    cpu, (x, idx, w) = _dev_inputs(pattern="partial")
+
+    def general(self, *args):
+        raise AssertionError("step by step")
+
+    with monkeypatch.context() as patched, _buffer() as buffer:
+        patched.setattr(HostStagedEPBuffer, "_enqueue", general)
+        result = buffer.dispatch(x, idx, w, do_expand=True)
+        combined = buffer.combine(result[0], result[3])[0]
+        assert buffer._streams.sole() is not None and len(buffer._streams.consumers) == 1
+        _check(result, cpu, True)
+        want = combined.clone()
+        del result, combined
+    for elsewhere in (True, False):
+        with _buffer() as buffer:
+            if not elsewhere:
+                buffer._register_consumer_stream(torch.cuda.Stream())
+            with torch.cuda.stream(buffer.get_comm_stream() if elsewhere else torch.cuda.current_stream()):
+                assert buffer._sole_stream_and_event()[0] is None
+                result = buffer.dispatch(x, idx, w, do_expand=True)
+                combined = buffer.combine(result[0], result[3])[0]
+            torch.cuda.synchronize()
+            _check(result, cpu, True)
+            assert torch.equal(combined, want)
+            del result, combined
+
+
 @pytest.mark.parametrize("mode", ["auto", "inline"])
 def test_combine_weighted_and_unique(world1, mode):
     """Single rank: "auto" is the one-launch gather-reduce, "inline" the cooperative kernel writing straight to out."""
