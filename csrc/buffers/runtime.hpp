@@ -373,10 +373,7 @@ class Runtime {
             cuda_check(cudaDeviceGetAttribute(&local_sms_, cudaDevAttrMultiProcessorCount, device), "query the device");
             cuda_check(cudaDeviceGetAttribute(&l2_bytes_, cudaDevAttrL2CacheSize, device), "query the device");
             local_plan_ = plan_dispatch_local(lay_, local_sms_, max_smem_, l2_bytes_);
-            if (local_plan_.usable) {
-                cuda_check(load_dispatch_local(options_.recv_fp8, max_smem_), "load the dispatch kernels");
-                local_ints_ = static_cast<std::int64_t>(align_up(kLocalCounterInts + dispatch_local_hist_ints(lay_, local_sms_), 32));
-            }
+            if (local_plan_.usable) local_ints_ = static_cast<std::int64_t>(align_up(kLocalCounterInts + dispatch_local_hist_ints(lay_, local_sms_), 32));
         }
         block_hist_ = at::zeros({local_ints_ + static_cast<std::int64_t>(hist_scratch_ints(C, E + P))}, i32);
         sticky_ = at::zeros({8}, i32);

@@ -114,19 +114,25 @@ LocalShape shape_dispatch_local(const SegmentLayout& lay, const LocalPlan& plan,
     return local_shape(plan, tokens, lay.num_topk, lay.hidden * 2ll + (expand ? lay.num_topk : 1) * row_bytes, ctas, cached);
 }
 
-cudaError_t load_dispatch_local(bool recv_fp8, std::size_t smem_limit) {
-    for (int which = 0; which < 12; ++which) {
-        if ((which & 2) != (recv_fp8 ? 2 : 0)) continue;
-        const cudaError_t status = cudaFuncSetAttribute(kernels[which], cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_limit));
-        if (status != cudaSuccess) return status;
-    }
-    return cudaSuccess;
-}
-
 cudaError_t launch_dispatch_local(const DispatchArgs& a, const RankConst& rc, const LocalPlan& plan, int* hist, unsigned long long* counters, int sms, int max_ctas, cudaStream_t stream) {
     const int ctas = std::max(1, std::min(std::min(sms, max_ctas), dispatch_local_width(rc.lay, a.num_tokens, a.do_expand && a.zero_padding && a.alignment > 1)));
     const LocalShape shape = shape_dispatch_local(rc.lay, plan, a.num_tokens, a.do_expand != 0, rc.recv_fp8 != 0, ctas, a.cached != 0);
-    const auto kernel = kernels[shape.mode * 4 + (rc.recv_fp8 != 0 ? 2 : 0) + (shape.pooled ? 1 : 0)];
+    const int which = shape.mode * 4 + (rc.recv_fp8 != 0 ? 2 : 0) + (shape.pooled ? 1 : 0);
+    const auto kernel = kernels[which];
+    static std::mutex mutex;
+    static std::size_t configured[12][64] = {{0}};
+    {
+        std::lock_guard<std::mutex> guard(mutex);
+        int device = 0;
+        cudaError_t status = cudaGetDevice(&device);
+        if (status != cudaSuccess) return status;
+        if (device < 0 || device >= 64) return cudaErrorInvalidDevice;
+        if (shape.bytes > configured[which][device]) {
+            status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(shape.bytes));
+            if (status != cudaSuccess) return status;
+            configured[which][device] = shape.bytes;
+        }
+    }
     LocalDispatchArgs args{a, shape.plan, hist, counters, sms, rc.lay.num_experts, rc.lay.num_channels, rc.lay.num_topk, rc.lay.hidden,
                            rc.lay.slots_full, rc.expanded_cap, rc.unique_cap, shape.once};
     // A CTA waits for others at the barrier of a layout that they count together, and for their plans where tokens are claimed:

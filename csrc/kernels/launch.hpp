@@ -32,9 +32,6 @@ cudaError_t launch_combine(const CombineLaunch& launch, int channels, std::size_
 // A group of one rank: how the local dispatch kernel cuts up shared memory, the ints of its scratch, and the two launches.
 // `rc` is the host's copy of the rank's constants, `sms` is what the scratch was made for, `max_ctas` bounds the CTAs; `counters` and `hist` belong to one buffer, whose launches are stream-ordered.
 LocalPlan plan_dispatch_local(const SegmentLayout& lay, int sms, std::size_t smem_limit, long long l2_bytes);
-// Loads the kernels for buffers of this row type, with leave for `smem_limit` bytes of shared memory: before the first launch (each takes 60
-// to 500 us in a process, which batches of another size or kind would meet one by one).
-cudaError_t load_dispatch_local(bool recv_fp8, std::size_t smem_limit);
 std::size_t dispatch_local_hist_ints(const SegmentLayout& lay, int ctas);
 // CTAs that a dispatch has work for: one per token, or one per expert where the rows between their segments are zeroed.
 int dispatch_local_width(const SegmentLayout& lay, int tokens, bool padding);
