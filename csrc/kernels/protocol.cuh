@@ -284,14 +284,15 @@ struct DispatchLaunch {
 };
 
 // One rank: whether L2 is to give up first what a launch that reads and writes `bytes` reads once (token rows, expert rows), and the
-// E4M3 rows it writes.  Between a dispatch and its combine more than twice as much goes by.  From 3/8 of L2 on (50 MB of 126) the hint
-// gains or is even; with it / without, us a pass over the data of the pass before: 512 tokens, 8 rows of 14 KB (66 MB) 36.9 / 38.2,
-// 2048 single rows of 14 KB (59 MB) 34.7 / 35.2, 4096 tokens, 2 rows of 4 KB (50 MB) 42.4 / 42.9, E4M3 dispatch of 2048 tokens
-// 35.2 / 36.8, of 4096 68.7 / 72.2.  Below, what is soon read again is lost: 256 tokens (33 MB) 25.6 / 22.6, 777 tokens, 4 rows of 8 KB
-// (32 MB) 26.7 / 24.7.  Another kernel that reads the tokens right behind the dispatch loses at any size, but less than the hint gains
-// above the line: 64 tokens 1.6 / 1.3 us, 256 3.1 / 2.5, 2048 single rows 10.0 / 9.6, 1024 tokens top-8 and more 7.0 / 7.0.  So does one
-// that reads the experts' rows again behind the combine: 1024 tokens 37.9 / 35.1 (combine 20.5 / 24.4), 4096 142 / 139 (82.6 / 93.0).
-constexpr bool outgrows_l2(long long bytes, long long l2_bytes) { return 8 * bytes >= 3 * l2_bytes; }
+// E4M3 rows it writes.  Exchanges that take turns on three sets of buffers, so that every pass meets data that others have driven out,
+// us a pass with the hint / without: below a ninth of L2 (15 of 126 MB) it loses, 32 tokens, 8 rows of 14 KB (4 MB) 18.1 / 17.1, 96
+// (12 MB) 20.5 / 19.6, 200 tokens, 4 rows of 8 KB (8 MB) 18.5 / 17.4, 128 single rows of 14 KB 16.1 / 15.7; even at 512 of them (15 MB)
+// 20.5 / 20.5; then it gains, 128 tokens of 8 rows (17 MB) 20.7 / 20.9, 256 26.7 / 27.5, 512 37.3 / 39.1, 768 single rows (22 MB) 22.9 /
+// 24.0, E4M3 dispatch of 512 tokens (37 MB) 16.5 / 18.1, of 4096 68.7 / 72.2, combine of 4096 tokens by itself 82.6 / 93.0.  The price is
+// paid by who reads the same data again soon: another kernel behind the dispatch that reads the tokens, 256 tokens 3.1 / 2.5 us, 2048 single
+// rows 10.0 / 9.6, 1024 tokens top-8 and more 7.0 / 7.0; one behind the combine that reads the experts' rows, 256 tokens 9.7 / 9.4, 1024
+// 37.9 / 35.1, 4096 142 / 139; a pass over the very data of the pass before, with nothing in between, 256 tokens 25.6 / 22.6.
+constexpr bool outgrows_l2(long long bytes, long long l2_bytes) { return 9 * bytes >= l2_bytes; }
 
 // Dispatch of a group of one rank (dispatch_local.cuh): how a CTA's shared memory is cut up.
 constexpr int kLocalCounterInts = 32;  // its counters, in front of its scratch

@@ -143,10 +143,10 @@ def test_a_small_batch_gives_up_no_more_row_buffers_than_it_can_spare(ext, chann
     assert roomy["whole"] and roomy["buffers"] == roomy["most_buffers"]
 
 
-@pytest.mark.parametrize("tokens,expand,recv_fp8,once", [(383, True, False, False), (384, True, False, True), (1727, False, False, False), (1728, False, False, True),
-                                                         (691, True, True, False), (692, True, True, True), (1, True, False, False), (8192, True, True, True)])
-def test_rows_are_kept_in_l2_by_launches_that_move_less_than_it_holds(ext, tokens, expand, recv_fp8, once):
-    """From 3/8 of L2 on, token rows and received rows counted (and expert rows and results in the combine), what is read once leaves first."""
+@pytest.mark.parametrize("tokens,expand,recv_fp8,once", [(113, True, False, False), (114, True, False, True), (511, False, False, False), (512, False, False, True),
+                                                         (204, True, True, False), (205, True, True, True), (1, True, False, False), (8192, True, True, True)])
+def test_rows_are_kept_in_l2_by_launches_that_move_little(ext, tokens, expand, recv_fp8, once):
+    """From a ninth of L2 on, token rows and received rows counted (and expert rows and results in the combine), what is read once leaves first."""
     from pcie_ep_b200 import _C
 
     l2, limit = 126 << 20, 227 * 1024
