@@ -2,17 +2,16 @@
 // batches of short rows: combine_push.cuh, see combine_local_pays.  Launches that share the SMs with other work, too: a CTA
 // of this kernel takes nearly all of an SM's shared memory.)
 //
-// What bounds it: reading the expert rows from HBM (4096 tokens, hidden 7168, top-8: 470 MB in, 59 MB out).  The rows of a
-// token lie far apart, so how they are asked for matters more than how many loads are in flight: pieces of 1 KB per row
-// through 16-byte register loads read 4.3 TB/s however many of them were outstanding (110 us).  Here a piece is as long as
-// two stages in shared memory allow -- a whole row of 7168 with top-8 -- and one bulk copy: 95 us (91 since L2 gives up what was read first), and
-// 104 us with half rows.
+// What bounds it: reading the expert rows from HBM (4096 tokens, hidden 7168, top-8: 470 MB in, 59 MB out).  The rows of a token lie
+// far apart, so how they are asked for matters more than how many loads are in flight: pieces of 1 KB per row through 16-byte register
+// loads read 4.3 TB/s however many of them were outstanding (110 us).  Here a piece is as long as two stages in shared memory allow -- a
+// whole row of 7168 with top-8 -- and one bulk copy: 95 us (91 since L2 gives up what was read first), and 104 us with half rows.
 //
-// Work unit = (entry of the combine map, slice of its rows).  A CTA's first units are its own, the others come from a
-// counter (launches of a few units per CTA: in a fixed order, kCombineLocalFixed): SMs do not all get the same share of HBM, and equal shares waited for the slowest (125 us).  The producer warp
-// keeps the claim after next and the map entries of the next units on their way while it starts the copies of the present
-// ones; a round of that takes 1.4 us, so small units are claimed four at a time (2048 tokens, a row each: 25.5 -> 21.9 us).
-// Before, through the multi-rank reducers (combine_push.cuh): 111 us, 139 us for 8192 tokens top-4 (now 103), 22 us for 128
+// Work unit = (entry of the combine map, slice of its rows).  A CTA's first units are its own, the others come from a counter (launches
+// of a few units per CTA: in a fixed order, kCombineLocalFixed): SMs do not all get the same share of HBM, and equal shares waited for
+// the slowest (125 us).  The producer warp keeps the claim after next and the map entries of the next units on their way while it starts
+// the copies of the present ones; a round of that takes 1.4 us, so small units are claimed four at a time (2048 tokens, a row each: 25.5
+// -> 21.9 us).  Before, through the multi-rank reducers (combine_push.cuh): 111 us, 139 us for 8192 tokens top-4 (now 103), 22 us for 128
 // tokens (now 7.4).  The other warps add the rows out of shared memory in the order of the entry, in FP32, a thread per 16-byte chunk.
 #pragma once
 
@@ -61,11 +60,11 @@ constexpr int kCombineLocalThreads = 32 * (1 + kCombineLocalConsumers);
 constexpr int kCombineLocalSmallStage = 32 * 1024;
 // Launches with at most this many units per CTA (the second line: of stages up to kCombineLocalSmallStage) don't claim: CTA b takes the
 // units b, b + grid, ...  There is little to even out yet, the map entries of four units are asked for at once, and without counters no
-// CTA has to find out whether it is the last one: 16 tokens, 8 rows of 14 KB 7.0 -> 5.2 us, 128 tokens 11.3 -> 8.3.  From 4 units on, singly
-// claimed / in a fixed order: 777 tokens, 4 rows of 8 KB 14.7 / 12.5, 1000 tokens, 2 rows of 4 KB 14.6 / 9.5, 8 rows of 14 KB 30.9 / 28.7, 1800
-// tokens, 8 rows of 8 KB (12 units) 31.4 / 30.0; 2048 tokens, 8 rows of 14 KB (14 units) an exchange of 102.9 / 103.5.  Nobody is the last one
-// then, so the duration in `stats` is that of CTA 0 (3.0 us of such a launch of 16 tokens, 16.3 of 2048 single rows): counting the CTAs for the
-// sake of that number cost 0.3 to 0.6 us a launch.
+// CTA has to find out whether it is the last one: 16 tokens, 8 rows of 14 KB 7.0 -> 5.2 us.  Singly claimed / in a fixed order:
+//   4 units and more: 777 tokens, 4 rows of 8 KB 14.7 / 12.5, 1000 tokens, 2 rows of 4 KB 14.6 / 9.5, 8 rows of 14 KB 30.9 / 28.7;
+//   12 units: 1800 tokens, 8 rows of 8 KB 31.4 / 30.0;  14: 2048 tokens, 8 rows of 14 KB, the exchange 102.9 / 103.5.
+// Nobody is the last one then, so the duration in `stats` is that of CTA 0 (3.0 us of such a launch of 16 tokens, 16.3 of 2048 single
+// rows): counting the CTAs for the sake of that number cost 0.3 to 0.6 us a launch.
 constexpr int kCombineLocalFixed = 12;
 constexpr int kCombineLocalFixedSmall = 16;
 

@@ -16,9 +16,9 @@
 //
 // What bounds it.  Large batches: writing the expanded rows to HBM.  4096 tokens, hidden 7168, top-8 move 528 MB.
 // Small ones: the chain launch -> ids -> counts -> scan -> rows; between them, from kLocalWholePairs on, a barrier and a prefix.
-// Launch to end with a cold L2, general kernel -> this one: 128 tokens 46 -> 10.1 us (no flags to wait for, no prefix by a single
-// warp, no barrier), 4096 tokens 131 -> 99 us, the same with E4M3 rows 106 -> 67 us (fourteen row buffers per SM on all SMs instead of eight on 128), 256 tokens
-// with a cached layout 45 -> 10.1 us.
+// Launch to end with a cold L2, general kernel -> this one: 128 tokens 46 -> 10.1 us (no flags to wait for, no prefix by a single warp,
+// no barrier), 4096 tokens 131 -> 99 us, the same with E4M3 rows 106 -> 67 us (fourteen row buffers per SM on all SMs instead of eight
+// on 128), 256 tokens with a cached layout 45 -> 10.1 us.
 #pragma once
 
 #include "dispatch_common.cuh"
@@ -262,8 +262,8 @@ __global__ void __launch_bounds__(kLocalThreads, 1) local_dispatch_kernel(const 
     unsigned* const token_bits = pair_bits + pair_words;                                    // which tokens are routed,
     int* const routed_words = reinterpret_cast<int*>(token_bits + token_words);             // [token_words + 1] routed tokens before word w
     if constexpr (whole) {
-        // The pairs of the whole batch: 32 per warp and step, the ids of eight steps on their way at once (of four: 2048 tokens top-8 0.8 us more).  Few experts meet in
-        // a step again and again: there a lane counts two of them from ballots of the ids' bits.
+        // The pairs of the whole batch: 32 per warp and step, the ids of eight steps on their way at once (of four: 2048 tokens top-8 0.8 us
+        // more).  Few experts meet in a step again and again: there a lane counts two of them from ballots of the ids' bits.
         const int own_first = t0 * K;
         const bool few = E <= kLocalFewExperts;
         unsigned mine[2] = {0u, 0u};  // few: pairs of the experts lane and lane + 32, those of earlier CTAs in the upper half

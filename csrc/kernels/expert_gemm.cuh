@@ -72,7 +72,7 @@ struct ScatterTarget {
 // (its pairs do not end together: HBM does not serve all SMs alike), and go on as soon as their own expert is there.  The second finds
 // everything from before the first complete: the first has waited for that before it let the second start.
 struct Progress {
-    unsigned* counters;  // [E + 1]: CTAs' tiles written per expert, CTAs of the second launch that have ended; zero between the launches; nullptr: none
+    unsigned* counters;  // [E + 1]: CTAs' tiles written per expert, CTAs of the second launch that have ended; zero between passes; nullptr: none
     int per_chunk;       // second launch: what the first one counts for a row chunk (2 CTAs x its channel tiles); 0: this launch is the first
     unsigned long long timeout_ns;  // second launch: for the rows of an expert at most, while the first is at work on them
 };

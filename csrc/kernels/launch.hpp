@@ -30,7 +30,8 @@ cudaError_t launch_dispatch(const DispatchLaunch& launch, int ctas, int threads,
 cudaError_t launch_combine(const CombineLaunch& launch, int channels, std::size_t crow_stride, cudaStream_t stream);
 
 // A group of one rank: how the local dispatch kernel cuts up shared memory, the ints of its scratch, and the two launches.
-// `rc` is the host's copy of the rank's constants, `sms` is what the scratch was made for, `max_ctas` bounds the CTAs; `counters` and `hist` belong to one buffer, whose launches are stream-ordered.
+// `rc` is the host's copy of the rank's constants, `sms` is what the scratch was made for, `max_ctas` bounds the CTAs; `counters` and
+// `hist` belong to one buffer, whose launches are stream-ordered.  `shape_dispatch_local`: which kernel `ctas` CTAs run, and with what.
 LocalPlan plan_dispatch_local(const SegmentLayout& lay, int sms, std::size_t smem_limit, long long l2_bytes);
 std::size_t dispatch_local_hist_ints(const SegmentLayout& lay, int ctas);
 // CTAs that a dispatch has work for: one per token, or one per expert where the rows between their segments are zeroed.
